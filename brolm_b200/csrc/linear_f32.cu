@@ -2,55 +2,390 @@
 // (wlejon/brolm include/brolm/detail/compute.h:49-86, the float branch).
 //
 // No tensor cores and no reduced-precision mode: every product and sum is an
-// IEEE float fma.  Each output element is the sum over k in ascending order,
-// whatever M is and wherever the row stands in the batch, so a row gives the
-// same bits alone, in a prompt or in a batch.
+// IEEE float fma.  One order of sums holds for all kernels of this file,
+// whatever M is, wherever the row stands in the batch and however the work is
+// cut:
+//
+//     y = C_0 + C_1 + C_2 + ...                    in ascending order,
+//     C_s = (sum over the even k) + (sum over the odd k)   of k in [512 s, 512 s + 512),
+//
+// each of the two sums being a chain of fmas over ascending k from zero.  So
+// a row gives the same bits alone, in a prompt or in a batch, and there are
+// independent sums to give to different warps and blocks (one chain over
+// K = 9216 leaves a decode step nothing to run in parallel, and a chain that
+// long also rounds more).  Even and odd k are the two halves of a packed
+// fma.rn.f32x2, whose operands are neighbours in a row of X and of W: both
+// are read from shared memory as they lie in memory.
+//
+// Three kernels:
+//   rows_kernel   M <= 16: the product is a stream of W.  Bound by memory.
+//   tiles_kernel  M > 16: tiles of 32 or 64 rows by 128 columns.  Bound by the fma pipes.
+//   any_kernel    operands whose rows do not lie on 16-byte boundaries.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int SEG = 512;        // k of one C_s
 
-__global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ X, int ldx,
-                                                         const float* __restrict__ W, int ldw,
-                                                         float* __restrict__ Y, int ldy, int M, int N, int K) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float halves_sum(uint64_t v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo + hi;
+}
+struct Pair2 { uint64_t x, y; };       // four consecutive floats
+__device__ __forceinline__ Pair2 lds4(uint32_t addr) {
+    Pair2 v;
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
+}
+// 16 bytes from global into shared memory, zeros when !ok
+__device__ __forceinline__ void copy16(uint32_t dst, const float* p, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(p), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// ---------------------------------------------------------------------------
+// M <= MP <= 16.  A block owns RG * R rows of W over the whole of K, a lane R rows of one segment at a time: the
+// 32 / RG segments a warp works on lie side by side in its lanes, and its warps take them in turns.  Every warp has a
+// queue of its own in shared memory (cp.async, no barrier): slices of 32 k of its rows, 128 bytes each from memory,
+// rows 144 bytes apart so that eight lanes' 16-byte reads fall into different banks; x's part of the slice comes along
+// and is read by all lanes of a segment at once.  The sums of all segments meet in shared memory and are added in
+// ascending order.
+// A warp's 16-byte read takes shared memory four cycles even where all lanes read one address, so with one row a lane
+// the reads of x set the pace from M = 8 on (256,000 x 2,304: 680 us at M = 8 and 987 us at M = 16, against 370 us at
+// M = 1, which is 6.4 TB/s): a lane then takes two rows for every x it reads (533 and 836 us).  At M = 3 a layer's four
+// products take 15, 14, 41 and 24 us (q/k/v, o, gate and up, down of 2,304 / 9,216); the tiles below, which served all M
+// before, took 317 us each on average.
+constexpr int PITCH = 144;                       // bytes of a pair's 32 k, with padding
+
+template <int R> __host__ __device__ constexpr int slots() { return R == 1 ? 5 : 4; }
+template <int MP, int RG> __host__ __device__ constexpr int x_bytes() { return (32 / RG) * (MP * 128 + 16); }
+template <int MP, int RG, int R> __host__ __device__ constexpr int slot_bytes() { return 32 * R * PITCH + x_bytes<MP, RG>(); }
+
+template <int MP, int RG, int R>
+__global__ void __launch_bounds__(256) rows_kernel(const float* __restrict__ X, int ldx, const float* __restrict__ W, int ldw,
+                                                   float* __restrict__ Y, int ldy, int M, int N, int K) {
+    constexpr int SUBS = 32 / RG, SLOTS = slots<R>(), ROWS = RG * R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    const int n_seg = (K + SEG - 1) / SEG, units = (n_seg + SUBS - 1) / SUBS;
+    const int n0 = blockIdx.x * ROWS;
+    extern __shared__ __align__(16) uint8_t raw[];
+    const uint32_t queue = (uint32_t)__cvta_generic_to_shared(raw) + warp * (SLOTS * slot_bytes<MP, RG, R>());
+    float* sums = reinterpret_cast<float*>(raw + (size_t)n_warps * (SLOTS * slot_bytes<MP, RG, R>()));   // [seg][MP][ROWS]
+
+    constexpr int SLICES = SEG / 32;
+    const int my_units = warp < units ? (units - warp + n_warps - 1) / n_warps : 0;
+    // the last unit ends with K
+    const int tail = min(SLICES, (K - (units - 1) * SUBS * SEG + 31) / 32);
+    const int total = my_units * SLICES - (my_units && (units - 1) % n_warps == warp ? SLICES - tail : 0);
+    // slice i of this warp: unit warp + n_warps * (i / SLICES), k from 32 * (i % SLICES) of each of its segments
+    auto slice_k = [&](int i, int sub) {
+        return ((warp + n_warps * (i / SLICES)) * SUBS + sub) * SEG + (i % SLICES) * 32;
+    };
+    auto fetch_w = [&](int i) {
+        if (i >= total) return;
+        const uint32_t dst = queue + (i % SLOTS) * slot_bytes<MP, RG, R>();
+#pragma unroll
+        for (int j = 0; j < 8 * R; ++j) {                           // [row of the lane][segment][row]
+            const int p = j * 4 + (lane >> 3), row = n0 + p % RG + (p / 32) * RG, k = slice_k(i, p % 32 / RG) + (lane & 7) * 4;
+            const bool ok = row < N && k < K;                       // K is a multiple of 4
+            copy16(dst + p * PITCH + (lane & 7) * 16, W + (ok ? (size_t)row * ldw + k : 0), ok);
+        }
+    };
+    auto fetch_x = [&](int i) {
+        if (i >= total) return;
+        const uint32_t dst = queue + (i % SLOTS) * slot_bytes<MP, RG, R>() + 32 * R * PITCH;
+#pragma unroll
+        for (int j = 0; j < (SUBS * MP * 8 + 31) / 32; ++j) {
+            const int idx = j * 32 + lane, m = (idx >> 3) % MP, sub = idx / (MP * 8);
+            if (idx < SUBS * MP * 8) {
+                const int k = slice_k(i, sub) + (idx & 7) * 4;
+                const bool ok = m < M && k < K;
+                copy16(dst + sub * (MP * 128 + 16) + m * 128 + (idx & 7) * 16, X + (ok ? (size_t)m * ldx + k : 0), ok);
+            }
+        }
+    };
+
+    // W depends on nothing that ran before; X is the kernel before this one's result
+#pragma unroll
+    for (int i = 0; i < SLOTS - 1; ++i) fetch_w(i);
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < SLOTS - 1; ++i) {
+        fetch_x(i);
+        copy_commit();
+    }
+    uint64_t acc[R][MP];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int m = 0; m < MP; ++m) acc[r][m] = 0;
+    const int sub = lane / RG;
+    for (int i = 0; i < total; ++i) {
+        copy_wait<SLOTS - 2>();
+        __syncwarp();                            // the slice has landed for all lanes, and slice i - 1 has been read by all
+        fetch_w(i + SLOTS - 1);
+        fetch_x(i + SLOTS - 1);
+        copy_commit();
+        const uint32_t slot = queue + (i % SLOTS) * slot_bytes<MP, RG, R>();
+        const uint32_t wp = slot + lane * PITCH, xp = slot + 32 * R * PITCH + sub * (MP * 128 + 16);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            Pair2 w[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) w[r] = lds4(wp + r * 32 * PITCH + c * 16);
+#pragma unroll
+            for (int m = 0; m < MP; ++m) {
+                const Pair2 x = lds4(xp + m * 128 + c * 16);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    fma2(acc[r][m], w[r].x, x.x);
+                    fma2(acc[r][m], w[r].y, x.y);
+                }
+            }
+        }
+        if (i % SLICES == SLICES - 1 || i == total - 1) {
+            const int seg = (warp + n_warps * (i / SLICES)) * SUBS + sub;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int m = 0; m < MP; ++m) {
+                    if (seg < n_seg) sums[(seg * MP + m) * ROWS + r * RG + lane % RG] = halves_sum(acc[r][m]);
+                    acc[r][m] = 0;
+                }
+        }
+    }
+    copy_wait<0>();
+    pdl_trigger();
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < MP * ROWS; idx += blockDim.x) {
+        const int m = idx / ROWS, n = n0 + idx % ROWS;
+        if (m >= M || n >= N) continue;
+        float y = sums[idx];
+        for (int s = 1; s < n_seg; ++s) y += sums[s * MP * ROWS + idx];
+        Y[(size_t)m * ldy + n] = y;
+    }
+}
+
+template <int MP, int RG, int R>
+int launch_rows(const float* x, int ldx, const float* w, int ldw, float* y, int ldy, int M, int N, int K, cudaStream_t stream) {
+    const int n_seg = (K + SEG - 1) / SEG, units = (n_seg + 32 / RG - 1) / (32 / RG);
+    constexpr int ROWS = RG * R;
+    const size_t sums = (size_t)n_seg * MP * ROWS * sizeof(float);
+    constexpr size_t queue = (size_t)slots<R>() * slot_bytes<MP, RG, R>();
+    // two blocks an SM where that leaves at least two warps; of the counts that fit, the largest that leaves no warp
+    // of the last round of units without one
+    int fit = sums < 112 * 1024 ? (int)((112 * 1024 - sums) / queue) : 0;
+    if (fit < 2) fit = sums < 224 * 1024 ? (int)((224 * 1024 - sums) / queue) : 0;
+    if (fit < 1) return BROLM_ERR_TOO_LARGE;
+    fit = fit < 8 ? fit : 8;
+    int warps = fit < units ? fit : units;
+    warps = (units + (units + warps - 1) / warps - 1) / ((units + warps - 1) / warps);
+    const size_t smem = warps * queue + sums;
+    static bool raised = false;
+    if (!raised) {
+        cudaError_t e = cudaFuncSetAttribute(rows_kernel<MP, RG, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) return (int)e;
+        raised = true;
+    }
+    return launch_pdl(rows_kernel<MP, RG, R>, dim3((N + ROWS - 1) / ROWS), dim3(warps * 32), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K);
+}
+
+// Rows of W per block: as many as leave two blocks for every SM, since the memory wants all SMs at work (a block of
+// fewer rows has the segments beside one another in its lanes, and reads x once per segment instead of once).  Two rows
+// a lane for more than four tokens, if that leaves lanes for about four warps an SM: 2,304 x 9,216 with 8 tokens 38.8 ->
+// 28.6 us, 18,432 x 2,304 with 16 tokens 82 -> 63 us, but 2,304 x 2,048 with 16 tokens 18.8 -> 23.4 us, and with 3
+// tokens 256,000 x 2,304 takes 464 us with one and 494 us with two.
+template <int MP, int R>
+int dispatch_groups(const float* x, int ldx, const float* w, int ldw, float* y, int ldy, int M, int N, int K, cudaStream_t stream) {
+    const int want = 2 * device_sm_count() - 40;
+    if (N / (32 * R) >= want) return launch_rows<MP, 32, R>(x, ldx, w, ldw, y, ldy, M, N, K, stream);
+    if (N / (16 * R) >= want) return launch_rows<MP, 16, R>(x, ldx, w, ldw, y, ldy, M, N, K, stream);
+    return launch_rows<MP, 8, R>(x, ldx, w, ldw, y, ldy, M, N, K, stream);
+}
+template <int MP>
+int dispatch_rows(const float* x, int ldx, const float* w, int ldw, float* y, int ldy, int M, int N, int K, cudaStream_t stream) {
+    if constexpr (MP > 4)
+        if ((long long)N * ((K + SEG - 1) / SEG) >= 2 * 4 * 32 * (long long)device_sm_count())
+            return dispatch_groups<MP, 2>(x, ldx, w, ldw, y, ldy, M, N, K, stream);
+    return dispatch_groups<MP, 1>(x, ldx, w, ldw, y, ldy, M, N, K, stream);
+}
+
+// ---------------------------------------------------------------------------
+// Tiles of BM x 128, BM / 8 x 8 outputs a thread (rows 8 apart, columns 16 apart: the eight lanes of a 16-byte read take
+// eight neighbouring rows of W, 144 bytes apart).  Shared memory hands out 128 bytes a cycle, so a thread's outputs have
+// to be as many as its registers hold: 8 x 8 reads 64 bytes for 64 fmas, which is what the fma pipes take in that time
+// (18,432 x 2,304: 43 TFLOP/s at M = 300 and 47 at M = 1024, of which the fma pipes are busy 64 %; 38 and 42 with
+// 8 x 4 and twice the warps; 24 and 25 before, with 4 x 4 and scalar fmas).  Two stages of 32 k; the sum over
+// the finished segments waits in shared memory, [output][thread].  The segments of K may be dealt to blocks along
+// z; with `parts` every segment's sums go to its own slice of Y, with one block along z they are added here.
+constexpr int BN = 128, STAGES = 2;
+
+template <int BM>
+__global__ void __launch_bounds__(128, 2) tiles_kernel(const float* __restrict__ X, int ldx, const float* __restrict__ W, int ldw,
+                                                       float* __restrict__ Y, int ldy, int M, int N, int K, int seg_per_block,
+                                                       int parts, long long part_stride) {
+    constexpr int TM = BM / 8, TN = BN / 16;
+    constexpr int STAGE = (BM + BN) * PITCH;
+    extern __shared__ __align__(16) uint8_t raw[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tn = (lane & 7) + 8 * (warp & 1), tm = (lane >> 3) + 4 * (warp >> 1);
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int seg0 = blockIdx.z * seg_per_block;
+    const int k_end = min(K, (seg0 + seg_per_block) * SEG);
+    const int steps = (k_end - seg0 * SEG + 31) / 32;
+
+    auto fetch = [&](int i) {
+        if (i < steps) {
+            const int k = seg0 * SEG + i * 32 + (tid & 7) * 4;
+            const uint32_t dst = base + (i % STAGES) * STAGE + (tid >> 3) * PITCH + (tid & 7) * 16;
+#pragma unroll
+            for (int j = 0; j < (BM + BN) / 16; ++j) {
+                const int row = j * 16 + (tid >> 3);
+                const float* p = row < BM ? X : W;
+                const long long r = row < BM ? m0 + row : n0 + row - BM;
+                const bool ok = k < K && r < (row < BM ? M : N);
+                copy16(dst + j * 16 * PITCH, p + (ok ? r * (row < BM ? ldx : ldw) + k : 0), ok);
+            }
+        }
+        copy_commit();
+    };
+
+    uint64_t acc[TM][TN];
+    float* tot = reinterpret_cast<float*>(raw + STAGES * STAGE) + tid;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0;
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) fetch(i);
+    for (int i = 0; i < steps; ++i) {
+        copy_wait<STAGES - 2>();
+        __syncthreads();                         // stage i has landed for all threads, and stage i - 1 has been read
+        fetch(i + STAGES - 1);
+        const uint32_t xs = base + (i % STAGES) * STAGE + tm * PITCH, ws = base + (i % STAGES) * STAGE + (BM + tn) * PITCH;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            Pair2 w[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) w[j] = lds4(ws + j * 16 * PITCH + c * 16);
+#pragma unroll
+            for (int t = 0; t < TM; ++t) {
+                const Pair2 x = lds4(xs + t * 8 * PITCH + c * 16);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[t][j], w[j].x, x.x);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fma2(acc[t][j], w[j].y, x.y);
+            }
+        }
+        if (i % (SEG / 32) == SEG / 32 - 1 || i == steps - 1) {
+            const int seg = i / (SEG / 32);
+            if (parts) {
+                float* dst = Y + (seg0 + seg) * part_stride;
+#pragma unroll
+                for (int t = 0; t < TM; ++t)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        const int m = m0 + tm + 8 * t, n = n0 + tn + 16 * j;
+                        if (m < M && n < N) dst[(size_t)m * ldy + n] = halves_sum(acc[t][j]);
+                        acc[t][j] = 0;
+                    }
+            } else {
+#pragma unroll
+                for (int t = 0; t < TM; ++t)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        const float c = halves_sum(acc[t][j]);
+                        tot[(t * TN + j) * 128] = seg == 0 ? c : tot[(t * TN + j) * 128] + c;
+                        acc[t][j] = 0;
+                    }
+            }
+        }
+    }
+    pdl_trigger();
+    if (parts) return;
+#pragma unroll
+    for (int t = 0; t < TM; ++t)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int m = m0 + tm + 8 * t, n = n0 + tn + 16 * j;
+            if (m < M && n < N) Y[(size_t)m * ldy + n] = tot[(t * TN + j) * 128];
+        }
+}
+
+// y = parts[0] + parts[1] + ... in order; parts [n_parts][M][N]
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ parts, int n_parts, float* __restrict__ Y,
+                                                        int ldy, int M, int N) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t stride = (size_t)M * N;
+    for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < stride; idx += (size_t)gridDim.x * 256) {
+        float y = parts[idx];
+#pragma unroll 4
+        for (int s = 1; s < n_parts; ++s) y += parts[s * stride + idx];
+        Y[idx / N * ldy + idx % N] = y;
+    }
+}
+
+template <int BM>
+int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int ldy, int M, int N, int K, float* parts,
+                 int seg_per_block, cudaStream_t stream) {
+    constexpr int smem = STAGES * (BM + BN) * PITCH + BM * BN * (int)sizeof(float);
+    static bool raised = false;
+    if (!raised) {
+        cudaError_t e = cudaFuncSetAttribute(tiles_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+        raised = true;
+    }
+    const int n_seg = (K + SEG - 1) / SEG;
+    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, parts ? (n_seg + seg_per_block - 1) / seg_per_block : 1);
+    if (!parts)
+        return launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K, n_seg, 0, 0LL);
+    const int st = launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, parts, N, M, N, K, seg_per_block, 1,
+                              (long long)M * N);
+    if (st) return st;
+    const size_t blocks = ((size_t)M * N + 255) / 256;
+    return launch_pdl(sum_parts_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, parts, n_seg, y, ldy,
+                      M, N);
+}
+
+// ---------------------------------------------------------------------------
+// Any strides and sizes: 64 x 64 tiles, 4 x 4 outputs a thread, one element at a time.
+constexpr int AM = 64, AN = 64, AK = 16;
+
+__global__ void __launch_bounds__(256) any_kernel(const float* __restrict__ X, int ldx, const float* __restrict__ W, int ldw,
+                                                  float* __restrict__ Y, int ldy, int M, int N, int K) {
+    __shared__ float As[AK][AM + 4];
+    __shared__ float Bs[AK][AN + 4];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;            // 16 x 16 threads, 4 x 4 outputs each
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * AM, n0 = blockIdx.x * AN;
     const int lr = tid >> 2, lk = (tid & 3) * 4;        // loader: row lr, k offset lk..lk+3
-    const bool vec = (K % 4 == 0) && (ldx % 4 == 0) && (ldw % 4 == 0) &&
-                     ((reinterpret_cast<uintptr_t>(X) & 15) == 0) && ((reinterpret_cast<uintptr_t>(W) & 15) == 0);
 
-    float acc[4][4];
+    float acc[2][4][4], tot[4][4];                      // [parity of k]
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = tot[i][j] = 0.0f;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
+    for (int k0 = 0; k0 < K; k0 += AK) {
         float a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
         const int k = k0 + lk;
         if (m0 + lr < M) {
             const float* p = X + (size_t)(m0 + lr) * ldx + k;
-            if (vec && k + 3 < K) {
-                const float4 t = *reinterpret_cast<const float4*>(p);
-                a[0] = t.x; a[1] = t.y; a[2] = t.z; a[3] = t.w;
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) if (k + i < K) a[i] = p[i];
-            }
+            for (int i = 0; i < 4; ++i) if (k + i < K) a[i] = p[i];
         }
         if (n0 + lr < N) {
             const float* p = W + (size_t)(n0 + lr) * ldw + k;
-            if (vec && k + 3 < K) {
-                const float4 t = *reinterpret_cast<const float4*>(p);
-                b[0] = t.x; b[1] = t.y; b[2] = t.z; b[3] = t.w;
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) if (k + i < K) b[i] = p[i];
-            }
+            for (int i = 0; i < 4; ++i) if (k + i < K) b[i] = p[i];
         }
         __syncthreads();   // the tile before this one is consumed
 #pragma unroll
@@ -60,14 +395,24 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
         }
         __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
+        for (int kk = 0; kk < AK; ++kk) {
             const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
             const float4 bv = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
             const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], br[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[kk & 1][i][j] = fmaf(ar[i], br[j], acc[kk & 1][i][j]);
+        }
+        if ((k0 + AK) % SEG == 0 || k0 + AK >= K) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float c = acc[0][i][j] + acc[1][i][j];
+                    tot[i][j] = k0 < SEG ? c : tot[i][j] + c;
+                    acc[0][i][j] = acc[1][i][j] = 0.0f;
+                }
         }
     }
 #pragma unroll
@@ -77,20 +422,38 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            if (n < N) Y[(size_t)m * ldy + n] = acc[i][j];
+            if (n < N) Y[(size_t)m * ldy + n] = tot[i][j];
         }
     }
 }
 
 }  // namespace
 
+// M <= 16 rows, and more in tiles.  parts (M > 16 only): room for ceil(K / 512) * M * N floats, into which the blocks,
+// seg_per_block segments of 512 k each, put their sums before they are added; null: a block takes all of K.
 BROLM_API int brolm_linear_f32(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
-                               cudaStream_t stream) {
+                               void* parts, int seg_per_block, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;
-    if (K <= 0) return BROLM_ERR_BAD_SIZE;
-    const long long gy = (M + BM - 1) / BM;
+    if (K <= 0 || (parts && seg_per_block < 1)) return BROLM_ERR_BAD_SIZE;
+    const float *xf = (const float*)x, *wf = (const float*)w;
+    float* yf = (float*)y;
+    const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)w & 15);
+    if (vec && M <= 16) {
+        const int st = M <= 1 ? dispatch_rows<1>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
+                     : M <= 2 ? dispatch_rows<2>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
+                     : M <= 4 ? dispatch_rows<4>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
+                     : M <= 8 ? dispatch_rows<8>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
+                              : dispatch_rows<16>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream);
+        if (st != BROLM_ERR_TOO_LARGE) return st;        // a K beyond what the sums have room for goes on below
+    }
+    const long long tiles_n = (N + BN - 1) / BN;
+    if (vec && tiles_n <= 65535) {
+        if (M <= 32) return launch_tiles<32>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
+        return launch_tiles<64>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
+    }
+    const long long gy = (M + AM - 1) / AM;
     if (gy > 65535) return BROLM_ERR_TOO_LARGE;
-    dim3 grid((N + BN - 1) / BN, (unsigned)gy);
-    linear_f32_kernel<<<grid, 256, 0, stream>>>((const float*)x, ldx, (const float*)w, ldw, (float*)y, ldy, M, N, K);
+    dim3 grid((N + AN - 1) / AN, (unsigned)gy);
+    any_kernel<<<grid, 256, 0, stream>>>(xf, ldx, wf, ldw, yf, ldy, M, N, K);
     return launch_status();
 }

@@ -1039,18 +1039,44 @@ def rotate_heads(rows: torch.Tensor, q_off: int, k_off: int, heads: int, dim: in
              rows.shape[0], _stream()), "rotate_heads")
 
 
+F32_SEGMENT = 512          # k of one partial sum of the float32 product (linear_f32.cu)
+
+
+def linear_f32_cut(M: int, N: int, K: int, sms: Optional[int] = None) -> int:
+    """How many 512-wide segments of K a block of the tiled float32 product takes; 0: all of them, nothing to add.
+
+    Two blocks share an SM, a block's time is its segments and about a quarter of one to start and end, and the last
+    round of blocks lasts as long as a full one; cut blocks cost writing and adding the segments' sums, about a third of
+    a segment.  (M = 300: the 4096 x 2304 product is 160 tiles for 296 places, cut into single segments it fills three
+    rounds of a fifth of the length.)  At most 16 rows need no cut: that kernel gives the segments to its warps."""
+    if M <= 16:
+        return 0
+    places = 2 * (sms or device_sms())
+    tiles = -(-M // (32 if M <= 32 else 64)) * -(-N // 128)
+    segs = -(-K // F32_SEGMENT)
+    best, cut = -(-tiles // places) * (segs + 0.25), 0
+    for per in range(segs - 1, 0, -1):
+        cost = -(-tiles * -(-segs // per) // places) * (per + 0.25) + 0.3
+        if cost < best:
+            best, cut = cost, per
+    return cut
+
+
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
-    """out (M, N) = x (M, K) @ weight (N, K)^T, all float32, rows may be strided."""
+    """out (M, N) = x (M, K) @ weight (N, K)^T, all float32, rows may be strided.  A row's bits depend on neither M
+    nor its place among the rows."""
     assert x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32
     assert x.dim() == 2 and weight.dim() == 2 and out.dim() == 2
     assert x.stride(1) == 1 and weight.stride(1) == 1 and out.stride(1) == 1
     M, K = x.shape
     N = weight.shape[0]
     assert weight.shape[1] == K and tuple(out.shape) == (M, N)
+    cut = linear_f32_cut(M, N, K)
+    parts = torch.empty((-(-K // F32_SEGMENT), M, N), dtype=torch.float32, device=x.device) if cut else None
     f = _fn("linear_f32", "brolm_linear_f32", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
-                                               c_void_p])
-    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, _stream()),
-           "linear_f32")
+                                               c_void_p, c_int, c_void_p])
+    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(parts), cut,
+             _stream()), "linear_f32")
 
 
 SKINNY_MAX_ROWS = 16

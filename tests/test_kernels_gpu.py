@@ -130,6 +130,30 @@ def test_linear_f32(M, N, K):
     assert torch.equal(one[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 2, 5, 16, 17, 33, 70])
+@pytest.mark.parametrize("N,K", [(8, 4), (33, 516), (2304, 2304), (136, 9216), (4750, 1028), (9500, 512)])
+def test_linear_f32_kernels_and_cuts(M, N, K):
+    """Streams of 8, 16 and 32 rows a block, tiles of 32 and 64 rows, cut along K and not: float sums, one order."""
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    x = torch.randn(M, K, generator=g, device=DEV)
+    w = torch.randn(N, K, generator=g, device=DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    kernels.linear_f32(x, w, out)
+    ref = x.double() @ w.double().T
+    # chains of at most 256 fmas, then their sums: each rounding is at most 2^-24 of a partial sum
+    bound = (256 + K / 256) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    one = torch.empty(1, N, device=DEV)
+    kernels.linear_f32(x[M - 1:], w, one)
+    assert torch.equal(one[0], out[M - 1])
+    # the same numbers off the 16-byte boundaries: the kernel for any operands, in the same order
+    wide = torch.empty(M, K + 1, device=DEV)
+    wide[:, 1:] = x
+    again = torch.empty(M, N, device=DEV)
+    kernels.linear_f32(wide[:, 1:], w, again)
+    assert torch.equal(again, out)
+
+
 def test_linear_f32_strided_views():
     g = torch.Generator().manual_seed(6)
     big = torch.randn(9, 3 * 48, generator=g).to(DEV)
