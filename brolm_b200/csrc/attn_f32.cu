@@ -1,0 +1,470 @@
+// Float attention over a prompt's packed keys or the paged cache, on CUDA cores: the float model's path where rows are
+// whole 16-byte pieces of at most 256 elements (attn_simt.cu has the masks and options, and takes everything else).
+//
+// One order of operations for a query, whatever step, batch or split it runs in, so that a prompt pass and a decode pass
+// give the same bits.  Keys come in spans of 128, anchored at multiples of 128 of the absolute position:
+//
+//   score    s_j = (sum over even c of q_c k_c) + (sum over odd c), each a chain of fmas over ascending c; then the
+//            scale, the cap, the slope, the distance bias and the mask
+//   span     m = max s_j, p_j = exp(s_j - m), l = the 32-key sums of p (a butterfly over lanes) added in order,
+//            a_d = a chain of fmas p_j v_jd over ascending j
+//   merge    of the spans in ascending order: M' = max(M, m), L = L e^(M - M') + l e^(m - M'), A alike
+//
+// and the result is A / L (with a sink: A / (L + e^(sink - M))).
+//
+// A block owns 32 rows of one (sequence, kv head), a row being a (query token, query head of the group) pair, or 8 where
+// a step has no more (decode), and either walks all spans it sees or, where that leaves SMs idle, one of them, with
+// merge_kernel behind it (attn_f32_splits in kernels/__init__.py has the rule and what both take): a decode step of three
+// sequences of up to 420 keys is otherwise twelve blocks (30 us shared; 337 us in attn_simt.cu, which served all sizes
+// before; a prompt of 300 tokens 72 and 187 us).  K comes through a ring of cp.async stages in slices of 32 c of all 128 keys, V in
+// slices of 16 keys; both products run on packed fma.rn.f32x2, the scores paired along c, the values along d.  Bound by
+// shared memory: a thread's outputs are what its registers hold (4 x 8 scores, 4 x 16 values).
+#include "common.cuh"
+
+namespace {
+
+constexpr int SPAN = 128;
+constexpr int THREADS = 128;
+constexpr int STAGES = 3;
+constexpr int KC = 32;                        // c of a slice of keys
+constexpr int PITCH = 144;                    // its bytes, padded: eight neighbouring rows lie in different banks
+constexpr int VK = 16;                        // keys of a slice of values
+constexpr int STAGE = SPAN * PITCH;           // 18,432 bytes; a slice of values takes VK * vd * 4 <= 16,384
+constexpr int P_PITCH = SPAN + 4;             // floats
+
+struct F32Args {
+    const float* q;
+    float* out;
+    int q_stride, out_stride;
+    const int32_t* cu_q;
+    const int32_t* kv_len;
+    const float* k;
+    const float* v;
+    int k_stride, v_stride;
+    const float* k_pages;                     // null: packed keys
+    const float* v_pages;
+    const int32_t* page_table;
+    int pt_stride, ring, page_size;
+    int n_kv, group, hd, vd;
+    float scale, cap;
+    int window, chunk;
+    const float* sink;
+    const float* slopes;
+    const float* dist_bias;
+    int dist_len;
+    int splits;                               // spans a tile can see; 0: a block walks them all
+    float* part_acc;                          // [token][head][split][vd]
+    float* part_ml;                           // [token][head][split][2]
+};
+
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+struct Pair2 { uint64_t x, y; };
+__device__ __forceinline__ Pair2 lds4(const float* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return Pair2{v.x, v.y};
+}
+__device__ __forceinline__ void copy16(void* dst, const float* p, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(p),
+                 "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// The merge of one more span into (M, L): factors for what is held and for what comes.
+__device__ __forceinline__ void merge_factors(float& M, float& L, float m, float l, float& held, float& fresh) {
+    const float top = fmaxf(M, m);
+    held = M > -INFINITY ? expf(M - top) : 0.0f;
+    fresh = m > -INFINITY ? expf(m - top) : 0.0f;
+    L = __fmaf_rn(L, held, __fmul_rn(l, fresh));
+    M = top;
+}
+__device__ __forceinline__ float merged(float held_sum, float held, float fresh_sum, float fresh) {
+    return __fmaf_rn(held_sum, held, __fmul_rn(fresh_sum, fresh));
+}
+__device__ __forceinline__ float share(const F32Args& a, float M, float L, int head) {
+    if (a.sink && M > -INFINITY) L += expf(a.sink[head] - M);
+    return L > 0.0f ? 1.0f / L : 0.0f;
+}
+
+// The rows of a tile and the spans they see: [first, last].
+struct Tile { int q0, row0, rows, first_pos, key_lo, first, last; };
+template <int ROWS>
+__device__ __forceinline__ Tile tile_of(const F32Args& a, int b, int tile) {
+    Tile t;
+    t.q0 = a.cu_q[b];
+    const int q_len = a.cu_q[b + 1] - t.q0, kv_len = a.kv_len[b];
+    t.row0 = tile * ROWS;
+    t.rows = kv_len > 0 ? max(0, min(ROWS, q_len * a.group - t.row0)) : 0;
+    t.first_pos = kv_len - q_len;
+    if (t.rows <= 0) return t;
+    const int lo = t.first_pos + t.row0 / a.group;
+    int key = a.window > 0 ? max(0, lo - a.window + 1) : 0;
+    if (a.chunk > 0) key = max(key, lo - lo % a.chunk);
+    t.key_lo = key;
+    t.first = key / SPAN;
+    t.last = (t.first_pos + (t.row0 + t.rows - 1) / a.group) / SPAN;
+    return t;
+}
+
+template <int ROWS, int VJ>
+__global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
+    constexpr int LN = ROWS == 32 ? 16 : 32;           // threads side by side over keys, and over value dims
+    constexpr int RI = ROWS / (THREADS / LN);          // rows of a thread, THREADS / LN apart
+    constexpr int RSTEP = THREADS / LN, KJ = SPAN / LN;
+    extern __shared__ __align__(16) uint8_t raw[];
+    const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;  // floats; zeros behind hd
+    uint8_t* ring = raw;
+    float* Qs = reinterpret_cast<float*>(raw + STAGES * STAGE);
+    float* P = Qs + ROWS * q_pitch;
+    float* stats = P + ROWS * P_PITCH;                  // [ROWS]: M, L, factor of what is held, factor of what comes
+    long long* k_off = reinterpret_cast<long long*>(stats + 4 * ROWS);
+    long long* v_off = k_off + SPAN;
+
+    const int b = blockIdx.z, g = blockIdx.y;
+    const int tile = a.splits ? blockIdx.x / a.splits : blockIdx.x;
+    pdl_wait();
+    const Tile t = tile_of<ROWS>(a, b, tile);
+    if (t.rows <= 0) return;
+    int span = t.first, last = t.last;
+    if (a.splits) {
+        span += blockIdx.x % a.splits;
+        if (span > last) return;
+        last = span;
+    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tn = tid % LN, tm = tid / LN;
+    const int key_hi = t.first_pos + (t.row0 + t.rows - 1) / a.group;
+
+    for (int idx = tid; idx < ROWS * (q_pitch / 4); idx += THREADS) {
+        const int r = idx / (q_pitch / 4), c = (idx - r * (q_pitch / 4)) * 4;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < t.rows && c < a.hd) {
+            const int row = t.row0 + r;
+            v = *reinterpret_cast<const float4*>(a.q + (size_t)(t.q0 + row / a.group) * a.q_stride +
+                                                 (g * a.group + row % a.group) * a.hd + c);
+        }
+        *reinterpret_cast<float4*>(Qs + r * q_pitch + c) = v;
+    }
+    if (tid < ROWS) {
+        stats[tid] = -INFINITY;
+        stats[ROWS + tid] = 0.0f;
+    }
+
+    const int k_slices = (a.hd + KC - 1) / KC;
+    float tot[RI][VJ][4];
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+        for (int j = 0; j < VJ; ++j) tot[i][j][0] = tot[i][j][1] = tot[i][j][2] = tot[i][j][3] = 0.0f;
+
+    for (; span <= last; ++span) {
+        const int key0 = span * SPAN;
+        const int keys = min(SPAN, key_hi + 1 - key0);  // keys behind the tile's last query are not read
+        __syncthreads();                                // the span before this one is done with (and Q and stats are written)
+        {
+            const int kp = key0 + tid;
+            long long ko = -1, vo = -1;
+            if (tid < keys && kp >= t.key_lo) {          // (a ring's places of older positions hold other keys)
+                if (a.k_pages) {
+                    const int place = kp % a.ring, page = a.page_table[(size_t)b * a.pt_stride + place / a.page_size];
+                    const long long at = ((long long)page * a.n_kv + g) * a.page_size + place % a.page_size;
+                    ko = at * a.hd;
+                    vo = at * a.vd;
+                } else {
+                    ko = (long long)(t.q0 + kp) * a.k_stride + (long long)g * a.hd;
+                    vo = (long long)(t.q0 + kp) * a.v_stride + (long long)g * a.vd;
+                }
+            }
+            k_off[tid] = ko;
+            v_off[tid] = vo;
+        }
+        __syncthreads();
+        const float* kb = a.k_pages ? a.k_pages : a.k;
+        const float* vb = a.k_pages ? a.v_pages : a.v;
+        const int v_slices = (keys + VK - 1) / VK, slices = k_slices + v_slices;
+        auto fetch = [&](int i) {
+            uint8_t* dst = ring + (i % STAGES) * STAGE;
+            if (i < k_slices) {
+                const int c = i * KC + (tid & 7) * 4;
+#pragma unroll
+                for (int j = 0; j < SPAN / 16; ++j) {
+                    const int key = j * 16 + (tid >> 3);
+                    const long long o = k_off[key];
+                    const bool ok = o >= 0 && c < a.hd;
+                    copy16(dst + key * PITCH + (tid & 7) * 16, kb + (ok ? o + c : 0), ok);
+                }
+            } else if (i < slices) {
+                const int pieces = a.vd / 4;
+                for (int idx = tid; idx < VK * pieces; idx += THREADS) {
+                    const int j = idx / pieces, c = (idx - j * pieces) * 4;
+                    const long long o = v_off[(i - k_slices) * VK + j];
+                    copy16(dst + (j * a.vd + c) * 4, vb + (o >= 0 ? o + c : 0), o >= 0);
+                }
+            }
+            copy_commit();
+        };
+#pragma unroll
+        for (int i = 0; i < STAGES - 1; ++i) fetch(i);
+
+        uint64_t s[RI][KJ];
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) s[i][j] = 0;
+        for (int i = 0; i < k_slices; ++i) {
+            copy_wait<STAGES - 2>();
+            __syncthreads();
+            fetch(i + STAGES - 1);
+            const float* ks = reinterpret_cast<const float*>(ring + (i % STAGES) * STAGE) + tn * (PITCH / 4);
+            const float* qs = Qs + tm * q_pitch + i * KC;
+#pragma unroll
+            for (int c = 0; c < KC; c += 4) {
+                Pair2 q[RI];
+#pragma unroll
+                for (int r = 0; r < RI; ++r) q[r] = lds4(qs + r * RSTEP * q_pitch + c);
+#pragma unroll
+                for (int j = 0; j < KJ; ++j) {
+                    const Pair2 k = lds4(ks + j * LN * (PITCH / 4) + c);
+#pragma unroll
+                    for (int r = 0; r < RI; ++r) {
+                        fma2(s[r][j], q[r].x, k.x);
+                        fma2(s[r][j], q[r].y, k.y);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RI; ++r) {
+            const int rr = tm + r * RSTEP, row = t.row0 + rr;
+            const int pos = rr < t.rows ? t.first_pos + row / a.group : -1, head = g * a.group + row % a.group;
+            const float slope = a.slopes && pos >= 0 ? a.slopes[head] : 0.0f;
+            const int from = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 && pos >= 0 ? pos - pos % a.chunk : 0);
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+                const int kp = key0 + tn + j * LN;
+                float sc = -INFINITY;
+                if (kp <= pos && kp >= from) {
+                    const float2 h = unpack2(s[r][j]);
+                    sc = soft_cap(__fmul_rn(h.x + h.y, a.scale), a.cap);
+                    if (a.slopes) sc = __fmaf_rn(-slope, (float)(pos - kp), sc);
+                    if (a.dist_bias) sc += a.dist_bias[(size_t)head * a.dist_len + min(pos - kp, a.dist_len - 1)];
+                }
+                P[rr * P_PITCH + tn + j * LN] = sc;
+            }
+        }
+        __syncthreads();
+        for (int r = warp * (ROWS / 4); r < (warp + 1) * (ROWS / 4); ++r) {
+            float sc[4], m = -INFINITY, l = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sc[e] = P[r * P_PITCH + e * 32 + lane];
+                m = fmaxf(m, sc[e]);
+            }
+            m = warp_max(m);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float p = sc[e] == -INFINITY ? 0.0f : expf(sc[e] - m);       // (a NaN stays one)
+                P[r * P_PITCH + e * 32 + lane] = p;
+                const float part = warp_sum(p);
+                l = e == 0 ? part : l + part;
+            }
+            if (lane == 0) {
+                if (a.splits) {
+                    stats[r] = m;
+                    stats[ROWS + r] = l;
+                } else {
+                    float M = stats[r], L = stats[ROWS + r], held, fresh;
+                    merge_factors(M, L, m, l, held, fresh);
+                    stats[r] = M;
+                    stats[ROWS + r] = L;
+                    stats[2 * ROWS + r] = held;
+                    stats[3 * ROWS + r] = fresh;
+                }
+            }
+        }
+        uint64_t acc[RI][VJ][2];
+#pragma unroll
+        for (int r = 0; r < RI; ++r)
+#pragma unroll
+            for (int j = 0; j < VJ; ++j) acc[r][j][0] = acc[r][j][1] = 0;
+        for (int i = k_slices; i < slices; ++i) {
+            copy_wait<STAGES - 2>();
+            __syncthreads();                            // (the first time round: P and the factors are written, too)
+            fetch(i + STAGES - 1);
+            const float* vs = reinterpret_cast<const float*>(ring + (i % STAGES) * STAGE);
+            const float* ps = P + tm * P_PITCH + (i - k_slices) * VK;
+#pragma unroll
+            for (int j0 = 0; j0 < VK; j0 += 4) {
+                float p[RI][4];
+#pragma unroll
+                for (int r = 0; r < RI; ++r) {
+                    const float4 f = *reinterpret_cast<const float4*>(ps + r * RSTEP * P_PITCH + j0);
+                    p[r][0] = f.x; p[r][1] = f.y; p[r][2] = f.z; p[r][3] = f.w;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    uint64_t pp[RI];
+#pragma unroll
+                    for (int r = 0; r < RI; ++r) pp[r] = pack2(p[r][e], p[r][e]);
+#pragma unroll
+                    for (int j = 0; j < VJ; ++j) {
+                        const int d = 4 * (tn + j * LN);
+                        if (d < a.vd) {
+                            const Pair2 v = lds4(vs + (j0 + e) * a.vd + d);
+#pragma unroll
+                            for (int r = 0; r < RI; ++r) {
+                                fma2(acc[r][j][0], pp[r], v.x);
+                                fma2(acc[r][j][1], pp[r], v.y);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        copy_wait<0>();                                 // (only empty groups are left)
+#pragma unroll
+        for (int r = 0; r < RI; ++r) {
+            const int rr = tm + r * RSTEP;
+            const float held = a.splits ? 0.0f : stats[2 * ROWS + rr], fresh = a.splits ? 1.0f : stats[3 * ROWS + rr];
+#pragma unroll
+            for (int j = 0; j < VJ; ++j) {
+                const float2 lo = unpack2(acc[r][j][0]), hi = unpack2(acc[r][j][1]);
+                if (a.splits) {
+                    tot[r][j][0] = lo.x; tot[r][j][1] = lo.y; tot[r][j][2] = hi.x; tot[r][j][3] = hi.y;
+                } else {
+                    tot[r][j][0] = merged(tot[r][j][0], held, lo.x, fresh);
+                    tot[r][j][1] = merged(tot[r][j][1], held, lo.y, fresh);
+                    tot[r][j][2] = merged(tot[r][j][2], held, hi.x, fresh);
+                    tot[r][j][3] = merged(tot[r][j][3], held, hi.y, fresh);
+                }
+            }
+        }
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int r = 0; r < RI; ++r) {
+        const int rr = tm + r * RSTEP;
+        if (rr >= t.rows) continue;
+        const int row = t.row0 + rr, token = t.q0 + row / a.group, head = g * a.group + row % a.group;
+        float* dst;
+        float inv = 1.0f;
+        if (a.splits) {
+            const size_t at = ((size_t)token * a.n_kv * a.group + head) * a.splits + blockIdx.x % a.splits;
+            dst = a.part_acc + at * a.vd;
+            if (tn == 0) {
+                a.part_ml[2 * at] = stats[rr];
+                a.part_ml[2 * at + 1] = stats[ROWS + rr];
+            }
+        } else {
+            dst = a.out + (size_t)token * a.out_stride + (size_t)head * a.vd;
+            inv = share(a, stats[rr], stats[ROWS + rr], head);
+        }
+#pragma unroll
+        for (int j = 0; j < VJ; ++j) {
+            const int d = 4 * (tn + j * LN);
+            if (d < a.vd)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dst[d + e] = a.splits ? tot[r][j][e] : __fmul_rn(tot[r][j][e], inv);
+        }
+    }
+}
+
+// One row (blockIdx.x: a row of the sequence's, blockIdx.y: kv head, blockIdx.z: sequence): its spans in order.
+template <int ROWS>
+__global__ void __launch_bounds__(64) merge_kernel(F32Args a) {
+    const int b = blockIdx.z, row = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
+    const Tile t = tile_of<ROWS>(a, b, row / ROWS);
+    if (row - t.row0 >= t.rows) return;
+    const int token = t.q0 + row / a.group, head = blockIdx.y * a.group + row % a.group;
+    const size_t at = ((size_t)token * a.n_kv * a.group + head) * a.splits;
+    const int n = t.last - t.first + 1;
+    const float* acc = a.part_acc + at * a.vd + threadIdx.x * 4;
+    const bool mine = (int)threadIdx.x * 4 < a.vd;
+    float M = -INFINITY, L = 0.0f, A[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+    for (int s = 0; s < n; ++s) {
+        float held, fresh;
+        const float2 ml = reinterpret_cast<const float2*>(a.part_ml)[at + s];
+        const float4 f = mine ? *reinterpret_cast<const float4*>(acc + (size_t)s * a.vd) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        merge_factors(M, L, ml.x, ml.y, held, fresh);
+        A[0] = merged(A[0], held, f.x, fresh);
+        A[1] = merged(A[1], held, f.y, fresh);
+        A[2] = merged(A[2], held, f.z, fresh);
+        A[3] = merged(A[3], held, f.w, fresh);
+    }
+    const float inv = share(a, M, L, head);
+    if (!mine) return;
+    float* dst = a.out + (size_t)token * a.out_stride + (size_t)head * a.vd + threadIdx.x * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dst[e] = __fmul_rn(A[e], inv);
+}
+
+template <int ROWS, int VJ>
+int launch(const F32Args& a, int batch, int max_q_len, cudaStream_t stream) {
+    const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;
+    const int smem = STAGES * STAGE + (ROWS * q_pitch + ROWS * P_PITCH + 4 * ROWS) * (int)sizeof(float) + 2 * SPAN * 8;
+    static bool raised = false;
+    if (!raised) {
+        cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<ROWS, VJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        if (e != cudaSuccess) return (int)e;
+        raised = true;
+    }
+    const int rows = max_q_len * a.group, tiles = (rows + ROWS - 1) / ROWS;
+    int st = launch_pdl(attn_f32_kernel<ROWS, VJ>, dim3(tiles * (a.splits ? a.splits : 1), a.n_kv, batch), dim3(THREADS), smem,
+                        stream, a);
+    if (st || !a.splits) return st;
+    return launch_pdl(merge_kernel<ROWS>, dim3(rows, a.n_kv, batch), dim3(64), 0, stream, a);
+}
+
+}  // namespace
+
+// Sizes: hd and vd multiples of 8, at most 256; all rows and strides whole 16-byte pieces.  splits > 0: at least as many
+// spans of 128 keys as any tile of rows sees, with part_acc [tokens][heads][splits][vd] and part_ml [..][splits][2].
+BROLM_API int brolm_attn_f32(const void* q, int q_stride, void* out, int out_stride, const void* cu_q, const void* kv_len,
+                             const void* k, const void* v, int k_stride, int v_stride, const void* k_pages, const void* v_pages,
+                             const void* page_table, int pt_stride, int ring, int page_size, int n_kv, int group, int hd, int vd,
+                             float scale, float cap, int window, int chunk, const void* sink, const void* slopes,
+                             const void* dist_bias, int dist_len, int batch, int max_q_len, int splits, void* part_acc,
+                             void* part_ml, cudaStream_t stream) {
+    if (batch <= 0 || max_q_len <= 0) return BROLM_OK;
+    if (hd <= 0 || hd > 256 || vd <= 0 || vd > 256 || group <= 0 || n_kv <= 0 || splits < 0) return BROLM_ERR_BAD_SIZE;
+    if (hd % 8 || vd % 8 || q_stride % 4 || ((uintptr_t)q & 15)) return BROLM_ERR_ALIGNMENT;
+    if (splits && (!part_acc || !part_ml)) return BROLM_ERR_BAD_SIZE;
+    if (dist_bias && dist_len <= 0) return BROLM_ERR_BAD_SIZE;
+    if (batch > 65535 || n_kv > 65535) return BROLM_ERR_TOO_LARGE;
+    if (k_pages) {
+        if (ring <= 0 || page_size <= 0 || page_size % 32 != 0 || ring % page_size != 0) return BROLM_ERR_BAD_SIZE;
+    } else if (!k || !v || k_stride % 4 || v_stride % 4 || ((uintptr_t)k & 15) || ((uintptr_t)v & 15)) {
+        return BROLM_ERR_ALIGNMENT;
+    }
+    F32Args a;
+    a.q = (const float*)q; a.out = (float*)out; a.q_stride = q_stride; a.out_stride = out_stride;
+    a.cu_q = (const int32_t*)cu_q; a.kv_len = (const int32_t*)kv_len;
+    a.k = (const float*)k; a.v = (const float*)v; a.k_stride = k_stride; a.v_stride = v_stride;
+    a.k_pages = (const float*)k_pages; a.v_pages = (const float*)v_pages; a.page_table = (const int32_t*)page_table;
+    a.pt_stride = pt_stride; a.ring = ring; a.page_size = page_size;
+    a.n_kv = n_kv; a.group = group; a.hd = hd; a.vd = vd; a.scale = scale; a.cap = cap; a.window = window; a.chunk = chunk;
+    a.sink = (const float*)sink; a.slopes = (const float*)slopes; a.dist_bias = (const float*)dist_bias; a.dist_len = dist_len;
+    a.splits = splits; a.part_acc = (float*)part_acc; a.part_ml = (float*)part_ml;
+    if ((long long)max_q_len * group <= 8) {
+        if (vd <= 128) return launch<8, 1>(a, batch, max_q_len, stream);
+        return launch<8, 2>(a, batch, max_q_len, stream);
+    }
+    if (vd <= 64) return launch<32, 1>(a, batch, max_q_len, stream);
+    if (vd <= 128) return launch<32, 2>(a, batch, max_q_len, stream);
+    return launch<32, 4>(a, batch, max_q_len, stream);
+}

@@ -1388,6 +1388,56 @@ def gemm_stream_status(reset: bool = False) -> int:
     return f(1 if reset else 0)
 
 
+F32_SPAN = 128             # keys of a span of the float attention (attn_f32.cu)
+
+
+def _attn_f32_ok(head_dim: int, vd: int, q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Tensor], kv_stride: int,
+                 v_stride: int) -> bool:
+    """Whether rows are whole 16-byte pieces of the sizes the float kernel takes (pages are, if these sizes are)."""
+    if head_dim % 8 or vd % 8 or head_dim > 256 or vd > 256 or q.stride(0) % 4 or q.data_ptr() % 16:
+        return False
+    return k is None or not (kv_stride % 4 or v_stride % 4 or k.data_ptr() % 16 or v.data_ptr() % 16)
+
+
+def attn_f32_splits(batch: int, n_kv: int, group: int, vd: int, tokens: int, max_q_len: int, max_keys: Optional[int],
+                    window: int = 0, chunk: int = 0, sms: Optional[int] = None) -> int:
+    """How many blocks share the spans of a tile of rows (0: a block walks them all): one per span as long as the tiles
+    alone are fewer than four to an SM and the partial results stay below 64 MB.
+
+    Measured, 8 heads of 256 over 4 kv heads, walked / shared: a prompt of 300 tokens (76 tiles) 130 / 71 us, one token of
+    three sequences of 420 keys 84 / 30 us, of eight of 1,024 183 / 42 us, of 64 of 1,280 265 / 204 us.  ``max_keys``: a bound on a sequence's keys (None: none is known)."""
+    rows = 8 if max_q_len * group <= 8 else 32
+    tiles = -(-max_q_len * group // rows)
+    spans = [-(-max_keys // F32_SPAN)] if max_keys else []
+    spans += [(s + rows // group + 1) // F32_SPAN + 2 for s in (window, chunk) if s > 0]
+    if not spans or min(spans) < 2 or tiles * n_kv * batch >= 4 * (sms or device_sms()):
+        return 0
+    return min(spans) if tokens * n_kv * group * min(spans) * (vd + 2) * 4 <= 64 << 20 else 0
+
+
+def _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group, head_dim,
+                   vd, scale, cap, window, chunk, sink, slopes, dist_bias, batch, max_q_len) -> None:
+    if k_pages is None:
+        max_keys = max_q_len
+    else:
+        places = page_table.shape[1] * page_size
+        max_keys = places if ring >= places else None          # a ring that wraps bounds nothing by itself
+    splits = attn_f32_splits(batch, n_kv, group, vd, q.shape[0], max_q_len, max_keys, window, chunk)
+    acc = ml = None
+    if splits:
+        acc = torch.empty((q.shape[0], n_kv * group, splits, vd), dtype=torch.float32, device=q.device)
+        ml = torch.empty((q.shape[0], n_kv * group, splits, 2), dtype=torch.float32, device=q.device)
+    f = _fn("attn_f32", "brolm_attn_f32", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
+                                           c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                           c_void_p, c_void_p, c_void_p])
+    _check(f(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(cu_q), _ptr(kv_len), _ptr(k), _ptr(v),
+             k.stride(0) if k is not None else 0, v.stride(0) if v is not None else 0, _ptr(k_pages), _ptr(v_pages),
+             _ptr(page_table), pt_stride, ring, page_size, n_kv, group, head_dim, vd, scale, cap, window, chunk, _ptr(sink),
+             _ptr(slopes), _ptr(dist_bias), dist_bias.shape[1] if dist_bias is not None else 0, batch, max_q_len, splits,
+             _ptr(acc), _ptr(ml), _stream()), "attention_f32")
+
+
 def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_len: torch.Tensor, *, n_kv: int,
                    group: int, head_dim: int, scale: float, cap: float, window: int, batch: int, max_q_len: int,
                    k: Optional[torch.Tensor] = None, v: Optional[torch.Tensor] = None,
@@ -1427,6 +1477,11 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_le
         assert k is not None and v is not None and k.dtype == q.dtype and v.dtype == q.dtype
         assert k.stride(-1) == 1 and v.stride(-1) == 1
         kv_stride, v_stride = k.stride(0), v.stride(0)
+    if q.dtype == torch.float32 and out.dtype == torch.float32 and not v_all and not ring_from and not (keep_first and window > 0) \
+            and _attn_f32_ok(head_dim, vd, q, k, v, kv_stride, v_stride):
+        _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group,
+                       head_dim, vd, scale, cap, window, int(chunk), sink, slopes, dist_bias, batch, max_q_len)
+        return
     f = _fn("attn_simt", "brolm_attn_simt", [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                              c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                              c_int, c_int, c_int, c_float, c_float, c_int, c_void_p, c_int, c_int,

@@ -764,6 +764,51 @@ def test_attention_prompt_and_decode_agree_bitwise():
     assert torch.equal(one[0], out[n - 1])
 
 
+@pytest.mark.parametrize("options", ["plain", "window", "chunk", "scores"])
+@pytest.mark.parametrize("n,n_q,n_kv,hd,vd", [(1, 2, 1, 8, 8), (127, 4, 2, 64, 64), (129, 8, 4, 256, 256), (300, 6, 2, 40, 72),
+                                              (260, 16, 1, 128, 200), (385, 3, 3, 256, 128)])
+def test_float_attention_gives_the_same_bits_however_it_is_cut(monkeypatch, options, n, n_q, n_kv, hd, vd):
+    """Spans of 128 keys walked by one block and shared by several, tiles of 8 and 32 rows, packed keys and pages; against
+    the kernel for any sizes, which rows off the 16-byte boundaries go to."""
+    g = torch.Generator(device=DEV).manual_seed(n + hd)
+    q, k, v = (torch.randn(n, w, generator=g, device=DEV) for w in (n_q * hd, n_kv * hd, n_kv * vd))
+    extra = dict(window=0)
+    if options == "window":
+        extra = dict(window=70)
+    if options == "chunk":
+        extra = dict(window=0, chunk=100)
+    if options == "scores":
+        extra = dict(window=0, sink=torch.randn(n_q, generator=g, device=DEV), slopes=torch.rand(n_q, generator=g, device=DEV) / 8,
+                     dist_bias=torch.randn(n_q, 50, generator=g, device=DEV))
+    cu = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+    length = torch.tensor([n], dtype=torch.int32, device=DEV)
+    kw = dict(n_kv=n_kv, group=n_q // n_kv, head_dim=hd, v_dim=vd, scale=1.5 / math.sqrt(hd), cap=20.0, batch=1, **extra)
+    shared, walked, other = (torch.full((n, n_q * vd), float("nan"), device=DEV) for _ in range(3))
+    kernels.attention_simt(q, shared, cu, length, k=k, v=v, max_q_len=n, **kw)
+    cut = kernels.attn_f32_splits(1, n_kv, n_q // n_kv, vd, n, n, n, extra["window"], extra.get("chunk", 0))
+    assert (cut > 1) == (n > 128)
+    off = torch.empty(n, n_q * hd + 1, device=DEV)
+    off[:, 1:] = q
+    kernels.attention_simt(off[:, 1:], other, cu, length, k=k, v=v, max_q_len=n, **kw)
+    close(shared, other.double().cpu(), torch.float32, scale=float(other.abs().max()))
+    monkeypatch.setattr(kernels, "attn_f32_splits", lambda *a, **b: 0)
+    kernels.attention_simt(q, walked, cu, length, k=k, v=v, max_q_len=n, **kw)
+    assert torch.equal(shared, walked)
+    # the last query as a decode step over pages in another order, walked and shared
+    pages = -(-n // 64)
+    order = torch.randperm(pages, generator=g, device=DEV)
+    kp, vp = (torch.full((pages, n_kv, 64, w), float("nan"), device=DEV) for w in (hd, vd))
+    for p in range(n):
+        kp[order[p // 64], :, p % 64], vp[order[p // 64], :, p % 64] = k[p].view(n_kv, hd), v[p].view(n_kv, vd)
+    table = order.to(torch.int32).view(1, -1)
+    for splits in (0, pages):
+        monkeypatch.setattr(kernels, "attn_f32_splits", lambda *a, **b: splits)
+        one = torch.full((1, n_q * vd), float("nan"), device=DEV)
+        kernels.attention_simt(q[n - 1:], one, torch.tensor([0, 1], dtype=torch.int32, device=DEV), length, k_pages=kp, v_pages=vp,
+                               page_table=table, ring=1 << 30, page_size=64, max_q_len=1, **kw)
+        assert torch.equal(one[0], shared[n - 1])
+
+
 def test_kernels_refuse_what_they_cannot_do():
     q = torch.zeros(2, 2 * 520, device=DEV)
     with pytest.raises(kernels.KernelError):                # a head beyond the exact kernel's 512
