@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(64) merge_kernel(F32Args a) {
     if (row - t.row0 >= t.rows) return;
     const int token = t.q0 + row / a.group, head = blockIdx.y * a.group + row % a.group;
     const size_t at = ((size_t)token * a.n_kv * a.group + head) * a.splits;
-    const int n = t.last - t.first + 1;
+    const int n = min(t.last - t.first + 1, a.splits);  // (never more: the caller's bound; and no read behind its room)
     const float* acc = a.part_acc + at * a.vd + threadIdx.x * 4;
     const bool mine = (int)threadIdx.x * 4 < a.vd;
     float M = -INFINITY, L = 0.0f, A[4] = {0.0f, 0.0f, 0.0f, 0.0f};

@@ -1415,13 +1415,18 @@ def attn_f32_splits(batch: int, n_kv: int, group: int, vd: int, tokens: int, max
     return min(spans) if tokens * n_kv * group * min(spans) * (vd + 2) * 4 <= 64 << 20 else 0
 
 
+def attn_f32_max_keys(places: int, ring: int) -> Optional[int]:
+    """A bound on the keys of a sequence whose page table has ``places`` places; None: the pages bound nothing, because
+    the positions go round.  (A ring of exactly as many places goes round, too.)"""
+    return places if ring > places else None
+
+
 def _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group, head_dim,
                    vd, scale, cap, window, chunk, sink, slopes, dist_bias, batch, max_q_len) -> None:
     if k_pages is None:
         max_keys = max_q_len
     else:
-        places = page_table.shape[1] * page_size
-        max_keys = places if ring >= places else None          # a ring that wraps bounds nothing by itself
+        max_keys = attn_f32_max_keys(page_table.shape[1] * page_size, ring)
     splits = attn_f32_splits(batch, n_kv, group, vd, q.shape[0], max_q_len, max_keys, window, chunk)
     acc = ml = None
     if splits:

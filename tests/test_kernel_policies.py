@@ -65,3 +65,17 @@ def test_which_product_takes_which_operands():
     # the tcgen05 prompt attention: head sizes 64, 128, 256 and groups that divide 128
     assert kernels.attention_prefill_tc_ok(256, 2) and kernels.attention_prefill_tc_ok(128, 8)
     assert not kernels.attention_prefill_tc_ok(80, 2) and not kernels.attention_prefill_tc_ok(128, 3)
+
+
+def test_float_attention_shares_as_many_spans_as_a_tile_can_see():
+    """Pages bound the keys only where positions never go round; a window or a chunk bounds them otherwise, wherever it
+    lies over the spans."""
+    assert kernels.attn_f32_max_keys(448, 1 << 30) == 448 and kernels.attn_f32_max_keys(192, 256) == 192
+    assert kernels.attn_f32_max_keys(256, 256) is None and kernels.attn_f32_max_keys(512, 256) is None
+    for window in (1, 65, 128, 129, 200, 256, 300):
+        ring = -(-window // 64) * 64
+        for group in (1, 4, 8, 40):
+            splits = kernels.attn_f32_splits(1, 1, group, 64, 1, 1, kernels.attn_f32_max_keys(ring, ring), window)
+            for pos in range(1000):
+                seen = pos // kernels.F32_SPAN - max(0, pos - window + 1) // kernels.F32_SPAN + 1
+                assert splits == 0 or seen <= splits, (window, group, pos)
