@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
         const int pos = tok0 + r / a.group;                 // position of the row's token (prompts start at 0)
         const float c0 = a.cap > 0.0f ? a.scale / a.cap * (2.0f * LOG2E) : a.scale * LOG2E;
         const float c1 = a.cap * LOG2E, c2 = 2.0f * a.cap * LOG2E;
+        const bool foreign = b + 1 < (int)gridDim.z && (t_first + n_tiles) * BN > q_len;   // the last tile goes beyond the sequence
         float m_ref = -INFINITY, l = 0.0f;                  // l: the sum over this thread's columns only
         bool ok = true;
         for (int j = 0; j < n_tiles; ++j) {
@@ -388,6 +389,22 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
             }
             l += sum;
             tmem_st32(tmem + lane_addr + S_COL + s * BN + half * (W / 2), pw);
+            if (foreign && j == n_tiles - 1) {
+                // the rows of the next sequence in this tile's values: their probabilities are zero, but zero times an
+                // infinity or a NaN is not
+                const int u0 = KU * n_tiles + 2 * (n_tiles - 1), kept = q_len - key_base;
+                for (int vu = 0; vu < 2; ++vu) {
+                    const int sl = (u0 + vu) % SLOTS, first = max(0, kept - 64 * vu);
+                    ok = wait_on(bar(U_FULL + sl), ((u0 + vu) / SLOTS) & 1, give_up, 14);
+                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                    for (int i = threadIdx.x - 64; i < (64 - first) * DB * 8; i += 256) {
+                        const int piece = i & 7, d = (i >> 3) % DB, row = first + (i >> 3) / DB;
+                        st_shared_zero16(ring + sl * SH::SLOT + d * (64 * 128) + row * 128 + piece * 16);
+                    }
+                }
+                if (!ok) break;
+                fence_proxy_async();
+            }
             tmem_wait_st();
             fence_before_sync();
             __syncwarp();

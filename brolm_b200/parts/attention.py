@@ -399,7 +399,8 @@ class Attention(Part):
         scored = bool(self.softcap or self.has_sink or self.dist_bias is not None)     # options of the score itself
         special = self.talk or self.gate or self.slopes is not None or self.keep_first or self.chunk
         same_size = self.v_dim == self.head_dim and self.head_dim % 16 == 0 and self._tensor_cores(ctx)
-        if not special and same_size and scored and (ctx.mode == "prefill" or page == 64):
+        plain = self.sink is None and self.dist_bias is None                # the cap, if any, is a plain layer's too
+        if not special and same_size and scored and not (plain and ctx.mode == "prefill") and (ctx.mode == "prefill" or page == 64):
             # key and value rows of one size: the plain layers' mma.sync kernels, which know the cap, the sink and
             # the distance table (and stage keys and values through more buffers than the head-wise ones)
             more = dict(sink=self.sink, dist_bias=self.dist_bias)
@@ -411,8 +412,10 @@ class Attention(Part):
                 kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
                                              page_size=page, n_splits=splits, **more,
                                              **{n: a for n, a in common.items() if n != "max_q_len"})
-        elif not special and not scored and same_size:
-            # nothing the tensor-core kernels do not know: the same attention as a plain layer's
+        elif not special and same_size and (not scored or (plain and ctx.mode == "prefill")):
+            # nothing the tensor-core kernels do not know: the same attention as a plain layer's.  (A prompt with a
+            # cap, 16 heads on 4 kv heads of 128 entries, one sequence of 37 / 256 / 2048 / 4096 tokens: 9.7 / 20.6 /
+            # 131.8 / 409.6 us on the mma.sync kernel, 7.1 / 9.4 / 44.3 / 149.7 us on the tcgen05 one)
             if ctx.mode == "prefill":
                 self.attend_packed(q, k, v, out, ctx, common)
             else:

@@ -472,6 +472,29 @@ def test_attention_packed(dtype, kernel, n_q, n_kv, hd, window, cap):
         t += n
 
 
+@pytest.mark.parametrize("hd,n_q,n_kv", [(64, 4, 2), (128, 16, 4), (256, 16, 1)])
+@pytest.mark.parametrize("first", [1, 63, 64, 65, 127, 128, 129, 300])
+def test_attention_tc_keeps_broken_values_of_the_next_sequence_out(hd, n_q, n_kv, first):
+    """The last key tile of a sequence holds rows of the next one; their infinities and NaNs stay there."""
+    g = torch.Generator().manual_seed(first + hd)
+    qkv = torch.randn(first + 90, (n_q + 2 * n_kv) * hd, generator=g).to(torch.bfloat16).to(DEV)
+    args = dict(n_kv=n_kv, group=n_q // n_kv, head_dim=hd, scale=hd ** -0.5, cap=30.0, window=0)
+    k_at, v_at = n_q * hd, (n_q + n_kv) * hd
+
+    def run(rows, lengths):
+        out = torch.empty(rows.shape[0], n_q * hd, dtype=torch.bfloat16, device=DEV)
+        cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device=DEV)
+        kernels.attention_prefill_tc(rows[:, :k_at], out, cu, rows[:, k_at:v_at], rows[:, v_at:], batch=len(lengths),
+                                     max_q_len=max(lengths), n_split=0, **args)
+        assert kernels.attention_tc_status() == 0
+        return out
+
+    alone = run(qkv[:first].contiguous(), [first])
+    qkv[first::2, v_at:] = float("nan")
+    qkv[first + 1::2, v_at:] = float("inf")
+    assert torch.equal(run(qkv, [first, 90])[:first], alone)
+
+
 @pytest.mark.parametrize("n_q,n_kv,hd,window,cap,gain", [(8, 4, 256, 0, 50.0, 40.0), (4, 2, 64, 100, 30.0, 25.0),
                                                          (4, 4, 128, 0, 20.0, 200.0)])
 def test_attention_tc_scores_beyond_the_cap(n_q, n_kv, hd, window, cap, gain):
