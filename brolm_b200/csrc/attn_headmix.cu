@@ -25,6 +25,8 @@
 
 namespace {
 
+constexpr int STAGES = 3;      // tiles of keys and values that a decode kernel holds
+
 struct HmArgs {
     const bf16* q;          // rows of q_stride elements; head h at h * hd
     void* out;              // rows of out_stride elements; head h, value head c at (h * n_vh + c) * vd

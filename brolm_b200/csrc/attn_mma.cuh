@@ -108,6 +108,7 @@ struct MmaArgs {
     float* part_o;          // [B][n_q][n_splits][hd]
     float* part_ml;         // [B][n_q][n_splits][2]  (max in log2 units, sum)
     int merge_here;         // decoding: the last block of a (sequence, kv head) merges the splits itself
+    int by_length;            // decode: blocks take the sequences in order of falling length
     const float* sink;      // [n_q] or null: exp(sink[head]) joins the softmax's denominator, with no value
     int shared_kv;          // decoding: the values are the keys' rows themselves (one tile serves both)
     // a learned bias by distance, or null: [n_q][dist_len] floats, of which key j adds entry
@@ -347,26 +348,52 @@ __global__ void __launch_bounds__(NTHREADS) attn_prefill_mma_kernel(MmaArgs a) {
 // ===========================================================================
 // decoding over the paged cache
 // ===========================================================================
-constexpr int STAGES = 3;
+// Keys and values come through a ring of three slots.  A slot holds a tile's keys and values, and with heads of more than
+// 128 entries a block then has its SM to itself; or (APART) the keys or the values, 32 KB at a head size of 256, so that
+// two blocks share an SM and one streams while the other starts, merges or waits.  Where there are more blocks than SMs
+// that is what keeps the memory busy (heads of 256 entries, a block alone / two: 64 sequences of 1,280 keys on 4 kv heads
+// 61.3 / 53.1 us, which is 6.3 TB/s; 8 of 8,190 in 4 / 9 splits 49.4 / 46.3 us; 16 of 128 to 6,144 on 8 kv heads
+// 89.5 / 81.7); with fewer a block's own run is what counts, and a whole tile in flight more shortens it (one sequence
+// of 1,280 keys in 10 splits 8.6 / 9.6 us, of 8,190 in 37 splits 14.1 / 17.0 us).
+constexpr int SLOTS = 3;
+template <bool APART> __host__ __device__ constexpr size_t decode_slot(int hd) { return (APART ? 1 : 2) * (size_t)KT * hd * 2; }
 constexpr int PT_ROW = 512;          // entries of a page-table row kept in shared memory (32768 keys)
 
-template <int HD_MAX, bool EXACT, bool BIAS = false>
+template <int HD_MAX, bool EXACT, bool BIAS, bool APART>
 __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int hd = EXACT ? HD_MAX : a.hd, hd16 = hd >> 4, cpr = hd >> 3;
     const bool swz = (hd & 63) == 0;
     const uint32_t rowb = (uint32_t)hd * 2u;
     bf16* Qs = reinterpret_cast<bf16*>(smem_raw);            // [16][hd]
-    bf16* stage0 = Qs + 16 * hd;                             // STAGES x ([KT][hd] keys, [KT][hd] values)
+    bf16* stage0 = Qs + 16 * hd;                             // SLOTS x ([KT][hd] keys and/or [KT][hd] values)
     const uint32_t qs_base = smem_u32(Qs), st_base = smem_u32(stage0);
-    const uint32_t stage_bytes = 2u * KT * hd * 2u;
+    const uint32_t slot_bytes = (uint32_t)decode_slot<APART>(hd);
 
-    const int split = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
+    const int split = blockIdx.x, g = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int pt_row[PT_ROW];
+    int b = blockIdx.z;
+    if (a.by_length) {
+        // several rounds of blocks: those of the longest sequences start first (equal ones in their order), so that
+        // the last round is made of short runs.  (16 sequences of 128 to 6,144 keys, 8 kv heads of 256 entries, 4 splits:
+        // 85.6 -> 67.0 us)
+        const int n = gridDim.z;
+        for (int i = threadIdx.x; i < n; i += NTHREADS) pt_row[i] = a.kv_len[i];
+        __syncthreads();
+        __shared__ int mine;
+        for (int i = threadIdx.x; i < n; i += NTHREADS) {
+            const int len = pt_row[i];
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += pt_row[j] > len || (pt_row[j] == len && j < i);
+            if (rank == b) mine = i;
+        }
+        __syncthreads();
+        b = mine;
+    }
     // The sequence's length and its row of the page table were written by the host before the step's
     // first kernel: they are fetched together, ahead of the wait, so that the first tile's address
     // does not take two more round trips to the L2 after it.
-    __shared__ int pt_row[PT_ROW];
     for (int i = threadIdx.x; i < min(a.pt_stride, PT_ROW); i += NTHREADS) pt_row[i] = a.page_table[(size_t)b * a.pt_stride + i];
     const int kv_len = a.kv_len[b];
     const int q_row = a.cu_q[b];                              // (also the host's)
@@ -398,33 +425,45 @@ __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
         const int entry = ridx / KT;
         return entry < PT_ROW ? pt_row[entry] : a.page_table[(size_t)b * a.pt_stride + entry];
     };
-    auto load_tile = [&](int i, int page) {                   // i-th tile of the split into stage i % STAGES
-        const int t = t_begin + i;
+    // a unit is what a slot takes: a tile, or its keys or its values (a row that is both comes once)
+    const int upt = APART && !a.shared_kv ? 2 : 1, n_units = n_tiles * upt;
+    int page = n_tiles > 0 ? page_of(0) : 0;                  // of the tile whose units are being asked for
+    auto load_unit = [&](int u) {                             // unit u into slot u % SLOTS; units are asked for in order
+        const int i = u / upt, which = u - i * upt, t = t_begin + i;
         const size_t src = ((size_t)page * a.n_kv + g) * KT * hd;
-        const uint32_t kb = st_base + (i % STAGES) * stage_bytes, vb = kb + KT * hd * 2u;
+        const uint32_t kb = st_base + (u % SLOTS) * slot_bytes;
+        const bf16* first = which ? a.v_pages : a.k_pages;
         for (int idx = threadIdx.x; idx < KT * cpr; idx += NTHREADS) {
             const int r = idx / cpr, c = idx - r * cpr;
             const uint32_t off = tile_off(r, c, hd, swz);
             const int kp = t * KT + r;
             const int bytes = (kp >= key_lo && kp <= pos) ? 16 : 0;   // places never written read as zero
-            cp_async16(kb + off, a.k_pages + src + r * hd + c * 8, bytes);
-            if (!a.shared_kv) cp_async16(vb + off, a.v_pages + src + r * hd + c * 8, bytes);
+            cp_async16(kb + off, first + src + r * hd + c * 8, bytes);
+            if (!APART && !a.shared_kv) cp_async16(kb + KT * rowb + off, a.v_pages + src + r * hd + c * 8, bytes);
         }
+        // the page of the next tile is looked up one unit ahead of its first use
+        if (which == upt - 1 && i + 1 < n_tiles) page = page_of(i + 1);
     };
 #pragma unroll
-    for (int i = 0; i < STAGES - 1; ++i) {
-        if (i < n_tiles) load_tile(i, page_of(i));
+    for (int u = 0; u < SLOTS - 1; ++u) {
+        if (u < n_units) load_unit(u);
         cp_async_commit();
     }
-    // the page id of the tile that the next iteration will load is fetched one iteration early
-    int page_next = (STAGES - 1 < n_tiles) ? page_of(STAGES - 1) : 0;
+    int unit = 0;
+    auto next_unit = [&]() -> uint32_t {                      // waits for the next unit and asks for one more; its address
+        cp_async_wait<SLOTS - 2>();
+        __syncthreads();                       // the unit has landed; everyone is done with the one before it
+        if (unit + SLOTS - 1 < n_units) load_unit(unit + SLOTS - 1);
+        cp_async_commit();
+        return st_base + (unit++ % SLOTS) * slot_bytes;
+    };
 
     const uint32_t x = lane & 7;
     const uint32_t xhi = swz ? (x & 6u) << 4 : 0u;
     const uint32_t jq = lane >> 4, jk = (lane >> 3) & 1, jv = lane >> 4;
     const uint32_t q_addr = qs_base + (lane & 15) * rowb + ((swz ? (jq ^ (x & 1u)) : jq) << 4);
     const uint32_t k_thr = (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * rowb + ((swz ? (jk ^ (x & 1u)) : jk) << 4);
-    const uint32_t v_thr = (a.shared_kv ? 0u : KT * rowb) + (warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * rowb +
+    const uint32_t v_thr = (a.shared_kv || APART ? 0u : KT * rowb) + (warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * rowb +
                            ((swz ? (jv ^ (x & 1u)) : jv) << 4);
 
     float o[HD_MAX / 8][4];
@@ -442,12 +481,7 @@ __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
     }
 
     for (int i = 0; i < n_tiles; ++i) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();                       // tile i has landed; everyone is done with tile i - 1
-        if (i + STAGES - 1 < n_tiles) load_tile(i + STAGES - 1, page_next);
-        cp_async_commit();
-        if (i + STAGES < n_tiles) page_next = page_of(i + STAGES);
-        const uint32_t sb = st_base + (i % STAGES) * stage_bytes;
+        uint32_t sb = next_unit();
         const int t = t_begin + i;
 
         float s[2][4];
@@ -508,6 +542,7 @@ __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
         pf[1] = pack_bf16(s[0][2], s[0][3]);
         pf[2] = pack_bf16(s[1][0], s[1][1]);
         pf[3] = pack_bf16(s[1][2], s[1][3]);
+        if (upt == 2) sb = next_unit();
 #pragma unroll
         for (int dp = 0; dp < HD_MAX / 16; ++dp) {
             if (dp < hd16) {
@@ -742,17 +777,14 @@ int launch_prefill(const MmaArgs& a, int batch, int max_q_len, cudaStream_t stre
     return launch_status();
 }
 
-template <int HD_MAX, bool EXACT, bool BIAS = false>
-int launch_decode(const MmaArgs& a, int batch, cudaStream_t stream) {
-    if constexpr (!BIAS) {
-        if (a.dist_bias) return launch_decode<HD_MAX, EXACT, true>(a, batch, stream);
-    }
-    size_t smem = (size_t)(16 + STAGES * 2 * KT) * a.hd * sizeof(bf16);
+template <int HD_MAX, bool EXACT, bool BIAS, bool APART>
+int launch_decode_as(const MmaArgs& a, int batch, cudaStream_t stream) {
+    size_t smem = (size_t)16 * a.hd * sizeof(bf16) + SLOTS * decode_slot<APART>(a.hd);
     const size_t merge = (size_t)(8 * 16 + 4 * a.group * a.hd) * sizeof(float) + 16 * a.hd * sizeof(bf16);
     if (merge > smem) smem = merge;
     static size_t allowed = 0;
     if (smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD_MAX, EXACT, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD_MAX, EXACT, BIAS, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         allowed = smem;
     }
@@ -760,12 +792,24 @@ int launch_decode(const MmaArgs& a, int batch, cudaStream_t stream) {
     MmaArgs b = a;
     b.merge_here = a.n_splits > 1 && a.n_splits <= MAX_MERGED_SPLITS && (long long)batch * a.n_kv <= MAX_TICKETS &&
                    (size_t)(a.group * a.n_splits + a.group) * sizeof(float) <= smem - 16 * a.hd * sizeof(bf16);
-    int st = launch_pdl(attn_decode_mma_kernel<HD_MAX, EXACT, BIAS>, grid, dim3(NTHREADS), smem, stream, b);
+    b.by_length = batch > 1 && batch <= PT_ROW && (long long)a.n_splits * a.n_kv * batch > 2LL * device_sm_count();
+    int st = launch_pdl(attn_decode_mma_kernel<HD_MAX, EXACT, BIAS, APART>, grid, dim3(NTHREADS), smem, stream, b);
     if (st != 0 || a.n_splits == 1 || b.merge_here) return st;
     dim3 cgrid(a.n_kv * a.group, batch);
     return launch_pdl(attn_combine_kernel, cgrid, dim3(128), (a.n_splits + 33) * sizeof(float), stream,
                       (const float*)a.part_o, (const float*)a.part_ml, a.out, a.cu_q, a.out_stride,
                       a.n_kv * a.group, a.n_splits, a.hd);
+}
+
+template <int HD_MAX, bool EXACT>
+int launch_decode(const MmaArgs& a, int batch, cudaStream_t stream) {
+    if constexpr (HD_MAX > 128) {
+        if ((long long)a.n_splits * a.n_kv * batch > device_sm_count())
+            return a.dist_bias ? launch_decode_as<HD_MAX, EXACT, true, true>(a, batch, stream)
+                               : launch_decode_as<HD_MAX, EXACT, false, true>(a, batch, stream);
+    }
+    return a.dist_bias ? launch_decode_as<HD_MAX, EXACT, true, false>(a, batch, stream)
+                       : launch_decode_as<HD_MAX, EXACT, false, false>(a, batch, stream);
 }
 
 int check_common(int hd, int group, int n_kv, int q_stride, int out_stride, int batch) {

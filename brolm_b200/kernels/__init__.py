@@ -1709,11 +1709,12 @@ def attention_tc_status(reset: bool = False) -> int:
     return f(1 if reset else 0)
 
 
+RAGGED_WAVES_SHARED = 2.2       # the same where blocks share an SM
 RAGGED_WAVES = int(os.environ.get("BROLM_RAGGED_WAVES", "5"))
 
 
 def decode_splits(batch: int, n_kv: int, max_kv_len: int, window: int, sms: Optional[int] = None,
-                  ragged: bool = False) -> int:
+                  ragged: bool = False, per_sm: int = 1) -> int:
     """How many blocks share the keys of one (sequence, kv head): as many as make one wave of blocks
     over the SMs (a block holds an SM's shared memory alone), at least two pages per block and at
     most 40 splits (the last block's merge reads every split's partial result).
@@ -1727,14 +1728,35 @@ def decode_splits(batch: int, n_kv: int, max_kv_len: int, window: int, sms: Opti
     1,280 to 6,400 keys and 8 kv heads (128 pairs): 1 / 2 / 4 / 6 / 8 / 12 splits 147 / 128 / 118 / 114 /
     116 / 126 us; with equal lengths more than one round only costs (152 / 163 / 167 us for 1 / 2 / 4).
     (Pieces of one size for all sequences, so that a short sequence is one block and a long one many,
-    were measured too: 111 to 113 us, no better than equal shares, and are not in the kernel.)"""
+    were measured too: 111 to 113 us, no better than equal shares, and are not in the kernel.)
+
+    ``per_sm``: so many blocks share an SM (``decode_blocks_per_sm``), and one wave is as many times the SMs, if the keys
+    give well more blocks than SMs: 8 sequences of 8,190 keys on 4 kv heads of 256 entries 49.4 us in 4 splits and 46.3
+    in 9, 16 of 1,280 keys 19.7 in 2 and 18.8 in 4; one sequence of 8,190 keys 14.1 in 37 and 17.5 in 40 (160 blocks).
+    With the blocks of the longest sequences first, about two waves are enough for ragged batches.  A decode step by
+    1.4 / 1.75 / 2.2 / 2.6 / 3.5 waves: 9B sizes, 16 sequences of 128 to 6,144 tokens 7,419 / 7,179 / 7,252 / 7,291 / 7,367
+    us; 2B, 24 of 100 to 4,000 3,201 / 2,932 / 2,786 / 2,834 / 2,916 us; 50 of 300 to 1,700 3,440 / 2,884 / 2,786 / 2,856 /
+    2,938 us.  The attention alone: 16 sequences of 128 to 6,144 keys, 8 kv heads: 80 / 67 / 68 / 73 / 74 us in 3 / 4 / 5 / 6 / 8 splits (89.5 in 6, with
+    one block an SM and the sequences in their own order); 12 of 100 to 8,000, 4 kv heads: 44 / 38 / 39 / 43 us in 8 / 10 /
+    12 / 16 (52 in 16); 64 of 500 to 1,900: 72 / 57 / 62 us in 1 / 2 / 3 (75 in 3)."""
     sms = sms or device_sms()
     keys = min(max_kv_len, window + 63) if window > 0 else max_kv_len
     tiles = max(1, (keys + 63) // 64)
-    want = max(1, sms // max(1, batch * n_kv))
-    if ragged:
-        want = max(want, -(-RAGGED_WAVES * sms // max(1, batch * n_kv)))
-    return max(1, min(want, (tiles + 1) // 2, 40))
+    most = min((tiles + 1) // 2, 40)
+    pairs = max(1, batch * n_kv)
+    want = max(1, sms // pairs)
+    if per_sm > 1 and min(per_sm * sms // pairs, most) * pairs > 1.5 * sms:
+        want = per_sm * sms // pairs
+    if ragged and per_sm > 1:
+        want = max(want, int(RAGGED_WAVES_SHARED * per_sm * sms / pairs))
+    elif ragged:
+        want = max(want, -(-RAGGED_WAVES * sms // pairs))
+    return max(1, min(want, most))
+
+
+def decode_blocks_per_sm(head_dim: int) -> int:
+    """How many blocks of the decode attention share an SM, where there are more blocks than SMs (``attn_mma.cuh``)."""
+    return 2 if head_dim > 128 else 1
 
 
 def attention_decode_mma(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_len: torch.Tensor,

@@ -338,7 +338,8 @@ class Attention(Part):
         elif tensor and page == 64:
             span = min(self.window or (1 << 30), self.chunk or (1 << 30))
             splits = kernels.decode_splits(ctx.batch, self.n_kv, ctx.max_kv_len, span if span < (1 << 30) else 0,
-                                           ragged=getattr(ctx, "ragged", False))
+                                           ragged=getattr(ctx, "ragged", False),
+                                           per_sm=kernels.decode_blocks_per_sm(self.head_dim))
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring, page_size=page,
                                          n_splits=splits, **{n: a for n, a in common.items() if n not in ("v_dim", "max_q_len")})
         else:
@@ -408,7 +409,8 @@ class Attention(Part):
                 kernels.attention_prefill_mma(q, out, ctx.cu_q, k, v, **common, **more)
             else:
                 splits = kernels.decode_splits(ctx.batch, self.n_kv, ctx.max_kv_len, self.window or 0,
-                                               ragged=getattr(ctx, "ragged", False))
+                                               ragged=getattr(ctx, "ragged", False),
+                                               per_sm=kernels.decode_blocks_per_sm(self.head_dim))
                 kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
                                              page_size=page, n_splits=splits, **more,
                                              **{n: a for n, a in common.items() if n != "max_q_len"})
@@ -489,7 +491,8 @@ class Attention(Part):
         if self._tensor_cores(ctx) and ctx.mode == "decode" and page == 64:
             args = {k: v for k, v in common.items() if k != "max_q_len"}
             splits = kernels.decode_splits(ctx.batch, self.n_kv, ctx.max_kv_len, self.window or 0,
-                                           ragged=getattr(ctx, "ragged", False))
+                                           ragged=getattr(ctx, "ragged", False),
+                                           per_sm=kernels.decode_blocks_per_sm(self.head_dim))
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
                                          page_size=page, n_splits=splits, **args)
         else:

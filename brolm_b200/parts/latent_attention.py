@@ -174,7 +174,8 @@ class LatentAttention(Part):
                 kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k=lat, v=lat, max_q_len=ctx.max_q_len, **common)
         elif tensor_cores and ctx.mode == "decode" and page == 64 and H <= 16:
             splits = kernels.decode_splits(ctx.batch, 1, ctx.max_kv_len, self.window or 0,
-                                           ragged=getattr(ctx, "ragged", False))
+                                           ragged=getattr(ctx, "ragged", False),
+                                           per_sm=kernels.decode_blocks_per_sm(D))
             if H * D >= 2048:
                 # every split leaves H * D floats for the block that merges them; up to four are merged in one
                 # round trip, and with all heads on one cached row a split is cheap to run and dear to merge

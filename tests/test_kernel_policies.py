@@ -79,3 +79,16 @@ def test_float_attention_shares_as_many_spans_as_a_tile_can_see():
             for pos in range(1000):
                 seen = pos // kernels.F32_SPAN - max(0, pos - window + 1) // kernels.F32_SPAN + 1
                 assert splits == 0 or seen <= splits, (window, group, pos)
+
+
+def test_decode_splits_where_two_blocks_share_an_sm():
+    two = dict(sms=148, per_sm=kernels.decode_blocks_per_sm(256))
+    assert kernels.decode_blocks_per_sm(128) == 1 and two["per_sm"] == 2
+    assert kernels.decode_splits(8, 4, 8192, 0, **two) == 9                       # 288 blocks for 296 places
+    assert kernels.decode_splits(1, 4, 8192, 0, **two) == 37                      # 40 would be little more than one round
+    assert kernels.decode_splits(64, 4, 2048, 0, **two) == 1
+    assert kernels.decode_splits(16, 8, 8192, 0, ragged=True, **two) == 5
+    assert kernels.decode_splits(3, 4, 700, 0, **two) == kernels.decode_splits(3, 4, 700, 0, sms=148)
+    for batch in (1, 2, 3, 5, 8, 13, 16, 30, 64):
+        for keys in (60, 300, 1280, 8192):
+            assert 1 <= kernels.decode_splits(batch, 4, keys, 0, **two) <= max(1, ((keys + 63) // 64 + 1) // 2)

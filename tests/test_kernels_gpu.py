@@ -832,6 +832,34 @@ def test_float_attention_gives_the_same_bits_however_it_is_cut(monkeypatch, opti
         assert torch.equal(one[0], shared[n - 1])
 
 
+@pytest.mark.parametrize("options", ["plain", "sink", "bias", "one row"])
+@pytest.mark.parametrize("hd,n_kv,splits", [(256, 4, 2), (144, 2, 4), (64, 4, 3)])
+def test_decode_attention_gives_the_same_bits_whatever_runs_beside_it(options, hd, n_kv, splits):
+    """More blocks than two rounds hold (two blocks to an SM with large heads, the longest sequences first) against every
+    sequence alone (a block to an SM): unequal and equal lengths, one key, a page's edges, padding rows in between."""
+    g = torch.Generator(device=DEV).manual_seed(hd + splits)
+    lengths = [0, 1, 64, 65, 700, 128, 0, 129, 63, 64] + [1 + 37 * i % 500 for i in range(88)]
+    B, group, W = len(lengths), 2, 11
+    assert splits * n_kv * B > 2 * kernels.device_sms(DEV)
+    pages = torch.randn(B * W, n_kv, 64, hd, generator=g, device=DEV).to(torch.bfloat16)
+    values = pages if options == "one row" else torch.randn(B * W, n_kv, 64, hd, generator=g, device=DEV).to(torch.bfloat16)
+    table = torch.randperm(B * W, generator=g, device=DEV).to(torch.int32).view(B, W)
+    q = torch.randn(B, n_kv * group * hd, generator=g, device=DEV).to(torch.bfloat16)
+    extra = dict(sink=torch.randn(n_kv * group, generator=g, device=DEV)) if options == "sink" else {}
+    if options == "bias":
+        extra = dict(dist_bias=torch.randn(n_kv * group, 100, generator=g, device=DEV))
+    kw = dict(ring=1 << 30, page_size=64, n_kv=n_kv, group=group, head_dim=hd, scale=hd ** -0.5, cap=20.0, window=300,
+              n_splits=splits, **extra)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    out = torch.full_like(q, 7.0)
+    kernels.attention_decode_mma(q, out, torch.arange(B + 1, dtype=torch.int32, device=DEV), i32(*lengths), pages, values, table,
+                                 batch=B, **kw)
+    for b in range(B):
+        one = torch.full_like(q[b:b + 1], 7.0)
+        kernels.attention_decode_mma(q[b:b + 1], one, i32(0, 1), i32(lengths[b]), pages, values, table[b:b + 1], batch=1, **kw)
+        assert torch.equal(out[b], one[0]), (b, lengths[b])
+
+
 def test_kernels_refuse_what_they_cannot_do():
     q = torch.zeros(2, 2 * 520, device=DEV)
     with pytest.raises(kernels.KernelError):                # a head beyond the exact kernel's 512
