@@ -3,10 +3,9 @@
 //
 // With few tokens the product is a stream of W from memory, and the kernel is
 // built as one: the roles of the operands are swapped (128 rows of W fill the M
-// side of tcgen05.mma, the tokens the N side), and a persistent block per SM
-// pulls its share of W through a deep ring of TMA stages (up to ten 16 KB
-// tiles in flight per SM), so the stream never drains between the block's work
-// items.  A work item is a (128-row tile of W, slice of K) pair; for the
+// side of tcgen05.mma, the tokens the N side), and persistent blocks pull their
+// share of W through deep rings of TMA stages (up to ten 16 KB tiles in flight
+// per SM), so the stream never drains between a block's work items.  A work item is a (128-row tile of W, slice of K) pair; for the
 // 2304-wide outputs of the model K is cut into slices so that every SM has an
 // item, and the float partial sums of the slices are added, in order, by the
 // kernel that reads them (the residual kernel).
@@ -36,7 +35,12 @@ using namespace tc;
 constexpr int BR = 128, BK = 64;
 constexpr int THREADS = 192;
 constexpr int W_BYTES = BR * BK * 2;
-constexpr int RING_BYTES = 200 * 1024;
+// One block an SM with a ring of 200 KB, or, where there are more items than SMs, two with 108 KB each: as many bytes in
+// flight, but one block streams while the other starts or stores, a round holds twice as many items (9B gate and up are
+// 224 for 148 SMs, two rounds of which the second is half empty), and the next kernel's first block finds room as soon
+// as one of the two is done.  At 16 tokens, one / two blocks an SM: 28,672 x 3,584 gated 46.8 / 34.0 us (31.9 at the
+// memory's rate), 3,584 x 14,336 in 5 / 10 slices 20.2 / 18.9 us (15.9), 8,192 x 3,584 in 2 / 4 slices 13.5 / 11.8 us.
+template <int PER_SM> constexpr int ring_bytes() { return PER_SM == 2 ? 108 * 1024 : 200 * 1024; }
 
 enum : int { EPI_STORE = 0, EPI_GATED = 1, EPI_SOFTCAP = 2 };
 
@@ -62,22 +66,22 @@ __device__ __forceinline__ bool drain_on(uint32_t bar, uint32_t parity, volatile
     return mbar_wait(bar, parity, give_up, &g_gemm_stream_error, code, true);
 }
 
-template <int BT, int EPI>
+template <int BT, int EPI, int PER_SM>
 struct Shape {
     static constexpr int OUT_ROWS = EPI == EPI_GATED ? BR / 2 : BR;        // output columns of a tile
     static constexpr int X_BYTES = BT * BK * 2;
     static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
-    static constexpr int STAGES = RING_BYTES / STAGE_BYTES > 10 ? 10 : RING_BYTES / STAGE_BYTES;
+    static constexpr int STAGES = ring_bytes<PER_SM>() / STAGE_BYTES > 10 ? 10 : ring_bytes<PER_SM>() / STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BT < 32 ? 32 : 2 * BT;            // two accumulators; a power of two
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 +
-                                   (EPI == EPI_GATED ? (size_t)64 * BT * 4 : 0);
+                                   (EPI == EPI_GATED ? (size_t)64 * 16 * 4 : 0);
 };
 
-template <int BT, int EPI>
-__global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w,
+template <int BT, int EPI, int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM) gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                  const __grid_constant__ CUtensorMap map_x,
                                                                  StreamArgs g) {
-    using S = Shape<BT, EPI>;
+    using S = Shape<BT, EPI, PER_SM>;
     constexpr int STAGES = S::STAGES;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;
@@ -226,12 +230,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(const __grid_co
                     col = rt * 64 + (lrow & 63);
                     if (quarter >= 2) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) upx[(lrow - 64) * BT + c + i] = o[i];
+                        for (int i = 0; i < 16; ++i) upx[i * 64 + lrow - 64] = o[i];
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (quarter < 2) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = fast_gate_pair(o[i], upx[lrow * BT + c + i], g.act, g.cap);   // code 2: cap is its limit
+                        for (int i = 0; i < 16; ++i) o[i] = fast_gate_pair(o[i], upx[i * 64 + lrow], g.act, g.cap);   // code 2: cap is its limit
                     }
                     writer = quarter < 2;
                     asm volatile("bar.sync 1, 128;" ::: "memory");          // upx may be written again
@@ -262,17 +266,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_stream_kernel(const __grid_co
     if (warp == 1) tmem_dealloc(tmem, S::TMEM_COLS);
 }
 
-template <int BT, int EPI>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const StreamArgs& g, cudaStream_t stream) {
-    using S = Shape<BT, EPI>;
+template <int BT, int EPI, int PER_SM>
+int launch_as(const CUtensorMap& mw, const CUtensorMap& mx, const StreamArgs& g, cudaStream_t stream) {
+    using S = Shape<BT, EPI, PER_SM>;
+    static_assert((S::SMEM + 1024) * PER_SM <= 228 * 1024 && S::TMEM_COLS * PER_SM <= 512, "the blocks of an SM");
     static bool raised = false;
     if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<BT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<BT, EPI, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
         if (e != cudaSuccess) return (int)e;
         raised = true;
     }
-    const int sms = device_sms();
-    return launch_pdl(gemm_stream_kernel<BT, EPI>, dim3(g.items < sms ? g.items : sms), dim3(THREADS), S::SMEM, stream, mw, mx, g);
+    const int places = PER_SM * device_sms();
+    return launch_pdl(gemm_stream_kernel<BT, EPI, PER_SM>, dim3(g.items < places ? g.items : places), dim3(THREADS), S::SMEM, stream, mw, mx, g);
+}
+
+template <int BT, int EPI>
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const StreamArgs& g, cudaStream_t stream) {
+    return g.items > device_sms() ? launch_as<BT, EPI, 2>(mw, mx, g, stream) : launch_as<BT, EPI, 1>(mw, mx, g, stream);
 }
 
 template <int EPI>

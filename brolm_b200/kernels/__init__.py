@@ -1330,6 +1330,25 @@ def stream_rows(x: torch.Tensor, weight: torch.Tensor) -> bool:
     return x.dim() == 2 and SKINNY_MAX_ROWS < x.shape[0] <= STREAM_ROWS and gemm_stream_ok(x, weight)
 
 
+def stream_instead_of_skinny(x: torch.Tensor, gate_up: torch.Tensor, sms: Optional[int] = None) -> bool:
+    """Whether gate and up with the activation of at most 16 tokens are better on the tcgen05 weight stream than on the
+    few-token product.
+
+    The mma.sync kernel reads the tokens anew for every 32 rows of W, from the L2 and through registers; the stream reads
+    them per 128 rows and keeps its weights in flight without registers, but starts later and works in pieces of 128 rows.
+    It is better where those pieces are more than the SMs and fill their last round of two an SM: 9B, 224 pieces, a
+    decode step of 1 / 4 / 8 / 16 sequences 4,081 / 4,297 / 4,642 / 7,180 us on mma.sync, 3,995 / 4,239 / 4,503 / 6,796 here
+    (the largest ragged); 27B, 576 pieces, the product alone at 8 / 16 tokens 104.0 / 113.4 and 101.2 / 102.7 us; but 2B,
+    144 pieces, 16.2 and 18.1 us at 8 tokens.  Both results differ from 64 bits by their rounding to bfloat16 (1.649e-3).
+    (Down, whose float sums the reader adds, stays: the stream is faster at 9B from nine tokens on, 25.5 -> 18.9 us, but
+    its sums differ from 64 bits by 1.4e-6 where those of the mma.sync kernel do by 0.6e-6.)"""
+    if not gemm_stream_ok(x, gate_up) or gate_up.shape[0] % 128:
+        return False
+    places = 2 * (sms or device_sms(x.device if x.is_cuda else None))
+    pieces = gate_up.shape[0] // 128
+    return pieces > places // 2 and pieces >= 0.7 * places * -(-pieces // places)
+
+
 def gemm_stream_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether the tcgen05 weight-streaming product (few tokens) takes these operands."""
     return (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and
@@ -1339,11 +1358,15 @@ def gemm_stream_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def gemm_stream_parts(x: torch.Tensor, weight: torch.Tensor, sms: Optional[int] = None) -> int:
-    """Slices of K so that every SM gets a (128-row tile, slice) item of the weight stream."""
+    """Slices of K so that every SM gets a (128-row tile, slice) item of the weight stream, two items where the weights
+    are many enough to be worth twice the slices (which the kernel after it adds): a decode step of 24 sequences at the 9B
+    sizes, whose matrices have 59 and 103 MB, 6,323 us with one and 6,081 with two; at the 2B sizes (19 and 42 MB) no
+    difference."""
     sms = sms or device_sms(x.device if x.is_cuda else None)
     row_tiles = (weight.shape[0] + 127) // 128
     nkb = (x.shape[1] + 63) // 64
-    want = max(1, sms // row_tiles)
+    many = weight.shape[0] * x.shape[1] * 2 >= 48 << 20
+    want = max(1, (2 if many else 1) * sms // row_tiles)
     # at least a ring's worth of K blocks (8) per item: a shorter run is over before its loads are all
     # in flight, and every further slice is another float copy of the output for the reader to add
     per = max(min(8, nkb), (nkb + want - 1) // want)
@@ -1819,7 +1842,7 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, s
 __all__ = ["KernelBuildError", "KernelError", "build_all", "launch_count", "device_sms", "wait_control", "embed_scale",
            "embed_pairs", "concat_cast", "latent_rows", "route_topk", "route_pick", "group_tiles", "group_pairs", "experts_tc_ok", "gather_rows", "experts_linear_tc", "grouped_tc_status", "heads_linear",
            "experts_linear", "rmsnorm", "residual_rmsnorm",
-           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "gemm_stream_ok", "gemm_stream_parts", "stream_rows",
+           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
            "gemm_stream_status", "attention_simt", "attention_prefill_mma", "attention_prefill_tc", "attention_prefill_tc_ok", "attention_prefill_tc_split", "attention_tc_status", "attention_decode_mma",
            "decode_splits", "argmax", "sample", "cast", "bias_act", "scaled_sum", "qkv_norm_write", "gate_group_norm", "head_norm_gate", "rotate_heads",
            "layernorm", "residual_layernorm", "table_gate", "delta_step", "delta_prompt", "experts_combine", "causal_conv", "conv_tail", "gated_scan", "ssm_scan", "block_matvec_f32", "block_matvec_ok", "split_halves"]

@@ -40,11 +40,13 @@ class GatedFeedForward(Part):
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """x (tokens, hidden) -> (tokens, hidden) float32."""
         act = torch.empty((x.shape[0], self.inter), dtype=ctx.dtype, device=x.device)
-        if kernels.skinny_ok(x, self.w_gate_up):
+        few = kernels.skinny_ok(x, self.w_gate_up)
+        stream = kernels.stream_rows(x, self.w_gate_up) or (few and kernels.stream_instead_of_skinny(x, self.w_gate_up))
+        if few and not (stream and self.inter % 64 == 0):
             # few tokens: both products and the activation in one pass over the weights
             kernels.skinny_gemm(x, self.w_gate_up, act, "gated", self.activation, limit=self.limit)
-        elif self.inter % 64 == 0 and kernels.stream_rows(x, self.w_gate_up):
-            # 17 to 128 tokens: the same on the tcgen05 weight stream
+        elif self.inter % 64 == 0 and stream:
+            # more of them, or many weights: the same on the tcgen05 weight stream
             kernels.gemm_stream(x, self.w_gate_up, act, "gated", self.activation, limit=self.limit)
         elif self.inter % 128 == 0 and kernels.gemm_tc_ok(x, self.w_gate_up, gated=True):
             # many tokens: the activation is the epilogue of the product; [gate | up] never reaches memory

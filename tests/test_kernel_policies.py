@@ -92,3 +92,14 @@ def test_decode_splits_where_two_blocks_share_an_sm():
     for batch in (1, 2, 3, 5, 8, 13, 16, 30, 64):
         for keys in (60, 300, 1280, 8192):
             assert 1 <= kernels.decode_splits(batch, 4, keys, 0, **two) <= max(1, ((keys + 63) // 64 + 1) // 2)
+
+
+def test_which_few_token_products_stream(monkeypatch):
+    monkeypatch.setattr(kernels, "gemm_stream_ok", lambda x, w: True)             # (tensors without memory have no address)
+    like = lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device="meta")
+    of = lambda M, N, K: kernels.stream_instead_of_skinny(like(M, K), like(N, K), sms=148)
+    assert of(1, 28672, 3584) and of(16, 73728, 4608)                 # 9B, 27B gate and up
+    assert not of(16, 18432, 2304) and not of(8, 8192, 2048)          # no more pieces than SMs
+    assert not of(8, 128 * 300, 512)                                        # a second round of four pieces
+    slices = lambda N, K: kernels.gemm_stream_parts(like(16, K), like(N, K), sms=148)
+    assert slices(3584, 14336) == 10 and slices(8192, 3584) == 4 and slices(2304, 9216) == 8

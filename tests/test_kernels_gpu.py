@@ -293,6 +293,26 @@ def test_gemm_stream_gated(M, F, K, act):
     assert kernels.gemm_stream_parts(torch.empty(8, 2304), torch.empty(256000, 2304)) == 1
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 128])
+@pytest.mark.parametrize("kind,N,K", [("store", 128 * 150 - 40, 72), ("store", 128 * 310 + 8, 200), ("parts", 1000, 64 * 44),
+                                      ("gated", 64 * 150, 72), ("gated", 64 * 300, 392)])
+def test_gemm_stream_with_two_blocks_an_sm(M, kind, N, K):
+    """More items than SMs: one round of two blocks an SM, and more than a round; remainders of rows and of K."""
+    g = torch.Generator(device=DEV).manual_seed(N + M)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(2 * N if kind == "gated" else N, K, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    if kind == "gated":
+        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        kernels.gemm_stream(x, w, out, "gated", "gelu_tanh")
+        close(out, plain.gelu_tanh(ref[:, :N]) * ref[:, N:], torch.bfloat16)
+    else:
+        out = torch.empty((22, M, N) if kind == "parts" else (M, N), dtype=torch.float32, device=DEV)
+        kernels.gemm_stream(x, w, out)
+        close(out.sum(0) if kind == "parts" else out, ref, torch.float32, scale=float(ref.abs().max()) * 50)
+    assert kernels.gemm_stream_status() == 0
+
+
 def test_gemm_tc_strided_views():
     g = torch.Generator().manual_seed(2)
     big = torch.randn(40, 3 * 64, generator=g).to(torch.bfloat16).to(DEV)
