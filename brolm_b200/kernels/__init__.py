@@ -48,7 +48,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle, without a Python object around it: 0.3 us instead of 3.2 for each launch."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 B200_SMS = 148
@@ -58,13 +59,16 @@ _sms: dict = {}
 def device_sms(device=None) -> int:
     """How many SMs the device of the kernels' launches has, asked once per device.  Without a CUDA
     device (the policy functions below are plain arithmetic and are tested on the CPU) the B200's 148."""
-    if not torch.cuda.is_available():
-        return B200_SMS
-    index = torch.device(device).index if device is not None else None
+    index = device.index if isinstance(device, torch.device) else torch.device(device).index if device is not None else None
     if index is None:
+        # (asking whether there is a device at all takes several microseconds: only until one has been seen)
+        if not _sms and not torch.cuda.is_available():
+            return B200_SMS
         index = torch.cuda.current_device()
     n = _sms.get(index)
     if n is None:
+        if not torch.cuda.is_available():
+            return B200_SMS
         n = _sms[index] = int(torch.cuda.get_device_properties(index).multi_processor_count)
     return n
 
