@@ -1183,7 +1183,11 @@ def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilog
         # 2B 17.4 against 16.2 us): their last, thin round of blocks streams twice the bytes per block
         tiles = 2
     else:
-        tiles = 2 if N >= 64 * device_sms(x.device) else 1
+        # two tiles a block for very wide outputs, and where one block to a place makes the better rounds (8,224 x 2,048 at
+        # 1 / 8 / 16 tokens, one tile 8.6 / 10.7 / 11.4 us, two 7.3 / 7.8 / 8.7; 8,192 x 3,584 13.7 / 16.0 / 16.8 and 11.3 / 11.8 /
+        # 12.8; up to 6,144 x 2,048 they are even)
+        sms = device_sms(x.device)
+        tiles = 2 if N >= 64 * sms or (ksplit == 1 and skinny_rope_tiles(N, K, sms) == 2) else 1
     if code == 2:
         assert out.dtype == torch.float32
     f = _fn("skinny_gemm", "brolm_skinny_gemm", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
