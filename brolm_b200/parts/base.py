@@ -37,6 +37,9 @@ class Part:
     # nothing that depends on values read back to the host: the decode step may
     # then be captured in a CUDA graph and replayed.
     graph_safe: bool = False
+    # True when its kernels may run at the same time as another part's: none of them keeps tickets, counters or scratch
+    # of its own on the device that another kernel of the step uses, too.
+    runs_beside: bool = False
 
     def param_specs(self) -> dict[str, ParamSpec]:
         """Local tensor name -> what it must look like."""

