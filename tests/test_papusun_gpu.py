@@ -289,3 +289,27 @@ def test_greedy_from_the_command_line(setups):
             row = plain.forward(config, weights, ids)[-1]
             assert float(row.max() - row[tok]) <= 1e-4 * float(row.abs().max())
             ids.append(tok)
+
+
+@pytest.mark.parametrize("batch", [1, 8, 20, 40])
+def test_captured_steps_run_the_two_mixers_as_branches(setups, batch):
+    """A captured step (the delta rule on a forked stream; the library's product beyond 32 tokens) against the same step
+    launch by launch, several steps on, and the same captured steps over again bit for bit."""
+    _, config, _, model = setups[("S", "bfloat16")]
+    g = np.random.default_rng(batch)
+    prompts = random_prompts(config["vocab"], [int(n) for n in g.integers(1, 90, batch)], seed=batch)
+    more = g.integers(0, config["vocab"], (6, batch)).tolist()
+
+    def run(eng):
+        slots = eng.open(batch)
+        rows = [eng.step(slots, prompts).clone()] + [eng.step(slots, [[t] for t in ids]).clone() for ids in more]
+        eng.close(slots)
+        return torch.stack(rows)
+
+    captured = bb.Engine(model, max_tokens=128 * batch, max_slots=batch)
+    assert captured.use_graphs
+    first = run(captured)
+    assert torch.equal(run(captured), first)
+    plainly = run(bb.Engine(model, max_tokens=128 * batch, max_slots=batch, use_graphs=False))
+    # other cuts of the keys and other products by the padded batch: what bfloat16 leaves of a logit, as the oracle bounds it
+    assert float((first - plainly).abs().max()) <= 2 * ROUNDING["S"][1] * float(plainly.abs().max())
