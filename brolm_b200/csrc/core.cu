@@ -13,6 +13,8 @@ template <typename W>
 __global__ void embed_scale_kernel(const int32_t* __restrict__ ids, const W* __restrict__ table,
                                    float scale, float* __restrict__ out, int hidden) {
     const int t = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
     const W* row = table + (size_t)ids[t] * hidden;
     float* dst = out + (size_t)t * hidden;
 #pragma unroll 4
@@ -23,14 +25,12 @@ BROLM_API int brolm_embed_scale(const void* ids, const void* table, int table_dt
                                 void* out, int tokens, int hidden, cudaStream_t stream) {
     if (tokens <= 0) return BROLM_OK;
     if (table_dtype == BROLM_F32)
-        embed_scale_kernel<float><<<tokens, 256, 0, stream>>>((const int32_t*)ids, (const float*)table, scale,
-                                                              (float*)out, hidden);
-    else if (table_dtype == BROLM_BF16)
-        embed_scale_kernel<bf16><<<tokens, 256, 0, stream>>>((const int32_t*)ids, (const bf16*)table, scale,
-                                                             (float*)out, hidden);
-    else
-        return BROLM_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(embed_scale_kernel<float>, dim3(tokens), dim3(256), 0, stream, (const int32_t*)ids, (const float*)table,
+                          scale, (float*)out, hidden);
+    if (table_dtype == BROLM_BF16)
+        return launch_pdl(embed_scale_kernel<bf16>, dim3(tokens), dim3(256), 0, stream, (const int32_t*)ids, (const bf16*)table,
+                          scale, (float*)out, hidden);
+    return BROLM_ERR_BAD_DTYPE;
 }
 
 // ---------------------------------------------------------------------------
@@ -574,6 +574,9 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, const int32_t* __restr
                                      T* __restrict__ k_pages, T* __restrict__ v_pages,
                                      const int32_t* __restrict__ cache_rows, int page_size) {
     const int t = blockIdx.x, head = blockIdx.y;          // head: q heads, then k heads, then v heads
+    // (no early trigger here nor in gated_act_kernel: the float product behind them streams from few warps an SM, and let in
+    // early its blocks lie unevenly: a float decode step at the 2B sizes 3,781 -> 3,858 us)
+    pdl_wait();
     const int pos = positions[t];
     if (pos < 0) return;
     const bool is_v = head >= n_q + n_kv, is_k = !is_v && head >= n_q;
@@ -764,16 +767,14 @@ BROLM_API int brolm_rope_kv_write(void* qkv, int dtype, const void* positions, c
     int threads = ((hd >> 1) + 31) / 32 * 32;
     if (threads > 256) threads = 256;
     if (dtype == BROLM_F32)
-        rope_kv_write_kernel<float><<<grid, threads, 0, stream>>>(
-            (float*)qkv, (const int32_t*)positions, (const float2*)cos_sin, n_q, n_kv, hd, rot, (float*)k_pages,
-            (float*)v_pages, (const int32_t*)cache_rows, page_size);
-    else if (dtype == BROLM_BF16)
-        rope_kv_write_kernel<bf16><<<grid, threads, 0, stream>>>(
-            (bf16*)qkv, (const int32_t*)positions, (const float2*)cos_sin, n_q, n_kv, hd, rot, (bf16*)k_pages,
-            (bf16*)v_pages, (const int32_t*)cache_rows, page_size);
-    else
-        return BROLM_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(rope_kv_write_kernel<float>, grid, dim3(threads), 0, stream, (float*)qkv, (const int32_t*)positions,
+                          (const float2*)cos_sin, n_q, n_kv, hd, rot, (float*)k_pages, (float*)v_pages,
+                          (const int32_t*)cache_rows, page_size);
+    if (dtype == BROLM_BF16)
+        return launch_pdl(rope_kv_write_kernel<bf16>, grid, dim3(threads), 0, stream, (bf16*)qkv, (const int32_t*)positions,
+                          (const float2*)cos_sin, n_q, n_kv, hd, rot, (bf16*)k_pages, (bf16*)v_pages,
+                          (const int32_t*)cache_rows, page_size);
+    return BROLM_ERR_BAD_DTYPE;
 }
 
 // ---------------------------------------------------------------------------
@@ -794,6 +795,7 @@ __device__ __forceinline__ float act_apply(float z, int act) {
 template <typename T>
 __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int inter, int act, float limit) {
     const size_t t = blockIdx.x;
+    pdl_wait();
     const T* g = gate_up + t * 2 * (size_t)inter;
     const T* u = g + inter;
     T* o = out + t * (size_t)inter;
@@ -806,6 +808,8 @@ __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ 
 __global__ void __launch_bounds__(256) gated_act_vec_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out,
                                                             int inter, int act, float limit) {
     const size_t t = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
     const bf16* g = gate_up + t * 2 * (size_t)inter;
     const bf16* u = g + inter;
     bf16* o = out + t * (size_t)inter;
@@ -832,19 +836,17 @@ BROLM_API int brolm_gated_act(const void* gate_up, void* out, int dtype, int tok
     if (dtype == BROLM_BF16 && inter % 8 == 0 && ((uintptr_t)gate_up & 15) == 0 && ((uintptr_t)out & 15) == 0) {
         int by = (inter / 8 + 255) / 256;
         if (by > 65535) by = 65535;
-        gated_act_vec_kernel<<<dim3(tokens, by), 256, 0, stream>>>((const bf16*)gate_up, (bf16*)out, inter, act, limit);
-        return launch_status();
+        return launch_pdl(gated_act_vec_kernel, dim3(tokens, by), dim3(256), 0, stream, (const bf16*)gate_up, (bf16*)out, inter, act,
+                          limit);
     }
     int by = (inter + 1023) / 1024;
     if (by > 65535) by = 65535;
     dim3 grid(tokens, by);
     if (dtype == BROLM_F32)
-        gated_act_kernel<float><<<grid, 256, 0, stream>>>((const float*)gate_up, (float*)out, inter, act, limit);
-    else if (dtype == BROLM_BF16)
-        gated_act_kernel<bf16><<<grid, 256, 0, stream>>>((const bf16*)gate_up, (bf16*)out, inter, act, limit);
-    else
-        return BROLM_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(gated_act_kernel<float>, grid, dim3(256), 0, stream, (const float*)gate_up, (float*)out, inter, act, limit);
+    if (dtype == BROLM_BF16)
+        return launch_pdl(gated_act_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)gate_up, (bf16*)out, inter, act, limit);
+    return BROLM_ERR_BAD_DTYPE;
 }
 
 // ---------------------------------------------------------------------------
@@ -854,6 +856,8 @@ BROLM_API int brolm_gated_act(const void* gate_up, void* out, int dtype, int tok
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void softcap_kernel(const T* __restrict__ x, float* __restrict__ out, size_t n, float cap, float mul) {
+    pdl_trigger();
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = soft_cap(to_float(x[i]) * mul, cap);
 }
@@ -863,10 +867,10 @@ BROLM_API int brolm_softcap(const void* x, int dtype, void* out, long long n, fl
     long long blocks = (n + 255) / 256;
     if (blocks > device_sm_count() * 32) blocks = device_sm_count() * 32;
     if (dtype == BROLM_F32)
-        softcap_kernel<float><<<(int)blocks, 256, 0, stream>>>((const float*)x, (float*)out, (size_t)n, cap, mul);
-    else if (dtype == BROLM_BF16)
-        softcap_kernel<bf16><<<(int)blocks, 256, 0, stream>>>((const bf16*)x, (float*)out, (size_t)n, cap, mul);
-    else
-        return BROLM_ERR_BAD_DTYPE;
-    return launch_status();
+        return launch_pdl(softcap_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, (const float*)x, (float*)out, (size_t)n,
+                          cap, mul);
+    if (dtype == BROLM_BF16)
+        return launch_pdl(softcap_kernel<bf16>, dim3((unsigned)blocks), dim3(256), 0, stream, (const bf16*)x, (float*)out, (size_t)n,
+                          cap, mul);
+    return BROLM_ERR_BAD_DTYPE;
 }

@@ -621,6 +621,8 @@ __global__ void __launch_bounds__(256) grouped_bf16_fast_kernel(GroupedArgs g) {
     constexpr int LD = BK + 8, CPR = BK / 8, WN = FBN / 4, NP = WN / 16;   // a warp: 32 rows x WN outputs
     extern __shared__ __align__(128) unsigned char fsm[];
     __shared__ RowInfo info[GBM];
+    pdl_trigger();
+    pdl_wait();
     const int group = tile_rows(g, blockIdx.y, info);
     if (group < 0) return;
     __syncthreads();
@@ -722,8 +724,7 @@ int launch_fast(const GroupedArgs& g, int row_tiles, cudaStream_t stream) {
         raised = true;
     }
     dim3 grid((g.N + FBN - 1) / FBN, row_tiles);
-    grouped_bf16_fast_kernel<FBN, BK, STAGES, HEADS><<<grid, 256, smem, stream>>>(g);
-    return launch_status();
+    return launch_pdl(grouped_bf16_fast_kernel<FBN, BK, STAGES, HEADS>, grid, dim3(256), smem, stream, g);
 }
 
 // `few`: the groups have a handful of rows each (decoding), so the matrices are streamed rather than tiled

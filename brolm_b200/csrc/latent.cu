@@ -36,6 +36,8 @@ template <typename T>
 __global__ void __launch_bounds__(128) latent_rows_kernel(LatentArgs<T> p) {
     __shared__ float red[33];
     const int t = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
     const int pos = p.positions[t];
     const T* row = p.proj + (size_t)t * p.ld_proj;
     const int half = p.rd >> 1;
@@ -102,8 +104,7 @@ int launch_latent(const void* proj, long ld_proj, int kv_col, const void* q, lon
     p.positions = (const int32_t*)positions; p.cos_sin = (const float*)cos_sin; p.rd = rd; p.inter = inter;
     p.gain = (const T*)gain; p.eps = eps; p.heads = heads; p.dn = dn; p.dr = dr; p.R = R; p.Dp = Dp;
     p.lat = (T*)lat; p.qlat = (T*)qlat; p.pages = (T*)pages; p.cache_rows = (const int32_t*)cache_rows;
-    latent_rows_kernel<T><<<tokens, 128, 0, stream>>>(p);
-    return launch_status();
+    return launch_pdl(latent_rows_kernel<T>, dim3(tokens), dim3(128), 0, stream, p);
 }
 
 }  // namespace
