@@ -356,62 +356,70 @@ int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int
 }
 
 // ---------------------------------------------------------------------------
-// Any strides and sizes: 64 x 64 tiles, 4 x 4 outputs a thread, one element at a time.
+// Any strides and sizes, one element at a time: 64 x 64 tiles, 4 x 4 outputs a thread, pairs of an even and an odd k side
+// by side in shared memory; the next 16 k are on their way while a tile is multiplied.
 constexpr int AM = 64, AN = 64, AK = 16;
+constexpr int APITCH = AM + 4;                         // pairs
 
 __global__ void __launch_bounds__(256) any_kernel(const float* __restrict__ X, int ldx, const float* __restrict__ W, int ldw,
                                                   float* __restrict__ Y, int ldy, int M, int N, int K) {
-    __shared__ float As[AK][AM + 4];
-    __shared__ float Bs[AK][AN + 4];
+    __shared__ __align__(16) float2 As[2][AK / 2][APITCH];
+    __shared__ __align__(16) float2 Bs[2][AK / 2][APITCH];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;            // 16 x 16 threads, 4 x 4 outputs each
+    const int tx = tid & 15, ty = tid >> 4;            // rows 4 ty .. 4 ty + 3; columns 2 tx, 2 tx + 1 and the two 32 further on
     const int m0 = blockIdx.y * AM, n0 = blockIdx.x * AN;
-    const int lr = tid >> 2, lk = (tid & 3) * 4;        // loader: row lr, k offset lk..lk+3
+    const int lr = tid >> 2, lk = (tid & 3) * 4;       // loader: row lr, k offset lk..lk+3
+    const float* xp = X + (size_t)min(m0 + lr, M - 1) * ldx + lk;
+    const float* wp = W + (size_t)min(n0 + lr, N - 1) * ldw + lk;
+    const bool x_ok = m0 + lr < M, w_ok = n0 + lr < N;
 
-    float acc[2][4][4], tot[4][4];                      // [parity of k]
+    float a[4], b[4];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool ok = k0 + lk + i < K;
+            a[i] = ok && x_ok ? xp[k0 + i] : 0.0f;
+            b[i] = ok && w_ok ? wp[k0 + i] : 0.0f;
+        }
+    };
+    uint64_t acc[4][4];
+    float tot[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = tot[i][j] = 0.0f;
-
+        for (int j = 0; j < 4; ++j) {
+            acc[i][j] = 0;
+            tot[i][j] = 0.0f;
+        }
+    load(0);
     for (int k0 = 0; k0 < K; k0 += AK) {
-        float a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
-        const int k = k0 + lk;
-        if (m0 + lr < M) {
-            const float* p = X + (size_t)(m0 + lr) * ldx + k;
+        const int st = (k0 / AK) & 1;
+        As[st][lk / 2][lr] = make_float2(a[0], a[1]);
+        As[st][lk / 2 + 1][lr] = make_float2(a[2], a[3]);
+        Bs[st][lk / 2][lr] = make_float2(b[0], b[1]);
+        Bs[st][lk / 2 + 1][lr] = make_float2(b[2], b[3]);
+        __syncthreads();   // this tile is written, and the one before it is consumed by all (its stage is written next)
+        if (k0 + AK < K) load(k0 + AK);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) if (k + i < K) a[i] = p[i];
-        }
-        if (n0 + lr < N) {
-            const float* p = W + (size_t)(n0 + lr) * ldw + k;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) if (k + i < K) b[i] = p[i];
-        }
-        __syncthreads();   // the tile before this one is consumed
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            As[lk + i][lr] = a[i];
-            Bs[lk + i][lr] = b[i];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < AK; ++kk) {
-            const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-            const float4 bv = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-            const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+        for (int kk = 0; kk < AK / 2; ++kk) {
+            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[st][kk][ty * 4]);
+            const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[st][kk][ty * 4 + 2]);
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[st][kk][tx * 2]);
+            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[st][kk][tx * 2 + 32]);
+            const uint64_t ar[4] = {a0.x, a0.y, a1.x, a1.y}, br[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[kk & 1][i][j] = fmaf(ar[i], br[j], acc[kk & 1][i][j]);
+                for (int j = 0; j < 4; ++j) fma2(acc[i][j], ar[i], br[j]);
         }
         if ((k0 + AK) % SEG == 0 || k0 + AK >= K) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float c = acc[0][i][j] + acc[1][i][j];
+                    const float c = halves_sum(acc[i][j]);
                     tot[i][j] = k0 < SEG ? c : tot[i][j] + c;
-                    acc[0][i][j] = acc[1][i][j] = 0.0f;
+                    acc[i][j] = 0;
                 }
         }
     }
@@ -421,7 +429,7 @@ __global__ void __launch_bounds__(256) any_kernel(const float* __restrict__ X, i
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
+            const int n = n0 + tx * 2 + (j & 1) + (j >> 1) * 32;
             if (n < N) Y[(size_t)m * ldy + n] = tot[i][j];
         }
     }
