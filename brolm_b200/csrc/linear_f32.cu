@@ -222,13 +222,13 @@ int dispatch_rows(const float* x, int ldx, const float* w, int ldw, float* y, in
 // (18,432 x 2,304: 43 TFLOP/s at M = 300 and 47 at M = 1024, of which the fma pipes are busy 64 %; 38 and 42 with
 // 8 x 4 and twice the warps; 24 and 25 before, with 4 x 4 and scalar fmas).  Two stages of 32 k; the sum over
 // the finished segments waits in shared memory, [output][thread].  The segments of K may be dealt to blocks along
-// z; with `parts` every segment's sums go to its own slice of Y, with one block along z they are added here.
+// z: the first of them adds its own in slice 0 of Y, the others leave every segment's sums in a slice of its own.
 constexpr int BN = 128, STAGES = 2;
 
 template <int BM>
 __global__ void __launch_bounds__(128, 2) tiles_kernel(const float* __restrict__ X, int ldx, const float* __restrict__ W, int ldw,
                                                        float* __restrict__ Y, int ldy, int M, int N, int K, int seg_per_block,
-                                                       int parts, long long part_stride) {
+                                                       long long part_stride) {
     constexpr int TM = BM / 8, TN = BN / 16;
     constexpr int STAGE = (BM + BN) * PITCH;
     extern __shared__ __align__(16) uint8_t raw[];
@@ -239,6 +239,8 @@ __global__ void __launch_bounds__(128, 2) tiles_kernel(const float* __restrict__
     const int seg0 = blockIdx.z * seg_per_block;
     const int k_end = min(K, (seg0 + seg_per_block) * SEG);
     const int steps = (k_end - seg0 * SEG + 31) / 32;
+    // the slice of this block's first segment; -1: the segments are added here (into slice 0, where there are several)
+    const int slice = seg0 > 0 ? seg0 - seg_per_block + 1 : -1;
 
     auto fetch = [&](int i) {
         if (i < steps) {
@@ -286,8 +288,8 @@ __global__ void __launch_bounds__(128, 2) tiles_kernel(const float* __restrict__
         }
         if (i % (SEG / 32) == SEG / 32 - 1 || i == steps - 1) {
             const int seg = i / (SEG / 32);
-            if (parts) {
-                float* dst = Y + (seg0 + seg) * part_stride;
+            if (slice >= 0) {
+                float* dst = Y + (slice + seg) * part_stride;
 #pragma unroll
                 for (int t = 0; t < TM; ++t)
 #pragma unroll
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(128, 2) tiles_kernel(const float* __restrict__
         }
     }
     pdl_trigger();
-    if (parts) return;
+    if (slice >= 0) return;
 #pragma unroll
     for (int t = 0; t < TM; ++t)
 #pragma unroll
@@ -346,13 +348,13 @@ int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int
     const int n_seg = (K + SEG - 1) / SEG;
     const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, parts ? (n_seg + seg_per_block - 1) / seg_per_block : 1);
     if (!parts)
-        return launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K, n_seg, 0, 0LL);
-    const int st = launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, parts, N, M, N, K, seg_per_block, 1,
+        return launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K, n_seg, 0LL);
+    const int st = launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, parts, N, M, N, K, seg_per_block,
                               (long long)M * N);
     if (st) return st;
     const size_t blocks = ((size_t)M * N + 255) / 256;
-    return launch_pdl(sum_parts_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, parts, n_seg, y, ldy,
-                      M, N);
+    return launch_pdl(sum_parts_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, parts,
+                      1 + (n_seg > seg_per_block ? n_seg - seg_per_block : 0), y, ldy, M, N);
 }
 
 // ---------------------------------------------------------------------------
@@ -437,8 +439,8 @@ __global__ void __launch_bounds__(256) any_kernel(const float* __restrict__ X, i
 
 }  // namespace
 
-// M <= 16 rows, and more in tiles.  parts (M > 16 only): room for ceil(K / 512) * M * N floats, into which the blocks,
-// seg_per_block segments of 512 k each, put their sums before they are added; null: a block takes all of K.
+// M <= 16 rows, and more in tiles.  parts (M > 16 only): the blocks take seg_per_block segments of 512 k each, and their
+// sums lie here before they are added, 1 + ceil(K / 512) - seg_per_block times M * N floats; null: a block takes all of K.
 BROLM_API int brolm_linear_f32(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
                                void* parts, int seg_per_block, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;

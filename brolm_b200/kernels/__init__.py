@@ -7,6 +7,7 @@ library fallback: a missing build or a CPU tensor raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_long, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
@@ -1046,24 +1047,54 @@ def rotate_heads(rows: torch.Tensor, q_off: int, k_off: int, heads: int, dim: in
 F32_SEGMENT = 512          # k of one partial sum of the float32 product (linear_f32.cu)
 
 
-def linear_f32_cut(M: int, N: int, K: int, sms: Optional[int] = None) -> int:
+F32_PARTS_LIMIT = 256 << 20  # bytes of partial sums
+
+
+def linear_f32_slices(K: int, per: int) -> int:
+    """How many partial sums of an output the tiled float32 product adds where a block takes ``per`` segments: one of the
+    first block, which adds its own, and one for each segment behind it."""
+    return 1 + max(0, -(-K // F32_SEGMENT) - per)
+
+
+@functools.lru_cache(maxsize=1024)
+def linear_f32_cut(M: int, N: int, K: int, sms: int) -> int:
     """How many 512-wide segments of K a block of the tiled float32 product takes; 0: all of them, nothing to add.
 
-    Two blocks share an SM, a block's time is its segments and about a quarter of one to start and end, and the last
-    round of blocks lasts as long as a full one; cut blocks cost writing and adding the segments' sums, about a third of
-    a segment.  (M = 300: the 4096 x 2304 product is 160 tiles for 296 places, cut into single segments it fills three
-    rounds of a fifth of the length.)  At most 16 rows need no cut: that kernel gives the segments to its warps."""
+    A segment takes a block 18 (tiles of 32 rows) or 30 us (64) alone on its SM, and two blocks that share one 31 or 52 us.
+    Blocks that take single segments fill a last round better; their sums (``linear_f32_slices`` of an output) are written
+    and read once more, and are not cut if they would take more than 256 MB.  At most 16 rows need no cut: that kernel
+    gives the segments to its warps."""
     if M <= 16:
         return 0
-    places = 2 * (sms or device_sms())
-    tiles = -(-M // (32 if M <= 32 else 64)) * -(-N // 128)
     segs = -(-K // F32_SEGMENT)
-    best, cut = -(-tiles // places) * (segs + 0.25), 0
-    for per in range(segs - 1, 0, -1):
-        cost = -(-tiles * -(-segs // per) // places) * (per + 0.25) + 0.3
-        if cost < best:
-            best, cut = cost, per
-    return cut
+    best = None
+    for rows, alone, shared in ((32, 18.2, 31.0),) if M <= 32 else ((64, 30.4, 52.0),):
+        tiles = -(-M // rows) * -(-N // 128)
+        for per in range(segs, 0, -1):
+            cuts = -(-segs // per)
+            adding, last = 0.0, K / F32_SEGMENT - (cuts - 1) * per
+            if cuts > 1:
+                size = linear_f32_slices(K, per) * M * N * 4
+                if size > F32_PARTS_LIMIT:
+                    break
+                adding = 2.0 + size / 5e6
+            # the blocks of full length in rounds (a last, thin one alone on the SMs), the shorter ones of the last cut behind
+            # them; and never faster than all places busy to the end
+            blocks, longest = tiles * cuts, min(per, K / F32_SEGMENT)
+            whole = blocks if last == longest else blocks - tiles
+            rounds, rest = divmod(whole, 2 * sms)
+            if rest:
+                beyond = max(0, rest + blocks - whole - sms) / sms
+                rounds += (alone + (shared - alone) * (1.0 if beyond and whole == blocks else min(1.0, beyond))) / shared
+            run = rounds * shared * longest
+            if cuts > 1 and blocks > 2 * sms:
+                if last != longest:
+                    run += 0.5 * shared * last
+                run = max(run, (tiles * K / F32_SEGMENT + 0.02 * blocks) * shared / (2 * sms) + 0.2 * shared * last)
+            cost = (run + 3.0 + adding) * (1.0 if cuts == 1 else 1.02)        # (cut where it is clearly the better way)
+            if best is None or cost < best[0]:
+                best = cost, per if cuts > 1 else 0
+    return best[1]
 
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
@@ -1075,8 +1106,9 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None
     M, K = x.shape
     N = weight.shape[0]
     assert weight.shape[1] == K and tuple(out.shape) == (M, N)
-    cut = linear_f32_cut(M, N, K)
-    parts = torch.empty((-(-K // F32_SEGMENT), M, N), dtype=torch.float32, device=x.device) if cut else None
+    aligned = not (K % 4 or x.stride(0) % 4 or weight.stride(0) % 4 or x.data_ptr() % 16 or weight.data_ptr() % 16)
+    cut = linear_f32_cut(M, N, K, device_sms(x.device)) if aligned else 0
+    parts = torch.empty((linear_f32_slices(K, cut), M, N), dtype=torch.float32, device=x.device) if cut else None
     f = _fn("linear_f32", "brolm_linear_f32", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                                c_void_p, c_int, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(parts), cut,

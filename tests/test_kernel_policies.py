@@ -103,3 +103,18 @@ def test_which_few_token_products_stream(monkeypatch):
     assert not of(8, 128 * 300, 512)                                        # a second round of four pieces
     slices = lambda N, K: kernels.gemm_stream_parts(like(16, K), like(N, K), sms=148)
     assert slices(3584, 14336) == 10 and slices(8192, 3584) == 4 and slices(2304, 9216) == 8
+
+
+def test_partial_sums_of_the_float_product_are_bounded():
+    """A cut along K pays for the sums it writes and reads again, and never takes more than a fixed scratch."""
+    assert kernels.linear_f32_slices(9216, 18) == 1 and kernels.linear_f32_slices(9216, 1) == 18
+    assert kernels.linear_f32_slices(9216 + 4, 9) == 11
+    cuts = 0
+    for M in (17, 40, 300, 1024, 4096, 4196, 8192, 16384):
+        for N, K in ((2304, 2304), (2304, 9216), (3584, 14336), (4608, 36864), (36864, 4608), (256000, 2304), (64, 100)):
+            cut = kernels.linear_f32_cut(M, N, K, 148)
+            assert 0 <= cut < -(-K // kernels.F32_SEGMENT)
+            if cut:
+                cuts += 1
+                assert kernels.linear_f32_slices(K, cut) * M * N * 4 <= 256 << 20, (M, N, K, cut)
+    assert cuts > 10

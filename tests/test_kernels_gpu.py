@@ -154,6 +154,17 @@ def test_linear_f32_kernels_and_cuts(M, N, K):
     assert torch.equal(again, out)
 
 
+def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
+    x = torch.zeros(300, 2305, device=DEV)[:, 1:]
+    w, out = torch.zeros(2304, 2304, device=DEV), torch.empty(300, 2304, device=DEV)
+    assert kernels.linear_f32_cut(300, 2304, 2304, kernels.device_sms()) > 0
+    kernels.linear_f32(x, w, out)
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    kernels.linear_f32(x, w, out)
+    assert torch.cuda.max_memory_allocated() == before
+
+
 def test_linear_f32_strided_views():
     g = torch.Generator().manual_seed(6)
     big = torch.randn(9, 3 * 48, generator=g).to(DEV)
