@@ -20,7 +20,8 @@
 // Three kernels:
 //   rows_kernel   M <= 16: the product is a stream of W.  Bound by memory.
 //   tiles_kernel  M > 16: tiles of 32 or 64 rows by 128 columns.  Bound by the fma pipes.
-//   any_kernel    operands whose rows do not lie on 16-byte boundaries.
+//   any_kernel    operands whose rows do not lie on 16-byte boundaries, and K of a few elements.
+// Which one, and how K is cut: linear_f32_plan in kernels/__init__.py.
 #include "common.cuh"
 
 namespace {
@@ -347,10 +348,15 @@ int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int
     }
     const int n_seg = (K + SEG - 1) / SEG;
     const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, parts ? (n_seg + seg_per_block - 1) / seg_per_block : 1);
-    if (!parts)
-        return launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K, n_seg, 0LL);
-    const int st = launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, parts, N, M, N, K, seg_per_block,
-                              (long long)M * N);
+    // Blocks that are let in early lie two on one SM and none on another, which costs where they do not fill all places:
+    // 64 x 1,024 x 1,024 in 16 blocks 51 us and 34 in order
+    const bool in_order = (long long)grid.x * grid.y * grid.z < 2LL * device_sm_count();
+    auto run = [&](float* dst, int ld, int per, long long stride) {
+        return in_order ? launch_in_order(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, dst, ld, M, N, K, per, stride)
+                        : launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, dst, ld, M, N, K, per, stride);
+    };
+    if (!parts) return run(y, ldy, n_seg, 0LL);
+    const int st = run(parts, N, seg_per_block, (long long)M * N);
     if (st) return st;
     const size_t blocks = ((size_t)M * N + 255) / 256;
     return launch_pdl(sum_parts_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, parts,
@@ -439,27 +445,31 @@ __global__ void __launch_bounds__(256) any_kernel(const float* __restrict__ X, i
 
 }  // namespace
 
-// M <= 16 rows, and more in tiles.  parts (M > 16 only): the blocks take seg_per_block segments of 512 k each, and their
-// sums lie here before they are added, 1 + ceil(K / 512) - seg_per_block times M * N floats; null: a block takes all of K.
+// kind: which kernel (rows and tiles want operands whose rows lie on 16-byte boundaries, K % 4 == 0; rows M <= 16).
+// parts (tiles only): the blocks take seg_per_block segments of 512 k each, and their sums lie here before they are added,
+// 1 + ceil(K / 512) - seg_per_block times M * N floats; null: a block takes all of K.
+enum : int { KIND_ANY = 0, KIND_ROWS = 1, KIND_TILES32 = 32, KIND_TILES64 = 64 };
+
 BROLM_API int brolm_linear_f32(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
-                               void* parts, int seg_per_block, cudaStream_t stream) {
+                               int kind, void* parts, int seg_per_block, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;
     if (K <= 0 || (parts && seg_per_block < 1)) return BROLM_ERR_BAD_SIZE;
     const float *xf = (const float*)x, *wf = (const float*)w;
     float* yf = (float*)y;
-    const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)w & 15);
-    if (vec && M <= 16) {
+    if (kind != KIND_ANY && (K % 4 || ldx % 4 || ldw % 4 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))) return BROLM_ERR_ALIGNMENT;
+    if (kind == KIND_ROWS) {
+        if (M > 16) return BROLM_ERR_BAD_SIZE;
         const int st = M <= 1 ? dispatch_rows<1>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
                      : M <= 2 ? dispatch_rows<2>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
                      : M <= 4 ? dispatch_rows<4>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
                      : M <= 8 ? dispatch_rows<8>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream)
                               : dispatch_rows<16>(xf, ldx, wf, ldw, yf, ldy, M, N, K, stream);
-        if (st != BROLM_ERR_TOO_LARGE) return st;        // a K beyond what the sums have room for goes on below
+        if (st != BROLM_ERR_TOO_LARGE) return st;
+        kind = KIND_TILES32;                             // a K beyond what the sums have room for
     }
-    const long long tiles_n = (N + BN - 1) / BN;
-    if (vec && tiles_n <= 65535) {
-        if (M <= 32) return launch_tiles<32>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
-        return launch_tiles<64>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
+    if ((N + BN - 1) / BN <= 65535) {
+        if (kind == KIND_TILES32) return launch_tiles<32>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
+        if (kind == KIND_TILES64) return launch_tiles<64>(xf, ldx, wf, ldw, yf, ldy, M, N, K, (float*)parts, seg_per_block, stream);
     }
     const long long gy = (M + AM - 1) / AM;
     if (gy > 65535) return BROLM_ERR_TOO_LARGE;

@@ -1057,18 +1057,25 @@ def linear_f32_slices(K: int, per: int) -> int:
 
 
 @functools.lru_cache(maxsize=1024)
-def linear_f32_cut(M: int, N: int, K: int, sms: int) -> int:
-    """How many 512-wide segments of K a block of the tiled float32 product takes; 0: all of them, nothing to add.
+def linear_f32_plan(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
+    """Which kernel of the float32 product takes these sizes (rows on 16-byte boundaries), and how many 512-wide segments
+    of K a block of it takes; 0: all of them, nothing to add.
 
-    A segment takes a block 18 (tiles of 32 rows) or 30 us (64) alone on its SM, and two blocks that share one 31 or 52 us.
-    Blocks that take single segments fill a last round better; their sums (``linear_f32_slices`` of an output) are written
-    and read once more, and are not cut if they would take more than 256 MB.  At most 16 rows need no cut: that kernel
-    gives the segments to its warps."""
-    if M <= 16:
-        return 0
+    At most 16 rows stream the weights (1); where K is so short that the streams never fill, the other kernels start
+    faster (K = 16: 2.6 us for 16 x 16 x 16 against 3.2; K = 100: 6.8 against 7.8 for 16 x 100).
+
+    More rows go in tiles of 32 or 64 rows by 128 columns.  A segment takes a block 18 or 30 us alone on its SM, and two
+    blocks that share one 31 or 52 us, so the larger tile is the better one where the SMs are full and the smaller where
+    they are not (100 x 256 x 1,024: 21.6 and 33.9 us).  Blocks that take single segments fill a last round better; their
+    sums (``linear_f32_slices`` of an output) are written and read once more, and are not cut if they would take more than
+    256 MB."""
+    if K <= 16 and M >= 8:
+        return 0, 0
+    if M <= 8 or (M <= 16 and K > 128):
+        return 1, 0
     segs = -(-K // F32_SEGMENT)
     best = None
-    for rows, alone, shared in ((32, 18.2, 31.0),) if M <= 32 else ((64, 30.4, 52.0),):
+    for rows, alone, shared in ((32, 18.2, 31.0), (64, 30.4, 52.0)):
         tiles = -(-M // rows) * -(-N // 128)
         for per in range(segs, 0, -1):
             cuts = -(-segs // per)
@@ -1093,8 +1100,8 @@ def linear_f32_cut(M: int, N: int, K: int, sms: int) -> int:
                 run = max(run, (tiles * K / F32_SEGMENT + 0.02 * blocks) * shared / (2 * sms) + 0.2 * shared * last)
             cost = (run + 3.0 + adding) * (1.0 if cuts == 1 else 1.02)        # (cut where it is clearly the better way)
             if best is None or cost < best[0]:
-                best = cost, per if cuts > 1 else 0
-    return best[1]
+                best = cost, rows, per if cuts > 1 else 0
+    return best[1:]
 
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
@@ -1107,11 +1114,16 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None
     N = weight.shape[0]
     assert weight.shape[1] == K and tuple(out.shape) == (M, N)
     aligned = not (K % 4 or x.stride(0) % 4 or weight.stride(0) % 4 or x.data_ptr() % 16 or weight.data_ptr() % 16)
-    cut = linear_f32_cut(M, N, K, device_sms(x.device)) if aligned else 0
+    kind, cut = linear_f32_plan(M, N, K, device_sms(x.device)) if aligned else (0, 0)
+    _linear_f32(x, weight, out, kind, cut)
+
+
+def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, kind: int, cut: int) -> None:
+    (M, K), N = x.shape, weight.shape[0]
     parts = torch.empty((linear_f32_slices(K, cut), M, N), dtype=torch.float32, device=x.device) if cut else None
     f = _fn("linear_f32", "brolm_linear_f32", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
-                                               c_void_p, c_int, c_void_p])
-    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(parts), cut,
+                                               c_int, c_void_p, c_int, c_void_p])
+    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, kind, _ptr(parts), cut,
              _stream()), "linear_f32")
 
 

@@ -112,9 +112,21 @@ def test_partial_sums_of_the_float_product_are_bounded():
     cuts = 0
     for M in (17, 40, 300, 1024, 4096, 4196, 8192, 16384):
         for N, K in ((2304, 2304), (2304, 9216), (3584, 14336), (4608, 36864), (36864, 4608), (256000, 2304), (64, 100)):
-            cut = kernels.linear_f32_cut(M, N, K, 148)
+            cut = kernels.linear_f32_plan(M, N, K, 148)[1]
             assert 0 <= cut < -(-K // kernels.F32_SEGMENT)
             if cut:
                 cuts += 1
                 assert kernels.linear_f32_slices(K, cut) * M * N * 4 <= 256 << 20, (M, N, K, cut)
     assert cuts > 10
+
+
+def test_which_kernel_takes_a_float_product():
+    """Streams for few rows, small tiles where large ones leave SMs idle, large ones where there are enough of them."""
+    plan = lambda M, N, K: kernels.linear_f32_plan(M, N, K, 148)
+    assert plan(1, 2304, 9216) == plan(16, 2304, 2304) == plan(1, 16, 16) == (1, 0)
+    assert plan(12, 100, 100) == (32, 0)                         # too short a K for streams
+    assert plan(8, 16, 16) == plan(300, 16, 16) == (0, 0)
+    assert plan(300, 64, 64) == plan(100, 2304, 256) == (32, 0)
+    assert plan(100, 256, 1024) == (32, 1)
+    assert plan(2048, 2304, 9216) == plan(300, 18432, 2304) == (64, 0)
+    assert plan(300, 2304, 9216) == (64, 1)

@@ -154,10 +154,24 @@ def test_linear_f32_kernels_and_cuts(M, N, K):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("M", [1, 8, 16, 31, 33, 64, 100])
+@pytest.mark.parametrize("N,K", [(5, 4), (128, 16), (130, 100), (257, 1540), (96, 3072)])
+def test_linear_f32_every_kernel_gives_the_same_bits(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N * K)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    ref = torch.empty(M, N, device=DEV)
+    kernels._linear_f32(x, w, ref, 0, 0)
+    segs = -(-K // kernels.F32_SEGMENT)
+    for kind, cut in [(k, c) for k in (1, 32, 64) for c in range(segs if k > 1 else 1) if k > 1 or M <= 16]:
+        out = torch.full((M, N), float("nan"), device=DEV)
+        kernels._linear_f32(x, w, out, kind, cut)
+        assert torch.equal(out, ref), (kind, cut)
+
+
 def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
     x = torch.zeros(300, 2305, device=DEV)[:, 1:]
     w, out = torch.zeros(2304, 2304, device=DEV), torch.empty(300, 2304, device=DEV)
-    assert kernels.linear_f32_cut(300, 2304, 2304, kernels.device_sms()) > 0
+    assert kernels.linear_f32_plan(300, 2304, 2304, kernels.device_sms())[1] > 0
     kernels.linear_f32(x, w, out)
     before = torch.cuda.memory_allocated()
     torch.cuda.reset_peak_memory_stats()
