@@ -417,12 +417,8 @@ template <int ROWS, int VJ>
 int launch(const F32Args& a, int batch, int max_q_len, cudaStream_t stream) {
     const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;
     const int smem = STAGES * STAGE + (ROWS * q_pitch + ROWS * P_PITCH + 4 * ROWS) * (int)sizeof(float) + 2 * SPAN * 8;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<ROWS, VJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        raised = true;
-    }
+    static OncePerDevice allowed;
+    if (const int e = allow_shared_memory(attn_f32_kernel<ROWS, VJ>, 112 * 1024, allowed)) return e;
     const int rows = max_q_len * a.group, tiles = (rows + ROWS - 1) / ROWS;
     int st = launch_pdl(attn_f32_kernel<ROWS, VJ>, dim3(tiles * (a.splits ? a.splits : 1), a.n_kv, batch), dim3(THREADS), smem,
                         stream, a);

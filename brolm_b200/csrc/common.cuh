@@ -9,6 +9,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "once_per_device.h"
+
 #define BROLM_API extern "C" __attribute__((visibility("default")))
 
 // Element type codes used across the C interface.
@@ -141,6 +143,15 @@ static inline int device_sm_count() {
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
     return sms;
+}
+
+// The kernel's limit of dynamic shared memory, once for each device; `done` is the caller's static.
+template <typename K>
+static inline int allow_shared_memory(K kernel, size_t bytes, OncePerDevice& done) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return (int)e;
+    return done.run(device, [&] { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 // Programmatic dependent launch.  A kernel launched through launch_pdl may begin

@@ -187,12 +187,8 @@ int launch_rows(const float* x, int ldx, const float* w, int ldw, float* y, int 
     int warps = fit < units ? fit : units;
     warps = (units + (units + warps - 1) / warps - 1) / ((units + warps - 1) / warps);
     const size_t smem = warps * queue + sums;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(rows_kernel<MP, RG, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        raised = true;
-    }
+    static OncePerDevice allowed;
+    if (const int e = allow_shared_memory(rows_kernel<MP, RG, R>, 227 * 1024, allowed)) return e;
     return launch_pdl(rows_kernel<MP, RG, R>, dim3((N + ROWS - 1) / ROWS), dim3(warps * 32), smem, stream, x, ldx, w, ldw, y, ldy, M, N, K);
 }
 
@@ -340,12 +336,8 @@ template <int BM>
 int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int ldy, int M, int N, int K, float* parts,
                  int seg_per_block, cudaStream_t stream) {
     constexpr int smem = STAGES * (BM + BN) * PITCH + BM * BN * (int)sizeof(float);
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(tiles_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-        raised = true;
-    }
+    static OncePerDevice allowed;
+    if (const int e = allow_shared_memory(tiles_kernel<BM>, smem, allowed)) return e;
     const int n_seg = (K + SEG - 1) / SEG;
     const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, parts ? (n_seg + seg_per_block - 1) / seg_per_block : 1);
     // Blocks that are let in early lie two on one SM and none on another, which costs where they do not fill all places:

@@ -54,7 +54,7 @@ LIBRARIES: dict[str, list[str]] = {
     "layernorm": ["layernorm.cu"],
     "delta_rule": ["delta_rule.cu"],
 }
-HEADERS = ["common.cuh", "attn_mma.cuh", "attn_decode_noalloc.h", "tcgen05.cuh"]
+HEADERS = ["common.cuh", "once_per_device.h", "attn_mma.cuh", "attn_decode_noalloc.h", "tcgen05.cuh"]
 
 _loaded: dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

@@ -2,9 +2,12 @@
 blocks share the keys of a sequence, into how many slices of K a product is
 cut, which product kernel takes which operands.  Pure arithmetic on shapes;
 no GPU."""
+import subprocess
+
 import torch
 
 from brolm_b200 import kernels
+from brolm_b200.kernels import build
 
 
 def test_decode_splits_make_one_wave_and_keep_two_pages_a_block():
@@ -130,3 +133,24 @@ def test_which_kernel_takes_a_float_product():
     assert plan(100, 256, 1024) == (32, 1)
     assert plan(2048, 2304, 9216) == plan(300, 18432, 2304) == (64, 0)
     assert plan(300, 2304, 9216) == (64, 1)
+
+
+def test_what_belongs_to_a_device_is_done_for_each(tmp_path):
+    """A limit raised on one device says nothing of another, and a call that failed is made again."""
+    (tmp_path / "t.cpp").write_text("""
+#include "once_per_device.h"
+#include <cstdio>
+#include <initializer_list>
+int main() {
+    OncePerDevice once;
+    int calls[70] = {}, failing = 1;
+    auto on = [&](int d) { return once.run(d, [&] { ++calls[d + 1]; return d == 3 ? failing : 0; }); };
+    int bad = 0;
+    for (int round = 0; round < 3; ++round)
+        for (int d : {0, 1, 63, 64, -1}) bad += on(d) != 0;
+    bad += on(3) != 1; failing = 0; bad += on(3) != 0; bad += on(3) != 0;
+    std::printf("%d %d %d %d %d %d", bad, calls[1], calls[2], calls[64], calls[65], calls[4]);
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-I", build.CSRC, "-o", str(tmp_path / "t"), str(tmp_path / "t.cpp")], check=True)
+    assert subprocess.run([str(tmp_path / "t")], capture_output=True, text=True, check=True).stdout == "0 1 1 1 3 2"
