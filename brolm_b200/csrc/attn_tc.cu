@@ -32,7 +32,14 @@
 // The reference maximum of a row is only raised when the tile's maximum exceeds
 // it by more than 8 (in log2 units): probabilities then stay below 2^8, and the
 // accumulator in tensor memory has to be rescaled (read, multiply, write back)
-// only on those rare tiles instead of on every tile.  Scores, statistics and
+// only on those rare tiles instead of on every tile.  Where a few keys lead, that
+// costs precision: the leading probability, exactly 1 under the row's own maximum,
+// is then some number below 2^8 that bfloat16 rounds.  TIGHT launches raise the
+// reference to every new maximum and sum the probabilities as they were rounded;
+// they serve the layers whose prompts ran on the mma.sync kernel before, which
+// keeps the running maximum (error against 64 bits, 128 entries, scores of deviation
+// 3 under a cap of 30, 2,048 keys: 0.67e-3 on mma.sync, 1.37e-3 with the gap, TIGHT
+// 0.67e-3, before the result is rounded).  Scores, statistics and
 // the accumulator are float (wlejon/brolm src/gemma2.cpp:360-367 for the order:
 // scale, cap * tanh(s / cap), mask, softmax).  Key j is visible from position p
 // iff 0 <= p - j < window.
@@ -110,7 +117,7 @@ struct Shape {
 enum : int { Q_FULL = 0, S_FULL = 1, P_FULL = 3, PV_DONE = 5, U_FULL = 7, U_EMPTY = U_FULL + MAX_SLOTS,
              N_BARS = U_EMPTY + MAX_SLOTS };
 
-template <int HD>
+template <int HD, bool TIGHT>
 __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                      const __grid_constant__ CUtensorMap map_k,
                                                                      const __grid_constant__ CUtensorMap map_v, TcArgs a) {
@@ -352,13 +359,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
             // may go over the partner's score columns
             asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
             m_t = fmaxf(m_t, xch[(s * 2 + (half ^ 1)) * BM + r]);
-            // raise the reference only when the tile goes well beyond it
-            const bool raise = m_t > m_ref + RESCALE_GAP;       // also true for the first visible tile of a row
+            // raise the reference only when the tile goes well beyond it (TIGHT: beyond it)
+            const bool raise = m_t > m_ref + (TIGHT ? 0.0f : RESCALE_GAP);       // also true for the first visible tile of a row
             const float m_new = raise ? m_t : m_ref;
             const float corr = (raise && m_ref > -INFINITY) ? fast_exp2(m_ref - m_new) : 1.0f;
 
             if (j > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
-                // rare: the accumulator has to be at rest (the product of the tile before is done), then every
+                // rare but for TIGHT: the accumulator has to be at rest (the product of the tile before is done), then every
                 // row of the warp is rescaled (rows that keep their reference multiply by 1); each warp of the
                 // pair takes half of the head size
                 ok = wait_on(bar(PV_DONE + (s ^ 1)), ((j - 1) >> 1) & 1, give_up, 12);
@@ -383,9 +390,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
 #pragma unroll
             for (int c = 0; c < W / 2; ++c) {
                 const float p0 = fast_exp2(sc[2 * c] - m_sub), p1 = fast_exp2(sc[2 * c + 1] - m_sub);
-                sum += p0 + p1;
                 __nv_bfloat162 t = __floats2bfloat162_rn(p0, p1);
                 pw[c] = *reinterpret_cast<uint32_t*>(&t);
+                if constexpr (TIGHT) sum += __uint_as_float(pw[c] << 16) + __uint_as_float(pw[c] & 0xffff0000u);
+                else sum += p0 + p1;
             }
             l += sum;
             tmem_st32(tmem + lane_addr + S_COL + s * BN + half * (W / 2), pw);
@@ -529,19 +537,25 @@ int make_map(CUtensorMap* map, const void* ptr, long long tokens, int heads, int
     return make_map_bf16(map, ptr, 3, dims, strides, box);
 }
 
-template <int HD>
-int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const TcArgs& a, dim3 grid,
-           cudaStream_t stream) {
+template <int HD, bool TIGHT>
+int launch_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const TcArgs& a, dim3 grid,
+              cudaStream_t stream) {
     using SH = Shape<HD>;
     constexpr size_t smem = (size_t)SH::Q_BYTES + (size_t)SH::SLOTS * SH::SLOT + N_BARS * 8 + 32 + 4 * BM * 4;
     static_assert(smem <= 232448, "shared memory of a block");
     static bool raised = false;
     if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, TIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         raised = true;
     }
-    return launch_pdl(attn_prefill_tc_kernel<HD>, grid, dim3(THREADS), smem, stream, mq, mk, mv, a);
+    return launch_pdl(attn_prefill_tc_kernel<HD, TIGHT>, grid, dim3(THREADS), smem, stream, mq, mk, mv, a);
+}
+
+template <int HD>
+int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const TcArgs& a, dim3 grid, bool tight,
+           cudaStream_t stream) {
+    return tight ? launch_as<HD, true>(mq, mk, mv, a, grid, stream) : launch_as<HD, false>(mq, mk, mv, a, grid, stream);
 }
 
 }  // namespace
@@ -614,11 +628,12 @@ BROLM_API int brolm_attn_prefill_tc_plan(int max_q_len, int n_kv, int group, int
 // rows of q_stride / kv_stride elements (token major; head h at h * hd).  v_lbo and v_sbo are the two
 // strides of the value operand's shared-memory descriptor in bytes (0: the defaults).  n_split > 0: the
 // heaviest n_split row blocks run as two halves of their keys; part_o holds n_split * n_kv * batch * 2 *
-// 128 * hd floats, part_ml n_split * n_kv * batch * 2 * 128 * 2 (n_split * n_kv * batch <= 1024).
+// 128 * hd floats, part_ml n_split * n_kv * batch * 2 * 128 * 2 (n_split * n_kv * batch <= 1024).  tight: the
+// reference is every row's running maximum, and the sum that of the rounded probabilities.
 BROLM_API int brolm_attn_prefill_tc(const void* q, int q_stride, void* out, int out_stride, const void* cu_q,
                                     const void* k, const void* v, int kv_stride, int total_tokens, int n_kv, int group,
                                     int hd, float scale, float cap, int window, int batch, int max_q_len, int v_lbo,
-                                    int v_sbo, int n_split, void* part_o, void* part_ml, cudaStream_t stream) {
+                                    int v_sbo, int n_split, void* part_o, void* part_ml, int tight, cudaStream_t stream) {
     if (batch <= 0 || max_q_len <= 0) return BROLM_OK;
     if (hd != 64 && hd != 128 && hd != 256) return BROLM_ERR_BAD_SIZE;
     if (group <= 0 || BM % group != 0 || n_kv <= 0 || batch > 65535 || n_kv > 65535) return BROLM_ERR_BAD_SIZE;
@@ -641,9 +656,9 @@ BROLM_API int brolm_attn_prefill_tc(const void* q, int q_stride, void* out, int 
     a.v_sbo = (uint32_t)((v_sbo > 0 ? v_sbo : 1024) >> 4);          // next eight keys
     a.n_split = n_split; a.part_o = (float*)part_o; a.part_ml = (float*)part_ml;
     dim3 grid(row_tiles + n_split, n_kv, batch);
-    if (hd == 64) return launch<64>(mq, mk, mv, a, grid, stream);
-    if (hd == 128) return launch<128>(mq, mk, mv, a, grid, stream);
-    return launch<256>(mq, mk, mv, a, grid, stream);
+    if (hd == 64) return launch<64>(mq, mk, mv, a, grid, tight != 0, stream);
+    if (hd == 128) return launch<128>(mq, mk, mv, a, grid, tight != 0, stream);
+    return launch<256>(mq, mk, mv, a, grid, tight != 0, stream);
 }
 
 BROLM_API int brolm_attn_tc_status(int reset) {

@@ -1747,10 +1747,13 @@ _split_memo: dict = {}
 
 def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *,
                          n_kv: int, group: int, head_dim: int, scale: float, cap: float, window: int, batch: int,
-                         max_q_len: int, v_lbo: int = 0, v_sbo: int = 0, n_split: Optional[int] = None) -> None:
+                         max_q_len: int, v_lbo: int = 0, v_sbo: int = 0, n_split: Optional[int] = None,
+                         tight: bool = False) -> None:
     """tcgen05 attention of whole prompts that start at position 0 (bfloat16; head_dim 64, 128 or 256).
     ``n_split``: how many of the heaviest row blocks run as two halves of their keys, merged by the half
-    that finishes second (None: ``attention_prefill_tc_split`` decides)."""
+    that finishes second (None: ``attention_prefill_tc_split`` decides).  ``tight``: probabilities under the
+    row's running maximum, and the sum of those as they were rounded: as precise as ``attention_prefill_mma``
+    or better, for a little more time."""
     assert q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and k.dtype == torch.bfloat16
     assert q.stride(-1) == 1 and out.stride(-1) == 1 and k.stride(-1) == 1 and v.stride(-1) == 1
     assert k.stride(0) == v.stride(0) and cu_q.dtype == torch.int32 and q.shape[0] == k.shape[0] == v.shape[0]
@@ -1763,10 +1766,10 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor,
         part_o, part_ml = both[:pairs * 2 * 128 * head_dim], both[pairs * 2 * 128 * head_dim:]
     f = _fn("attn_tc", "brolm_attn_prefill_tc", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                                  c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int,
-                                                 c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
+                                                 c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p])
     _check(f(_ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(cu_q), _ptr(k), _ptr(v), k.stride(0), q.shape[0],
              n_kv, group, head_dim, scale, cap, window, batch, max_q_len, v_lbo, v_sbo, n_split, _ptr(part_o),
-             _ptr(part_ml), _stream()),
+             _ptr(part_ml), 1 if tight else 0, _stream()),
            "attention_prefill_tc")
 
 

@@ -419,7 +419,7 @@ class Attention(Part):
             # cap, 16 heads on 4 kv heads of 128 entries, one sequence of 37 / 256 / 2048 / 4096 tokens: 9.7 / 20.6 /
             # 131.8 / 409.6 us on the mma.sync kernel, 7.1 / 9.4 / 44.3 / 149.7 us on the tcgen05 one)
             if ctx.mode == "prefill":
-                self.attend_packed(q, k, v, out, ctx, common)
+                self.attend_packed(q, k, v, out, ctx, common, tight=scored)
             else:
                 self.attend_paged(q, out, ctx, common, k_pages, v_pages, table, ring, page)
         else:
@@ -479,9 +479,9 @@ class Attention(Part):
     def _tensor_cores(self, ctx) -> bool:
         return ctx.dtype == torch.bfloat16 and self.head_dim <= 256 and self.n_q // self.n_kv <= 16
 
-    def attend_packed(self, q, k, v, out, ctx, common):
+    def attend_packed(self, q, k, v, out, ctx, common, tight=False):
         if self._tensor_cores(ctx) and kernels.attention_prefill_tc_ok(self.head_dim, self.n_q // self.n_kv):
-            kernels.attention_prefill_tc(q, out, ctx.cu_q, k, v, **common)         # tcgen05, scores in tensor memory
+            kernels.attention_prefill_tc(q, out, ctx.cu_q, k, v, tight=tight, **common)         # tcgen05, scores in tensor memory
         elif self._tensor_cores(ctx):
             kernels.attention_prefill_mma(q, out, ctx.cu_q, k, v, **common)
         else:

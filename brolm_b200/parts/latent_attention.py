@@ -166,7 +166,7 @@ class LatentAttention(Part):
             if tensor_cores and self.sink is None and kernels.attention_prefill_tc_ok(D, H):
                 # all heads on one row that is key and value: 16 heads, rows of 256, window 1024, one sequence of 37 /
                 # 256 / 2048 / 4096 tokens: 8.5 / 9.9 / 41.2 / 80.9 us here, 13.4 / 24.7 / 141.8 / 276.6 us on mma.sync
-                kernels.attention_prefill_tc(q, out, ctx.cu_q, lat, lat, max_q_len=ctx.max_q_len,
+                kernels.attention_prefill_tc(q, out, ctx.cu_q, lat, lat, max_q_len=ctx.max_q_len, tight=True,
                                              **{n: a for n, a in common.items() if n != "sink"})
             elif tensor_cores:
                 kernels.attention_prefill_mma(q, out, ctx.cu_q, lat, lat, max_q_len=ctx.max_q_len, **common)

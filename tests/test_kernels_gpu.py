@@ -540,6 +540,43 @@ def test_attention_tc_keeps_broken_values_of_the_next_sequence_out(hd, n_q, n_kv
     assert torch.equal(run(qkv, [first, 90])[:first], alone)
 
 
+@pytest.mark.parametrize("hd,n_q,n_kv", [(64, 4, 2), (128, 16, 4), (256, 16, 1)])
+@pytest.mark.parametrize("cap,gain", [(0.0, 0.3), (30.0, 1.0), (30.0, 3.0), (50.0, 5.0)])
+def test_attention_tc_tight_is_as_precise_as_mma(hd, n_q, n_kv, cap, gain):
+    """Scores of deviation ``gain``, from flat to a few leading keys: the error against 64 bits of the whole result, over
+    some 10^6 entries, is that of the mma.sync kernel (whose tiles are half as wide) but for one part in a hundred."""
+    g = torch.Generator().manual_seed(hd + int(10 * gain))
+    lengths = [900, 389, 64]
+    T = sum(lengths)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * hd, generator=g).to(torch.bfloat16)
+    dq = qkv.to(DEV)
+    cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device=DEV)
+    k_at, v_at = n_q * hd, (n_q + n_kv) * hd
+    kw = dict(n_kv=n_kv, group=n_q // n_kv, head_dim=hd, scale=gain * hd ** -0.5, cap=cap, window=0, batch=len(lengths),
+              max_q_len=max(lengths))
+    ref = torch.empty(T, k_at, dtype=torch.float64, device=DEV)
+    for b, n in enumerate(lengths):
+        at = sum(lengths[:b])
+        rows = dq[at:at + n].double()
+        heads = lambda part, count: part.view(n, count, hd).transpose(0, 1)
+        q, k, v = heads(rows[:, :k_at], n_q), heads(rows[:, k_at:v_at], n_kv), heads(rows[:, v_at:], n_kv)
+        k, v = (t.repeat_interleave(n_q // n_kv, 0) for t in (k, v))
+        s = q @ k.transpose(1, 2) * kw["scale"]
+        s = cap * torch.tanh(s / cap) if cap else s
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), -torch.inf)
+        ref[at:at + n] = (torch.softmax(s, -1) @ v).transpose(0, 1).reshape(n, k_at)
+
+    def error(kernel, **more):
+        out = torch.empty(T, k_at, dtype=torch.bfloat16, device=DEV)
+        kernel(dq[:, :k_at], out, cu, dq[:, k_at:v_at], dq[:, v_at:], **kw, **more)
+        return float((out.double() - ref).norm() / ref.norm())
+
+    mma = error(kernels.attention_prefill_mma)
+    for n_split in (0, 5):
+        assert error(kernels.attention_prefill_tc, tight=True, n_split=n_split) <= 1.01 * mma
+    assert kernels.attention_tc_status() == 0
+
+
 @pytest.mark.parametrize("n_q,n_kv,hd,window,cap,gain", [(8, 4, 256, 0, 50.0, 40.0), (4, 2, 64, 100, 30.0, 25.0),
                                                          (4, 4, 128, 0, 20.0, 200.0)])
 def test_attention_tc_scores_beyond_the_cap(n_q, n_kv, hd, window, cap, gain):

@@ -13,6 +13,7 @@ import pytest
 import torch
 
 import brolm_b200 as bb
+from brolm_b200 import kernels
 from tests.papusun_helpers import make_folder, oracle_inputs, random_prompts
 from tests.plain import papusun_plain as plain
 
@@ -313,3 +314,14 @@ def test_captured_steps_run_the_two_mixers_as_branches(setups, batch):
     plainly = run(bb.Engine(model, max_tokens=128 * batch, max_slots=batch, use_graphs=False))
     # other cuts of the keys and other products by the padded batch: what bfloat16 leaves of a logit, as the oracle bounds it
     assert float((first - plainly).abs().max()) <= 2 * ROUNDING["S"][1] * float(plainly.abs().max())
+
+
+def test_prompts_on_the_tcgen05_kernel_keep_the_precision_of_mma(setups, monkeypatch):
+    """Layers of one latent row ran on the mma.sync kernel before: on the tcgen05 one they ask for its precision."""
+    _, config, _, model = setups[("U", "bfloat16")]               # rows of 64 in its first two latent layers
+    asked = []
+    real = kernels.attention_prefill_tc
+    monkeypatch.setattr(kernels, "attention_prefill_tc", lambda *a, **kw: (asked.append(kw.get("tight", False)), real(*a, **kw)))
+    eng = bb.Engine(model, max_tokens=128, max_slots=1)
+    eng.step(eng.open(1), random_prompts(config["vocab"], [70], seed=1))
+    assert len(asked) >= 2 and all(asked)
