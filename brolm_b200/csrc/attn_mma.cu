@@ -30,13 +30,14 @@ BROLM_API int brolm_attn_prefill_mma(const void* q, int q_stride, void* out, int
 
 // One query token per sequence (row cu_q[b] of q) over the paged cache.  The page size is
 // 64 keys.  group <= 16.  With n_splits > 1, part_o holds batch * n_q * n_splits * hd floats
-// and part_ml batch * n_q * n_splits * 2 floats of scratch.
+// and part_ml batch * n_q * n_splits * 2 floats of scratch.  longest_first: the sequences' lengths are far from
+// equal, and their blocks start in order of falling length where there is more than one round of them.
 BROLM_API int brolm_attn_decode_mma(const void* q, int q_stride, void* out, int out_stride, const void* cu_q,
                                     const void* kv_len, const void* k_pages, const void* v_pages,
                                     const void* page_table, int pt_stride, int ring, int page_size, int n_kv,
                                     int group, int hd, float scale, float cap, int window, const void* sink,
                                     int batch, int n_splits, void* part_o, void* part_ml, int chunk,
-                                    const void* dist_bias, int dist_len, cudaStream_t stream) {
+                                    const void* dist_bias, int dist_len, int longest_first, cudaStream_t stream) {
     if (batch <= 0) return BROLM_OK;
     int st = check_common(hd, group, n_kv, q_stride, out_stride, batch);
     if (st) return st;
@@ -51,7 +52,7 @@ BROLM_API int brolm_attn_decode_mma(const void* q, int q_stride, void* out, int 
     a.pt_stride = pt_stride; a.ring = ring;
     a.n_kv = n_kv; a.group = group; a.hd = hd; a.scale = scale; a.cap = cap; a.window = window; a.chunk = chunk;
     a.n_splits = n_splits; a.part_o = (float*)part_o; a.part_ml = (float*)part_ml;
-    a.sink = (const float*)sink; a.shared_kv = k_pages == v_pages;
+    a.sink = (const float*)sink; a.shared_kv = k_pages == v_pages; a.by_length = longest_first;
     if (dist_bias && dist_len <= 0) return BROLM_ERR_BAD_SIZE;
     a.dist_bias = (const float*)dist_bias; a.dist_len = dist_bias ? dist_len : 0;
     if (hd == 64) return launch_decode<64, true>(a, batch, stream);

@@ -108,7 +108,9 @@ struct MmaArgs {
     float* part_o;          // [B][n_q][n_splits][hd]
     float* part_ml;         // [B][n_q][n_splits][2]  (max in log2 units, sum)
     int merge_here;         // decoding: the last block of a (sequence, kv head) merges the splits itself
-    int by_length;            // decode: blocks take the sequences in order of falling length
+    int by_length;            // decode: blocks take the sequences in order of falling length.  In several rounds of blocks those
+                              // of the longest then start first, and the last round is made of short runs (16 sequences of
+                              // 128 to 6,144 keys, 8 kv heads of 256 entries, 4 splits: 85.6 -> 67.0 us)
     const float* sink;      // [n_q] or null: exp(sink[head]) joins the softmax's denominator, with no value
     int shared_kv;          // decoding: the values are the keys' rows themselves (one tile serves both)
     // a learned bias by distance, or null: [n_q][dist_len] floats, of which key j adds entry
@@ -359,6 +361,32 @@ constexpr int SLOTS = 3;
 template <bool APART> __host__ __device__ constexpr size_t decode_slot(int hd) { return (APART ? 1 : 2) * (size_t)KT * hd * 2; }
 constexpr int PT_ROW = 512;          // entries of a page-table row kept in shared memory (32768 keys)
 
+// The sequence of place `rank` when n <= MAX_BY_LENGTH sequences stand in order of falling length, equal ones in their own:
+// the largest bound that more than `rank` of them reach is that sequence's (length, place from behind), found bit by bit
+// by each warp for itself.  (Counting, for every sequence, those ahead of it took a block of 512 some 10 us.)
+constexpr int MAX_BY_LENGTH = 512;
+__device__ __forceinline__ int by_falling_length(const int* kv_len, int n, int rank) {
+    const int lane = threadIdx.x & 31;
+    uint32_t key[MAX_BY_LENGTH / 32], most = 0;
+#pragma unroll
+    for (int j = 0; j < MAX_BY_LENGTH / 32; ++j) {
+        const int i = j * 32 + lane;
+        key[j] = i < n ? (uint32_t)min(max(kv_len[i], 0), (1 << 22) - 1) * MAX_BY_LENGTH + (MAX_BY_LENGTH - 1 - i) : 0u;
+        most = max(most, key[j]);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    uint32_t bound = 0;
+    for (int bit = 31 - __clz(most | 1); bit >= 0; --bit) {
+        const uint32_t next = bound | (1u << bit);
+        int reach = 0;
+#pragma unroll
+        for (int j = 0; j < MAX_BY_LENGTH / 32; ++j)
+            if (j * 32 < n) reach += key[j] >= next;
+        if (__reduce_add_sync(0xffffffffu, reach) > rank) bound = next;
+    }
+    return MAX_BY_LENGTH - 1 - (int)(bound % MAX_BY_LENGTH);
+}
+
 template <int HD_MAX, bool EXACT, bool BIAS, bool APART>
 __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -374,23 +402,7 @@ __global__ void __launch_bounds__(NTHREADS) attn_decode_mma_kernel(MmaArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ int pt_row[PT_ROW];
     int b = blockIdx.z;
-    if (a.by_length) {
-        // several rounds of blocks: those of the longest sequences start first (equal ones in their order), so that
-        // the last round is made of short runs.  (16 sequences of 128 to 6,144 keys, 8 kv heads of 256 entries, 4 splits:
-        // 85.6 -> 67.0 us)
-        const int n = gridDim.z;
-        for (int i = threadIdx.x; i < n; i += NTHREADS) pt_row[i] = a.kv_len[i];
-        __syncthreads();
-        __shared__ int mine;
-        for (int i = threadIdx.x; i < n; i += NTHREADS) {
-            const int len = pt_row[i];
-            int rank = 0;
-            for (int j = 0; j < n; ++j) rank += pt_row[j] > len || (pt_row[j] == len && j < i);
-            if (rank == b) mine = i;
-        }
-        __syncthreads();
-        b = mine;
-    }
+    if (a.by_length) b = by_falling_length(a.kv_len, gridDim.z, b);
     // The sequence's length and its row of the page table were written by the host before the step's
     // first kernel: they are fetched together, ahead of the wait, so that the first tile's address
     // does not take two more round trips to the L2 after it.
@@ -831,7 +843,7 @@ int launch_decode_as(const MmaArgs& a, int batch, cudaStream_t stream) {
     MmaArgs b = a;
     b.merge_here = a.n_splits > 1 && a.n_splits <= MAX_MERGED_SPLITS && (long long)batch * a.n_kv <= MAX_TICKETS &&
                    (size_t)(a.group * a.n_splits + a.group) * sizeof(float) <= smem - 16 * a.hd * sizeof(bf16);
-    b.by_length = batch > 1 && batch <= PT_ROW && (long long)a.n_splits * a.n_kv * batch > 2LL * device_sm_count();
+    b.by_length = a.by_length && batch > 1 && batch <= MAX_BY_LENGTH && (long long)a.n_splits * a.n_kv * batch > 2LL * device_sm_count();
     int st = launch_pdl(attn_decode_mma_kernel<HD_MAX, EXACT, BIAS, APART>, grid, dim3(NTHREADS), smem, stream, b);
     if (st != 0 || a.n_splits == 1 || b.merge_here) return st;
     dim3 cgrid(a.n_kv * a.group, batch);

@@ -341,7 +341,7 @@ class Attention(Part):
                                            ragged=getattr(ctx, "ragged", False),
                                            per_sm=kernels.decode_blocks_per_sm(self.head_dim))
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring, page_size=page,
-                                         n_splits=splits, **{n: a for n, a in common.items() if n not in ("v_dim", "max_q_len")})
+                                         n_splits=splits, longest_first=self._longest_first(ctx, splits), **{n: a for n, a in common.items() if n not in ("v_dim", "max_q_len")})
         else:
             kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table,
                                    ring=ring, page_size=page, **common)
@@ -412,7 +412,7 @@ class Attention(Part):
                                                ragged=getattr(ctx, "ragged", False),
                                                per_sm=kernels.decode_blocks_per_sm(self.head_dim))
                 kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
-                                             page_size=page, n_splits=splits, **more,
+                                             page_size=page, n_splits=splits, longest_first=self._longest_first(ctx, splits), **more,
                                              **{n: a for n, a in common.items() if n != "max_q_len"})
         elif not special and same_size and (not scored or (plain and ctx.mode == "prefill")):
             # nothing the tensor-core kernels do not know: the same attention as a plain layer's.  (A prompt with a
@@ -479,6 +479,11 @@ class Attention(Part):
     def _tensor_cores(self, ctx) -> bool:
         return ctx.dtype == torch.bfloat16 and self.head_dim <= 256 and self.n_q // self.n_kv <= 16
 
+    def _longest_first(self, ctx, splits: int) -> bool:
+        span = min(self.window or (1 << 30), self.chunk or (1 << 30))
+        return kernels.decode_longest_first(getattr(ctx, "ragged", False), splits, ctx.max_kv_len, span if span < (1 << 30) else 0,
+                                            self.head_dim)
+
     def attend_packed(self, q, k, v, out, ctx, common, tight=False):
         if self._tensor_cores(ctx) and kernels.attention_prefill_tc_ok(self.head_dim, self.n_q // self.n_kv):
             kernels.attention_prefill_tc(q, out, ctx.cu_q, k, v, tight=tight, **common)         # tcgen05, scores in tensor memory
@@ -494,7 +499,7 @@ class Attention(Part):
                                            ragged=getattr(ctx, "ragged", False),
                                            per_sm=kernels.decode_blocks_per_sm(self.head_dim))
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
-                                         page_size=page, n_splits=splits, **args)
+                                         page_size=page, n_splits=splits, longest_first=self._longest_first(ctx, splits), **args)
         else:
             kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table,
                                    ring=ring, page_size=page, **common)

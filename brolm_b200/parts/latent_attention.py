@@ -181,7 +181,9 @@ class LatentAttention(Part):
                 # round trip, and with all heads on one cached row a split is cheap to run and dear to merge
                 splits = min(splits, 4)
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, pages, pages, table, ring=ring, page_size=page,
-                                         n_splits=splits, **common)
+                                         n_splits=splits, **common,
+                                         longest_first=kernels.decode_longest_first(getattr(ctx, "ragged", False), splits,
+                                                                                    ctx.max_kv_len, self.window or 0, D))
         else:
             if ctx.mode == "prefill" and self.window and ctx.max_kv_len > ring:
                 raise NotImplementedError("a layer that reads another layer's windowed cache cannot take a "

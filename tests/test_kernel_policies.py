@@ -154,3 +154,12 @@ int main() {
 """)
     subprocess.run(["g++", "-std=c++17", "-I", build.CSRC, "-o", str(tmp_path / "t"), str(tmp_path / "t.cpp")], check=True)
     assert subprocess.run([str(tmp_path / "t")], capture_output=True, text=True, check=True).stdout == "0 1 1 1 3 2"
+
+
+def test_decode_blocks_start_by_length_only_where_runs_are_long():
+    first = kernels.decode_longest_first
+    assert not first(False, 1, 8192, 0, 256)                                      # equal lengths keep their own order
+    assert first(True, 5, 8192, 0, 256) and first(True, 2, 1024, 0, 256)
+    assert not first(True, 6, 1024, 0, 256) and not first(True, 1, 256, 0, 256)
+    assert not first(True, 1, 8192, 64, 256) and first(True, 1, 8192, 4096, 256)  # a window bounds a run, too
+    assert not first(True, 2, 1024, 0, 128) and first(True, 2, 4096, 0, 128)

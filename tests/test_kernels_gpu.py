@@ -916,11 +916,12 @@ def test_float_attention_gives_the_same_bits_however_it_is_cut(monkeypatch, opti
 
 @pytest.mark.parametrize("options", ["plain", "sink", "bias", "one row"])
 @pytest.mark.parametrize("hd,n_kv,splits", [(256, 4, 2), (144, 2, 4), (64, 4, 3)])
-def test_decode_attention_gives_the_same_bits_whatever_runs_beside_it(options, hd, n_kv, splits):
+@pytest.mark.parametrize("batch,longest_first", [(98, True), (98, False), (512, True), (513, True)])
+def test_decode_attention_gives_the_same_bits_whatever_runs_beside_it(options, hd, n_kv, splits, batch, longest_first):
     """More blocks than two rounds hold (two blocks to an SM with large heads, the longest sequences first) against every
     sequence alone (a block to an SM): unequal and equal lengths, one key, a page's edges, padding rows in between."""
     g = torch.Generator(device=DEV).manual_seed(hd + splits)
-    lengths = [0, 1, 64, 65, 700, 128, 0, 129, 63, 64] + [1 + 37 * i % 500 for i in range(88)]
+    lengths = [0, 1, 64, 65, 700, 128, 0, 129, 63, 64] + [1 + 37 * i % 500 for i in range(batch - 10)]
     B, group, W = len(lengths), 2, 11
     assert splits * n_kv * B > 2 * kernels.device_sms(DEV)
     pages = torch.randn(B * W, n_kv, 64, hd, generator=g, device=DEV).to(torch.bfloat16)
@@ -935,8 +936,8 @@ def test_decode_attention_gives_the_same_bits_whatever_runs_beside_it(options, h
     i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
     out = torch.full_like(q, 7.0)
     kernels.attention_decode_mma(q, out, torch.arange(B + 1, dtype=torch.int32, device=DEV), i32(*lengths), pages, values, table,
-                                 batch=B, **kw)
-    for b in range(B):
+                                 batch=B, longest_first=longest_first, **kw)
+    for b in range(B) if batch < 100 else range(0, B, 17):
         one = torch.full_like(q[b:b + 1], 7.0)
         kernels.attention_decode_mma(q[b:b + 1], one, i32(0, 1), i32(lengths[b]), pages, values, table[b:b + 1], batch=1, **kw)
         assert torch.equal(out[b], one[0]), (b, lengths[b])
