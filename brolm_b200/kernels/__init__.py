@@ -1809,8 +1809,15 @@ def decode_splits(batch: int, n_kv: int, max_kv_len: int, window: int, sms: Opti
     were measured too: 111 to 113 us, no better than equal shares, and are not in the kernel.)
 
     ``per_sm``: so many blocks share an SM (``decode_blocks_per_sm``), and one wave is as many times the SMs, if the keys
-    give well more blocks than SMs: 8 sequences of 8,190 keys on 4 kv heads of 256 entries 49.4 us in 4 splits and 46.3
-    in 9, 16 of 1,280 keys 19.7 in 2 and 18.8 in 4; one sequence of 8,190 keys 14.1 in 37 and 17.5 in 40 (160 blocks).
+    give well more blocks than SMs.  It is the better way where one block an SM leaves a tenth of the SMs idle, or does not
+    cut at all, and the runs stay long enough; a kv head of 256 entries, one wave / per SM:
+      128 of 148 SMs busy: 32 pairs of 1,500 keys 14.0 in 4 splits / 14.6 us in 9 (3.6 pages a block under the bound of
+      2,048), of 3,000 22.2 / 22.0 (7.1), of 8,190 49.5 / 46.1; 64 pairs of 520 12.2 in 2 / 13.0 in 4 (4), of 1,500 22.3 /
+      21.0 (8); 128 pairs of 520 keys 16.4 whole / 18.2 in 2 (8), of 1,500 36.8 / 35.5 (16);
+      120 busy: 40 pairs of 520 keys 9.5 in 3 / 10.7 in 7 (2.3), of 2,000 20.6 / 19.2 (4.6); 112: 56 of 1,500 22.0 in 2 / 19.4
+      in 5; 80 and 96: 80 pairs of 520 keys 15.4 whole / 13.4 in 3 (5.3), 96 of 8,190 178 / 116;
+      144 busy: 36 pairs of 520, 1,030 and 8,190 keys 9.3 / 10.7, 12.7 / 13.7 and 50.3 / 49.3; 144 of 1,500 and 8,190 keys 37.2
+      / 37.6 and 178.6 / 169.9.
     With the blocks of the longest sequences first, about two waves are enough for ragged batches.  A decode step by
     1.4 / 1.75 / 2.2 / 2.6 / 3.5 waves: 9B sizes, 16 sequences of 128 to 6,144 tokens 7,419 / 7,179 / 7,252 / 7,291 / 7,367
     us; 2B, 24 of 100 to 4,000 3,201 / 2,932 / 2,786 / 2,834 / 2,916 us; 50 of 300 to 1,700 3,440 / 2,884 / 2,786 / 2,856 /
@@ -1823,8 +1830,12 @@ def decode_splits(batch: int, n_kv: int, max_kv_len: int, window: int, sms: Opti
     most = min((tiles + 1) // 2, 40)
     pairs = max(1, batch * n_kv)
     want = max(1, sms // pairs)
-    if per_sm > 1 and min(per_sm * sms // pairs, most) * pairs > 1.5 * sms:
-        want = per_sm * sms // pairs
+    shared = min(per_sm * sms // pairs, most)
+    busy = want * pairs / sms
+    if per_sm > 1 and shared * pairs > 1.5 * sms and (busy < 0.9 or want == 1):
+        pages = (3 if busy <= 0.7 else 16 if busy < 0.9 else 32) if want == 1 else 4.5 if busy > 0.8 else 3
+        if tiles >= pages * shared:
+            want = shared
     if ragged and per_sm > 1:
         want = max(want, int(RAGGED_WAVES_SHARED * per_sm * sms / pairs))
     elif ragged:

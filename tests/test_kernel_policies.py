@@ -90,6 +90,12 @@ def test_decode_splits_where_two_blocks_share_an_sm():
     assert kernels.decode_splits(8, 4, 8192, 0, **two) == 9                       # 288 blocks for 296 places
     assert kernels.decode_splits(1, 4, 8192, 0, **two) == 37                      # 40 would be little more than one round
     assert kernels.decode_splits(64, 4, 2048, 0, **two) == 1
+    assert kernels.decode_splits(8, 4, 2048, 0, **two) == 4                       # nine would be runs of three or four pages
+    assert kernels.decode_splits(8, 4, 4096, 0, **two) == 9
+    assert kernels.decode_splits(12, 4, 8192, 0, **two) == 3                      # 144 blocks keep all SMs busy
+    assert kernels.decode_splits(16, 8, 1024, 0, **two) == 1 and kernels.decode_splits(16, 8, 2048, 0, **two) == 2
+    assert kernels.decode_splits(12, 8, 1024, 0, **two) == 3                      # 96 of 148 SMs busy
+    assert kernels.decode_splits(36, 4, 8192, 0, **two) == 2 and kernels.decode_splits(36, 4, 2048, 0, **two) == 1
     assert kernels.decode_splits(16, 8, 8192, 0, ragged=True, **two) == 5
     assert kernels.decode_splits(3, 4, 700, 0, **two) == kernels.decode_splits(3, 4, 700, 0, sms=148)
     for batch in (1, 2, 3, 5, 8, 13, 16, 30, 64):
