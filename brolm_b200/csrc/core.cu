@@ -874,3 +874,13 @@ BROLM_API int brolm_softcap(const void* x, int dtype, void* out, long long n, fl
                           cap, mul);
     return BROLM_ERR_BAD_DTYPE;
 }
+
+// ---------------------------------------------------------------------------
+// A stream that belongs to nobody else (a framework's streams come from a pool that the whole process shares).
+// ---------------------------------------------------------------------------
+BROLM_API int brolm_stream_create(void** stream) {
+    cudaStream_t made = nullptr;
+    const cudaError_t e = cudaStreamCreateWithFlags(&made, cudaStreamNonBlocking);
+    *stream = made;
+    return (int)e;
+}

@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import dataclasses
 import gc
+import weakref
 from typing import Optional, Sequence
 
 import numpy as np
@@ -97,7 +98,8 @@ class _DecodeGraph:
         self.ctx = StepContext(
             mode="decode", dtype=engine.model.dtype, device=dev, cache=cache, batch=rows, n_tokens=rows, slots=[],
             positions=seg[1], tok_seq=ar[:rows].clone(), cu_q=ar, kv_len=seg[2], slots_dev=seg[3], max_q_len=1,
-            page_tables=tables, cache_rows=cache_rows, host_lengths=[], max_kv_len=kv_cap, ragged=ragged)
+            page_tables=tables, cache_rows=cache_rows, host_lengths=[], max_kv_len=kv_cap, ragged=ragged,
+            beside=engine.beside)
         self.all_rows = ar[:rows].clone()
         # an all-padding state: the warm-up pass touches no cache
         self.hv[:] = 0
@@ -196,6 +198,12 @@ class Engine:
         self._graphs: dict[tuple, _DecodeGraph] = {}
         self._graphs_generation = model.generation
         self._graph_pool = torch.cuda.graph_pool_handle() if self.use_graphs else None
+        # a stream of the engine's own for the branches of its captured steps
+        self.beside: Optional[torch.cuda.Stream] = None
+        if self.use_graphs and any(p.branches for p in parts):
+            index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+            self.beside = kernels.take_stream(index)
+            weakref.finalize(self, kernels.give_stream, index, self.beside)
         self.last_h2d_bytes = 0          # bytes the last step copied from the host
         self._pin: Optional[torch.Tensor] = None      # pinned staging buffer of the steps that are not captured
         self._pin_copied = None

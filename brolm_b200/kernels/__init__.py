@@ -6,6 +6,7 @@ library fallback: a missing build or a CPU tensor raises.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import functools
 import os
@@ -51,6 +52,31 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 def _stream() -> int:
     """The current stream's handle, without a Python object around it: 0.3 us instead of 3.2 for each launch."""
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def _new_stream(index: int) -> torch.cuda.Stream:
+    handle = c_void_p()
+    with torch.cuda.device(index):
+        _check(_fn("core", "brolm_stream_create", [ctypes.POINTER(c_void_p)])(ctypes.byref(handle)), "stream_create")
+    return torch.cuda.ExternalStream(handle.value, device=index)
+
+
+_free_streams: dict = {}       # device index -> streams given back
+
+
+def take_stream(index: int) -> torch.cuda.Stream:
+    """A stream of the device that is the caller's alone until ``give_stream``.  (``torch.cuda.Stream()`` is one of 32 that the process
+    shares: while a capture forks onto it, another thread's launches there become part of the graph.)  As many exist as
+    were ever taken at one time; memory and workspaces that torch keeps by stream are found again by the next taker."""
+    free = _free_streams.setdefault(index, collections.deque())
+    try:
+        return free.pop()
+    except IndexError:
+        return _new_stream(index)
+
+
+def give_stream(index: int, stream: torch.cuda.Stream) -> None:
+    _free_streams.setdefault(index, collections.deque()).append(stream)
 
 
 B200_SMS = 148

@@ -40,6 +40,8 @@ class Part:
     # True when its kernels may run at the same time as another part's: none of them keeps tickets, counters or scratch
     # of its own on the device that another kernel of the step uses, too.
     runs_beside: bool = False
+    # True when it forks a branch of a captured step onto the context's second stream.
+    branches: bool = False
 
     def param_specs(self) -> dict[str, ParamSpec]:
         """Local tensor name -> what it must look like."""

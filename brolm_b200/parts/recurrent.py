@@ -394,6 +394,10 @@ class SideBySide(Part):
     def graph_safe(self) -> bool:
         return self.left.graph_safe and self.right.graph_safe
 
+    @property
+    def branches(self) -> bool:
+        return self.right.runs_beside
+
     def cache_spec(self):
         return (self.left.cache_spec(), self.right.cache_spec())
 
@@ -402,13 +406,13 @@ class SideBySide(Part):
         self.right.prepare(max_positions, device)
 
     def forward(self, x: torch.Tensor, ctx, entry, writes_cache: bool = True) -> torch.Tensor:
-        if self.right.runs_beside and x.is_cuda and torch.cuda.is_current_stream_capturing():
+        beside = getattr(ctx, "beside", None)
+        if beside is not None and self.branches and torch.cuda.is_current_stream_capturing():
             # A captured step of single tokens is a chain of short kernels, none of which fills the device: the two
             # mixers become two branches of the graph.  The second stream's memory goes back to that stream, and whoever
             # forks it again lets it wait first, so nothing is written again before this stream has read it.
             # (8 sequences, 2,048 wide, 16 heads on either side, two such layers of four: a step of 395 us takes 375.)
             here = torch.cuda.current_stream(x.device)
-            beside = torch.cuda.Stream(device=x.device)
             beside.wait_stream(here)
             with torch.cuda.stream(beside):
                 b = self.right.forward(x, ctx, entry.parts[1], writes_cache)

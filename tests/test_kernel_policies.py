@@ -169,3 +169,14 @@ def test_decode_blocks_start_by_length_only_where_runs_are_long():
     assert not first(True, 6, 1024, 0, 256) and not first(True, 1, 256, 0, 256)
     assert not first(True, 1, 8192, 64, 256) and first(True, 1, 8192, 4096, 256)  # a window bounds a run, too
     assert not first(True, 2, 1024, 0, 128) and first(True, 2, 4096, 0, 128)
+
+
+def test_streams_are_nobody_elses_until_given_back(monkeypatch):
+    made = []
+    monkeypatch.setattr(kernels, "_free_streams", {})
+    monkeypatch.setattr(kernels, "_new_stream", lambda index: made.append(index) or object())
+    a, b, c = kernels.take_stream(0), kernels.take_stream(0), kernels.take_stream(1)
+    assert len({id(a), id(b), id(c)}) == 3 and made == [0, 0, 1]
+    kernels.give_stream(0, a)
+    assert kernels.take_stream(1) is not a and kernels.take_stream(0) is a
+    assert len(made) == 4

@@ -3,6 +3,7 @@
 prompt and then decoding around the rings, batches of unequal requests against each alone with slots, pages and
 states used again, the first tokens, long decoding, greedy generation through the entry point, and the trace replay
 and the command line as a user runs them."""
+import gc
 import json
 import os
 import subprocess
@@ -325,3 +326,29 @@ def test_prompts_on_the_tcgen05_kernel_keep_the_precision_of_mma(setups, monkeyp
     eng = bb.Engine(model, max_tokens=128, max_slots=1)
     eng.step(eng.open(1), random_prompts(config["vocab"], [70], seed=1))
     assert len(asked) >= 2 and all(asked)
+
+
+def test_captures_leave_the_streams_of_the_process_alone(setups, monkeypatch):
+    """The branches of captured steps run on a stream of the engine's own, not on ones that all of torch shares: a capture
+    draws the one for its warm-up pass (and the first of all the one it captures on), whatever pairs of mixers it has."""
+    _, config, _, model = setups[("U", "bfloat16")]
+    drawn = []
+
+    class Drawn(torch.cuda.Stream):
+        def __new__(cls, *a, **kw):
+            drawn.append(cls)
+            return super().__new__(cls, *a, **kw)
+
+    engines = [bb.Engine(model, max_tokens=512, max_slots=4) for _ in range(2)]
+    handles = {e.beside.cuda_stream for e in engines}
+    assert len(handles) == 2
+    monkeypatch.setattr(torch.cuda, "Stream", Drawn)
+    for n in (1, 2, 4):
+        slots = engines[0].open(n)
+        engines[0].step(slots, random_prompts(config["vocab"], [5] * n, seed=n))
+        engines[0].step(slots, [[1]] * n)
+        engines[0].close(slots)
+    assert len(drawn) <= 3 + 1
+    del engines
+    gc.collect()
+    assert bb.Engine(model, max_tokens=128, max_slots=1).beside.cuda_stream in handles
