@@ -130,6 +130,18 @@ __device__ __forceinline__ float clamped_gate(float g, float u, float limit) {
     return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
 }
 
+// The activations of a gated feed-forward, codes 0 (the tanh form of gelu) and 1 (silu), and the gated pair of all codes.
+__device__ __forceinline__ float gate_act(float z, int act) {
+    if (act == 0) {
+        const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
+        return 0.5f * z * (1.0f + tanhf(u));
+    }
+    return z / (1.0f + expf(-z));
+}
+__device__ __forceinline__ float gate_pair(float g, float u, int act, float limit) {
+    return act == 2 ? clamped_gate(g, u, limit) : gate_act(g, act) * u;
+}
+
 static inline int launch_status() {
     return (int)cudaGetLastError();
 }

@@ -784,14 +784,6 @@ BROLM_API int brolm_rope_kv_write(void* qkv, int dtype, const void* positions, c
 // act 1: silu             z / (1 + exp(-z))
 // act 2: the clamped gate of common.cuh, a function of gate, up and a limit
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float act_apply(float z, int act) {
-    if (act == 0) {
-        const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-        return 0.5f * z * (1.0f + tanhf(u));
-    }
-    return z / (1.0f + expf(-z));
-}
-
 template <typename T>
 __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int inter, int act, float limit) {
     const size_t t = blockIdx.x;
@@ -800,8 +792,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ 
     const T* u = g + inter;
     T* o = out + t * (size_t)inter;
     for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < inter; j += gridDim.y * blockDim.x)
-        o[j] = from_float<T>(act == 2 ? clamped_gate(to_float(g[j]), to_float(u[j]), limit)
-                                      : act_apply(to_float(g[j]), act) * to_float(u[j]));
+        o[j] = from_float<T>(gate_pair(to_float(g[j]), to_float(u[j]), act, limit));
 }
 
 // bfloat16 with inter a multiple of 8: eight elements per thread, 16-byte accesses.
@@ -821,10 +812,7 @@ __global__ void __launch_bounds__(256) gated_act_vec_kernel(const bf16* __restri
         __nv_bfloat162* r2 = reinterpret_cast<__nv_bfloat162*>(&r);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            r2[e] = act == 2 ? __floats2bfloat162_rn(clamped_gate(gv[2 * e], uv[2 * e], limit),
-                                                     clamped_gate(gv[2 * e + 1], uv[2 * e + 1], limit))
-                             : __floats2bfloat162_rn(act_apply(gv[2 * e], act) * uv[2 * e],
-                                                     act_apply(gv[2 * e + 1], act) * uv[2 * e + 1]);
+            r2[e] = __floats2bfloat162_rn(gate_pair(gv[2 * e], uv[2 * e], act, limit), gate_pair(gv[2 * e + 1], uv[2 * e + 1], act, limit));
         *reinterpret_cast<uint4*>(o + j) = r;
     }
 }

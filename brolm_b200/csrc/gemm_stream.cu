@@ -235,7 +235,11 @@ __global__ void __launch_bounds__(THREADS, PER_SM) gemm_stream_kernel(const __gr
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (quarter < 2) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = fast_gate_pair(o[i], upx[i * 64 + lrow], g.act, g.cap);   // code 2: cap is its limit
+                        for (int i = 0; i < 16; ++i) {                       // code 2: cap is its limit
+                            // up to 16 tokens: the activation of the few-token product, which serves the other sizes
+                            const float u = upx[i * 64 + lrow];
+                            o[i] = BT == 16 ? gate_pair(o[i], u, g.act, g.cap) : fast_gate_pair(o[i], u, g.act, g.cap);
+                        }
                     }
                     writer = quarter < 2;
                     asm volatile("bar.sync 1, 128;" ::: "memory");          // upx may be written again

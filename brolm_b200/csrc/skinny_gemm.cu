@@ -59,14 +59,6 @@ __device__ __forceinline__ uint4 ldg16_cached(const bf16* p, bool ok) {
     return v;
 }
 
-__device__ __forceinline__ float act_apply(float z, int act) {
-    if (act == 0) {
-        const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-        return 0.5f * z * (1.0f + tanhf(u));
-    }
-    return z / (1.0f + expf(-z));
-}
-
 enum : int { EPI_STORE = 0, EPI_GATED = 1, EPI_SOFTCAP = 2, EPI_ROPE = 3 };
 
 struct SkinnyArgs {
@@ -290,7 +282,7 @@ __global__ void __launch_bounds__(WARPS * 32) skinny_kernel(SkinnyArgs a) {
                 gsum += red[w][((2 * ot) * NT + j) * 4 + e][ln];
                 usum += red[w][((2 * ot + 1) * NT + j) * 4 + e][ln];
             }
-            v = a.act == 2 ? clamped_gate(gsum, usum, a.cap) : act_apply(gsum, a.act) * usum;   // code 2: cap is its limit
+            v = gate_pair(gsum, usum, a.act, a.cap);   // code 2: cap is its limit
         } else {
             v = 0.0f;
 #pragma unroll

@@ -943,6 +943,18 @@ def test_decode_attention_gives_the_same_bits_whatever_runs_beside_it(options, h
         assert torch.equal(out[b], one[0]), (b, lengths[b])
 
 
+@pytest.mark.parametrize("activation,limit", [("gelu_tanh", 0.0), ("silu", 0.0), ("clamped_gate", 7.0)])
+def test_few_tokens_have_the_same_activation_on_both_products(activation, limit):
+    """One weight for every output, so that the sums are exact: what is left is the activation, to the last bit."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.eye(16, 64, device=DEV).to(torch.bfloat16)
+    w = (3 * torch.randn(2 * 8192, 64, generator=g, device=DEV)).to(torch.bfloat16)
+    few, stream = (torch.empty(16, 8192, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    kernels.skinny_gemm(x, w, few, "gated", activation, limit=limit)
+    kernels.gemm_stream(x, w, stream, "gated", activation, limit=limit)
+    assert torch.equal(few, stream)
+
+
 def test_kernels_refuse_what_they_cannot_do():
     q = torch.zeros(2, 2 * 520, device=DEV)
     with pytest.raises(kernels.KernelError):                # a head beyond the exact kernel's 512
