@@ -1417,13 +1417,17 @@ def stream_instead_of_skinny(x: torch.Tensor, gate_up: torch.Tensor, sms: Option
     It is better where those pieces are more than the SMs and fill their last round of two an SM: 9B, 224 pieces, a
     decode step of 1 / 4 / 8 / 16 sequences 4,081 / 4,297 / 4,642 / 7,180 us on mma.sync, 3,995 / 4,239 / 4,503 / 6,796 here
     (the largest ragged); 27B, 576 pieces, the product alone at 8 / 16 tokens 104.0 / 113.4 and 101.2 / 102.7 us; but 2B,
-    144 pieces, 16.2 and 18.1 us at 8 tokens.  Both results differ from 64 bits by their rounding to bfloat16 (1.649e-3), and the activation is the same.
+    144 pieces, 16.2 and 18.1 us at 8 tokens.  In several rounds the late start counts until the tokens' reads do: 27B at 1 / 4
+    / 6 / 8 tokens 98.9 / 99.9 / 102.8 / 104.3 us on mma.sync and 102.5 / 101.2 / 100.7 / 101.6 here, 57,344 x 4,096 at 6 / 8 75.7
+    / 77.9 and 77.7 / 77.0.  Both results differ from 64 bits by their rounding to bfloat16 (1.649e-3), and the activation is the same.
     (Down, whose float sums the reader adds, stays: the stream is faster at 9B from nine tokens on, 25.5 -> 18.9 us, but
     its sums differ from 64 bits by 1.4e-6 where those of the mma.sync kernel do by 0.6e-6.)"""
     if not gemm_stream_ok(x, gate_up) or gate_up.shape[0] % 128:
         return False
     places = 2 * (sms or device_sms(x.device if x.is_cuda else None))
     pieces = gate_up.shape[0] // 128
+    if pieces > places and x.shape[0] < 8:
+        return False
     return pieces > places // 2 and pieces >= 0.7 * places * -(-pieces // places)
 
 

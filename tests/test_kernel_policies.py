@@ -109,6 +109,7 @@ def test_which_few_token_products_stream(monkeypatch):
     of = lambda M, N, K: kernels.stream_instead_of_skinny(like(M, K), like(N, K), sms=148)
     assert of(1, 28672, 3584) and of(16, 73728, 4608)                 # 9B, 27B gate and up
     assert not of(16, 18432, 2304) and not of(8, 8192, 2048)          # no more pieces than SMs
+    assert of(8, 73728, 4608) and not of(1, 73728, 4608) and not of(7, 57344, 4096)     # several rounds: not for the fewest
     assert not of(8, 128 * 300, 512)                                        # a second round of four pieces
     slices = lambda N, K: kernels.gemm_stream_parts(like(16, K), like(N, K), sms=148)
     assert slices(3584, 14336) == 10 and slices(8192, 3584) == 4 and slices(2304, 9216) == 8
