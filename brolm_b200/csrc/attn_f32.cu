@@ -14,9 +14,11 @@
 //
 // A block owns 32 rows of one (sequence, kv head), a row being a (query token, query head of the group) pair, or 8 where
 // a step has no more (decode), and either walks all spans it sees or, where that leaves SMs idle, one of them, with
-// merge_kernel behind it (attn_f32_splits in kernels/__init__.py has the rule and what both take): a decode step of three
+// merge_kernel behind it (attn_f32_splits and attn_f32_worth_sharing in kernels/__init__.py have the rule and what both take): a decode step of three
 // sequences of up to 420 keys is otherwise twelve blocks (30 us shared; 337 us in attn_simt.cu, which served all sizes
-// before; a prompt of 300 tokens 72 and 187 us).  K comes through a ring of cp.async stages in slices of 32 c of all 128 keys, V in
+// before; a prompt of 300 tokens 63 and 173 us).  Of a span only the 32-key parts that some row sees are worked on: one,
+// two or all four (16 tokens, 4 heads of 16: 8.9 us, 13.8 with whole spans; 1,000 tokens, 32 heads of 128 on 8 kv heads, window 64:
+// 129 and 183).  K comes through a ring of cp.async stages in slices of 32 c of all 128 keys, V in
 // slices of 16 keys; both products run on packed fma.rn.f32x2, the scores paired along c, the values along d.  Bound by
 // shared memory: a thread's outputs are what its registers hold (4 x 8 scores, 4 x 16 values).
 #include "common.cuh"
@@ -29,7 +31,6 @@ constexpr int STAGES = 3;
 constexpr int KC = 32;                        // c of a slice of keys
 constexpr int PITCH = 144;                    // its bytes, padded: eight neighbouring rows lie in different banks
 constexpr int VK = 16;                        // keys of a slice of values
-constexpr int STAGE = SPAN * PITCH;           // 18,432 bytes; a slice of values takes VK * vd * 4 <= 16,384
 constexpr int P_PITCH = SPAN + 4;             // floats
 
 struct F32Args {
@@ -52,6 +53,7 @@ struct F32Args {
     const float* slopes;
     const float* dist_bias;
     int dist_len;
+    int max_parts;                            // 32-key parts of a span that hold keys: 4, or fewer in steps of so few keys
     int splits;                               // spans a tile can see; 0: a block walks them all
     float* part_acc;                          // [token][head][split][vd]
     float* part_ml;                           // [token][head][split][2]
@@ -81,6 +83,12 @@ __device__ __forceinline__ void copy16(void* dst, const float* p, bool ok) {
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// a slice of keys, or of values
+__host__ __device__ __forceinline__ int stage_bytes(const F32Args& a) {
+    const int k = a.max_parts * 32 * PITCH, v = VK * a.vd * 4;
+    return k > v ? k : v;
+}
 
 // The merge of one more span into (M, L): factors for what is held and for what comes.
 __device__ __forceinline__ void merge_factors(float& M, float& L, float m, float l, float& held, float& fresh) {
@@ -118,15 +126,18 @@ __device__ __forceinline__ Tile tile_of(const F32Args& a, int b, int tile) {
     return t;
 }
 
+template <int N> struct Count { static constexpr int value = N; };
+
 template <int ROWS, int VJ>
-__global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
+__global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn_f32_kernel(F32Args a) {
     constexpr int LN = ROWS == 32 ? 16 : 32;           // threads side by side over keys, and over value dims
     constexpr int RI = ROWS / (THREADS / LN);          // rows of a thread, THREADS / LN apart
-    constexpr int RSTEP = THREADS / LN, KJ = SPAN / LN;
+    constexpr int RSTEP = THREADS / LN;
     extern __shared__ __align__(16) uint8_t raw[];
     const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;  // floats; zeros behind hd
+    const int stage = stage_bytes(a);
     uint8_t* ring = raw;
-    float* Qs = reinterpret_cast<float*>(raw + STAGES * STAGE);
+    float* Qs = reinterpret_cast<float*>(raw + STAGES * stage);
     float* P = Qs + ROWS * q_pitch;
     float* stats = P + ROWS * P_PITCH;                  // [ROWS]: M, L, factor of what is held, factor of what comes
     long long* k_off = reinterpret_cast<long long*>(stats + 4 * ROWS);
@@ -139,24 +150,15 @@ __global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
     if (t.rows <= 0) return;
     int span = t.first, last = t.last;
     if (a.splits) {
-        span += blockIdx.x % a.splits;
+        const int share = blockIdx.x % a.splits;
+        span += share;
         if (span > last) return;
-        last = span;
+        if (share < a.splits - 1) last = span;          // (the last block walks what is left, should the bound not have held)
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tn = tid % LN, tm = tid / LN;
     const int key_hi = t.first_pos + (t.row0 + t.rows - 1) / a.group;
 
-    for (int idx = tid; idx < ROWS * (q_pitch / 4); idx += THREADS) {
-        const int r = idx / (q_pitch / 4), c = (idx - r * (q_pitch / 4)) * 4;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (r < t.rows && c < a.hd) {
-            const int row = t.row0 + r;
-            v = *reinterpret_cast<const float4*>(a.q + (size_t)(t.q0 + row / a.group) * a.q_stride +
-                                                 (g * a.group + row % a.group) * a.hd + c);
-        }
-        *reinterpret_cast<float4*>(Qs + r * q_pitch + c) = v;
-    }
     if (tid < ROWS) {
         stats[tid] = -INFINITY;
         stats[ROWS + tid] = 0.0f;
@@ -169,10 +171,13 @@ __global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
 #pragma unroll
         for (int j = 0; j < VJ; ++j) tot[i][j][0] = tot[i][j][1] = tot[i][j][2] = tot[i][j][3] = 0.0f;
 
-    for (; span <= last; ++span) {
+    for (bool first = true; span <= last; ++span, first = false) {
         const int key0 = span * SPAN;
-        const int keys = min(SPAN, key_hi + 1 - key0);  // keys behind the tile's last query are not read
-        __syncthreads();                                // the span before this one is done with (and Q and stats are written)
+        const int keys = min(a.max_parts * 32, key_hi + 1 - key0);      // keys behind the tile's last query are not read
+        // the 32-key parts of the span that any row sees: part0 and as many as make one, two or all four
+        int part0 = max(0, t.key_lo - key0) / 32, n_parts = (keys - 1) / 32 - part0 + 1;
+        if (n_parts > 2) part0 = 0, n_parts = 4;
+        __syncthreads();                                // the span before this one is done with
         {
             const int kp = key0 + tid;
             long long ko = -1, vo = -1;
@@ -193,107 +198,145 @@ __global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
         __syncthreads();
         const float* kb = a.k_pages ? a.k_pages : a.k;
         const float* vb = a.k_pages ? a.v_pages : a.v;
-        const int v_slices = (keys + VK - 1) / VK, slices = k_slices + v_slices;
-        auto fetch = [&](int i) {
-            uint8_t* dst = ring + (i % STAGES) * STAGE;
-            if (i < k_slices) {
-                const int c = i * KC + (tid & 7) * 4;
-#pragma unroll
-                for (int j = 0; j < SPAN / 16; ++j) {
-                    const int key = j * 16 + (tid >> 3);
-                    const long long o = k_off[key];
-                    const bool ok = o >= 0 && c < a.hd;
-                    copy16(dst + key * PITCH + (tid & 7) * 16, kb + (ok ? o + c : 0), ok);
-                }
-            } else if (i < slices) {
+        const int v_from = part0 * 32, slices = k_slices + (keys - v_from + VK - 1) / VK;
+        auto fetch_v = [&](int i) {
+            if (i < slices) {
+                uint8_t* dst = ring + (i % STAGES) * stage;
                 const int pieces = a.vd / 4;
                 for (int idx = tid; idx < VK * pieces; idx += THREADS) {
                     const int j = idx / pieces, c = (idx - j * pieces) * 4;
-                    const long long o = v_off[(i - k_slices) * VK + j];
+                    const long long o = v_off[v_from + (i - k_slices) * VK + j];
                     copy16(dst + (j * a.vd + c) * 4, vb + (o >= 0 ? o + c : 0), o >= 0);
                 }
             }
             copy_commit();
         };
+        auto parts = [&](auto count) {
+            constexpr int N = decltype(count)::value, NJ = N * 32 / LN;
+            auto fetch = [&](int i) {
+                if (i >= k_slices) return fetch_v(i);
+                uint8_t* dst = ring + (i % STAGES) * stage;
+                const int c = i * KC + (tid & 7) * 4;
 #pragma unroll
-        for (int i = 0; i < STAGES - 1; ++i) fetch(i);
-
-        uint64_t s[RI][KJ];
+                for (int j = 0; j < N * 2; ++j) {
+                    const int key = part0 * 32 + j * 16 + (tid >> 3);
+                    const long long o = k_off[key];
+                    const bool ok = o >= 0 && c < a.hd;
+                    copy16(dst + key * PITCH + (tid & 7) * 16, kb + (ok ? o + c : 0), ok);
+                }
+                copy_commit();
+            };
 #pragma unroll
-        for (int i = 0; i < RI; ++i)
+            for (int i = 0; i < STAGES - 1; ++i) fetch(i);
+            if (first) {                                    // (seen by all behind the first slice's barrier)
+                for (int idx = tid; idx < ROWS * (q_pitch / 4); idx += THREADS) {
+                    const int r = idx / (q_pitch / 4), c = (idx - r * (q_pitch / 4)) * 4;
+                    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (r < t.rows && c < a.hd) {
+                        const int row = t.row0 + r;
+                        v = *reinterpret_cast<const float4*>(a.q + (size_t)(t.q0 + row / a.group) * a.q_stride +
+                                                             (g * a.group + row % a.group) * a.hd + c);
+                    }
+                    *reinterpret_cast<float4*>(Qs + r * q_pitch + c) = v;
+                }
+            }
+            uint64_t s[RI][NJ];
 #pragma unroll
-            for (int j = 0; j < KJ; ++j) s[i][j] = 0;
-        for (int i = 0; i < k_slices; ++i) {
-            copy_wait<STAGES - 2>();
-            __syncthreads();
-            fetch(i + STAGES - 1);
-            const float* ks = reinterpret_cast<const float*>(ring + (i % STAGES) * STAGE) + tn * (PITCH / 4);
-            const float* qs = Qs + tm * q_pitch + i * KC;
+            for (int i = 0; i < RI; ++i)
 #pragma unroll
-            for (int c = 0; c < KC; c += 4) {
-                Pair2 q[RI];
+                for (int j = 0; j < NJ; ++j) s[i][j] = 0;
+            for (int i = 0; i < k_slices; ++i) {
+                copy_wait<STAGES - 2>();
+                __syncthreads();
+                fetch(i + STAGES - 1);
+                const float* ks = reinterpret_cast<const float*>(ring + (i % STAGES) * stage) + (part0 * 32 + tn) * (PITCH / 4);
+                const float* qs = Qs + tm * q_pitch + i * KC;
 #pragma unroll
-                for (int r = 0; r < RI; ++r) q[r] = lds4(qs + r * RSTEP * q_pitch + c);
+                for (int c = 0; c < KC; c += 4) {
+                    Pair2 q[RI];
 #pragma unroll
-                for (int j = 0; j < KJ; ++j) {
-                    const Pair2 k = lds4(ks + j * LN * (PITCH / 4) + c);
+                    for (int r = 0; r < RI; ++r) q[r] = lds4(qs + r * RSTEP * q_pitch + c);
 #pragma unroll
-                    for (int r = 0; r < RI; ++r) {
-                        fma2(s[r][j], q[r].x, k.x);
-                        fma2(s[r][j], q[r].y, k.y);
+                    for (int j = 0; j < NJ; ++j) {
+                        const Pair2 k = lds4(ks + j * LN * (PITCH / 4) + c);
+#pragma unroll
+                        for (int r = 0; r < RI; ++r) {
+                            fma2(s[r][j], q[r].x, k.x);
+                            fma2(s[r][j], q[r].y, k.y);
+                        }
                     }
                 }
             }
-        }
 #pragma unroll
-        for (int r = 0; r < RI; ++r) {
-            const int rr = tm + r * RSTEP, row = t.row0 + rr;
-            const int pos = rr < t.rows ? t.first_pos + row / a.group : -1, head = g * a.group + row % a.group;
-            const float slope = a.slopes && pos >= 0 ? a.slopes[head] : 0.0f;
-            const int from = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 && pos >= 0 ? pos - pos % a.chunk : 0);
+            for (int r = 0; r < RI; ++r)
 #pragma unroll
-            for (int j = 0; j < KJ; ++j) {
-                const int kp = key0 + tn + j * LN;
-                float sc = -INFINITY;
-                if (kp <= pos && kp >= from) {
+                for (int j = 0; j < NJ; ++j) {
                     const float2 h = unpack2(s[r][j]);
-                    sc = soft_cap(__fmul_rn(h.x + h.y, a.scale), a.cap);
-                    if (a.slopes) sc = __fmaf_rn(-slope, (float)(pos - kp), sc);
-                    if (a.dist_bias) sc += a.dist_bias[(size_t)head * a.dist_len + min(pos - kp, a.dist_len - 1)];
+                    P[(tm + r * RSTEP) * P_PITCH + part0 * 32 + tn + j * LN] = h.x + h.y;
                 }
-                P[rr * P_PITCH + tn + j * LN] = sc;
-            }
-        }
-        __syncthreads();
-        for (int r = warp * (ROWS / 4); r < (warp + 1) * (ROWS / 4); ++r) {
-            float sc[4], m = -INFINITY, l = 0.0f;
+            __syncthreads();
+            // a warp's rows, two at a time: scores out of the products, then the span's maximum, probabilities and sum
+            constexpr int RB = 2;
+            for (int r0 = warp * (ROWS / 4); r0 < (warp + 1) * (ROWS / 4); r0 += RB) {
+                float sc[RB][N], m[RB], l[RB];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                sc[e] = P[r * P_PITCH + e * 32 + lane];
-                m = fmaxf(m, sc[e]);
-            }
-            m = warp_max(m);
+                for (int r = 0; r < RB; ++r) {
+                    const int row = t.row0 + r0 + r, head = g * a.group + row % a.group;
+                    const int pos = r0 + r < t.rows ? t.first_pos + row / a.group : -1;
+                    const float slope = a.slopes && pos >= 0 ? a.slopes[head] : 0.0f;
+                    const int from = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 && pos >= 0 ? pos - pos % a.chunk : 0);
+                    m[r] = -INFINITY;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float p = sc[e] == -INFINITY ? 0.0f : expf(sc[e] - m);       // (a NaN stays one)
-                P[r * P_PITCH + e * 32 + lane] = p;
-                const float part = warp_sum(p);
-                l = e == 0 ? part : l + part;
-            }
-            if (lane == 0) {
-                if (a.splits) {
-                    stats[r] = m;
-                    stats[ROWS + r] = l;
-                } else {
+                    for (int e = 0; e < N; ++e) {
+                        const int kp = key0 + (part0 + e) * 32 + lane;
+                        float v = -INFINITY;
+                        if (kp <= pos && kp >= from) {
+                            v = soft_cap(__fmul_rn(P[(r0 + r) * P_PITCH + (part0 + e) * 32 + lane], a.scale), a.cap);
+                            if (a.slopes) v = __fmaf_rn(-slope, (float)(pos - kp), v);
+                            if (a.dist_bias) v += a.dist_bias[(size_t)head * a.dist_len + min(pos - kp, a.dist_len - 1)];
+                        }
+                        sc[r][e] = v;
+                        m[r] = fmaxf(m[r], v);
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], o));
+#pragma unroll
+                for (int r = 0; r < RB; ++r)
+#pragma unroll
+                    for (int e = 0; e < N; ++e) {
+                        sc[r][e] = sc[r][e] == -INFINITY ? 0.0f : expf(sc[r][e] - m[r]);       // (a NaN stays one)
+                        P[(r0 + r) * P_PITCH + (part0 + e) * 32 + lane] = sc[r][e];
+                    }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < RB; ++r)
+#pragma unroll
+                        for (int e = 0; e < N; ++e) sc[r][e] += __shfl_xor_sync(0xffffffffu, sc[r][e], o);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    l[r] = sc[r][0];
+#pragma unroll
+                    for (int e = 1; e < N; ++e) l[r] += sc[r][e];
+                }
+                if (lane < RB) {
+                    const float mine = lane == 0 ? m[0] : m[1], sum = lane == 0 ? l[0] : l[1];
+                    const int r = r0 + lane;
                     float M = stats[r], L = stats[ROWS + r], held, fresh;
-                    merge_factors(M, L, m, l, held, fresh);
+                    merge_factors(M, L, mine, sum, held, fresh);
                     stats[r] = M;
                     stats[ROWS + r] = L;
                     stats[2 * ROWS + r] = held;
                     stats[3 * ROWS + r] = fresh;
                 }
             }
-        }
+        };
+        if (n_parts == 1) parts(Count<1>());
+        else if (n_parts == 2) parts(Count<2>());
+        else parts(Count<4>());
         uint64_t acc[RI][VJ][2];
 #pragma unroll
         for (int r = 0; r < RI; ++r)
@@ -302,9 +345,9 @@ __global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
         for (int i = k_slices; i < slices; ++i) {
             copy_wait<STAGES - 2>();
             __syncthreads();                            // (the first time round: P and the factors are written, too)
-            fetch(i + STAGES - 1);
-            const float* vs = reinterpret_cast<const float*>(ring + (i % STAGES) * STAGE);
-            const float* ps = P + tm * P_PITCH + (i - k_slices) * VK;
+            fetch_v(i + STAGES - 1);
+            const float* vs = reinterpret_cast<const float*>(ring + (i % STAGES) * stage);
+            const float* ps = P + tm * P_PITCH + v_from + (i - k_slices) * VK;
 #pragma unroll
             for (int j0 = 0; j0 < VK; j0 += 4) {
                 float p[RI][4];
@@ -337,18 +380,14 @@ __global__ void __launch_bounds__(THREADS) attn_f32_kernel(F32Args a) {
 #pragma unroll
         for (int r = 0; r < RI; ++r) {
             const int rr = tm + r * RSTEP;
-            const float held = a.splits ? 0.0f : stats[2 * ROWS + rr], fresh = a.splits ? 1.0f : stats[3 * ROWS + rr];
+            const float held = stats[2 * ROWS + rr], fresh = stats[3 * ROWS + rr];
 #pragma unroll
             for (int j = 0; j < VJ; ++j) {
                 const float2 lo = unpack2(acc[r][j][0]), hi = unpack2(acc[r][j][1]);
-                if (a.splits) {
-                    tot[r][j][0] = lo.x; tot[r][j][1] = lo.y; tot[r][j][2] = hi.x; tot[r][j][3] = hi.y;
-                } else {
-                    tot[r][j][0] = merged(tot[r][j][0], held, lo.x, fresh);
-                    tot[r][j][1] = merged(tot[r][j][1], held, lo.y, fresh);
-                    tot[r][j][2] = merged(tot[r][j][2], held, hi.x, fresh);
-                    tot[r][j][3] = merged(tot[r][j][3], held, hi.y, fresh);
-                }
+                tot[r][j][0] = merged(tot[r][j][0], held, lo.x, fresh);
+                tot[r][j][1] = merged(tot[r][j][1], held, lo.y, fresh);
+                tot[r][j][2] = merged(tot[r][j][2], held, hi.x, fresh);
+                tot[r][j][3] = merged(tot[r][j][3], held, hi.y, fresh);
             }
         }
     }
@@ -416,7 +455,7 @@ __global__ void __launch_bounds__(64) merge_kernel(F32Args a) {
 template <int ROWS, int VJ>
 int launch(const F32Args& a, int batch, int max_q_len, cudaStream_t stream) {
     const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;
-    const int smem = STAGES * STAGE + (ROWS * q_pitch + ROWS * P_PITCH + 4 * ROWS) * (int)sizeof(float) + 2 * SPAN * 8;
+    const int smem = STAGES * stage_bytes(a) + (ROWS * q_pitch + ROWS * P_PITCH + 4 * ROWS) * (int)sizeof(float) + 2 * SPAN * 8;
     static OncePerDevice allowed;
     if (const int e = allow_shared_memory(attn_f32_kernel<ROWS, VJ>, 112 * 1024, allowed)) return e;
     const int rows = max_q_len * a.group, tiles = (rows + ROWS - 1) / ROWS;
@@ -456,6 +495,9 @@ BROLM_API int brolm_attn_f32(const void* q, int q_stride, void* out, int out_str
     a.n_kv = n_kv; a.group = group; a.hd = hd; a.vd = vd; a.scale = scale; a.cap = cap; a.window = window; a.chunk = chunk;
     a.sink = (const float*)sink; a.slopes = (const float*)slopes; a.dist_bias = (const float*)dist_bias; a.dist_len = dist_len;
     a.splits = splits; a.part_acc = (float*)part_acc; a.part_ml = (float*)part_ml;
+    // a prompt's keys are its tokens: with few of them a block takes less of an SM (16 prompts of 20 tokens, 32 heads of 128 on
+    // 8 kv heads, 384 blocks: 27 us where two share an SM)
+    a.max_parts = k_pages || max_q_len > 64 ? 4 : max_q_len > 32 ? 2 : 1;
     if ((long long)max_q_len * group <= 8) {
         if (vd <= 128) return launch<8, 1>(a, batch, max_q_len, stream);
         return launch<8, 2>(a, batch, max_q_len, stream);

@@ -1520,6 +1520,38 @@ def attn_f32_splits(batch: int, n_kv: int, group: int, vd: int, tokens: int, max
     return min(spans) if tokens * n_kv * group * min(spans) * (vd + 2) * 4 <= 64 << 20 else 0
 
 
+def attn_f32_worth_sharing(batch: int, n_kv: int, group: int, head_dim: int, vd: int, max_q_len: int, max_keys: Optional[int],
+                           window: int = 0, chunk: int = 0, sms: Optional[int] = None) -> bool:
+    """Whether blocks that share a tile's spans, and the launch that merges what they leave, are clearly faster than blocks
+    that walk them.
+
+    A span takes a block of 32 rows some 21 us with heads of 64, 30 with 128 and 48 with 256, of 8 rows 10, 14 and 24; two or
+    three blocks share an SM and slow each other down a little.  Measured, walked / shared: a prompt of 300 tokens with 8
+    heads of 256 on 4 kv heads (76 tiles) 147 / 79 us, with a window of 100 92 / 76; with 32 heads of 128 on 8 (304) 93 / 86, with a
+    window of 64 51 / 66; one token of 200 keys, 32 heads of 128 on 8, of one sequence 27 / 18, of 32 sequences 29 / 36."""
+    sms = sms or device_sms()
+    rows = 8 if max_q_len * group <= 8 else 32
+    size = (head_dim + vd) / 512
+    span, places, slower = (8 + 16 * size, 3 * sms, 0.3) if rows == 8 else (12 + 36 * size, 2 * sms, 0.2)
+    tiles = -(-max_q_len * group // rows) * n_kv * batch
+    walks = []                           # spans that a block walks, and blocks with something to do where they are shared
+    if max_keys:
+        full = max_keys / F32_SPAN
+        walks.append((full, -(-3 * max_keys // (4 * F32_SPAN)), 1.0) if max_q_len == 1 else (full + 0.2, (full + 1.2) / 2, 1.0))
+    for keys in (window, chunk):
+        if keys > 0:
+            seen = (keys + rows // group) / F32_SPAN
+            walks.append((max(1 + 0.3 * seen, seen + 0.3), 1 + seen, 0.85))        # (no block sees a whole span)
+    if not walks:
+        return False
+    walked, busy, part = (min(w[i] for w in walks) for i in range(3))
+
+    def round_of(blocks: float) -> float:
+        return span * max(1.0, blocks / places) * (1 + slower * min(places / sms - 1, max(0.0, blocks / sms - 1)))
+    merging = 5 + (max_q_len * group * n_kv * batch / 400 if rows == 8 else 0)
+    return part * round_of(tiles * busy) + merging < 0.93 * walked * round_of(tiles)
+
+
 def attn_f32_max_keys(places: int, ring: int) -> Optional[int]:
     """A bound on the keys of a sequence whose page table has ``places`` places; None: the pages bound nothing, because
     the positions go round.  (A ring of exactly as many places goes round, too.)"""
@@ -1532,7 +1564,9 @@ def _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_
         max_keys = max_q_len
     else:
         max_keys = attn_f32_max_keys(page_table.shape[1] * page_size, ring)
-    splits = attn_f32_splits(batch, n_kv, group, vd, q.shape[0], max_q_len, max_keys, window, chunk)
+    splits = 0
+    if attn_f32_worth_sharing(batch, n_kv, group, head_dim, vd, max_q_len, max_keys, window, chunk):
+        splits = attn_f32_splits(batch, n_kv, group, vd, q.shape[0], max_q_len, max_keys, window, chunk)
     acc = ml = None
     if splits:
         acc = torch.empty((q.shape[0], n_kv * group, splits, vd), dtype=torch.float32, device=q.device)

@@ -181,3 +181,12 @@ def test_streams_are_nobody_elses_until_given_back(monkeypatch):
     kernels.give_stream(0, a)
     assert kernels.take_stream(1) is not a and kernels.take_stream(0) is a
     assert len(made) == 4
+
+
+def test_float_attention_shares_spans_only_where_the_merge_is_worth_it():
+    worth = lambda *a, **kw: kernels.attn_f32_worth_sharing(*a, sms=148, **kw)
+    assert worth(1, 4, 2, 256, 256, 300, 300) and worth(3, 4, 2, 256, 256, 1, 512) and worth(64, 4, 2, 256, 256, 1, 512)
+    assert not worth(1, 4, 2, 256, 256, 100, 100) and not worth(1, 4, 2, 256, 256, 1, 128)     # one span
+    assert not worth(1, 2, 2, 32, 32, 300, 300, window=16) and not worth(1, 8, 4, 128, 128, 300, 300, window=64)
+    assert worth(1, 4, 2, 256, 256, 300, 300, window=100) and not worth(32, 8, 4, 128, 128, 1, 256)
+    assert not worth(1, 4, 2, 256, 256, 1, None)                                               # no bound

@@ -914,6 +914,67 @@ def test_float_attention_gives_the_same_bits_however_it_is_cut(monkeypatch, opti
         assert torch.equal(one[0], shared[n - 1])
 
 
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("lengths", [[3], [32, 5, 1], [33, 64, 20], [65, 7, 96], [97, 40], [129, 160, 31]])
+@pytest.mark.parametrize("window,chunk", [(0, 0), (1, 0), (40, 0), (70, 0), (0, 33)])
+def test_float_attention_of_parts_of_spans(monkeypatch, lengths, window, chunk, shared):
+    """One, two and all 32-key parts of a span, at either end of it, with prompts short enough for small stages; a row's bits
+    are those of a launch with stages for whole spans, and all is close to 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(sum(lengths) + window)
+    n_q, n_kv, hd, vd = 6, 3, 24, 40
+    T, B = sum(lengths), len(lengths)
+    q, k, v = (torch.randn(T, w, generator=g, device=DEV) for w in (n_q * hd, n_kv * hd, n_kv * vd))
+    cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device=DEV)
+    length = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: shared)
+    kw = dict(n_kv=n_kv, group=2, head_dim=hd, v_dim=vd, scale=hd ** -0.5, cap=20.0, window=window, chunk=chunk, batch=B, k=k, v=v)
+    out, wide = (torch.full((T, n_q * vd), float("nan"), device=DEV) for _ in range(2))
+    kernels.attention_simt(q, out, cu, length, max_q_len=max(lengths), **kw)
+    kernels.attention_simt(q, wide, cu, length, max_q_len=max(max(lengths), 300), **kw)      # stages for whole spans
+    assert torch.equal(out, wide)
+    for b, n in enumerate(lengths):
+        at = int(cu[b])
+        heads = lambda t, count: t[at:at + n].double().view(n, count, -1).transpose(0, 1)
+        kk, vv = (heads(t, n_kv).repeat_interleave(2, 0) for t in (k, v))
+        s = heads(q, n_q) @ kk.transpose(1, 2) * hd ** -0.5
+        s = 20.0 * torch.tanh(s / 20.0)
+        p, j = torch.arange(n, device=DEV).view(-1, 1), torch.arange(n, device=DEV)
+        seen = (j <= p) & ((p - j < window) if window else (j >= 0)) & ((j >= p - p % chunk) if chunk else (j >= 0))
+        ref = torch.softmax(s.masked_fill(~seen, -torch.inf), -1) @ vv
+        close(out[at:at + n], ref.transpose(0, 1).reshape(n, -1).cpu(), torch.float32, scale=float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("window", [1, 100, 128, 129, 257, 300, 400])
+@pytest.mark.parametrize("shared", [False, True])
+def test_float_attention_in_wrapped_rings_gives_the_bits_of_the_prompt(monkeypatch, window, shared):
+    """Several sequences decoded from rings of their window's pages, up to four spans wide and many times wrapped, against
+    the last tokens of the same sequences as packed prompts: the same bits, walked and shared."""
+    g = torch.Generator(device=DEV).manual_seed(window)
+    n_q, n_kv, hd, vd = 4, 2, 16, 24
+    lengths = [1, 130, 700, 641, 385, 512]
+    T, B, ring = sum(lengths), len(lengths), -(-window // 64) * 64
+    q, k, v = (torch.randn(T, w, generator=g, device=DEV) for w in (n_q * hd, n_kv * hd, n_kv * vd))
+    cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device=DEV)
+    length = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: shared)
+    kw = dict(n_kv=n_kv, group=2, head_dim=hd, v_dim=vd, scale=0.5, cap=0.0, window=window, batch=B)
+    packed = torch.full((T, n_q * vd), float("nan"), device=DEV)
+    kernels.attention_simt(q, packed, cu, length, max_q_len=max(lengths), k=k, v=v, **kw)
+    per = ring // 64
+    table = torch.randperm(B * per, generator=g, device=DEV).to(torch.int32).view(B, per)
+    kp, vp = torch.zeros(B * per, n_kv, 64, hd, device=DEV), torch.zeros(B * per, n_kv, 64, vd, device=DEV)
+    for b, n in enumerate(lengths):
+        at = int(cu[b])
+        for p in range(max(0, n - ring), n):
+            page = int(table[b, p % ring // 64])
+            kp[page, :, p % 64], vp[page, :, p % 64] = k[at + p].view(n_kv, hd), v[at + p].view(n_kv, vd)
+    ends = (cu[1:] - 1).long()
+    one = torch.full((B, n_q * vd), float("nan"), device=DEV)
+    kernels.attention_simt(q[ends], one, torch.arange(B + 1, dtype=torch.int32, device=DEV), length, max_q_len=1, k_pages=kp,
+                           v_pages=vp, page_table=table, ring=ring, page_size=64, **kw)
+    assert torch.equal(one, packed[ends])
+
+
 @pytest.mark.parametrize("options", ["plain", "sink", "bias", "one row"])
 @pytest.mark.parametrize("hd,n_kv,splits", [(256, 4, 2), (144, 2, 4), (64, 4, 3)])
 @pytest.mark.parametrize("batch,longest_first", [(98, True), (98, False), (512, True), (513, True)])
