@@ -1552,18 +1552,20 @@ def attn_f32_worth_sharing(batch: int, n_kv: int, group: int, head_dim: int, vd:
     return part * round_of(tiles * busy) + merging < 0.93 * walked * round_of(tiles)
 
 
-def attn_f32_max_keys(places: int, ring: int) -> Optional[int]:
-    """A bound on the keys of a sequence whose page table has ``places`` places; None: the pages bound nothing, because
-    the positions go round.  (A ring of exactly as many places goes round, too.)"""
-    return places if ring > places else None
+def attn_f32_max_keys(places: int, ring: int, max_keys: Optional[int] = None) -> Optional[int]:
+    """A bound on the keys of a sequence whose page table has ``places`` places, and of which the caller may know one of
+    its own; None: none is known, because the positions go round in the pages.  (A ring of exactly as many places goes
+    round, too.)"""
+    bounds = [n for n in (places if ring > places else None, max_keys) if n]
+    return min(bounds) if bounds else None
 
 
 def _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group, head_dim,
-                   vd, scale, cap, window, chunk, sink, slopes, dist_bias, batch, max_q_len) -> None:
+                   vd, scale, cap, window, chunk, sink, slopes, dist_bias, batch, max_q_len, max_keys) -> None:
     if k_pages is None:
         max_keys = max_q_len
     else:
-        max_keys = attn_f32_max_keys(page_table.shape[1] * page_size, ring)
+        max_keys = attn_f32_max_keys(page_table.shape[1] * page_size, ring, max_keys)
     splits = 0
     if attn_f32_worth_sharing(batch, n_kv, group, head_dim, vd, max_q_len, max_keys, window, chunk):
         splits = attn_f32_splits(batch, n_kv, group, vd, q.shape[0], max_q_len, max_keys, window, chunk)
@@ -1589,7 +1591,8 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_le
                    page_table: Optional[torch.Tensor] = None, ring: int = 0, page_size: int = 0,
                    sink: Optional[torch.Tensor] = None, v_dim: Optional[int] = None, chunk: int = 0,
                    slopes: Optional[torch.Tensor] = None, keep_first: int = 0, ring_from: int = 0,
-                   v_all: int = 0, v_from: int = 0, dist_bias: Optional[torch.Tensor] = None) -> None:
+                   v_all: int = 0, v_from: int = 0, dist_bias: Optional[torch.Tensor] = None,
+                   max_keys: Optional[int] = None) -> None:
     """Exact attention on CUDA cores.  Keys come from (k, v) packed like q, or from cache pages.
     ``sink``: float32 [query heads]; exp(sink) joins every softmax's denominator (a key with no value).
     ``v_dim``: size of a value row and of an output row when it is not ``head_dim``.
@@ -1602,7 +1605,9 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_le
     the call fills those kv heads' part (``attention_all_values`` covers all of them).
     ``out`` may be float32 whatever the element type of q.
     ``dist_bias``: float32 [query heads, L]; key j adds entry min(p - j, L - 1) of its head's row to the score
-    after the scale and the cap."""
+    after the scale and the cap.
+    ``max_keys``: with pages, a bound on the sequences' lengths, by which the work is cut (the page table may be
+    much wider)."""
     _check_dist_bias(dist_bias, n_kv * group)
     _check_sink(sink, n_kv * group)
     _check_sink(slopes, n_kv * group)
@@ -1624,7 +1629,7 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_le
     if q.dtype == torch.float32 and out.dtype == torch.float32 and not v_all and not ring_from and not (keep_first and window > 0) \
             and _attn_f32_ok(head_dim, vd, q, k, v, kv_stride, v_stride):
         _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group,
-                       head_dim, vd, scale, cap, window, int(chunk), sink, slopes, dist_bias, batch, max_q_len)
+                       head_dim, vd, scale, cap, window, int(chunk), sink, slopes, dist_bias, batch, max_q_len, max_keys)
         return
     f = _fn("attn_simt", "brolm_attn_simt", [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                              c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,

@@ -343,7 +343,7 @@ class Attention(Part):
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring, page_size=page,
                                          n_splits=splits, longest_first=self._longest_first(ctx, splits), **{n: a for n, a in common.items() if n not in ("v_dim", "max_q_len")})
         else:
-            kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table,
+            kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table, max_keys=ctx.max_kv_len,
                                    ring=ring, page_size=page, **common)
         return linear(out, self.w_o, out_dtype=torch.float32, parts_ok=True)
 
@@ -429,7 +429,7 @@ class Attention(Part):
                 source = dict(k=k, v=v)
             else:
                 source = dict(k_pages=k_pages, v_pages=v_pages, page_table=table, ring=ring, page_size=page,
-                              ring_from=ctx.ring_from(kv_entry))
+                              ring_from=ctx.ring_from(kv_entry), max_keys=ctx.max_kv_len)
             # bfloat16 without a chunked mask runs on the tensor cores, all else on the exact kernel
             tensor = self._tensor_cores(ctx) and not self.chunk and not (scored and self.talk) and \
                 kernels.attention_headmix_ok(self.head_dim, self.v_dim, group, ctx.mode != "prefill", page)
@@ -501,7 +501,7 @@ class Attention(Part):
             kernels.attention_decode_mma(q, out, ctx.cu_q, ctx.kv_len, k_pages, v_pages, table, ring=ring,
                                          page_size=page, n_splits=splits, longest_first=self._longest_first(ctx, splits), **args)
         else:
-            kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table,
+            kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=k_pages, v_pages=v_pages, page_table=table, max_keys=ctx.max_kv_len,
                                    ring=ring, page_size=page, **common)
 
 

@@ -189,7 +189,7 @@ class LatentAttention(Part):
                 raise NotImplementedError("a layer that reads another layer's windowed cache cannot take a "
                                           "prompt longer than the ring in one step")
             kernels.attention_simt(q, out, ctx.cu_q, ctx.kv_len, k_pages=pages, v_pages=pages, page_table=table,
-                                   ring=ring, page_size=page, max_q_len=ctx.max_q_len, **common)
+                                   ring=ring, page_size=page, max_q_len=ctx.max_q_len, max_keys=ctx.max_kv_len, **common)
         o = torch.empty((T, H * self.dv), dtype=x.dtype, device=x.device)
         head_gate = proj[:, self.gate_from:self.gate_from + H] if self.head_gate else None
         kernels.heads_linear(out, D, self.w_uv, o, self.dv, gate=head_gate)

@@ -190,3 +190,13 @@ def test_float_attention_shares_spans_only_where_the_merge_is_worth_it():
     assert not worth(1, 2, 2, 32, 32, 300, 300, window=16) and not worth(1, 8, 4, 128, 128, 300, 300, window=64)
     assert worth(1, 4, 2, 256, 256, 300, 300, window=100) and not worth(32, 8, 4, 128, 128, 1, 256)
     assert not worth(1, 4, 2, 256, 256, 1, None)                                               # no bound
+
+
+def test_float_attention_is_cut_by_the_lengths_not_by_the_table():
+    """A page table for 32,768 tokens and sequences of at most 512: four spans, not 256, and no more scratch than for those."""
+    bound = kernels.attn_f32_max_keys
+    assert bound(32768, 1 << 30, 512) == 512 and bound(32768, 1 << 30) == 32768 and bound(256, 1 << 30, 512) == 256
+    assert bound(256, 256, 300) == 300 and bound(256, 256) is None and bound(256, 256, 0) is None
+    splits = lambda keys, batch: kernels.attn_f32_splits(batch, 4, 2, 256, batch, 1, keys, sms=148)
+    assert splits(bound(32768, 1 << 30, 512), 3) == 4
+    assert splits(bound(32768, 1 << 30, 512), 32) == 4 and splits(bound(32768, 1 << 30), 32) == 0

@@ -944,6 +944,28 @@ def test_float_attention_of_parts_of_spans(monkeypatch, lengths, window, chunk, 
         close(out[at:at + n], ref.transpose(0, 1).reshape(n, -1).cpu(), torch.float32, scale=float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("bound", [700, 512, 100])
+def test_float_attention_with_a_bound_on_the_keys(monkeypatch, bound):
+    """A bound cuts the work; one that does not hold costs no keys."""
+    g = torch.Generator(device=DEV).manual_seed(bound)
+    lengths, n_kv, hd = [700, 3, 450, 128], 2, 32
+    B = len(lengths)
+    table = torch.randperm(64 * B, generator=g, device=DEV).to(torch.int32).view(B, 64)
+    kp, vp = (torch.randn(64 * B, n_kv, 64, hd, generator=g, device=DEV) for _ in range(2))
+    q = torch.randn(B, n_kv * 2 * hd, generator=g, device=DEV)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: True)
+    outs = []
+    for keys in (None, bound):
+        outs.append(torch.full_like(q, float("nan")))
+        kernels.attention_simt(q, outs[-1], torch.arange(B + 1, dtype=torch.int32, device=DEV),
+                               torch.tensor(lengths, dtype=torch.int32, device=DEV), n_kv=n_kv, group=2, head_dim=hd, scale=0.2, cap=0.0,
+                               window=0, batch=B, max_q_len=1, k_pages=kp, v_pages=vp, page_table=table, ring=1 << 30, page_size=64,
+                               max_keys=keys)
+    if bound >= max(lengths):
+        assert torch.equal(*outs)
+    close(outs[1], outs[0].double().cpu(), torch.float32)
+
+
 @pytest.mark.parametrize("window", [1, 100, 128, 129, 257, 300, 400])
 @pytest.mark.parametrize("shared", [False, True])
 def test_float_attention_in_wrapped_rings_gives_the_bits_of_the_prompt(monkeypatch, window, shared):
