@@ -1626,7 +1626,9 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, kv_le
         assert k is not None and v is not None and k.dtype == q.dtype and v.dtype == q.dtype
         assert k.stride(-1) == 1 and v.stride(-1) == 1
         kv_stride, v_stride = k.stride(0), v.stride(0)
-    if q.dtype == torch.float32 and out.dtype == torch.float32 and not v_all and not ring_from and not (keep_first and window > 0) \
+    # (kept first keys without a window are all keys; what the kernel for all options refuses goes to it to be refused)
+    kept = keep_first != 0 and not (keep_first > 0 and window <= 0 and chunk <= 0)
+    if q.dtype == torch.float32 and out.dtype == torch.float32 and not v_all and not ring_from and not kept \
             and _attn_f32_ok(head_dim, vd, q, k, v, kv_stride, v_stride):
         _attention_f32(q, out, cu_q, kv_len, k, v, k_pages, v_pages, page_table, pt_stride, ring, page_size, n_kv, group,
                        head_dim, vd, scale, cap, window, int(chunk), sink, slopes, dist_bias, batch, max_q_len, max_keys)

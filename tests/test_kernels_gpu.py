@@ -944,6 +944,15 @@ def test_float_attention_of_parts_of_spans(monkeypatch, lengths, window, chunk, 
         close(out[at:at + n], ref.transpose(0, 1).reshape(n, -1).cpu(), torch.float32, scale=float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("options", [dict(keep_first=4, chunk=8), dict(keep_first=-1), dict(keep_first=-1, window=5)])
+def test_float_attention_refuses_the_options_that_exclude_each_other(options):
+    x = torch.zeros(8, 32, device=DEV)
+    with pytest.raises(kernels.KernelError):
+        kernels.attention_simt(x, torch.empty_like(x), torch.tensor([0, 8], dtype=torch.int32, device=DEV),
+                               torch.tensor([8], dtype=torch.int32, device=DEV), k=x, v=x, batch=1, max_q_len=8,
+                               **{**dict(n_kv=1, group=1, head_dim=32, scale=1.0, cap=0.0, window=0), **options})
+
+
 @pytest.mark.parametrize("bound", [700, 512, 100])
 def test_float_attention_with_a_bound_on_the_keys(monkeypatch, bound):
     """A bound cuts the work; one that does not hold costs no keys."""
