@@ -2,7 +2,9 @@
 // whole 16-byte pieces of at most 256 elements (attn_simt.cu has the masks and options, and takes everything else).
 //
 // One order of operations for a query, whatever step, batch or split it runs in, so that a prompt pass and a decode pass
-// give the same bits.  Keys come in spans of 128, anchored at multiples of 128 of the absolute position:
+// give the same bits for finite values.  (A tile reads the values of all keys that any of its rows sees, and gives those
+// that a row does not see the weight zero: zero times an infinity or a NaN of a later token reaches the rows before it in the
+// tile, and a decode pass does not read it.)  Keys come in spans of 128, anchored at multiples of 128 of the absolute position:
 //
 //   score    s_j = (sum over even c of q_c k_c) + (sum over odd c), each a chain of fmas over ascending c; then the
 //            scale, the cap, the slope, the distance bias and the mask

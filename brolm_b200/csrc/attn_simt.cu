@@ -1,9 +1,9 @@
 // Soft-capped, windowed, causal grouped-query attention on CUDA cores, for
 // float and bfloat16 elements, with every product, score and sum in float.
 //
-// This is the exact path: the float model uses it for prompts and for
-// decoding, and it is the reference the tensor-core kernels are checked
-// against.  One block handles one (sequence, kv head) and a tile of 32
+// This is the path for all sizes, masks and options (attn_f32.cu has the
+// float model's usual ones), and the reference the tensor-core kernels are
+// checked against.  One block handles one (sequence, kv head) and a tile of 32
 // "rows"; a row is a (query token, query head of the group) pair, so all
 // query heads that share a kv head reuse the same staged keys and values.
 //
@@ -14,7 +14,8 @@
 // order with one online-softmax update per tile.  The order of operations for
 // one query therefore does not depend on how the tokens were cut into steps
 // or on what else is in the batch: a prompt pass and a decode pass give the
-// same bits for the same inputs.
+// same bits for the same finite inputs (a key that a row of the tile does not
+// see has the weight zero, and zero times an infinity is a NaN).
 //
 // Scores follow wlejon/brolm src/gemma2.cpp:360-367: s = (q.k) * scale, then
 // cap * tanh(s / cap), then the mask, then softmax.  Key j is visible from a

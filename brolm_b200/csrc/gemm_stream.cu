@@ -4,8 +4,10 @@
 // With few tokens the product is a stream of W from memory, and the kernel is
 // built as one: the roles of the operands are swapped (128 rows of W fill the M
 // side of tcgen05.mma, the tokens the N side), and persistent blocks pull their
-// share of W through deep rings of TMA stages (up to ten 16 KB tiles in flight
-// per SM), so the stream never drains between a block's work items.  A work item is a (128-row tile of W, slice of K) pair; for the
+// share of W through deep rings of TMA stages (a 16 KB tile and its tokens; up
+// to ten in a block, or six in each of the two blocks of an SM), so the stream
+// never drains between a block's work items.  A work item is a (128-row tile of
+// W, slice of K) pair; for the
 // 2304-wide outputs of the model K is cut into slices so that every SM has an
 // item, and the float partial sums of the slices are added, in order, by the
 // kernel that reads them (the residual kernel).
@@ -35,11 +37,12 @@ using namespace tc;
 constexpr int BR = 128, BK = 64;
 constexpr int THREADS = 192;
 constexpr int W_BYTES = BR * BK * 2;
-// One block an SM with a ring of 200 KB, or, where there are more items than SMs, two with 108 KB each: as many bytes in
-// flight, but one block streams while the other starts or stores, a round holds twice as many items (9B gate and up are
-// 224 for 148 SMs, two rounds of which the second is half empty), and the next kernel's first block finds room as soon
-// as one of the two is done.  At 16 tokens, one / two blocks an SM: 28,672 x 3,584 gated 46.8 / 34.0 us (31.9 at the
-// memory's rate), 3,584 x 14,336 in 5 / 10 slices 20.2 / 18.9 us (15.9), 8,192 x 3,584 in 2 / 4 slices 13.5 / 11.8 us.
+// One block an SM with a ring of 200 KB, or, where there are more items than SMs, two with 108 KB each (at 16 tokens
+// twice six stages for ten, at 128 twice three for six): one block streams while the other starts or stores, a round holds
+// twice as many items (9B gate and up are 224 for 148 SMs, two rounds of which the second is half empty), and the next
+// kernel's first block finds room as soon as one of the two is done.  At 16 tokens, one / two blocks an SM: 28,672 x
+// 3,584 gated 46.8 / 34.0 us (31.9 at the memory's rate), 3,584 x 14,336 in 5 / 10 slices 20.2 / 18.9 us (15.9), 8,192 x
+// 3,584 in 2 / 4 slices 13.5 / 11.8 us.
 template <int PER_SM> constexpr int ring_bytes() { return PER_SM == 2 ? 108 * 1024 : 200 * 1024; }
 
 enum : int { EPI_STORE = 0, EPI_GATED = 1, EPI_SOFTCAP = 2 };
