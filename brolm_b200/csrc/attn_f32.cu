@@ -61,9 +61,6 @@ struct F32Args {
     float* part_ml;                           // [token][head][split][2]
 };
 
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t v;
     asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(lo), "f"(hi));
@@ -74,17 +71,10 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
     asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
     return f;
 }
-struct Pair2 { uint64_t x, y; };
 __device__ __forceinline__ Pair2 lds4(const float* p) {
     const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
     return Pair2{v.x, v.y};
 }
-__device__ __forceinline__ void copy16(void* dst, const float* p, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(p),
-                 "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // a slice of keys, or of values
 __host__ __device__ __forceinline__ int stage_bytes(const F32Args& a) {
@@ -139,6 +129,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
     const int q_pitch = (a.hd + KC - 1) / KC * KC + 4;  // floats; zeros behind hd
     const int stage = stage_bytes(a);
     uint8_t* ring = raw;
+    const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
     float* Qs = reinterpret_cast<float*>(raw + STAGES * stage);
     float* P = Qs + ROWS * q_pitch;
     float* stats = P + ROWS * P_PITCH;                  // [ROWS]: M, L, factor of what is held, factor of what comes
@@ -203,7 +194,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
         const int v_from = part0 * 32, slices = k_slices + (keys - v_from + VK - 1) / VK;
         auto fetch_v = [&](int i) {
             if (i < slices) {
-                uint8_t* dst = ring + (i % STAGES) * stage;
+                const uint32_t dst = ring_at + (i % STAGES) * stage;
                 const int pieces = a.vd / 4;
                 for (int idx = tid; idx < VK * pieces; idx += THREADS) {
                     const int j = idx / pieces, c = (idx - j * pieces) * 4;
@@ -217,7 +208,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
             constexpr int N = decltype(count)::value, NJ = N * 32 / LN;
             auto fetch = [&](int i) {
                 if (i >= k_slices) return fetch_v(i);
-                uint8_t* dst = ring + (i % STAGES) * stage;
+                const uint32_t dst = ring_at + (i % STAGES) * stage;
                 const int c = i * KC + (tid & 7) * 4;
 #pragma unroll
                 for (int j = 0; j < N * 2; ++j) {

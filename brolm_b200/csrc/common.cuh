@@ -121,6 +121,19 @@ __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
     }
 }
 
+// Two float fmas in one instruction: the halves of a 64-bit register.
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+struct Pair2 { uint64_t x, y; };       // four consecutive floats
+
+// 16 bytes on their way from global into shared memory, zeros when !ok
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
 // A gate that is clamped from above and a partner that is clamped on both sides and shifted by one:
 //     g' = min(g, limit),  u' = clamp(u, -limit, limit),  g' * sigmoid(1.702 g') * (u' + 1)
 // (activation code 2 of the gated feed-forward; codes 0 and 1 are act(g) * u with gelu and silu).

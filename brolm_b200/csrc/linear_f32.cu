@@ -28,26 +28,16 @@ namespace {
 
 constexpr int SEG = 512;        // k of one C_s
 
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ float halves_sum(uint64_t v) {
     float lo, hi;
     asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v));
     return lo + hi;
 }
-struct Pair2 { uint64_t x, y; };       // four consecutive floats
 __device__ __forceinline__ Pair2 lds4(uint32_t addr) {
     Pair2 v;
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
     return v;
 }
-// 16 bytes from global into shared memory, zeros when !ok
-__device__ __forceinline__ void copy16(uint32_t dst, const float* p, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(p), "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // ---------------------------------------------------------------------------
 // M <= MP <= 16.  A block owns RG * R rows of W over the whole of K, a lane R rows of one segment at a time: the
