@@ -330,9 +330,12 @@ int launch_tiles(const float* x, int ldx, const float* w, int ldw, float* y, int
     if (const int e = allow_shared_memory(tiles_kernel<BM>, smem, allowed)) return e;
     const int n_seg = (K + SEG - 1) / SEG;
     const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, parts ? (n_seg + seg_per_block - 1) / seg_per_block : 1);
-    // Blocks that are let in early lie two on one SM and none on another, which costs where they do not fill all places:
-    // 64 x 1,024 x 1,024 in 16 blocks 51 us and 34 in order
-    const bool in_order = (long long)grid.x * grid.y * grid.z < 2LL * device_sm_count();
+    // Blocks that are let in early, beside what is left of the kernel before them, lie two on one SM and none on another,
+    // which costs where they do not fill all places (300 x 2,304 x 256, 90 blocks: 22.1 us and 19.7 in order; 17 x 2,304 x 2,304
+    // in 90, behind the sums of the product before: 30.9 and 22.5); a handful finds SMs of its own, and starts sooner
+    // (17 x 1,000 x 516, 8 blocks: 21.2 and 22.5).
+    const long long blocks_all = (long long)grid.x * grid.y * grid.z;
+    const bool in_order = blocks_all < 2LL * device_sm_count() && (parts || blocks_all > device_sm_count() / 4);
     auto run = [&](float* dst, int ld, int per, long long stride) {
         return in_order ? launch_in_order(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, dst, ld, M, N, K, per, stride)
                         : launch_pdl(tiles_kernel<BM>, grid, dim3(128), smem, stream, x, ldx, w, ldw, dst, ld, M, N, K, per, stride);
