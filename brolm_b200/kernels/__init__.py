@@ -1441,9 +1441,10 @@ def gemm_stream_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 def gemm_stream_parts(x: torch.Tensor, weight: torch.Tensor, sms: Optional[int] = None) -> int:
     """Slices of K so that every SM gets a (128-row tile, slice) item of the weight stream, two items where the weights
-    are many enough to be worth twice the slices (which the kernel after it adds): a decode step of 24 sequences at the 9B
-    sizes, whose matrices have 59 and 103 MB, 6,323 us with one and 6,081 with two; at the 2B sizes (19 and 42 MB) no
-    difference."""
+    are many enough to be worth twice the slices, which the kernel after it adds.  Product and residual kernel at 24 tokens,
+    one / two items an SM: 2,304 x 9,216 (42 MB) 19.5 / 16.2 us, 3,072 x 8,064 (50) 21.0 / 16.6, 8,192 x 3,584 (59) 25.9 / 19.7, 3,584
+    x 14,336 (103) 30.8 / 27.5; a decode step of 24 sequences at the 9B sizes 6,323 / 6,081 us, at the 2B sizes (19 and
+    42 MB), where the slices' sums are the larger share, no difference."""
     sms = sms or device_sms(x.device if x.is_cuda else None)
     row_tiles = (weight.shape[0] + 127) // 128
     nkb = (x.shape[1] + 63) // 64

@@ -4,6 +4,7 @@
     python -m brolm_b200.kernels.microbench attn_prefill --tokens 2048
     python -m brolm_b200.kernels.microbench norms --batch 8
     python -m brolm_b200.kernels.microbench stream --batch 64            (the weight stream against the library)
+    python -m brolm_b200.kernels.microbench float --tokens 300           (a float layer's products and its attention)
     python -m brolm_b200.kernels.microbench timeline_decode --batch 8 --ctx 8192 --layers 6
     python -m brolm_b200.kernels.microbench timeline_prefill --tokens 2048 --layers 4
 
@@ -17,8 +18,9 @@ import math
 
 import torch
 
-from . import (attention_decode_mma, attention_prefill_mma, attention_prefill_tc, attention_prefill_tc_split, attention_tc_status, decode_splits, gemm_tc, gemm_tc_status, residual_rmsnorm,
-               rmsnorm, skinny_gemm)
+from . import (attention_decode_mma, attention_prefill_mma, attention_prefill_tc, attention_prefill_tc_split, attention_simt,
+               attention_tc_status, decode_blocks_per_sm, decode_longest_first, decode_splits, gemm_tc, gemm_tc_status, linear_f32,
+               residual_rmsnorm, rmsnorm, skinny_gemm)
 
 DEV = "cuda:0"
 
@@ -54,14 +56,15 @@ def attn_decode(args) -> None:
     kv_len = torch.full((B,), ctx, dtype=torch.int32, device=DEV)
     if args.ragged:              # lengths spread evenly between a fifth of the context and all of it
         kv_len = torch.linspace(ctx / 5, ctx, B).round().int()[torch.randperm(B, generator=torch.Generator().manual_seed(1))].to(DEV)
-    splits = args.splits or decode_splits(B, n_kv, ctx, args.window, ragged=args.ragged)
+    splits = args.splits or decode_splits(B, n_kv, ctx, args.window, ragged=args.ragged, per_sm=decode_blocks_per_sm(hd))
     n = B * n_q * splits
     scratch = (torch.empty(n * hd, dtype=torch.float32, device=DEV), torch.empty(n * 2, dtype=torch.float32, device=DEV))
 
     def run():
         attention_decode_mma(q, out, cu, kv_len, kp, vp, table, ring=ring, page_size=64, n_kv=n_kv, group=n_q // n_kv,
                              head_dim=hd, scale=1 / math.sqrt(hd), cap=50.0, window=args.window, batch=B,
-                             n_splits=splits, scratch=scratch)
+                             n_splits=splits, scratch=scratch,
+                             longest_first=decode_longest_first(args.ragged, splits, ctx, args.window, hd))
 
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=DEV)
     ms = timed(run, args.reps, flush)
@@ -99,6 +102,24 @@ def attn_prefill(args) -> None:
         cut = f" cut={attention_prefill_tc_split(T, n_kv, n_q // n_kv, args.window, 1) if n_split is None else n_split}" if fn is run_tc else ""
         print(f"attn_prefill {name} tokens={T} window={args.window}{cut}: {ms * 1e3:.1f} us, {flops / ms / 1e9:.1f} TFLOP/s")
     print("attention_tc status", attention_tc_status())
+
+
+def float_layer(args) -> None:
+    """The four products of a float32 layer and the attention of one prompt, at --tokens tokens."""
+    T, n_q, n_kv, hd = args.tokens, args.heads, args.kv_heads, args.head_dim
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=DEV)
+    for name, N, K in (("q/k/v", (n_q + 2 * n_kv) * hd, args.hidden), ("o", args.hidden, n_q * hd),
+                       ("gate+up", 2 * args.inter, args.hidden), ("down", args.hidden, args.inter)):
+        x, w, y = torch.randn(T, K, device=DEV), torch.randn(N, K, device=DEV), torch.empty(T, N, device=DEV)
+        ms = timed(lambda: linear_f32(x, w, y), args.reps, flush)
+        print(f"{name} {T} x {N} x {K}: {ms * 1e3:.1f} us, {2e-9 * T * N * K / ms:.1f} TFLOP/s, {4e-6 * N * K / ms:.0f} GB/s of weights")
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * hd, device=DEV)
+    out = torch.empty(T, n_q * hd, device=DEV)
+    cu, length = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.tensor([T], dtype=torch.int32, device=DEV)
+    ms = timed(lambda: attention_simt(qkv[:, :n_q * hd], out, cu, length, k=qkv[:, n_q * hd:(n_q + n_kv) * hd],
+                                      v=qkv[:, (n_q + n_kv) * hd:], n_kv=n_kv, group=n_q // n_kv, head_dim=hd,
+                                      scale=1 / math.sqrt(hd), cap=args.cap, window=args.window, batch=1, max_q_len=T), args.reps, flush)
+    print(f"attention: {ms * 1e3:.1f} us")
 
 
 def model_prefill(args) -> None:
@@ -279,7 +300,7 @@ def timeline_prefill(args) -> None:
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("what", choices=["attn_decode", "attn_prefill", "model_prefill", "norms", "skinny", "gemm", "stream",
+    ap.add_argument("what", choices=["attn_decode", "attn_prefill", "model_prefill", "norms", "skinny", "gemm", "stream", "float",
                                      "timeline_decode", "timeline_prefill"])
     ap.add_argument("--inter", type=int, default=9216)
     ap.add_argument("--layers", type=int, default=2)
@@ -302,7 +323,7 @@ def main() -> None:
         from .. import kernels
         kernels.USE_TC_GEMM = False
     {"attn_decode": attn_decode, "attn_prefill": attn_prefill, "model_prefill": model_prefill,
-     "norms": norms, "skinny": skinny, "gemm": gemm, "stream": stream,
+     "norms": norms, "skinny": skinny, "gemm": gemm, "stream": stream, "float": float_layer,
      "timeline_decode": timeline_decode, "timeline_prefill": timeline_prefill}[args.what](args)
 
 

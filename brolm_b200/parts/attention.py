@@ -285,7 +285,7 @@ class Attention(Part):
             kernels.skinny_qkv_rope(x, self.w_qkv, qkv, ctx.positions, cos_sin, self.n_q, self.n_kv, self.head_dim,
                                     *kept, page)
         elif kernels.stream_rows(x, self.w_qkv) and (cos_sin is None or rot == self.head_dim):
-            # 17 to 128 tokens: the weights stream once through tcgen05, cut along K so that every SM takes
+            # 17 to 32 tokens: the weights stream once through tcgen05, cut along K so that every SM takes
             # part; the kernel that rotates q and k and fills the cache adds the slices on its way
             slices = kernels.gemm_stream_parts(x, self.w_qkv)
             sums = torch.empty((slices, x.shape[0], self.q_dim + 2 * self.kv_dim), dtype=torch.float32, device=x.device)

@@ -5,14 +5,16 @@ element type in the same way).
 * float32 weight: the framework's own CUDA-core kernel, true 32-bit.
 * bfloat16 weight, up to 16 rows (decode steps): the framework's own
   weight-streaming tensor-core kernel, float32 accumulation.
-* bfloat16 weight, 17 to 128 rows (wider decode batches, short prompts): the
-  framework's tcgen05 weight stream (TMA ring, tokens on the N side of the
-  instruction), float32 accumulation.
+* bfloat16 weight, 17 to 32 rows (``kernels.STREAM_ROWS``; wider decode
+  batches, short prompts): the framework's tcgen05 weight stream (TMA ring,
+  tokens on the N side of the instruction), float32 accumulation.
 * bfloat16 weight, more rows: the framework's tcgen05 kernel (TMA loads,
-  accumulator in tensor memory), float32 accumulation; the library product
-  (cuBLAS through torch) only for operands that kernel does not take (a width
-  that is no multiple of 8) or that leave most SMs without a tile.  The result
-  is bfloat16 or, on request, float32.
+  accumulator in tensor memory), float32 accumulation, where there are at
+  least as many output tiles as SMs; else, and for operands that kernel does
+  not take (a width that is no multiple of 8), the library product (cuBLAS
+  through torch), which so has most products of 33 to 128 rows and, at 2,048
+  rows, the narrow ones (o and down of the 2B sizes).  The result is bfloat16
+  or, on request, float32.
 """
 from __future__ import annotations
 
@@ -56,7 +58,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
             kernels.skinny_gemm(x, weight, y)
             return y
         if kernels.stream_rows(x, weight) and want in (torch.bfloat16, torch.float32):
-            # 17 to 128 tokens: still a stream of the weights, on tcgen05 with the tokens on the N side
+            # 17 to 32 tokens: still a stream of the weights, on tcgen05 with the tokens on the N side
             parts = kernels.gemm_stream_parts(x, weight) if (parts_ok and want == torch.float32 and out is None) else 1
             if parts > 1:
                 y = torch.empty((parts, M, N), dtype=torch.float32, device=x.device)
