@@ -361,30 +361,45 @@ constexpr int SLOTS = 3;
 template <bool APART> __host__ __device__ constexpr size_t decode_slot(int hd) { return (APART ? 1 : 2) * (size_t)KT * hd * 2; }
 constexpr int PT_ROW = 512;          // entries of a page-table row kept in shared memory (32768 keys)
 
-// The sequence of place `rank` when n <= MAX_BY_LENGTH sequences stand in order of falling length, equal ones in their own:
-// the largest bound that more than `rank` of them reach is that sequence's (length, place from behind), found bit by bit
-// by each warp for itself.  (Counting, for every sequence, those ahead of it took a block of 512 some 10 us.)
+// The sequence of place `rank` when n <= MAX_BY_LENGTH sequences stand in order of falling length in pages, equal ones in
+// their own.  Each warp finds it for itself: up to 32 sequences are counted against one another by shuffles; of more, the
+// largest bound that more than `rank` of them reach is that sequence's (pages, place from behind), found bit by bit.  (A
+// decode step's launch of 16 sequences of 128 to 6,144 keys, 8 kv heads: 70 us; a block that counted all pairs took 10 us to
+// start with 512 sequences.)
 constexpr int MAX_BY_LENGTH = 512;
-__device__ __forceinline__ int by_falling_length(const int* kv_len, int n, int rank) {
-    const int lane = threadIdx.x & 31;
-    uint32_t key[MAX_BY_LENGTH / 32], most = 0;
+__device__ __forceinline__ uint32_t length_key(const int* kv_len, int n, int i) {
+    return i < n ? (uint32_t)((max(kv_len[i], 0) + KT - 1) / KT) * MAX_BY_LENGTH + (MAX_BY_LENGTH - 1 - i) : 0u;
+}
+template <int J>
+__device__ __forceinline__ int by_bits(const int* kv_len, int n, int rank) {
+    uint32_t key[J], most = 0;
 #pragma unroll
-    for (int j = 0; j < MAX_BY_LENGTH / 32; ++j) {
-        const int i = j * 32 + lane;
-        key[j] = i < n ? (uint32_t)min(max(kv_len[i], 0), (1 << 22) - 1) * MAX_BY_LENGTH + (MAX_BY_LENGTH - 1 - i) : 0u;
+    for (int j = 0; j < J; ++j) {
+        key[j] = length_key(kv_len, n, j * 32 + (threadIdx.x & 31));
         most = max(most, key[j]);
     }
     most = __reduce_max_sync(0xffffffffu, most);
     uint32_t bound = 0;
-    for (int bit = 31 - __clz(most | 1); bit >= 0; --bit) {
+    for (int bit = 31 - __clz(most); bit >= 0; --bit) {
         const uint32_t next = bound | (1u << bit);
         int reach = 0;
 #pragma unroll
-        for (int j = 0; j < MAX_BY_LENGTH / 32; ++j)
-            if (j * 32 < n) reach += key[j] >= next;
+        for (int j = 0; j < J; ++j) reach += key[j] >= next;
         if (__reduce_add_sync(0xffffffffu, reach) > rank) bound = next;
     }
     return MAX_BY_LENGTH - 1 - (int)(bound % MAX_BY_LENGTH);
+}
+__device__ __forceinline__ int by_falling_length(const int* kv_len, int n, int rank) {
+    if (n <= 32) {
+        const uint32_t key = length_key(kv_len, n, threadIdx.x & 31);
+        int ahead = 0;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) ahead += __shfl_sync(0xffffffffu, key, j) > key;
+        return __ffs(__ballot_sync(0xffffffffu, key && ahead == rank)) - 1;
+    }
+    if (n <= 64) return by_bits<2>(kv_len, n, rank);
+    if (n <= 128) return by_bits<4>(kv_len, n, rank);
+    return by_bits<MAX_BY_LENGTH / 32>(kv_len, n, rank);
 }
 
 template <int HD_MAX, bool EXACT, bool BIAS, bool APART>
