@@ -226,25 +226,22 @@ __global__ void __launch_bounds__(THREADS, PER_SM) gemm_stream_kernel(const __gr
                 float o[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) o[i] = __uint_as_float(v[i]);
-                int col;
-                bool writer = true;
+                int col, first = 0;                             // of the sixteen tokens, the first that this lane stores
                 if (EPI == EPI_GATED) {
-                    // lanes 0-63 hold the gate values of 64 outputs, lanes 64-127 their up values
+                    // lanes 0-63 hold the gate values of 64 outputs, lanes 64-127 their up values: they exchange halves, and
+                    // each makes the results of eight tokens
                     col = rt * 64 + (lrow & 63);
-                    if (quarter >= 2) {
+                    first = quarter < 2 ? 0 : 8;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) upx[i * 64 + lrow - 64] = o[i];
-                    }
+                    for (int i = 0; i < 8; ++i) upx[(8 - first + i) * 64 + (lrow & 63)] = quarter < 2 ? o[8 + i] : o[i];
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (quarter < 2) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {                       // code 2: cap is its limit
-                            // up to 16 tokens: the activation of the few-token product, which serves the other sizes
-                            const float u = upx[i * 64 + lrow];
-                            o[i] = BT == 16 ? gate_pair(o[i], u, g.act, g.cap) : fast_gate_pair(o[i], u, g.act, g.cap);
-                        }
+                    for (int i = 0; i < 8; ++i) {                           // code 2: cap is its limit
+                        const float other = upx[(first + i) * 64 + (lrow & 63)];
+                        const float z = quarter < 2 ? o[i] : other, u = quarter < 2 ? other : o[8 + i];
+                        // up to 16 tokens: the activation of the few-token product, which serves the other sizes
+                        o[i] = BT == 16 ? gate_pair(z, u, g.act, g.cap) : fast_gate_pair(z, u, g.act, g.cap);
                     }
-                    writer = quarter < 2;
                     asm volatile("bar.sync 1, 128;" ::: "memory");          // upx may be written again
                 } else {
                     col = rt * BR + lrow;
@@ -253,10 +250,10 @@ __global__ void __launch_bounds__(THREADS, PER_SM) gemm_stream_kernel(const __gr
                         for (int i = 0; i < 16; ++i) o[i] = soft_cap(o[i] * g.mul, g.cap);
                     }
                 }
-                if (writer && col < g.N) {
+                if (col < g.N) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int tok = c + i;
+                    for (int i = 0; i < (EPI == EPI_GATED ? 8 : 16); ++i) {
+                        const int tok = c + first + i;
                         if (tok < g.M) {
                             if (g.ksplit > 1) reinterpret_cast<float*>(g.y)[ks * g.part_stride + (size_t)tok * g.ldy + col] = o[i];
                             else if (g.out_f32) reinterpret_cast<float*>(g.y)[(size_t)tok * g.ldy + col] = o[i];
