@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
     const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
     float* Qs = reinterpret_cast<float*>(raw + STAGES * stage);
     float* P = Qs + ROWS * q_pitch;
-    float* stats = P + ROWS * P_PITCH;                  // [ROWS]: M, L, factor of what is held, factor of what comes
+    float* stats = P + ROWS * P_PITCH;                  // [ROWS]: M, L, and from the second span on the factors of what is held and of what comes
     long long* k_off = reinterpret_cast<long long*>(stats + 4 * ROWS);
     long long* v_off = k_off + SPAN;
 
@@ -152,10 +152,19 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
     const int tn = tid % LN, tm = tid / LN;
     const int key_hi = t.first_pos + (t.row0 + t.rows - 1) / a.group;
 
-    if (tid < ROWS) {
-        stats[tid] = -INFINITY;
-        stats[ROWS + tid] = 0.0f;
-    }
+    auto load_q = [&] {
+        for (int idx = tid; idx < ROWS * (q_pitch / 4); idx += THREADS) {
+            const int r = idx / (q_pitch / 4), c = (idx - r * (q_pitch / 4)) * 4;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (r < t.rows && c < a.hd) {
+                const int row = t.row0 + r;
+                v = *reinterpret_cast<const float4*>(a.q + (size_t)(t.q0 + row / a.group) * a.q_stride +
+                                                     (g * a.group + row % a.group) * a.hd + c);
+            }
+            *reinterpret_cast<float4*>(Qs + r * q_pitch + c) = v;
+        }
+    };
+    if (ROWS == 8) load_q();
 
     const int k_slices = (a.hd + KC - 1) / KC;
     float tot[RI][VJ][4];
@@ -167,9 +176,11 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
     for (bool first = true; span <= last; ++span, first = false) {
         const int key0 = span * SPAN;
         const int keys = min(a.max_parts * 32, key_hi + 1 - key0);      // keys behind the tile's last query are not read
-        // the 32-key parts of the span that any row sees: part0 and as many as make one, two or all four
+        // the 32-key parts of the span that any row sees: part0 and as many as make one, two or all four.  (Tiles of eight
+        // rows, decoding, always work on all four: a step runs each instruction about once, and what a launch of three
+        // variants fetches of them is a tenth of its time, 30 us against 26 a layer of 4 kv heads of 256 at 420 keys.)
         int part0 = max(0, t.key_lo - key0) / 32, n_parts = (keys - 1) / 32 - part0 + 1;
-        if (n_parts > 2) part0 = 0, n_parts = 4;
+        if (ROWS == 8 || n_parts > 2) part0 = 0, n_parts = 4;
         __syncthreads();                                // the span before this one is done with
         {
             const int kp = key0 + tid;
@@ -221,18 +232,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
             };
 #pragma unroll
             for (int i = 0; i < STAGES - 1; ++i) fetch(i);
-            if (first) {                                    // (seen by all behind the first slice's barrier)
-                for (int idx = tid; idx < ROWS * (q_pitch / 4); idx += THREADS) {
-                    const int r = idx / (q_pitch / 4), c = (idx - r * (q_pitch / 4)) * 4;
-                    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (r < t.rows && c < a.hd) {
-                        const int row = t.row0 + r;
-                        v = *reinterpret_cast<const float4*>(a.q + (size_t)(t.q0 + row / a.group) * a.q_stride +
-                                                             (g * a.group + row % a.group) * a.hd + c);
-                    }
-                    *reinterpret_cast<float4*>(Qs + r * q_pitch + c) = v;
-                }
-            }
+            if (ROWS == 32 && first) load_q();              // (seen by all behind the first slice's barrier)
             uint64_t s[RI][NJ];
 #pragma unroll
             for (int i = 0; i < RI; ++i)
@@ -318,16 +318,22 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
                 if (lane < RB) {
                     const float mine = lane == 0 ? m[0] : m[1], sum = lane == 0 ? l[0] : l[1];
                     const int r = r0 + lane;
-                    float M = stats[r], L = stats[ROWS + r], held, fresh;
-                    merge_factors(M, L, mine, sum, held, fresh);
-                    stats[r] = M;
-                    stats[ROWS + r] = L;
-                    stats[2 * ROWS + r] = held;
-                    stats[3 * ROWS + r] = fresh;
+                    if (first) {                             // nothing is held: what comes is taken as it is
+                        stats[r] = mine;
+                        stats[ROWS + r] = sum;
+                    } else {
+                        float M = stats[r], L = stats[ROWS + r], held, fresh;
+                        merge_factors(M, L, mine, sum, held, fresh);
+                        stats[r] = M;
+                        stats[ROWS + r] = L;
+                        stats[2 * ROWS + r] = held;
+                        stats[3 * ROWS + r] = fresh;
+                    }
                 }
             }
         };
-        if (n_parts == 1) parts(Count<1>());
+        if constexpr (ROWS == 8) parts(Count<4>());
+        else if (n_parts == 1) parts(Count<1>());
         else if (n_parts == 2) parts(Count<2>());
         else parts(Count<4>());
         uint64_t acc[RI][VJ][2];
@@ -373,7 +379,7 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
 #pragma unroll
         for (int r = 0; r < RI; ++r) {
             const int rr = tm + r * RSTEP;
-            const float held = stats[2 * ROWS + rr], fresh = stats[3 * ROWS + rr];
+            const float held = first ? 0.0f : stats[2 * ROWS + rr], fresh = first ? 1.0f : stats[3 * ROWS + rr];
 #pragma unroll
             for (int j = 0; j < VJ; ++j) {
                 const float2 lo = unpack2(acc[r][j][0]), hi = unpack2(acc[r][j][1]);
@@ -490,7 +496,7 @@ BROLM_API int brolm_attn_f32(const void* q, int q_stride, void* out, int out_str
     a.splits = splits; a.part_acc = (float*)part_acc; a.part_ml = (float*)part_ml;
     // a prompt's keys are its tokens: with few of them a block takes less of an SM (16 prompts of 20 tokens, 32 heads of 128 on
     // 8 kv heads, 384 blocks: 27 us where two share an SM)
-    a.max_parts = k_pages || max_q_len > 64 ? 4 : max_q_len > 32 ? 2 : 1;
+    a.max_parts = k_pages || max_q_len > 64 || (long long)max_q_len * group <= 8 ? 4 : max_q_len > 32 ? 2 : 1;
     if ((long long)max_q_len * group <= 8) {
         if (vd <= 128) return launch<8, 1>(a, batch, max_q_len, stream);
         return launch<8, 2>(a, batch, max_q_len, stream);
