@@ -1095,7 +1095,7 @@ def linear_f32_plan(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
     they are not (100 x 256 x 1,024: 21.6 and 33.9 us).  Blocks that take single segments fill a last round better; their
     sums (``linear_f32_slices`` of an output) are written and read once more, and are not cut if they would take more than
     256 MB."""
-    if K <= 16 and M >= 8:
+    if K <= 16 and 8 <= M <= 64 * 65535:                 # (its grid has no more rows of tiles)
         return 0, 0
     if M <= 8 or (M <= 16 and K > 128):
         return 1, 0

@@ -135,7 +135,8 @@ def test_which_kernel_takes_a_float_product():
     plan = lambda M, N, K: kernels.linear_f32_plan(M, N, K, 148)
     assert plan(1, 2304, 9216) == plan(16, 2304, 2304) == plan(1, 16, 16) == (1, 0)
     assert plan(12, 100, 100) == (32, 0)                         # too short a K for streams
-    assert plan(8, 16, 16) == plan(300, 16, 16) == (0, 0)
+    assert plan(8, 16, 16) == plan(300, 16, 16) == plan(64 * 65535, 16, 16) == (0, 0)
+    assert plan(64 * 65535 + 1, 16, 16)[0] in (32, 64)           # more rows than that kernel's grid holds
     assert plan(300, 64, 64) == plan(100, 2304, 256) == (32, 0)
     assert plan(100, 256, 1024) == (32, 1)
     assert plan(2048, 2304, 9216) == plan(300, 18432, 2304) == (64, 0)
