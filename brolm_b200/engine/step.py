@@ -225,11 +225,13 @@ class Engine:
     def _check_waits(self, where: str, consequence: str) -> None:
         """Raise if a bounded wait inside one of the tcgen05 kernels ran out since the last check.
         Reads and resets every status word (each read waits for the device)."""
-        if self.device.type != "cuda" or self.model.dtype != torch.bfloat16:
+        if self.device.type != "cuda":
             return
-        codes = {"gemm_tc": kernels.gemm_tc_status(reset=True), "attn_tc": kernels.attention_tc_status(reset=True),
-                 "gemm_stream": kernels.gemm_stream_status(reset=True),
-                 "grouped_tc": kernels.grouped_tc_status(reset=True)}
+        codes = {"linear_f32_tc": kernels.linear_f32_tc_status(reset=True)}
+        if self.model.dtype == torch.bfloat16:
+            codes |= {"gemm_tc": kernels.gemm_tc_status(reset=True), "attn_tc": kernels.attention_tc_status(reset=True),
+                      "gemm_stream": kernels.gemm_stream_status(reset=True),
+                      "grouped_tc": kernels.grouped_tc_status(reset=True)}
         bad = {k: v for k, v in codes.items() if v}
         if bad:
             raise StepError(f"{where}: a wait inside a tensor-core kernel ran out ({bad}), in this step or in a "

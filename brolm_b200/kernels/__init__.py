@@ -1130,6 +1130,34 @@ def linear_f32_plan(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
     return best[1:]
 
 
+def linear_f32_tc_slices(N: int, K: int) -> int:
+    """Into how many slices of K the float32 product on tensor cores (linear_f32_tc.cu) is cut; 0: these weights are not
+    for it.  A function of the weights' size alone: every number of rows has to give a row the same bits."""
+    if N * K < 1 << 20 or K < 256 or N > 128 * 65535:
+        return 0
+    tiles, slices = -(-N // 128), 8
+    while slices > 1 and (tiles * slices > B200_SMS or K < 128 * slices or K <= (slices - 1) * _f32_tc_slice(K, slices)):
+        slices //= 2
+    return slices
+
+
+def _f32_tc_slice(K: int, slices: int) -> int:
+    return (-(-K // slices) + 63) // 64 * 64
+
+
+def linear_f32_tc_scratch(M: int, N: int, slices: int) -> bool:
+    """Whether the slices of a product of M rows are added by a kernel behind it rather than by clusters of blocks: for more
+    than 32 rows a block has an SM to itself, and only about sixteen clusters of eight such blocks find room at a time.
+    Many clusters fill their rounds all the same; then, and where the sums would take more than 256 MB, there is no scratch."""
+    return M > 32 and -(-M // 160) * -(-N // 128) < 64 and slices * M * N * 4 <= F32_PARTS_LIMIT
+
+
+def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
+    """Whether the float32 product with these weights runs on tensor cores, whatever the rows are."""
+    N, K = weight.shape
+    return not (K % 4 or weight.stride(0) % 4 or weight.data_ptr() % 16) and weight.stride(1) == 1 and linear_f32_tc_slices(N, K) > 0
+
+
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
     """out (M, N) = x (M, K) @ weight (N, K)^T, all float32, rows may be strided.  A row's bits depend on neither M
     nor its place among the rows."""
@@ -1139,9 +1167,35 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None
     M, K = x.shape
     N = weight.shape[0]
     assert weight.shape[1] == K and tuple(out.shape) == (M, N)
+    if linear_f32_tc_ok(weight) and M <= 160 * 65535:
+        _linear_f32_tc(x, weight, out, linear_f32_tc_slices(N, K))
+        return
     aligned = not (K % 4 or x.stride(0) % 4 or weight.stride(0) % 4 or x.data_ptr() % 16 or weight.data_ptr() % 16)
     kind, cut = linear_f32_plan(M, N, K, device_sms(x.device)) if aligned else (0, 0)
     _linear_f32(x, weight, out, kind, cut)
+
+
+def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, activation: str, limit: float = 0.0) -> None:
+    """out (M, F) = act(x @ gate^T) * (x @ up^T) for weight = [gate; up] (2 F, K), all float32: the bits of ``linear_f32``
+    and ``gated_act`` behind it, where ``linear_f32_tc_ok``."""
+    assert x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32
+    assert x.dim() == 2 and x.stride(1) == 1 and out.stride(1) == 1 and linear_f32_tc_ok(weight)
+    assert weight.shape == (2 * out.shape[1], x.shape[1]) and x.shape[0] == out.shape[0]
+    if activation not in ACTIVATIONS:
+        raise KernelError(f"linear_f32_gated: unknown activation '{activation}' (known: {sorted(ACTIVATIONS)})")
+    _linear_f32_tc(x, weight, out, linear_f32_tc_slices(*weight.shape), True, ACTIVATIONS[activation], limit)
+
+
+def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, slices: int, gated: bool = False, act: int = 0,
+                   limit: float = 0.0) -> None:
+    (M, K), N = x.shape, out.shape[1]
+    parts = None
+    if slices > 1 and not gated and linear_f32_tc_scratch(M, N, slices) and not (x.stride(0) % 4 or x.data_ptr() % 16):
+        parts = torch.empty((slices, M, N), dtype=torch.float32, device=x.device)
+    f = _fn("linear_f32_tc", "brolm_linear_f32_tc", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
+                                                     c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p])
+    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, slices,
+             _f32_tc_slice(K, slices), int(gated), act, limit, _ptr(parts), _stream()), "linear_f32_tc")
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, kind: int, cut: int) -> None:
@@ -1151,6 +1205,16 @@ def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, kind: 
                                                c_int, c_void_p, c_int, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, kind, _ptr(parts), cut,
              _stream()), "linear_f32")
+
+
+def linear_f32_tc_status(reset: bool = False) -> int:
+    """0 if no bounded wait inside linear_f32_tc ever ran out; otherwise its code.  Synchronises."""
+    if not library_loaded("linear_f32_tc"):
+        return 0
+    f = load_library("linear_f32_tc").brolm_linear_f32_tc_status
+    f.argtypes = [c_int]
+    f.restype = c_int
+    return f(1 if reset else 0)
 
 
 SKINNY_MAX_ROWS = 16
@@ -1374,7 +1438,7 @@ def gemm_tc_status(reset: bool = False) -> int:
     return f(1 if reset else 0)
 
 
-WAIT_LIBRARIES = ("gemm_tc", "gemm_tc2", "gemm_stream", "attn_tc", "grouped_tc")
+WAIT_LIBRARIES = ("linear_f32_tc", "gemm_tc", "gemm_tc2", "gemm_stream", "attn_tc", "grouped_tc")
 
 
 def wait_control(library: str, cycles: int = 0, stall_code: int = 0) -> None:
@@ -1992,7 +2056,7 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, s
 __all__ = ["KernelBuildError", "KernelError", "build_all", "launch_count", "device_sms", "wait_control", "embed_scale",
            "embed_pairs", "concat_cast", "latent_rows", "route_topk", "route_pick", "group_tiles", "group_pairs", "experts_tc_ok", "gather_rows", "experts_linear_tc", "grouped_tc_status", "heads_linear",
            "experts_linear", "rmsnorm", "residual_rmsnorm",
-           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
+           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "linear_f32_gated", "linear_f32_tc_ok", "linear_f32_tc_scratch", "linear_f32_tc_slices", "linear_f32_tc_status", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
            "gemm_stream_status", "attention_simt", "attention_prefill_mma", "attention_prefill_tc", "attention_prefill_tc_ok", "attention_prefill_tc_split", "attention_tc_status", "attention_decode_mma",
            "decode_splits", "decode_longest_first", "argmax", "sample", "cast", "bias_act", "scaled_sum", "qkv_norm_write", "gate_group_norm", "head_norm_gate", "rotate_heads",
            "layernorm", "residual_layernorm", "table_gate", "delta_step", "delta_prompt", "experts_combine", "causal_conv", "conv_tail", "gated_scan", "ssm_scan", "block_matvec_f32", "block_matvec_ok", "split_halves"]

@@ -32,6 +32,7 @@ NVCC_FLAGS = [
 LIBRARIES: dict[str, list[str]] = {
     "core": ["core.cu"],
     "linear_f32": ["linear_f32.cu"],
+    "linear_f32_tc": ["linear_f32_tc.cu"],
     "attn_simt": ["attn_simt.cu"],
     "attn_f32": ["attn_f32.cu"],
     "attn_mma": ["attn_mma.cu"],

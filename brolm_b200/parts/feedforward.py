@@ -40,6 +40,10 @@ class GatedFeedForward(Part):
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """x (tokens, hidden) -> (tokens, hidden) float32."""
         act = torch.empty((x.shape[0], self.inter), dtype=ctx.dtype, device=x.device)
+        if x.dtype == act.dtype == self.w_gate_up.dtype == torch.float32 and kernels.linear_f32_tc_ok(self.w_gate_up):
+            # float: the activation is the product's last step
+            kernels.linear_f32_gated(x, self.w_gate_up, act, self.activation, self.limit)
+            return linear(act, self.w_down, out_dtype=torch.float32)
         few = kernels.skinny_ok(x, self.w_gate_up)
         stream = kernels.stream_rows(x, self.w_gate_up) or (few and kernels.stream_instead_of_skinny(x, self.w_gate_up))
         if few and not (stream and self.inter % 64 == 0):

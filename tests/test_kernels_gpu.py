@@ -168,6 +168,77 @@ def test_linear_f32_every_kernel_gives_the_same_bits(M, N, K):
         assert torch.equal(out, ref), (kind, cut)
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 160, 161, 330])
+@pytest.mark.parametrize("N,K", [(4100, 260), (1024, 1028), (130, 9216), (20000, 256)])
+def test_linear_f32_on_tensor_cores(M, N, K):
+    """One, two, four and eight slices of K, ends of K and of the rows inside a tile, every width of the token tile."""
+    assert kernels.linear_f32_tc_slices(N, K) == {4100: 2, 1024: 4, 130: 8, 20000: 1}[N]
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    x[:, ::3] *= 1e-3                                        # (rows whose numbers differ widely)
+    wide = torch.full((M, N + 3), float("nan"), device=DEV)
+    kernels.linear_f32(x, w, wide[:, :N])
+    out = wide[:, :N]
+    assert kernels.linear_f32_tc_status(reset=True) == 0 and bool(wide[:, N:].isnan().all())
+    ref = x.double() @ w.double().T
+    # a product 3 * 2^-24; per 64 k twelve steps of the tensor core, each good to 2^-22 of what it adds; K / 64 float additions;
+    # what is too small for its row's scale 2^-38 of its largest
+    size = x.abs().double() @ w.abs().double().T
+    least = 2.0 ** -38 * K * x.abs().amax(1, keepdim=True).double() * w.abs().amax(1).double()
+    assert bool(((out.double() - ref).abs() <= (3 + 48 + K / 64) * 2.0 ** -24 * size + least).all())
+    plain_sums = torch.empty(M, N, device=DEV)
+    kernels._linear_f32(x, w, plain_sums, 0, 0)
+    assert float((out.double() - ref).norm()) <= 1.05 * float((plain_sums.double() - ref).norm())     # no less precise
+    for m in (0, M - 1):                                     # alone, and off the 16-byte boundaries
+        row = torch.empty(1, K + 1, device=DEV)
+        row[:, 1:] = x[m]
+        one = torch.empty(1, N, device=DEV)
+        kernels.linear_f32(row[:, 1:], w, one)
+        assert torch.equal(one[0], out[m])
+
+
+def test_linear_f32_on_tensor_cores_of_infinities_and_the_smallest_numbers():
+    """What a sum of parts cannot say is said by the floats themselves; the rows beside keep their bits."""
+    g = torch.Generator(device=DEV).manual_seed(12)
+    M, N, K = 40, 2048, 520
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    w[7, :] = w[7, :].to(torch.bfloat16).float()
+    before = torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, before)
+    x[3, 5], x[4, 77], x[5, 519], x[6, :4] = torch.inf, -torch.inf, torch.nan, 3.4e38
+    x[8] *= 1e-35
+    x[9] *= 1e30
+    w[9, 1], w[11] = torch.inf, 0.0
+    w[12] *= 1e-36
+    w[13] *= 1e-30
+    out, plain_sums = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, out)
+    kernels._linear_f32(x, w, plain_sums, 0, 0)
+    others = torch.arange(M, device=DEV) != 6               # (sums of the largest numbers run over on their way, or do not)
+    for same in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(same(out[others]), same(plain_sums[others]))
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    ok = ref.isfinite() & plain_sums.isfinite() & out.isfinite()
+    bound = 512 * 2.0 ** -24 * size + K * 2.0 ** -149
+    assert bool((((out.double() - ref).abs() <= bound) | ~ok).all())
+    rows = torch.tensor([m for m in range(M) if m not in (3, 4, 5, 6, 8, 9)], device=DEV)
+    cols = torch.tensor([n for n in range(N) if n not in (9, 11, 12, 13)], device=DEV)
+    assert torch.equal(out[rows][:, cols], before[rows][:, cols])
+
+
+@pytest.mark.parametrize("activation,limit", [("gelu_tanh", 0.0), ("silu", 0.0), ("clamped_gate", 1.5)])
+@pytest.mark.parametrize("M,F,K", [(1, 2048, 256), (16, 520, 1028), (33, 9472, 256), (170, 2100, 512)])
+def test_linear_f32_gated(M, F, K, activation, limit):
+    g = torch.Generator(device=DEV).manual_seed(M + F)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(2 * F, K, generator=g, device=DEV) / K ** 0.5
+    w[1, 3] = torch.inf
+    both, want, out = torch.empty(M, 2 * F, device=DEV), torch.empty(M, F, device=DEV), torch.empty(M, F, device=DEV)
+    kernels.linear_f32(x, w, both)
+    kernels.gated_act(both, want, activation, limit)
+    kernels.linear_f32_gated(x, w, out, activation, limit)
+    assert torch.equal(out.nan_to_num(7.0), want.nan_to_num(7.0))
+
+
 def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
     x = torch.zeros(300, 2305, device=DEV)[:, 1:]
     w, out = torch.zeros(2304, 2304, device=DEV), torch.empty(300, 2304, device=DEV)

@@ -46,6 +46,24 @@ def test_a_product_whose_wait_runs_out_reports_it_and_the_next_one_is_right(libr
     assert float((out.double().cpu() - ref).abs().max()) <= 2e-2 * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("code,M", [(2, 3), (5, 40), (6, 300), (8, 20), (9, 200)])
+def test_a_float_product_whose_wait_runs_out(code, M):
+    """The issuing thread's wait, those for fetched weights, for the room of their parts and of the tokens', for a sum."""
+    g = torch.Generator(device=DEV).manual_seed(6)
+    x, w = torch.randn(M, 2048, generator=g, device=DEV), torch.randn(1100, 2048, generator=g, device=DEV)
+    out, again = torch.empty(M, 1100, device=DEV), torch.empty(M, 1100, device=DEV)
+    kernels.linear_f32(x, w, out)
+    assert kernels.linear_f32_tc_status(reset=True) == 0
+    kernels.wait_control("linear_f32_tc", cycles=LIMIT, stall_code=code)
+    try:
+        kernels.linear_f32(x, w, again)
+        assert kernels.linear_f32_tc_status(reset=True) == code and kernels.linear_f32_tc_status() == 0
+    finally:
+        kernels.wait_control("linear_f32_tc", 0, 0)
+    kernels.linear_f32(x, w, again)
+    assert kernels.linear_f32_tc_status() == 0 and torch.equal(again, out)
+
+
 def test_prompt_attention_whose_wait_runs_out():
     n_q, n_kv, hd, T = 4, 2, 128, 300
     g = torch.Generator().manual_seed(2)
