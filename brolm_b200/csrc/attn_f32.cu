@@ -419,6 +419,187 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 ? 2 : 3) attn
     }
 }
 
+// Tiles of eight rows whose spans are shared (decode steps): a cluster of four blocks takes a span, each the scores of 32
+// keys for all rows, and then, with every score handed round through shared memory, a quarter of the value's entries for
+// all 128 keys.  All keys and values of a block are on their way at once, 64 KB with heads of 256, and every chain of fmas
+// has a thread of its own: what is left is the chains' length and the memory's latency.  The same order of operations.
+constexpr int FEW = 8, FEW_THREADS = 32 * FEW, SHARERS = 4;
+
+__host__ __device__ __forceinline__ int few_quarter(int vd) { return (vd + 15) / 16 * 4; }      // value entries of a block
+__host__ __device__ __forceinline__ int few_bytes(const F32Args& a) {
+    return 32 * (a.hd * 4 + 16) + SPAN * few_quarter(a.vd) * 4 + (FEW * a.hd + FEW * P_PITCH + 4 * FEW) * 4 + (32 + SPAN) * 8;
+}
+
+__global__ void __launch_bounds__(FEW_THREADS) __cluster_dims__(SHARERS, 1, 1) attn_f32_few_kernel(F32Args a) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    const int k_pitch = a.hd * 4 + 16, vq = few_quarter(a.vd);
+    const uint32_t ks = (uint32_t)__cvta_generic_to_shared(raw), vs = ks + 32 * k_pitch;
+    float* Vs = reinterpret_cast<float*>(raw + 32 * k_pitch);
+    float* Qs = Vs + SPAN * vq;
+    float* P = Qs + FEW * a.hd;
+    float* stats = P + FEW * P_PITCH;                   // [FEW]: M, L, the factors of what is held and of what comes
+    long long* k_off = reinterpret_cast<long long*>(stats + 4 * FEW);
+    long long* v_off = k_off + 32;
+    const int b = blockIdx.z, g = blockIdx.y, part = blockIdx.x % SHARERS, split = blockIdx.x / SHARERS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_wait();
+    const Tile t = tile_of<FEW>(a, b, 0);
+    if (t.rows <= 0) return;
+    int span = t.first + split, last = t.last;
+    if (span > last) return;
+    if (split < a.splits - 1) last = span;              // (the last one walks what is left, should the bound not have held)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    const int key_hi = t.first_pos + (t.row0 + t.rows - 1) / a.group;
+    const int v0 = part * vq, v_wide = min(vq, a.vd - v0);              // (nothing is left for the last blocks of small rows)
+    const float* kb = a.k_pages ? a.k_pages : a.k;
+    const float* vb = a.k_pages ? a.v_pages : a.v;
+    for (int idx = tid; idx < t.rows * (a.hd / 4); idx += FEW_THREADS) {
+        const int r = idx / (a.hd / 4), c = (idx - r * (a.hd / 4)) * 4, row = t.row0 + r;
+        copy16((uint32_t)__cvta_generic_to_shared(Qs + r * a.hd + c),
+               a.q + (size_t)(t.q0 + row / a.group) * a.q_stride + (g * a.group + row % a.group) * a.hd + c, true);
+    }
+    // a thread's chain over the keys: two neighbouring value entries of a row
+    const int chains = max(0, v_wide / 2), my_row = chains ? tid / chains : FEW, my_d = chains ? (tid - my_row * chains) * 2 : 0;
+    float tot[2] = {0.0f, 0.0f};
+    for (bool first = true; span <= last; ++span, first = false) {
+        const int key0 = span * SPAN, keys = min(SPAN, key_hi + 1 - key0);
+        if (tid < SPAN) {
+            const int kp = key0 + tid;
+            long long ko = -1, vo = -1;
+            if (tid < keys && kp >= t.key_lo) {          // (a ring's places of older positions hold other keys)
+                if (a.k_pages) {
+                    const int place = kp % a.ring, page = a.page_table[(size_t)b * a.pt_stride + place / a.page_size];
+                    const long long at = ((long long)page * a.n_kv + g) * a.page_size + place % a.page_size;
+                    ko = at * a.hd;
+                    vo = at * a.vd;
+                } else {
+                    ko = (long long)(t.q0 + kp) * a.k_stride + (long long)g * a.hd;
+                    vo = (long long)(t.q0 + kp) * a.v_stride + (long long)g * a.vd;
+                }
+            }
+            if (tid >> 5 == part) k_off[lane] = ko;
+            v_off[tid] = vo;
+        }
+        __syncthreads();
+        for (int key = warp; key < 32; key += FEW) {
+            const long long o = k_off[key];
+            for (int c = lane * 4; c < a.hd; c += 128) copy16(ks + key * k_pitch + c * 4, kb + (o >= 0 ? o + c : 0), o >= 0);
+        }
+        copy_commit();
+        if (v_wide > 0) {
+            const int pieces = v_wide / 4;
+            for (int idx = tid; idx < SPAN * pieces; idx += FEW_THREADS) {
+                const int j = idx / pieces, c = (idx - j * pieces) * 4;
+                const long long o = v_off[j];
+                copy16(vs + (j * vq + c) * 4, vb + (o >= 0 ? o + v0 + c : 0), o >= 0);
+            }
+        }
+        copy_commit();
+        copy_wait<1>();
+        __syncthreads();
+        float score = 0.0f;
+        if (warp < t.rows) {                             // a warp's row, a lane's key
+            uint64_t s = 0;
+            const float* q = Qs + warp * a.hd;
+            const float* k = reinterpret_cast<const float*>(raw + lane * k_pitch);
+#pragma unroll 8
+            for (int c = 0; c < a.hd; c += 4) {
+                const Pair2 qq = lds4(q + c), kk = lds4(k + c);
+                fma2(s, qq.x, kk.x);
+                fma2(s, qq.y, kk.y);
+            }
+            const float2 h = unpack2(s);
+            score = h.x + h.y;
+        }
+        if (first) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");          // (the other blocks are there)
+        if (warp < t.rows) {
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(P + warp * P_PITCH + part * 32 + lane);
+#pragma unroll
+            for (int r = 0; r < SHARERS; ++r) {
+                uint32_t far;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(r));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(far), "f"(score) : "memory");
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        if (warp < t.rows) {                             // as in the kernel above, one row a warp
+            const int row = t.row0 + warp, head = g * a.group + row % a.group, pos = t.first_pos + row / a.group;
+            const float slope = a.slopes ? a.slopes[head] : 0.0f;
+            const int from = max(a.window > 0 ? pos - a.window + 1 : 0, a.chunk > 0 ? pos - pos % a.chunk : 0);
+            float sc[4], m = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int kp = key0 + e * 32 + lane;
+                float v = -INFINITY;
+                if (kp <= pos && kp >= from) {
+                    v = soft_cap(__fmul_rn(P[warp * P_PITCH + e * 32 + lane], a.scale), a.cap);
+                    if (a.slopes) v = __fmaf_rn(-slope, (float)(pos - kp), v);
+                    if (a.dist_bias) v += a.dist_bias[(size_t)head * a.dist_len + min(pos - kp, a.dist_len - 1)];
+                }
+                sc[e] = v;
+                m = fmaxf(m, v);
+            }
+            m = warp_max(m);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sc[e] = sc[e] == -INFINITY ? 0.0f : expf(sc[e] - m);                    // (a NaN stays one)
+                P[warp * P_PITCH + e * 32 + lane] = sc[e];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sc[e] += __shfl_xor_sync(0xffffffffu, sc[e], o);
+            if (lane == 0) {
+                const float sum = ((sc[0] + sc[1]) + sc[2]) + sc[3];
+                if (first) {
+                    stats[warp] = m;
+                    stats[FEW + warp] = sum;
+                } else {
+                    float M = stats[warp], L = stats[FEW + warp], held, fresh;
+                    merge_factors(M, L, m, sum, held, fresh);
+                    stats[warp] = M;
+                    stats[FEW + warp] = L;
+                    stats[2 * FEW + warp] = held;
+                    stats[3 * FEW + warp] = fresh;
+                }
+            }
+        }
+        copy_wait<0>();
+        __syncthreads();
+        if (my_row < t.rows) {
+            uint64_t acc = 0;
+            const float* p = P + my_row * P_PITCH;
+            const float* v = Vs + my_d;
+#pragma unroll 4
+            for (int j = 0; j < SPAN; j += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(p + j);
+                fma2(acc, pack2(w.x, w.x), *reinterpret_cast<const uint64_t*>(v + j * vq));
+                fma2(acc, pack2(w.y, w.y), *reinterpret_cast<const uint64_t*>(v + (j + 1) * vq));
+                fma2(acc, pack2(w.z, w.z), *reinterpret_cast<const uint64_t*>(v + (j + 2) * vq));
+                fma2(acc, pack2(w.w, w.w), *reinterpret_cast<const uint64_t*>(v + (j + 3) * vq));
+            }
+            const float held = first ? 0.0f : stats[2 * FEW + my_row], fresh = first ? 1.0f : stats[3 * FEW + my_row];
+            const float2 f = unpack2(acc);
+            tot[0] = merged(tot[0], held, f.x, fresh);
+            tot[1] = merged(tot[1], held, f.y, fresh);
+        }
+        if (span < last) {                               // the scores of the next span come into P from all blocks
+            __syncthreads();
+            asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        }
+    }
+    pdl_trigger();
+    const auto place = [&](int r) {
+        const int row = t.row0 + r;
+        return ((size_t)(t.q0 + row / a.group) * a.n_kv * a.group + g * a.group + row % a.group) * a.splits + split;
+    };
+    if (part == 0 && tid < t.rows) {
+        a.part_ml[2 * place(tid)] = stats[tid];
+        a.part_ml[2 * place(tid) + 1] = stats[FEW + tid];
+    }
+    if (my_row < t.rows) *reinterpret_cast<float2*>(a.part_acc + place(my_row) * a.vd + v0 + my_d) = make_float2(tot[0], tot[1]);
+}
+
 // One row (blockIdx.x: a row of the sequence's, blockIdx.y: kv head, blockIdx.z: sequence): its spans in order.
 template <int ROWS>
 __global__ void __launch_bounds__(64) merge_kernel(F32Args a) {
@@ -449,6 +630,14 @@ __global__ void __launch_bounds__(64) merge_kernel(F32Args a) {
     float* dst = a.out + (size_t)token * a.out_stride + (size_t)head * a.vd + threadIdx.x * 4;
 #pragma unroll
     for (int e = 0; e < 4; ++e) dst[e] = __fmul_rn(A[e], inv);
+}
+
+int launch_few(const F32Args& a, int batch, int max_q_len, cudaStream_t stream) {
+    static OncePerDevice allowed;
+    if (const int e = allow_shared_memory(attn_f32_few_kernel, 112 * 1024, allowed)) return e;
+    const int st = launch_pdl(attn_f32_few_kernel, dim3(a.splits * SHARERS, a.n_kv, batch), dim3(FEW_THREADS), few_bytes(a), stream, a);
+    if (st) return st;
+    return launch_pdl(merge_kernel<FEW>, dim3(max_q_len * a.group, a.n_kv, batch), dim3(64), 0, stream, a);
 }
 
 template <int ROWS, int VJ>
@@ -498,6 +687,7 @@ BROLM_API int brolm_attn_f32(const void* q, int q_stride, void* out, int out_str
     // 8 kv heads, 384 blocks: 27 us where two share an SM)
     a.max_parts = k_pages || max_q_len > 64 || (long long)max_q_len * group <= 8 ? 4 : max_q_len > 32 ? 2 : 1;
     if ((long long)max_q_len * group <= 8) {
+        if (splits) return launch_few(a, batch, max_q_len, stream);
         if (vd <= 128) return launch<8, 1>(a, batch, max_q_len, stream);
         return launch<8, 2>(a, batch, max_q_len, stream);
     }

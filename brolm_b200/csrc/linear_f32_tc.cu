@@ -14,7 +14,8 @@
 // the slices are added through the shared memory of a cluster of blocks, or by a kernel behind this one.  Roles:
 //   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it;
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the two rows of halves into tensor memory (the A operand);
-//   X       these do the same for the tokens, into shared memory (the B operand);
+//   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
+//           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the halves in by TMA;
 //   MMA     one thread issues 12 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two accumulators;
 //   ADD     these add an accumulator to the sums in their registers, and at the end store them.
 // The thread that issues is what all wait for, so its stage of 64 k has one barrier to wait on, which all that its products
@@ -36,22 +37,28 @@ constexpr int W_SLOT = BR * KW * 4;
 constexpr int A_PLANE = KX / 2, A_COLS = 2 * A_PLANE;        // tensor memory: two k a column, two planes a stage
 constexpr int SCALES = 4;                          // stages whose scales are kept: one that is written is not read any more
 
-enum class Role { TMA, MMA, SPLIT, ADD, X, NONE };
+enum class Role { TMA, MMA, SPLIT, ADD, X, FETCH_X, NONE };
 
-// Up to 32 tokens two blocks share an SM; for more one block takes it, with 28 warps that share its registers by need.
-template <int NT>
+// Up to 32 tokens two blocks share an SM, or one has a ring of twice the slots where there are no more blocks than SMs and
+// their clusters are small enough to find room (18,432 x 2,304 with 3 tokens, 144 blocks: 40.6 us with four slots, %s with
+// ten; the memory's latency asks for more than two stages on their way).  For more tokens one block takes the SM, with 28 warps
+// that share its registers by need.
+template <int NT, int BLOCKS>
 struct Shape {
     static constexpr bool FEW = NT <= 32;
-    static constexpr int PER_SM = FEW ? 2 : 1;
+    static constexpr int PER_SM = BLOCKS;
+    static_assert(FEW || BLOCKS == 1, "many tokens take the SM");
     static constexpr int WARPS = FEW ? 16 : 28, THREADS = 32 * WARPS;
     static constexpr int GROUPS = FEW ? 1 : 2, COLS = NT / GROUPS;          // warps of a quarter that add, each its share of the tokens
     static constexpr int X_WARPS = FEW ? 2 : 8;
     static constexpr int READY = 4 + X_WARPS + 4 * GROUPS;                  // arrivals that a stage waits for
-    static constexpr int W_SLOTS = FEW ? 5 : 8;
+    static constexpr int X_RAW = NT * KX * 4;                               // bytes of a stage of X as it is
+    static constexpr int W_SLOTS = !FEW ? 8 : PER_SM == 1 ? 10 : NT == 16 ? 5 : 4;
+    static constexpr int AHEAD = !FEW ? 0 : PER_SM == 1 ? 4 : 3;           // stages of X that are on their way (FEW)
     static constexpr int X_PLANE = NT * KX * 2, X_SLOT = 2 * X_PLANE;
     static constexpr int TMEM = FEW ? 256 : 512;
-    static constexpr int RING = W_SLOTS * W_SLOT + 2 * X_SLOT;
-    static constexpr int BARS = 2 * W_SLOTS + 5;
+    static constexpr int RING = W_SLOTS * W_SLOT + 2 * X_SLOT + AHEAD * X_RAW;
+    static constexpr int BARS = 2 * W_SLOTS + 7;
     static constexpr int SMEM = RING + SCALES * (BR + NT) * 4 + BARS * 8 + 24;
     static_assert(2 * NT + 2 * A_COLS <= TMEM && TMEM * PER_SM <= 512, "accumulators and A");
     static_assert((SMEM + 1024) * PER_SM <= 228 * 1024, "the blocks of an SM");
@@ -59,7 +66,7 @@ struct Shape {
 
     static __device__ __forceinline__ Role role(int warp, int& index) {     // index: within the role
         if (warp < 2) return warp == 0 ? Role::TMA : Role::MMA;
-        if (warp < 4) return index = warp - 2, FEW ? Role::X : Role::NONE;
+        if (warp < 4) return index = warp - 2, FEW ? Role::X : warp == 3 ? Role::FETCH_X : Role::NONE;
         if (warp < 12) return index = warp - 4, Role::SPLIT;
         if (warp < 12 + 4 * GROUPS) return index = warp - 12, Role::ADD;
         return index = warp - 20, Role::X;
@@ -75,12 +82,14 @@ struct Args {
     const float* x;
     const float* w;
     float* y;
+    const float* x_scale;    // X taken apart ahead: [M][stages of K] scales, and the halves under a map of their own; null: here
     float* parts;            // the slices' sums, [slice][M][N], are added by the kernel behind; null: by the cluster
     int ldx, ldw, ldy;
     int M, N, K;
     int tokens;              // of a token tile: a multiple of 16
     int slice;               // k of a slice: a multiple of 64
     int x_vec;               // X's rows lie on 16-byte boundaries
+    int x_stages;            // columns of x_scale
     int gated;               // W is [gate; up] of 2 N rows, a block has 64 of each, and y = act(gate) * up
     int act;
     float limit;
@@ -139,9 +148,10 @@ __device__ __forceinline__ float checked(const Args& g, int token, int row, floa
     return y;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Args g) {
-    using S = Shape<NT>;
+template <int NT, int BLOCKS>
+__global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                                                                     const __grid_constant__ CUtensorMap map_x, Args g) {
+    using S = Shape<NT, BLOCKS>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t w_ring = smem_u32(smem_raw), x_ring = w_ring + S::W_SLOTS * W_SLOT;
     float* row_scale = reinterpret_cast<float*>(smem_raw + S::RING);        // [SCALES][BR]: what a partial sum is multiplied by
@@ -150,7 +160,7 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + S::BARS);
     volatile int* give_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * S::W_SLOTS, ready = w_empty + 8 * S::W_SLOTS, made = ready + 16,
-                   all_made = made + 16;
+                   all_made = made + 16, x_full = all_made + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     const int n_slices = gridDim.x, part = blockIdx.x;
@@ -162,7 +172,7 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::W_SLOTS; ++s) mbar_init(w_full + 8 * s, 1), mbar_init(w_empty + 8 * s, 4);
-        for (int s = 0; s < 2; ++s) mbar_init(ready + 8 * s, S::READY), mbar_init(made + 8 * s, 1);
+        for (int s = 0; s < 2; ++s) mbar_init(ready + 8 * s, S::READY), mbar_init(made + 8 * s, 1), mbar_init(x_full + 8 * s, 1);
         mbar_init(all_made, 1);
         give_up[0] = 0;
         give_up[1] = 0;
@@ -180,7 +190,7 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
 
     int index = 0;
     const Role role = S::role(warp, index);
-    if (role == Role::TMA || role == Role::MMA || role == Role::NONE) {
+    if (role == Role::TMA || role == Role::MMA || role == Role::FETCH_X || role == Role::NONE) {
         if constexpr (!S::FEW) fewer_registers<48>();
         if (role == Role::TMA && lane == 0) {
             int i = 0;
@@ -201,6 +211,7 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
             for (int j = 0; j < stages; ++j) {
                 const int s = j & 1;
                 if (!wait_on(ready + 8 * s, (j >> 1) & 1, 2)) break;
+                if (g.x_scale && !wait_on(x_full + 8 * s, (j >> 1) & 1, 3)) break;
                 fence_after_sync();
                 const uint32_t acc = tmem + s * NT, a = tmem_a + s * A_COLS;
                 const uint64_t b = desc_kmajor(x_ring + s * S::X_SLOT);
@@ -217,6 +228,20 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
                 umma_commit(all_made);
                 mbar_wait(all_made, 0, give_up, &g_linear_f32_tc_error, 10, true);
             }
+        }
+        if (role == Role::FETCH_X && lane == 0 && g.x_scale) {
+            pdl_wait();
+            int j = 0;
+            for (; j < stages; ++j) {
+                const int s = j & 1;
+                if (j >= 2 && !wait_on(made + 8 * s, ((j >> 1) & 1) ^ 1, 9)) break;
+                mbar_expect_tx(x_full + 8 * s, 2 * g.tokens * KX * 2);
+                for (int q = 0; q < 2; ++q)
+                    tma_load_3d(x_ring + s * S::X_SLOT + q * S::X_PLANE, &map_x, k_lo + j * KX, m0, q, x_full + 8 * s);
+            }
+            if (*give_up)
+                for (int i = max(0, j - 2); i < j; ++i)
+                    mbar_wait(x_full + 8 * (i & 1), (i >> 1) & 1, give_up, &g_linear_f32_tc_error, 11, true);
         }
     } else if (role == Role::SPLIT) {
         if constexpr (!S::FEW) fewer_registers<48>();
@@ -317,7 +342,7 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
                 const int token = u * (T / 8) + (xt >> 3);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[u][e] = 0.0f;
-                if (token < tokens && j < stages) {
+                if (token < tokens) {
                     const float* p = g.x + (size_t)(m0 + token) * g.ldx + k;
                     if (g.x_vec) {
 #pragma unroll
@@ -363,14 +388,58 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
             if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
             return true;
         };
-        if constexpr (NT == 16) {                               // what comes next is on its way
-            float va[PER][8], vb[PER][8];
-            load(0, va);
-            for (int j = 0; j < stages; j += 2) {
-                load(j + 1, vb);
-                if (!put(j, va) || j + 1 >= stages) break;
-                load(j + 2, va);
-                if (!put(j + 1, vb)) break;
+        if constexpr (S::FEW) {
+            // every thread brings in what it will take apart, some stages ahead
+            const uint32_t raw = x_ring + 2 * S::X_SLOT + xt * 32;
+            auto fetch = [&](int j) {
+                const int k = k_lo + j * KX + chunk * 8;
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int token = u * (T / 8) + (xt >> 3);
+                    const float* p = g.x + (size_t)(m0 + token) * g.ldx + k;
+                    const uint32_t dst = raw + (j % S::AHEAD) * S::X_RAW + u * T * 32;
+                    const bool there = token < tokens && j < stages;
+                    if (g.x_vec) {
+#pragma unroll
+                        for (int e = 0; e < 8; e += 4) copy16(dst + e * 4, there && k + e < g.K ? p + e : g.x, there && k + e < g.K);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const bool ok = there && k + e < g.K;
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst + e * 4), "l"(ok ? p + e : g.x), "r"(ok ? 4 : 0) : "memory");
+                        }
+                    }
+                }
+                copy_commit();
+            };
+#pragma unroll
+            for (int j = 0; j < S::AHEAD - 1; ++j) fetch(j);
+            for (int j = 0; j < stages; ++j) {
+                fetch(j + S::AHEAD - 1);
+                copy_wait<S::AHEAD - 1>();
+                float v[PER][8];
+#pragma unroll
+                for (int u = 0; u < PER; ++u)
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {
+                        const float4 f = lds_float4(raw + (j % S::AHEAD) * S::X_RAW + u * T * 32 + e * 4);
+                        v[u][e] = f.x, v[u][e + 1] = f.y, v[u][e + 2] = f.z, v[u][e + 3] = f.w;
+                    }
+                if (!put(j, v)) break;
+            }
+            copy_wait<0>();
+        } else if (g.x_scale) {
+            // the halves come by TMA: the scales alone
+            const float* src = g.x_scale + (size_t)(m0 + xt) * g.x_stages + k_lo / KX;
+            const bool there = xt < tokens;
+            float next = there ? src[0] : 1.0f;
+            for (int j = 0; j < stages; ++j) {
+                const float now = next;
+                if (there && j + 1 < stages) next = src[j + 1];
+                if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 9)) break;
+                if (xt < NT) token_scale[(j % SCALES) * NT + xt] = now;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
             }
         } else {
             float v[PER][8];
@@ -433,6 +502,38 @@ __global__ void __launch_bounds__(Shape<NT>::THREADS, Shape<NT>::PER_SM) linear_
     if (warp == 2) tmem_dealloc(tmem, S::TMEM);
 }
 
+// X taken apart ahead: eight lanes take 64 k of a token.  halves [2][M][Kp], Kp = 64 stages; scale [M][stages]
+__global__ void __launch_bounds__(256) split_rows_kernel(Args g, __half* __restrict__ halves, float* __restrict__ scale, int stages) {
+    pdl_trigger();
+    const size_t kp = (size_t)stages * KX;
+    const long long unit = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
+    const int chunk = threadIdx.x & 7, token = (int)(unit / stages), st = (int)(unit % stages), k = st * KX + chunk * 8;
+    pdl_wait();
+    const bool there = token < g.M;
+    const float* p = g.x + (size_t)(there ? token : 0) * g.ldx + k;
+    float v[8], most = 0.0f, up, down;
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) {                          // (X's rows lie on 16-byte boundaries)
+        const float4 f = there && k + e < g.K ? *reinterpret_cast<const float4*>(p + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[e] = f.x, v[e + 1] = f.y, v[e + 2] = f.z, v[e + 3] = f.w;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) most = fmaxf(most, fabsf(v[e]));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+    scales_of(most, up, down);
+    if (!there) return;
+    uint4 q[2];
+    uint32_t* q0 = &q[0].x;
+    uint32_t* q1 = &q[1].x;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) take_apart(v[2 * e], v[2 * e + 1], up, q0[e], q1[e]);
+    __half* dst = halves + (size_t)token * kp + k;
+    *reinterpret_cast<uint4*>(dst) = q[0];
+    *reinterpret_cast<uint4*>(dst + (size_t)g.M * kp) = q[1];
+    if (chunk == 0) scale[(size_t)token * stages + st] = down;
+}
+
 // y = parts[0] + parts[1] + ... in order
 __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
     pdl_trigger();
@@ -447,11 +548,11 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
     }
 }
 
-template <int NT>
-int launch(const CUtensorMap& mw, const Args& g, dim3 grid, cudaStream_t stream) {
-    using S = Shape<NT>;
+template <int NT, int BLOCKS>
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, dim3 grid, cudaStream_t stream) {
+    using S = Shape<NT, BLOCKS>;
     static OncePerDevice allowed;
-    if (const int e = allow_shared_memory(linear_f32_tc_kernel<NT>, S::SMEM, allowed)) return e;
+    if (const int e = allow_shared_memory(linear_f32_tc_kernel<NT, BLOCKS>, S::SMEM, allowed)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(S::THREADS);
@@ -465,7 +566,7 @@ int launch(const CUtensorMap& mw, const Args& g, dim3 grid, cudaStream_t stream)
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = grid.x > 1 && !g.parts ? 2 : 1;
-    const int st = (int)cudaLaunchKernelEx(&cfg, linear_f32_tc_kernel<NT>, mw, g);
+    const int st = (int)cudaLaunchKernelEx(&cfg, linear_f32_tc_kernel<NT, BLOCKS>, mw, mx, g);
     if (st || !g.parts) return st;
     const size_t blocks = ((size_t)g.M * g.N + 255) / 256;
     return launch_pdl(add_slices_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, g, (int)grid.x);
@@ -476,8 +577,10 @@ int launch(const CUtensorMap& mw, const Args& g, dim3 grid, cudaStream_t stream)
 // Y = X W^T over `slices` slices of K of `slice` k each (a multiple of 64, none empty; at most 8 slices); gated: Y =
 // act(X Wg^T) * (X Wu^T) for W = [Wg; Wu] of 2 N rows.  W's rows lie on 16-byte boundaries, K is a multiple of 4; X's rows
 // may lie anywhere.  parts: room for slices * M * N floats, with which a second kernel adds the slices; null: clusters do.
+// halves: room for X taken apart ahead (more than 32 rows on 16-byte boundaries), 16-byte aligned, M * ceil(K / 64) * 260 bytes;
+// null: every block does it.
 BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
-                                  int slices, int slice, int gated, int act, float limit, void* parts, cudaStream_t stream) {
+                                  int slices, int slice, int gated, int act, float limit, void* parts, void* halves, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;
     if (K <= 0 || K % 4 || ldw % 4 || ((uintptr_t)w & 15)) return BROLM_ERR_ALIGNMENT;
     if (slices < 1 || slices > 8 || slice < 64 || slice % 64 || (long long)(slices - 1) * slice >= K || (long long)slices * slice < K) return BROLM_ERR_BAD_SIZE;
@@ -504,10 +607,28 @@ BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw
     g.slice = slice;
     g.gated = gated; g.act = act; g.limit = limit;
     g.x_vec = ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
+    g.x_scale = nullptr;
+    g.x_stages = (K + KX - 1) / KX;
+    CUtensorMap mx = mw;
+    if (halves) {
+        if (most <= 32 || !g.x_vec || ((uintptr_t)halves & 15)) return BROLM_ERR_ALIGNMENT;
+        const cuuint64_t kp = (cuuint64_t)g.x_stages * KX;
+        const cuuint64_t xdims[3] = {kp, (cuuint64_t)M, 2}, xstrides[2] = {kp * 2, kp * M * 2};
+        const cuuint32_t xbox[3] = {KX, (cuuint32_t)g.tokens, 1}, xelem[3] = {1, 1, 1};
+        if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, halves, xdims, xstrides, xbox, xelem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return BROLM_ERR_ALIGNMENT;
+        float* scale = reinterpret_cast<float*>((uint8_t*)halves + (size_t)M * kp * 4);
+        g.x_scale = scale;
+        const long long units = (long long)M * g.x_stages;
+        const int st = launch_pdl(split_rows_kernel, dim3((unsigned)((units * 8 + 255) / 256)), dim3(256), 0, stream, g, (__half*)halves, scale, g.x_stages);
+        if (st) return st;
+    }
     const dim3 grid(slices, (M + g.tokens - 1) / g.tokens, (unsigned)row_tiles);
-    if (most == 16) return launch<16>(mw, g, grid, stream);
-    if (most == 32) return launch<32>(mw, g, grid, stream);
-    return launch<160>(mw, g, grid, stream);
+    const bool alone = grid.x <= 4 && (long long)grid.x * grid.y * grid.z <= device_sm_count();
+    if (most == 16) return alone ? launch<16, 1>(mw, mx, g, grid, stream) : launch<16, 2>(mw, mx, g, grid, stream);
+    if (most == 32) return alone ? launch<32, 1>(mw, mx, g, grid, stream) : launch<32, 2>(mw, mx, g, grid, stream);
+    return launch<160, 1>(mw, mx, g, grid, stream);
 }
 
 BROLM_API int brolm_linear_f32_tc_status(int reset) {
