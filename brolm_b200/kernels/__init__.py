@@ -1513,10 +1513,14 @@ def gemm_stream_parts(x: torch.Tensor, weight: torch.Tensor, sms: Optional[int] 
     one / two items an SM: 2,304 x 9,216 (42 MB) 19.5 / 16.2 us, 3,072 x 8,064 (50) 21.0 / 16.6, 8,192 x 3,584 (59) 25.9 / 19.7, 3,584
     x 14,336 (103) 30.8 / 27.5; a decode step of 24 sequences at the 9B sizes 6,323 / 6,081 us, at the 2B sizes (19 and
     42 MB), where the slices' sums are the larger share, no difference."""
-    sms = sms or device_sms(x.device if x.is_cuda else None)
-    row_tiles = (weight.shape[0] + 127) // 128
-    nkb = (x.shape[1] + 63) // 64
-    many = weight.shape[0] * x.shape[1] * 2 >= 48 << 20
+    return _stream_slices(weight.shape[0], x.shape[1], sms or device_sms(x.device if x.is_cuda else None))
+
+
+@functools.lru_cache(maxsize=1024)
+def _stream_slices(N: int, K: int, sms: int) -> int:
+    row_tiles = (N + 127) // 128
+    nkb = (K + 63) // 64
+    many = N * K * 2 >= 48 << 20
     want = max(1, (2 if many else 1) * sms // row_tiles)
     # at least a ring's worth of K blocks (8) per item: a shorter run is over before its loads are all
     # in flight, and every further slice is another float copy of the output for the reader to add
@@ -1550,6 +1554,87 @@ def gemm_stream(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilog
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(-2), M, N, K, code,
              1 if out.dtype == torch.float32 else 0, ACTIVATIONS[activation], limit if code == 1 else cap, scale, ksplit,
              part_stride, _stream()), "gemm_stream")
+
+
+class _PromptNorm(ctypes.Structure):
+    _fields_ = [("weight", c_void_p), ("eps", c_float), ("offset", c_float)]
+
+
+class _PromptLayer(ctypes.Structure):
+    _fields_ = ([(n, c_void_p) for n in ("gemm_stream", "rope_kv_write_parts", "attn_prefill_tc", "residual_rmsnorm", "h", "x", "next",
+                                         "w_qkv", "w_o", "w_gate_up", "w_down", "sums", "qkv", "attn", "mid", "act", "positions",
+                                         "cos_sin", "cu_q", "cache_rows", "k_pages", "v_pages")] +
+                [(n, _PromptNorm) for n in ("post_mixer", "pre_ffn", "post_ffn", "after")] +
+                [(n, c_int) for n in ("w_dtype_mid", "w_dtype_end", "tokens", "hidden", "inter", "n_q", "n_kv", "head_dim", "page_size",
+                                      "batch", "max_q_len", "window")] +
+                [(n, c_float) for n in ("scale", "cap", "limit")] +
+                [(n, c_int) for n in ("activation", "qkv_slices", "o_slices", "down_slices")])
+
+
+_prompt_fns: list = []       # the entry points of the four libraries, once they are loaded
+
+
+def _prompt_entry_points() -> list:
+    if not _prompt_fns:
+        if load_library("prompt_layer").brolm_prompt_layer_size() != ctypes.sizeof(_PromptLayer):
+            raise KernelError("prompt_layer: the library's arguments are laid out in another way")
+        _prompt_fns[:] = [ctypes.cast(getattr(load_library(lib), name), c_void_p).value for lib, name in
+                          (("gemm_stream", "brolm_gemm_stream"), ("core", "brolm_rope_kv_write_parts"),
+                           ("attn_tc", "brolm_attn_prefill_tc"), ("core", "brolm_residual_rmsnorm"))]
+    return _prompt_fns
+
+
+def prompt_layer_ok(tokens: int, head_dim: int, group: int, inter: int, max_q_len: int, n_kv: int, window: int, batch: int,
+                    *weights: torch.Tensor) -> bool:
+    """Whether the launches of a layer for a prompt of so many tokens go out from one call (``prompt_layer``): more than the
+    few-token product takes and at most what the weight stream does."""
+    return (SKINNY_MAX_ROWS < tokens <= STREAM_MAX_ROWS and PROMPT_LAYER and inter % 64 == 0 and group <= 16
+            and attention_prefill_tc_ok(head_dim, group)
+            and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights)
+            and not (PREFILL_SPLIT and attention_prefill_tc_split(max_q_len, n_kv, group, window, batch)))
+
+
+def prompt_layer(h: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor, w_o: torch.Tensor, w_gate_up: torch.Tensor,
+                 w_down: torch.Tensor, norms: list, positions: torch.Tensor, cos_sin: Optional[torch.Tensor], cu_q: torch.Tensor,
+                 cache_rows: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, *, n_q: int, n_kv: int, head_dim: int,
+                 page_size: int, batch: int, max_q_len: int, window: int, scale: float, cap: float, activation: str,
+                 limit: float) -> Optional[torch.Tensor]:
+    """A whole layer of a short prompt (``prompt_layer_ok``): h float32 (tokens, hidden) is updated, x bfloat16 is its norm.
+    ``norms``: (weight, eps, offset) of the mixer's result, ahead of the feed-forward, of its result, and ahead of the next layer
+    (None: there is none, and nothing is returned); the next layer's x otherwise."""
+    T, H = x.shape
+    q, cols, F = n_q * head_dim, (n_q + 2 * n_kv) * head_dim, w_down.shape[1]
+    assert h.dtype == torch.float32 and h.shape == x.shape and h.is_contiguous() and x.is_contiguous() and x.dtype == torch.bfloat16
+    assert w_qkv.shape == (cols, H) and w_o.shape == (H, q) and w_gate_up.shape == (2 * F, H) and w_down.shape == (H, F)
+    assert positions.dtype == cu_q.dtype == cache_rows.dtype == torch.int32 and positions.numel() == cache_rows.numel() == T
+    assert k_pages.dtype == v_pages.dtype == torch.bfloat16 and k_pages.is_contiguous() and v_pages.is_contiguous()
+    assert tuple(k_pages.shape[1:]) == (n_kv, page_size, head_dim) and k_pages.shape == v_pages.shape
+    assert cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[1:] == (head_dim // 2, 2))
+    assert all(n is None or (n[0].is_contiguous() and n[0].numel() == H) for n in norms)
+    assert norms[0][0].dtype == norms[1][0].dtype and (norms[3] is None or norms[2][0].dtype == norms[3][0].dtype)
+    sms = device_sms(x.device)
+    slices = [_stream_slices(n, k, sms) for n, k in ((cols, H), (H, q), (H, F))]
+    # scratch: the slices' sums, q/k/v, the attention's rows, the feed-forward's rows and its inner ones
+    sizes = [4 * T * max(slices[0] * cols, slices[1] * H, slices[2] * H), 2 * T * cols, 2 * T * q, 2 * T * H, 2 * T * F]
+    at, offs = 0, []
+    for n in sizes:
+        offs.append(at)
+        at += (n + 255) // 256 * 256
+    scratch = torch.empty(at, dtype=torch.uint8, device=x.device)
+    out = torch.empty_like(x) if norms[3] is not None else None
+    base = _ptr(scratch)
+    norm = lambda n: _PromptNorm(n[0].data_ptr(), n[1], n[2]) if n is not None else _PromptNorm(None, 0.0, 0.0)
+    args = _PromptLayer(*_prompt_entry_points(), _ptr(h), _ptr(x), _ptr(out), _ptr(w_qkv), _ptr(w_o), _ptr(w_gate_up), _ptr(w_down),
+                        *[base + o for o in offs], _ptr(positions), _ptr(cos_sin), _ptr(cu_q), _ptr(cache_rows), _ptr(k_pages),
+                        _ptr(v_pages), *[norm(n) for n in norms], _code(norms[0][0]), _code(norms[2][0]), T, H, F, n_q, n_kv, head_dim,
+                        page_size, batch, max_q_len, window, scale, cap, limit, ACTIVATIONS[activation], *slices)
+    _check(_fn("prompt_layer", "brolm_prompt_layer", [c_void_p, c_void_p])(ctypes.byref(args), _stream()), "prompt_layer")
+    add_launches(7)
+    return out
+
+
+# BROLM_PROMPT_LAYER=0: short prompts launch kernel by kernel
+PROMPT_LAYER = os.environ.get("BROLM_PROMPT_LAYER", "1") != "0"
 
 
 def gemm_stream_status(reset: bool = False) -> int:
@@ -2060,7 +2145,7 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, s
 __all__ = ["KernelBuildError", "KernelError", "build_all", "launch_count", "device_sms", "wait_control", "embed_scale",
            "embed_pairs", "concat_cast", "latent_rows", "route_topk", "route_pick", "group_tiles", "group_pairs", "experts_tc_ok", "gather_rows", "experts_linear_tc", "grouped_tc_status", "heads_linear",
            "experts_linear", "rmsnorm", "residual_rmsnorm",
-           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "linear_f32_gated", "linear_f32_tc_ok", "linear_f32_tc_scratch", "linear_f32_tc_slices", "linear_f32_tc_status", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
+           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "linear_f32_gated", "linear_f32_tc_ok", "linear_f32_tc_scratch", "linear_f32_tc_slices", "linear_f32_tc_status", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "prompt_layer", "prompt_layer_ok", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
            "gemm_stream_status", "attention_simt", "attention_prefill_mma", "attention_prefill_tc", "attention_prefill_tc_ok", "attention_prefill_tc_split", "attention_tc_status", "attention_decode_mma",
            "decode_splits", "decode_longest_first", "argmax", "sample", "cast", "bias_act", "scaled_sum", "qkv_norm_write", "gate_group_norm", "head_norm_gate", "rotate_heads",
            "layernorm", "residual_layernorm", "table_gate", "delta_step", "delta_prompt", "experts_combine", "causal_conv", "conv_tail", "gated_scan", "ssm_scan", "block_matvec_f32", "block_matvec_ok", "split_halves"]

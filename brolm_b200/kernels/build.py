@@ -54,6 +54,7 @@ LIBRARIES: dict[str, list[str]] = {
     "linear_attn": ["linear_attn.cu"],
     "layernorm": ["layernorm.cu"],
     "delta_rule": ["delta_rule.cu"],
+    "prompt_layer": ["prompt_layer.cu"],
 }
 HEADERS = ["common.cuh", "once_per_device.h", "attn_mma.cuh", "attn_decode_noalloc.h", "tcgen05.cuh"]
 

@@ -30,8 +30,11 @@ from typing import Optional
 
 import torch
 
+from .. import kernels
+from .attention import Attention
 from .base import Part, PartSpec, register_part
-from .norm import add_then_norm
+from .feedforward import GatedFeedForward
+from .norm import RMSNorm, add_then_norm
 
 
 @dataclasses.dataclass
@@ -84,12 +87,39 @@ class Block(Part):
                 next_norm: Optional[Part]) -> Optional[torch.Tensor]:
         """h: residual stream (updated in place); x = pre_mixer_norm(h).
         Returns next_norm(h) for the block that follows, if there is one."""
+        if ctx.mode == "prefill" and writes_cache and x.dtype == torch.bfloat16 and self._launches_at_once(x, ctx, next_norm):
+            return self._forward_at_once(h, x, ctx, entry, next_norm)
         y = self.mixer.forward(x, ctx, entry, writes_cache)
         if self.feedforward is None:
             return add_then_norm(h, y, self.post_mixer_norm, next_norm, ctx.dtype)
         x = add_then_norm(h, y, self.post_mixer_norm, self.pre_ffn_norm, ctx.dtype)
         y = self.feedforward.forward(x, ctx)
         return add_then_norm(h, y, self.post_ffn_norm, next_norm, ctx.dtype)
+
+
+    def _launches_at_once(self, x: torch.Tensor, ctx, next_norm: Optional[Part]) -> bool:
+        """Whether this is a plain layer (attention without options, a gated feed-forward, four norms) and the step's
+        tokens are so few that the host sets the pace."""
+        m, f = self.mixer, self.feedforward
+        norms = [self.post_mixer_norm, self.pre_ffn_norm, self.post_ffn_norm] + ([next_norm] if next_norm is not None else [])
+        if type(m) is not Attention or type(f) is not GatedFeedForward or m.headwise or m.rowwise or not x.is_contiguous() \
+                or (m.position is not None and m.position.rotary_dim != m.head_dim) \
+                or any(type(n) is not RMSNorm or n.groups != 1 for n in norms) \
+                or norms[0].weight.dtype != norms[1].weight.dtype or norms[2].weight.dtype != norms[-1].weight.dtype:
+            return False
+        return kernels.prompt_layer_ok(x.shape[0], m.head_dim, m.n_q // m.n_kv, f.inter, ctx.max_q_len, m.n_kv, m.window or 0,
+                                       ctx.batch, m.w_qkv, m.w_o, f.w_gate_up, f.w_down)
+
+    def _forward_at_once(self, h: torch.Tensor, x: torch.Tensor, ctx, entry, next_norm: Optional[Part]) -> Optional[torch.Tensor]:
+        m, f = self.mixer, self.feedforward
+        k_pages, v_pages, _, _, page = ctx.kv(entry)
+        norms = [(n.weight, n.eps, n.offset) if n is not None else None
+                 for n in (self.post_mixer_norm, self.pre_ffn_norm, self.post_ffn_norm, next_norm)]
+        return kernels.prompt_layer(h, x, m.w_qkv, m.w_o, f.w_gate_up, f.w_down, norms, ctx.positions,
+                                    m.position.table if m.position is not None else None, ctx.cu_q, ctx.cache_rows[entry.group_id],
+                                    k_pages, v_pages, n_q=m.n_q, n_kv=m.n_kv, head_dim=m.head_dim, page_size=page, batch=ctx.batch,
+                                    max_q_len=ctx.max_q_len, window=m.window or 0, scale=m.scale, cap=m.softcap,
+                                    activation=f.activation, limit=f.limit)
 
 
 register_part("block", "sandwich", Block)
