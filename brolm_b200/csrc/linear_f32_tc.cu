@@ -11,7 +11,7 @@
 // a row's bits depend neither on M nor on its place among the rows, nor on how X lies in memory.
 //
 // A block owns 128 rows of W (the M side of the instruction), up to NT tokens (the N side) and one slice of K.  The sums of
-// the slices are added through the shared memory of a cluster of blocks, or by a kernel behind this one.  Roles:
+// the slices are added through the shared memory of a cluster of blocks, or by the kernel behind this one.  Roles:
 //   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it;
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the two rows of halves into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
@@ -33,8 +33,8 @@
 // error against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.5 to 1.7e-7 here.  The same with three
 // bfloat16 parts a float and six products: 1.4e-7, but 170 us for 300 tokens of 18,432 x 2,304 and 69 us for 3.
 // An infinity or a NaN among the operands ends as a NaN here (infinity minus infinity, infinity times zero), and numbers
-// near the smallest lose their low parts: a result that is not finite, or so small that this may show, is made again
-// from the floats themselves by the thread that stores it.
+// near the smallest lose their low parts: a slice's sum that is not finite, or so small that this may show, is made again
+// from the floats themselves by the thread that has it.
 #include "tcgen05.cuh"
 
 #include <cuda_fp16.h>
@@ -139,24 +139,22 @@ __device__ __forceinline__ uint32_t idesc_half(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int k, int end) {
     float y = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += 512) {
+    for (; k < end; k += 512) {
         float even = 0.0f, odd = 0.0f;
-        const int end = min(K, k0 + 512);
-        for (int k = k0; k < end; k += 2) {                   // K is a multiple of 4
-            even = __fmaf_rn(x[k], w[k], even);
-            odd = __fmaf_rn(x[k + 1], w[k + 1], odd);
+        const int stop = min(end, k + 512);
+        for (int i = k; i < stop; i += 2) {                   // the ends are multiples of 4
+            even = __fmaf_rn(x[i], w[i], even);
+            odd = __fmaf_rn(x[i + 1], w[i + 1], odd);
         }
         y += even + odd;
     }
     return y;
 }
-__device__ __forceinline__ float checked(const Args& g, int token, int row, float y) {
+__device__ __forceinline__ bool doubtful(float y) {
     const float size = fabsf(y);
-    if (!(size <= 3.402823466e38f) || (size < 1e-25f && y != 0.0f))
-        y = plain_dot(g.x + (size_t)token * g.ldx, g.w + (size_t)row * g.ldw, g.K);
-    return y;
+    return !(size <= 3.402823466e38f) || (size < 1e-25f && y != 0.0f);
 }
 
 template <int NT, int BLOCKS>
@@ -325,20 +323,16 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
         }
         if (j == stages) {
-            if (g.parts) {
-                float* dst = g.parts + ((size_t)part * g.M + m0 + first) * g.N + n0 + row;
-                if (n0 + row < g.N) {
+            // the rings are done with: all products have been made
+            float* sums = reinterpret_cast<float*>(smem_raw) + row;
 #pragma unroll
-                    for (int c = 0; c < S::COLS; ++c)
-                        if (first + c < tokens) dst[(size_t)c * g.N] = sum[c];
-                }
-            } else {
-                // the rings are done with: all products have been made
-                float* sums = reinterpret_cast<float*>(smem_raw);
-#pragma unroll
-                for (int c = 0; c < S::COLS; ++c)
-                    if (first + c < tokens) sums[(first + c) * BR + row] = sum[c];
-            }
+            for (int c = 0; c < S::COLS; ++c)
+                if (first + c < tokens) sums[(first + c) * BR] = sum[c];
+            const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
+            if (w_row < (g.gated ? 2 * g.N : g.N))
+                for (int c = first; c < min(first + S::COLS, tokens); ++c)
+                    if (doubtful(sums[c * BR]))
+                        sums[c * BR] = plain_dot(g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo, min(g.K, k_lo + g.slice));
         }
     } else {
         // X: eight k of a token at a time, the eight lanes of a token side by side
@@ -467,37 +461,41 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         else __syncthreads();
     };
     all_here();
-    if (!g.parts && !give_up[0]) {
-        // the blocks of the cluster deal the tokens among them; a thread makes four neighbours of a row of Y
-        const int quads = out_rows / 4;
-        const bool wide_store = g.ldy % 4 == 0 && ((uintptr_t)g.y & 15) == 0;
+    if (!give_up[0]) {
+        // the blocks of the cluster deal the tokens among them; a thread makes four neighbours of a row of Y, or of this slice's sums
+        const int quads = out_rows / 4, ranks = g.parts ? 1 : n_slices, rank = g.parts ? 0 : part;
+        float* dst_rows = g.parts ? g.parts + (size_t)part * g.M * g.N : g.y;
+        const int ld = g.parts ? g.N : g.ldy;
+        const bool wide_store = ld % 4 == 0 && ((uintptr_t)dst_rows & 15) == 0;
         auto total = [&](int t, int row, float (&y)[4]) {
             const uint32_t at = w_ring + (t * BR + row) * 4;
-            for (int r = 0; r < n_slices; ++r) {
-                uint32_t far;
+            for (int r = 0; r < ranks; ++r) {
                 float4 v;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(r));
-                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(far) : "memory");
+                if (ranks > 1) {
+                    uint32_t far;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(r));
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(far) : "memory");
+                } else {
+                    v = lds_float4(at);
+                }
                 y[0] = r ? y[0] + v.x : v.x;
                 y[1] = r ? y[1] + v.y : v.y;
                 y[2] = r ? y[2] + v.z : v.z;
                 y[3] = r ? y[3] + v.w : v.w;
             }
         };
-        const int mine = (tokens - part + n_slices - 1) / n_slices;         // tokens part, part + n_slices, ...
+        const int mine = (tokens - rank + ranks - 1) / ranks;  // tokens rank, rank + ranks, ...
         for (int idx = threadIdx.x; idx < mine * quads; idx += S::THREADS) {
-            const int t = part + n_slices * (idx / quads), c = idx % quads * 4, left = g.N - n0 - c;
+            const int t = rank + ranks * (idx / quads), c = idx % quads * 4, left = g.N - n0 - c;
             if (left <= 0) continue;
             float y[4], u[4];
             total(t, c, y);
-            if (g.gated) total(t, c + BR / 2, u);
+            if (g.gated) {
+                total(t, c + BR / 2, u);
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (e < left) {
-                    y[e] = checked(g, m0 + t, c + e < BR / 2 ? n0 + c + e : second + c + e - BR / 2, y[e]);
-                    if (g.gated) y[e] = gate_pair(y[e], checked(g, m0 + t, second + c + e, u[e]), g.act, g.limit);
-                }
-            float* dst = g.y + (size_t)(m0 + t) * g.ldy + n0 + c;
+                for (int e = 0; e < 4; ++e) y[e] = gate_pair(y[e], u[e], g.act, g.limit);
+            }
+            float* dst = dst_rows + (size_t)(m0 + t) * ld + n0 + c;
             if (wide_store && left >= 4) {
                 *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
             } else {
@@ -554,8 +552,7 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
         float y = g.parts[idx];
 #pragma unroll 4
         for (int s = 1; s < slices; ++s) y += g.parts[s * total + idx];
-        const int token = (int)(idx / g.N), n = (int)(idx % g.N);
-        g.y[(size_t)token * g.ldy + n] = checked(g, token, n, y);
+        g.y[idx / g.N * g.ldy + idx % g.N] = y;
     }
 }
 
@@ -578,7 +575,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, dim3 gri
     cfg.attrs = attr;
     cfg.numAttrs = grid.x > 1 && !g.parts ? 2 : 1;
     const int st = (int)cudaLaunchKernelEx(&cfg, linear_f32_tc_kernel<NT, BLOCKS>, mw, mx, g);
-    if (st || !g.parts) return st;
+    if (st || !g.parts || !g.y) return st;
     const size_t blocks = ((size_t)g.M * g.N + 255) / 256;
     return launch_pdl(add_slices_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, stream, g, (int)grid.x);
 }
@@ -587,7 +584,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, dim3 gri
 
 // Y = X W^T over `slices` slices of K of `slice` k each (a multiple of 64, none empty; at most 8 slices); gated: Y =
 // act(X Wg^T) * (X Wu^T) for W = [Wg; Wu] of 2 N rows.  W's rows lie on 16-byte boundaries, K is a multiple of 4; X's rows
-// may lie anywhere.  parts: room for slices * M * N floats, with which a second kernel adds the slices; null: clusters do.
+// may lie anywhere.  parts: room for slices * M * N floats, with which a second kernel adds the slices (y null: the caller's does); null: clusters do.
 // halves: room for X taken apart ahead (more than 32 rows on 16-byte boundaries), 16-byte aligned, M * ceil(K / 64) * 260 bytes;
 // null: every block does it.
 BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
@@ -636,7 +633,7 @@ BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw
         if (st) return st;
     }
     const dim3 grid(slices, (M + g.tokens - 1) / g.tokens, (unsigned)row_tiles);
-    const bool alone = grid.x <= 4 && (long long)grid.x * grid.y * grid.z <= device_sm_count();
+    const bool alone = (grid.x <= 4 || parts) && (long long)grid.x * grid.y * grid.z <= device_sm_count();
     if (most == 16) return alone ? launch<16, 1>(mw, mx, g, grid, stream) : launch<16, 2>(mw, mx, g, grid, stream);
     if (most == 32) return alone ? launch<32, 1>(mw, mx, g, grid, stream) : launch<32, 2>(mw, mx, g, grid, stream);
     return launch<160, 1>(mw, mx, g, grid, stream);

@@ -1152,6 +1152,21 @@ def linear_f32_tc_scratch(M: int, N: int, slices: int) -> bool:
     return M > 32 and -(-M // 160) * -(-N // 128) < 64 and slices * M * N * 4 <= F32_PARTS_LIMIT
 
 
+def linear_f32_parts(x: torch.Tensor, weight: torch.Tensor) -> int:
+    """How many slices' sums ``linear_f32_slices_into`` leaves for a reader that adds them itself, in order (1: the product is
+    not cut, or is better added at once: 300 rows of 2,304 in eight slices take the residual kernel 21 us, added before it 13)."""
+    return max(1, linear_f32_tc_slices(*weight.shape)) if x.shape[0] <= 32 and linear_f32_tc_ok(weight) else 1
+
+
+def linear_f32_slices_into(x: torch.Tensor, weight: torch.Tensor, sums: torch.Tensor) -> None:
+    """sums (slices, M, N) float32: their sum in order is ``linear_f32``, bit by bit."""
+    (M, K), N = x.shape, weight.shape[0]
+    assert x.dtype == torch.float32 and weight.dtype == torch.float32 and sums.dtype == torch.float32 and sums.is_contiguous()
+    assert x.dim() == 2 and x.stride(1) == 1 and weight.shape[1] == K
+    assert tuple(sums.shape) == (linear_f32_parts(x, weight), M, N) and sums.shape[0] > 1
+    _linear_f32_tc(x, weight, None, sums.shape[0], parts=sums)
+
+
 def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
     """Whether the float32 product with these weights runs on tensor cores, whatever the rows are."""
     N, K = weight.shape
@@ -1186,19 +1201,19 @@ def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, a
     _linear_f32_tc(x, weight, out, linear_f32_tc_slices(*weight.shape), True, ACTIVATIONS[activation], limit)
 
 
-def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, slices: int, gated: bool = False, act: int = 0,
-                   limit: float = 0.0) -> None:
-    (M, K), N = x.shape, out.shape[1]
-    parts = halves = None
+def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], slices: int, gated: bool = False, act: int = 0,
+                   limit: float = 0.0, parts: Optional[torch.Tensor] = None) -> None:
+    (M, K), N = x.shape, out.shape[1] if out is not None else parts.shape[2]
+    halves = None
     if M > 32 and not (x.stride(0) % 4 or x.data_ptr() % 16):
-        if slices > 1 and not gated and linear_f32_tc_scratch(M, N, slices):
+        if parts is None and slices > 1 and not gated and linear_f32_tc_scratch(M, N, slices):
             parts = torch.empty((slices, M, N), dtype=torch.float32, device=x.device)
         size = M * -(-K // 64) * 260                         # the rows as halves, and a scale for every 64
         if size <= F32_PARTS_LIMIT:
             halves = torch.empty(size, dtype=torch.uint8, device=x.device)
     f = _fn("linear_f32_tc", "brolm_linear_f32_tc", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                                      c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p])
-    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0), M, N, K, slices,
+    _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0) if out is not None else N, M, N, K, slices,
              _f32_tc_slice(K, slices), int(gated), act, limit, _ptr(parts), _ptr(halves), _stream()), "linear_f32_tc")
 
 
@@ -2145,7 +2160,7 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, s
 __all__ = ["KernelBuildError", "KernelError", "build_all", "launch_count", "device_sms", "wait_control", "embed_scale",
            "embed_pairs", "concat_cast", "latent_rows", "route_topk", "route_pick", "group_tiles", "group_pairs", "experts_tc_ok", "gather_rows", "experts_linear_tc", "grouped_tc_status", "heads_linear",
            "experts_linear", "rmsnorm", "residual_rmsnorm",
-           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "linear_f32_gated", "linear_f32_tc_ok", "linear_f32_tc_scratch", "linear_f32_tc_slices", "linear_f32_tc_status", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "prompt_layer", "prompt_layer_ok", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
+           "rope_kv_write", "rope_kv_write_parts", "gated_act", "softcap", "linear_f32", "linear_f32_parts", "linear_f32_slices_into", "linear_f32_gated", "linear_f32_tc_ok", "linear_f32_tc_scratch", "linear_f32_tc_slices", "linear_f32_tc_status", "skinny_gemm", "skinny_qkv_rope", "skinny_ok", "skinny_parts", "skinny_rope_tiles", "gemm_tc", "gemm_tc2", "gemm_tc2_status", "gemm_tc_ok", "gemm_tc_status", "gemm_stream", "prompt_layer", "prompt_layer_ok", "gemm_stream_ok", "gemm_stream_parts", "stream_instead_of_skinny", "stream_rows",
            "gemm_stream_status", "attention_simt", "attention_prefill_mma", "attention_prefill_tc", "attention_prefill_tc_ok", "attention_prefill_tc_split", "attention_tc_status", "attention_decode_mma",
            "decode_splits", "decode_longest_first", "argmax", "sample", "cast", "bias_act", "scaled_sum", "qkv_norm_write", "gate_group_norm", "head_norm_gate", "rotate_heads",
            "layernorm", "residual_layernorm", "table_gate", "delta_step", "delta_prompt", "experts_combine", "causal_conv", "conv_tail", "gated_scan", "ssm_scan", "block_matvec_f32", "block_matvec_ok", "split_halves"]

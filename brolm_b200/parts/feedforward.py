@@ -43,7 +43,7 @@ class GatedFeedForward(Part):
         if x.dtype == act.dtype == self.w_gate_up.dtype == torch.float32 and kernels.linear_f32_tc_ok(self.w_gate_up):
             # float: the activation is the product's last step
             kernels.linear_f32_gated(x, self.w_gate_up, act, self.activation, self.limit)
-            return linear(act, self.w_down, out_dtype=torch.float32)
+            return linear(act, self.w_down, out_dtype=torch.float32, parts_ok=True)
         few = kernels.skinny_ok(x, self.w_gate_up)
         stream = kernels.stream_rows(x, self.w_gate_up) or (few and kernels.stream_instead_of_skinny(x, self.w_gate_up))
         if few and not (stream and self.inter % 64 == 0):
