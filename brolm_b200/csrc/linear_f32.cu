@@ -1,7 +1,8 @@
 // True 32-bit matrix product  Y[M,N] = X[M,K] * W[N,K]^T  on CUDA cores
 // (wlejon/brolm include/brolm/detail/compute.h:49-86, the float branch).
 //
-// No tensor cores and no reduced-precision mode: every product and sum is an
+// For weights of up to a million numbers, and those off 16-byte boundaries (linear_f32_tc.cu takes the others; the figures
+// below for larger ones are from before).  No tensor cores and no reduced-precision mode: every product and sum is an
 // IEEE float fma.  One order of sums holds for all kernels of this file,
 // whatever M is, wherever the row stands in the batch and however the work is
 // cut:

@@ -289,3 +289,26 @@ def test_decode_in_wider_batches(setups, name, dtype, batch, monkeypatch):
     eng = bb.Engine(model, max_tokens=64 * batch, max_slots=batch)
     run_batch_teacher_forced(eng, config, weights, prompts, [max(1, n - 4) for n in lengths], dtype)
     assert eng.cache.live_slots == 0
+
+
+@pytest.mark.parametrize("lengths", [[17], [33], [20, 1, 30], [128], [60, 68]])
+@pytest.mark.parametrize("n_kv,head_dim", [(2, 64), (1, 128), (4, 256)])
+def test_a_layer_launched_from_one_call_is_the_layer_launched_kernel_by_kernel(monkeypatch, lengths, n_kv, head_dim):
+    """The same kernels with the same arguments: every logit's bits, and those of a token decoded from the cache."""
+    from brolm_b200 import kernels
+    cfg = bb.Gemma2Config(vocab_size=300, hidden_size=192, intermediate_size=320, num_hidden_layers=3, num_attention_heads=4,
+                          num_key_value_heads=n_kv, head_dim=head_dim, sliding_window=24)
+    model = bb.Model(cfg, dtype="bfloat16", device=DEV).init_random(seed=5)
+    prompts = random_prompts(300, lengths, seed=9)
+    monkeypatch.setattr(kernels, "STREAM_ROWS", 128)         # the products of more than 32 tokens on the stream, too
+    got, launched = [], []
+    for at_once in (True, False):
+        monkeypatch.setattr(kernels, "PROMPT_LAYER", at_once)
+        eng = bb.Engine(model, max_tokens=1024, max_slots=4)
+        slots = eng.open(len(prompts))
+        before = kernels.launch_count()
+        logits = eng.step(slots, prompts, want=[list(range(n)) for n in lengths]).clone()
+        launched.append(kernels.launch_count() - before)
+        got.append((logits, eng.step(slots, [[7]] * len(prompts)).clone()))
+        eng.close(slots)
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and launched[0] == launched[1]

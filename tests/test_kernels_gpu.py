@@ -226,6 +226,23 @@ def test_linear_f32_on_tensor_cores_of_infinities_and_the_smallest_numbers():
     assert torch.equal(out[rows][:, cols], before[rows][:, cols])
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(4100, 260), (2050, 1028), (136, 9216)])
+def test_linear_f32_in_slices(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x, w = torch.randn(M, K + 1, generator=g, device=DEV)[:, 1:], torch.randn(N, K, generator=g, device=DEV)
+    x[0, 3], w[5] = torch.nan, w[5] * 1e-36
+    n = kernels.linear_f32_parts(x, w)
+    assert n == kernels.linear_f32_tc_slices(N, K) > 1 and kernels.linear_f32_parts(x.repeat(33, 1), w) == 1
+    sums, out = torch.full((n, M, N), 7.0, device=DEV), torch.empty(M, N, device=DEV)
+    kernels.linear_f32_slices_into(x, w, sums)
+    kernels.linear_f32(x, w, out)
+    total = sums[0].clone()
+    for s in sums[1:]:
+        total += s
+    assert torch.equal(total.nan_to_num(7.0), out.nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("activation,limit", [("gelu_tanh", 0.0), ("silu", 0.0), ("clamped_gate", 1.5)])
 @pytest.mark.parametrize("M,F,K", [(1, 2048, 256), (16, 520, 1028), (33, 9472, 256), (170, 2100, 512)])
 def test_linear_f32_gated(M, F, K, activation, limit):
@@ -983,6 +1000,30 @@ def test_float_attention_gives_the_same_bits_however_it_is_cut(monkeypatch, opti
         kernels.attention_simt(q[n - 1:], one, torch.tensor([0, 1], dtype=torch.int32, device=DEV), length, k_pages=kp, v_pages=vp,
                                page_table=table, ring=1 << 30, page_size=64, max_q_len=1, **kw)
         assert torch.equal(one[0], shared[n - 1])
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd,vd", [(8, 1, 256, 256), (8, 1, 8, 8), (5, 1, 40, 24), (6, 2, 136, 200), (16, 4, 64, 16)])
+@pytest.mark.parametrize("tokens", [1, 2])
+def test_float_attention_of_a_few_rows_gives_the_bits_of_more(monkeypatch, n_q, n_kv, hd, vd, tokens):
+    """Up to eight rows in clusters that share a span, value rows of fewer entries than the blocks' shares, several spans and a
+    bound that does not hold, against the same rows walked by one block."""
+    g = torch.Generator(device=DEV).manual_seed(hd + vd)
+    group = n_q // n_kv
+    tokens = 1 if tokens * group > 8 else tokens
+    lengths = [2, 128, 129, 500, 31]
+    B, table = len(lengths), torch.randperm(40, generator=g, device=DEV).to(torch.int32).view(5, 8)
+    kp, vp = torch.randn(40, n_kv, 64, hd, generator=g, device=DEV), torch.randn(40, n_kv, 64, vd, generator=g, device=DEV)
+    q = torch.randn(B * tokens, n_q * hd, generator=g, device=DEV)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: True)
+    outs = []
+    for splits in (0, 4, 2):                                 # walked; shared; shared, with spans left for the last share
+        monkeypatch.setattr(kernels, "attn_f32_splits", lambda *a, **kw: splits)
+        outs.append(torch.full((B * tokens, n_q * vd), float("nan"), device=DEV))
+        kernels.attention_simt(q, outs[-1], torch.arange(0, B * tokens + 1, tokens, dtype=torch.int32, device=DEV),
+                               torch.tensor(lengths, dtype=torch.int32, device=DEV), n_kv=n_kv, group=group, head_dim=hd, v_dim=vd,
+                               scale=hd ** -0.5, cap=30.0, window=0, batch=B, max_q_len=tokens, k_pages=kp, v_pages=vp,
+                               page_table=table, ring=1 << 30, page_size=64)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and not bool(outs[0].isnan().any())
 
 
 @pytest.mark.parametrize("shared", [False, True])
