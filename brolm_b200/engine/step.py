@@ -205,6 +205,7 @@ class Engine:
             self.beside = kernels.take_stream(index)
             weakref.finalize(self, kernels.give_stream, index, self.beside)
         self.last_h2d_bytes = 0          # bytes the last step copied from the host
+        self._checked_at = -1            # this library's launches when the kernels' status words were last read
         self._pin: Optional[torch.Tensor] = None      # pinned staging buffer of the steps that are not captured
         self._pin_copied = None
 
@@ -225,8 +226,9 @@ class Engine:
     def _check_waits(self, where: str, consequence: str) -> None:
         """Raise if a bounded wait inside one of the tcgen05 kernels ran out since the last check.
         Reads and resets every status word (each read waits for the device)."""
-        if self.device.type != "cuda":
-            return
+        if self.device.type != "cuda" or self._checked_at == kernels.launch_count():
+            return                       # (nothing of this library has run since: a prompt is checked at its step's end)
+        self._checked_at = kernels.launch_count()
         codes = {"linear_f32_tc": kernels.linear_f32_tc_status(reset=True)}
         if self.model.dtype == torch.bfloat16:
             codes |= {"gemm_tc": kernels.gemm_tc_status(reset=True), "attn_tc": kernels.attention_tc_status(reset=True),
