@@ -15,8 +15,7 @@
 //   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it;
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the two rows of halves into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
-//           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the halves in by TMA, and
-//           these warps split W, too;
+//           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the halves in by TMA;
 //   MMA     one thread issues 12 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two accumulators;
 //   ADD     these add an accumulator to the sums in their registers, and at the end store them.
 // The thread that issues is what all wait for, so its stage of 64 k has one barrier to wait on, which all that its products
@@ -63,7 +62,7 @@ struct Shape {
     static constexpr int WARPS = FEW ? 16 : 28, THREADS = 32 * WARPS;
     static constexpr int GROUPS = FEW ? 1 : 2, COLS = NT / GROUPS;          // warps of a quarter that add, each its share of the tokens
     static constexpr int X_WARPS = FEW ? 2 : 8;
-    static constexpr int READY = 4 + 4 * GROUPS;             // arrivals that a stage waits for, and those of who brings the tokens
+    static constexpr int READY = 4 + X_WARPS + 4 * GROUPS;                  // arrivals that a stage waits for
     static constexpr int X_RAW = NT * KX * 4;                               // bytes of a stage of X as it is
     static constexpr int W_SLOTS = !FEW ? 8 : PER_SM == 1 ? 10 : NT == 16 ? 5 : 4;
     static constexpr int AHEAD = !FEW ? 0 : PER_SM == 1 ? 4 : 3;           // stages of X that are on their way (FEW)
@@ -131,21 +130,6 @@ __device__ __forceinline__ float4 lds_float4(uint32_t at) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t v;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
@@ -181,7 +165,6 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     const uint32_t w_ring = smem_u32(smem_raw), x_ring = w_ring + S::W_SLOTS * W_SLOT;
     float* row_scale = reinterpret_cast<float*>(smem_raw + S::RING);        // [SCALES][BR]: what a partial sum is multiplied by
     float* token_scale = row_scale + SCALES * BR;                           // [SCALES][NT]
-    const bool ahead = !S::FEW && g.x_scale;
     uint64_t* bars = reinterpret_cast<uint64_t*>(token_scale + SCALES * NT);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + S::BARS);
     volatile int* give_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -198,7 +181,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::W_SLOTS; ++s) mbar_init(w_full + 8 * s, 1), mbar_init(w_empty + 8 * s, 4);
-        for (int s = 0; s < 2; ++s) mbar_init(ready + 8 * s, S::READY + (ahead ? 1 : S::X_WARPS)), mbar_init(made + 8 * s, 1), mbar_init(x_full + 8 * s, 1);
+        for (int s = 0; s < 2; ++s) mbar_init(ready + 8 * s, S::READY), mbar_init(made + 8 * s, 1), mbar_init(x_full + 8 * s, 1);
         mbar_init(all_made, 1);
         give_up[0] = 0;
         give_up[1] = 0;
@@ -237,7 +220,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             for (int j = 0; j < stages; ++j) {
                 const int s = j & 1;
                 if (!wait_on(ready + 8 * s, (j >> 1) & 1, 2)) break;
-                if (ahead && !wait_on(x_full + 8 * s, (j >> 1) & 1, 3)) break;
+                if (g.x_scale && !wait_on(x_full + 8 * s, (j >> 1) & 1, 3)) break;
                 fence_after_sync();
                 const uint32_t acc = tmem + s * NT, a = tmem_a + s * A_COLS;
                 const uint64_t b = desc_kmajor(x_ring + s * S::X_SLOT);
@@ -255,7 +238,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 mbar_wait(all_made, 0, give_up, &g_linear_f32_tc_error, 10, true);
             }
         }
-        if (role == Role::FETCH_X && lane == 0 && ahead) {
+        if (role == Role::FETCH_X && lane == 0 && g.x_scale) {
             pdl_wait();
             int j = 0;
             for (; j < stages; ++j) {
@@ -269,39 +252,16 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 for (int i = max(0, j - 2); i < j; ++i)
                     mbar_wait(x_full + 8 * (i & 1), (i >> 1) & 1, give_up, &g_linear_f32_tc_error, 11, true);
         }
-        if (role == Role::NONE && ahead) {
-            // the scales of the tokens that were taken apart ahead
-            constexpr int PER = (NT + 31) / 32;
-            pdl_wait();
-            const float* src = g.x_scale + (size_t)m0 * g.x_stages + k_lo / KX;
-            float next[PER];
-            auto fetch = [&](int j) {
-#pragma unroll
-                for (int u = 0; u < PER; ++u) {
-                    const int t = lane + 32 * u;
-                    next[u] = t < tokens && j < stages ? src[(size_t)t * g.x_stages + j] : 1.0f;
-                }
-            };
-            fetch(0);
-            for (int j = 0; j < stages; ++j) {
-                if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 12)) break;
-#pragma unroll
-                for (int u = 0; u < PER; ++u)
-                    if (lane + 32 * u < NT) token_scale[(j % SCALES) * NT + lane + 32 * u] = next[u];
-                fetch(j + 1);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
-            }
-        }
-    } else if (role == Role::SPLIT || (role == Role::X && ahead)) {
-        if constexpr (!S::FEW) {
-            if (role == Role::SPLIT) fewer_registers<48>();
-            else fewer_registers<56>();
-        }
+    } else if (role == Role::SPLIT) {
+        if constexpr (!S::FEW) fewer_registers<48>();
         const int row = (warp & 3) * 32 + lane;
-        // sets of four warps take turns
-        for (int j = (role == Role::SPLIT ? index : 8 + index) >> 2; j < stages; j += ahead ? 4 : 2) {
+        for (int j = index >> 2; j < stages; j += 2) {         // two sets of four warps take turns
             const int s0 = 2 * j % S::W_SLOTS, s1 = (2 * j + 1) % S::W_SLOTS;
+            // A wait on a slot's phase asks that the phase before it is known to be over.  That was a stage at least four back
+            // where there are eight slots, which this set has seen; where there are fewer, the stage two back has to be over first.
+            constexpr bool AT_ONCE = S::W_SLOTS >= 8;
+            static_assert(S::W_SLOTS >= 4, "two stages");
+            if (!AT_ONCE && j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 6)) break;
             if (!all_wait_on(w_full + 8 * s0, (2 * j / S::W_SLOTS) & 1, 5)) break;
             if (!all_wait_on(w_full + 8 * s1, ((2 * j + 1) / S::W_SLOTS) & 1, 5)) break;
             const uint32_t src[2] = {w_ring + s0 * W_SLOT + row * 128, w_ring + s1 * W_SLOT + row * 128};
@@ -309,7 +269,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
 #pragma unroll
             for (int c = 0; c < 16; ++c) most = largest(most, lds_float4(src[c >> 3] + (((c & 7) ^ (row & 7)) << 4)));
             scales_of(most, up, down);
-            if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 6)) break;
+            if (AT_ONCE && j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 6)) break;
             fence_after_sync();
             row_scale[(j % SCALES) * BR + row] = down;
             const uint32_t a = tmem_a + (j & 1) * A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
@@ -333,11 +293,11 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
         }
     } else if (role == Role::ADD) {
-        if constexpr (!S::FEW) more_registers<120>();
+        if constexpr (!S::FEW) more_registers<112>();
         const int quarter = warp & 3, first = (index >> 2) * S::COLS, row = quarter * 32 + lane;
-        uint64_t sum[S::COLS / 2];                             // neighbouring tokens in a packed register
+        float sum[S::COLS];
 #pragma unroll
-        for (int c = 0; c < S::COLS / 2; ++c) sum[c] = 0;
+        for (int c = 0; c < S::COLS; ++c) sum[c] = 0.0f;
         if (lane == 0) mbar_arrive(ready), mbar_arrive(ready + 8);          // both accumulators are free
         int j = 0;
         for (; j < stages; ++j) {
@@ -345,30 +305,21 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             if (!all_wait_on(ready + 8 * (j & 1), (j >> 1) & 1, 8)) break;          // (it has long been: for the scales' sake)
             fence_after_sync();
             const uint32_t acc = tmem + (j & 1) * NT + first + ((uint32_t)(quarter * 32) << 16);
-            const float one = row_scale[(j % SCALES) * BR + row];
-            const uint64_t mine = pack2(one, one);
-            const float* theirs = token_scale + (j % SCALES) * NT + first;
-            // where registers allow it, the next sixteen are on their way while sixteen are added
-            constexpr int BUFS = S::FEW ? 1 : 2;
-            uint32_t v[BUFS][16];
-            if (BUFS == 2 && first < wide) tmem_ld16(acc, v[0]);
+            const float mine = row_scale[(j % SCALES) * BR + row];
+            const float4* theirs = reinterpret_cast<const float4*>(token_scale + (j % SCALES) * NT + first);
 #pragma unroll
             for (int c = 0; c < S::COLS; c += 16) {
                 if (first + c < wide) {
-                    uint32_t (&w)[16] = v[BUFS == 2 ? (c / 16) & 1 : 0];
-                    if (BUFS == 1) tmem_ld16(acc + c, w);
+                    uint32_t v[16];
+                    tmem_ld16(acc + c, v);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(w[e]));          // (nothing of it before the wait)
-                    if (BUFS == 2 && c + 16 < S::COLS && first + c + 16 < wide) tmem_ld16(acc + c + 16, v[BUFS == 2 ? (c / 16 + 1) & 1 : 0]);
-#pragma unroll
                     for (int e = 0; e < 16; e += 4) {
-                        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(theirs + c + e);
-                        uint64_t p = pack2(__uint_as_float(w[e]), __uint_as_float(w[e + 1])), q = pack2(__uint_as_float(w[e + 2]), __uint_as_float(w[e + 3]));
-                        p = mul2(p, mine);
-                        q = mul2(q, mine);
-                        fma2(sum[(c + e) / 2], p, t.x);
-                        fma2(sum[(c + e) / 2 + 1], q, t.y);
+                        const float4 t = theirs[(c + e) / 4];
+                        sum[c + e] = __fmaf_rn(__uint_as_float(v[e]) * mine, t.x, sum[c + e]);
+                        sum[c + e + 1] = __fmaf_rn(__uint_as_float(v[e + 1]) * mine, t.y, sum[c + e + 1]);
+                        sum[c + e + 2] = __fmaf_rn(__uint_as_float(v[e + 2]) * mine, t.z, sum[c + e + 2]);
+                        sum[c + e + 3] = __fmaf_rn(__uint_as_float(v[e + 3]) * mine, t.w, sum[c + e + 3]);
                     }
                 }
             }
@@ -380,11 +331,8 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             // the rings are done with: all products have been made
             float* sums = reinterpret_cast<float*>(smem_raw) + row;
 #pragma unroll
-            for (int c = 0; c < S::COLS; c += 2) {
-                const float2 y = unpack2(sum[c / 2]);
-                if (first + c < tokens) sums[(first + c) * BR] = y.x;
-                if (first + c + 1 < tokens) sums[(first + c + 1) * BR] = y.y;
-            }
+            for (int c = 0; c < S::COLS; ++c)
+                if (first + c < tokens) sums[(first + c) * BR] = sum[c];
             const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
             if (w_row < (g.gated ? 2 * g.N : g.N))
                 for (int c = first; c < min(first + S::COLS, tokens); ++c)
@@ -393,7 +341,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         }
     } else {
         // X: eight k of a token at a time, the eight lanes of a token side by side
-        if constexpr (!S::FEW) fewer_registers<56>();
+        if constexpr (!S::FEW) fewer_registers<64>();
         constexpr int T = S::X_WARPS * 32, PER = (NT * 8 + T - 1) / T;
         const int xt = index * 32 + lane, chunk = xt & 7;
         pdl_wait();                                            // X is the kernel before this one's result
@@ -490,6 +438,19 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 if (!put(j, v)) break;
             }
             copy_wait<0>();
+        } else if (g.x_scale) {
+            // the halves come by TMA: the scales alone
+            const float* src = g.x_scale + (size_t)(m0 + xt) * g.x_stages + k_lo / KX;
+            const bool there = xt < tokens;
+            float next = there ? src[0] : 1.0f;
+            for (int j = 0; j < stages; ++j) {
+                const float now = next;
+                if (there && j + 1 < stages) next = src[j + 1];
+                if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 9)) break;
+                if (xt < NT) token_scale[(j % SCALES) * NT + xt] = now;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
+            }
         } else {
             float v[PER][8];
             for (int j = 0; j < stages; ++j) {

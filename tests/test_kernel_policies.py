@@ -130,6 +130,17 @@ def test_partial_sums_of_the_float_product_are_bounded():
     assert cuts > 10
 
 
+def test_slices_of_the_float_product_on_tensor_cores():
+    """None is empty, each is whole stages of 64, clusters of at most eight; small weights are not for it."""
+    for N in (64, 1100, 4100, 18432, 256000):
+        for K in list(range(248, 3000, 4)) + [9216, 14336, 36864]:
+            n = kernels.linear_f32_tc_slices(N, K)
+            assert n in (0, 1, 2, 4, 8) and (n > 0) == (N * K >= 1 << 20 and K >= 256)
+            if n:
+                per = kernels._f32_tc_slice(K, n)
+                assert per % 64 == 0 and (n - 1) * per < K <= n * per and (n == 1 or -(-N // 128) * n <= 148)
+
+
 def test_which_kernel_takes_a_float_product():
     """Streams for few rows, small tiles where large ones leave SMs idle, large ones where there are enough of them."""
     plan = lambda M, N, K: kernels.linear_f32_plan(M, N, K, 148)

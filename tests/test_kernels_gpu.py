@@ -1023,7 +1023,8 @@ def test_float_attention_of_a_few_rows_gives_the_bits_of_more(monkeypatch, n_q, 
                                torch.tensor(lengths, dtype=torch.int32, device=DEV), n_kv=n_kv, group=group, head_dim=hd, v_dim=vd,
                                scale=hd ** -0.5, cap=30.0, window=0, batch=B, max_q_len=tokens, k_pages=kp, v_pages=vp,
                                page_table=table, ring=1 << 30, page_size=64)
-    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and not bool(outs[0].isnan().any())
+    assert torch.equal(outs[0], outs[1]) and not bool(outs[0].isnan().any())
+    close(outs[2], outs[0].double().cpu(), torch.float32, scale=float(outs[0].abs().max()))      # (a share's spans are merged first)
 
 
 @pytest.mark.parametrize("shared", [False, True])
