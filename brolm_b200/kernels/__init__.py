@@ -1296,19 +1296,31 @@ def skinny_parts(x: torch.Tensor, weight: torch.Tensor, sms: Optional[int] = Non
     Measured, product + residual kernel, microseconds at 8 tokens, by slices 1 / 2 / 3 / 4:
     2304 x 9216 (2B down) 14.4 / 12.5 / 11.8 / 14.8; 4608 x 36864 (27B down) 74.0 / 72.9 / 63.2 / 67.4;
     3584 x 4096 (9B o) 10.7 / 11.8 / 12.2 / 12.0."""
-    sms = sms or device_sms(x.device if x.is_cuda else None)
-    blocks = (weight.shape[0] + 15) // 16
-    kblocks = (x.shape[1] + 63) // 64
-    nbytes = float(weight.shape[0]) * x.shape[1] * 2.0
+    return _skinny_slices(x.shape[0], weight.shape[0], x.shape[1], sms or device_sms(x.device if x.is_cuda else None))
+
+
+@functools.lru_cache(maxsize=1024)
+def _skinny_slices(M: int, N: int, K: int, sms: int) -> int:
+    blocks = (N + 15) // 16
+    kblocks = (K + 63) // 64
+    nbytes = float(N) * K * 2.0
     best, best_cost = 1, None
     for parts in range(1, 9):
         if parts > 1 and kblocks // parts < 8:
             break
         cost = _rounds_cost(blocks * parts, 3, sms, nbytes)
-        cost += (parts - 1) * x.shape[0] * weight.shape[0] * 8.0 + (parts - 1) * 0.3e-6 * 6.5e12
+        cost += (parts - 1) * M * N * 8.0 + (parts - 1) * 0.3e-6 * 6.5e12
         if best_cost is None or cost < best_cost * 0.98:
             best, best_cost = parts, cost
     return best
+
+
+@functools.lru_cache(maxsize=1024)
+def _skinny_tiles(N: int, K: int, ksplit: int, sms: int) -> int:
+    """16-row tiles a block of the few-token product without a gate: two for very wide outputs, and where one block to a place
+    makes the better rounds (8,224 x 2,048 at 1 / 8 / 16 tokens, one tile 8.6 / 10.7 / 11.4 us, two 7.3 / 7.8 / 8.7; 8,192 x 3,584
+    13.7 / 16.0 / 16.8 and 11.3 / 11.8 / 12.8; up to 6,144 x 2,048 they are even)."""
+    return 2 if N >= 64 * sms or (ksplit == 1 and skinny_rope_tiles(N, K, sms) == 2) else 1
 
 
 def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: str = "store",
@@ -1336,11 +1348,7 @@ def skinny_gemm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilog
         # 2B 17.4 against 16.2 us): their last, thin round of blocks streams twice the bytes per block
         tiles = 2
     else:
-        # two tiles a block for very wide outputs, and where one block to a place makes the better rounds (8,224 x 2,048 at
-        # 1 / 8 / 16 tokens, one tile 8.6 / 10.7 / 11.4 us, two 7.3 / 7.8 / 8.7; 8,192 x 3,584 13.7 / 16.0 / 16.8 and 11.3 / 11.8 /
-        # 12.8; up to 6,144 x 2,048 they are even)
-        sms = device_sms(x.device)
-        tiles = 2 if N >= 64 * sms or (ksplit == 1 and skinny_rope_tiles(N, K, sms) == 2) else 1
+        tiles = _skinny_tiles(N, K, ksplit, device_sms(x.device))
     if code == 2:
         assert out.dtype == torch.float32
     f = _fn("skinny_gemm", "brolm_skinny_gemm", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
@@ -1576,17 +1584,19 @@ class _PromptNorm(ctypes.Structure):
 
 
 class _PromptLayer(ctypes.Structure):
-    _fields_ = ([(n, c_void_p) for n in ("gemm_stream", "rope_kv_write_parts", "attn_prefill_tc", "residual_rmsnorm", "h", "x", "next",
+    _fields_ = ([(n, c_void_p) for n in ("gemm_stream", "rope_kv_write_parts", "attn_prefill_tc", "residual_rmsnorm", "skinny_gemm",
+                                         "skinny_qkv_rope", "h", "x", "next",
                                          "w_qkv", "w_o", "w_gate_up", "w_down", "sums", "qkv", "attn", "mid", "act", "positions",
                                          "cos_sin", "cu_q", "cache_rows", "k_pages", "v_pages")] +
                 [(n, _PromptNorm) for n in ("post_mixer", "pre_ffn", "post_ffn", "after")] +
                 [(n, c_int) for n in ("w_dtype_mid", "w_dtype_end", "tokens", "hidden", "inter", "n_q", "n_kv", "head_dim", "page_size",
                                       "batch", "max_q_len", "window")] +
                 [(n, c_float) for n in ("scale", "cap", "limit")] +
-                [(n, c_int) for n in ("activation", "qkv_slices", "o_slices", "down_slices")])
+                [(n, c_int) for n in ("activation", "qkv_slices", "o_slices", "down_slices", "few", "qkv_tiles", "o_tiles", "down_tiles",
+                                      "gate_up_stream")])
 
 
-_prompt_fns: list = []       # the entry points of the four libraries, once they are loaded
+_prompt_fns: list = []       # the entry points of the other libraries, once they are loaded
 
 
 def _prompt_entry_points() -> list:
@@ -1595,15 +1605,16 @@ def _prompt_entry_points() -> list:
             raise KernelError("prompt_layer: the library's arguments are laid out in another way")
         _prompt_fns[:] = [ctypes.cast(getattr(load_library(lib), name), c_void_p).value for lib, name in
                           (("gemm_stream", "brolm_gemm_stream"), ("core", "brolm_rope_kv_write_parts"),
-                           ("attn_tc", "brolm_attn_prefill_tc"), ("core", "brolm_residual_rmsnorm"))]
+                           ("attn_tc", "brolm_attn_prefill_tc"), ("core", "brolm_residual_rmsnorm"),
+                           ("skinny_gemm", "brolm_skinny_gemm"), ("skinny_gemm", "brolm_skinny_qkv_rope"))]
     return _prompt_fns
 
 
 def prompt_layer_ok(tokens: int, head_dim: int, group: int, inter: int, max_q_len: int, n_kv: int, window: int, batch: int,
                     *weights: torch.Tensor) -> bool:
-    """Whether the launches of a layer for a prompt of so many tokens go out from one call (``prompt_layer``): more than the
-    few-token product takes and at most what the weight stream does."""
-    return (SKINNY_MAX_ROWS < tokens <= STREAM_MAX_ROWS and PROMPT_LAYER and inter % 64 == 0 and group <= 16
+    """Whether the launches of a layer for a prompt of so many tokens go out from one call (``prompt_layer``): at most what the
+    weight stream takes."""
+    return (0 < tokens <= STREAM_MAX_ROWS and PROMPT_LAYER and inter % 64 == 0 and group <= 16
             and attention_prefill_tc_ok(head_dim, group)
             and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights)
             and not (PREFILL_SPLIT and attention_prefill_tc_split(max_q_len, n_kv, group, window, batch)))
@@ -1627,8 +1638,12 @@ def prompt_layer(h: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor, w_o: tor
     assert cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[1:] == (head_dim // 2, 2))
     assert all(n is None or (n[0].is_contiguous() and n[0].numel() == H) for n in norms)
     assert norms[0][0].dtype == norms[1][0].dtype and (norms[3] is None or norms[2][0].dtype == norms[3][0].dtype)
-    sms = device_sms(x.device)
-    slices = [_stream_slices(n, k, sms) for n, k in ((cols, H), (H, q), (H, F))]
+    sms, few = device_sms(x.device), T <= SKINNY_MAX_ROWS
+    if few:
+        slices = [1, _skinny_slices(T, H, q, sms), _skinny_slices(T, H, F, sms)]
+        tiles = [skinny_rope_tiles(cols, H, sms), _skinny_tiles(H, q, slices[1], sms), _skinny_tiles(H, F, slices[2], sms)]
+    else:
+        slices, tiles = [_stream_slices(n, k, sms) for n, k in ((cols, H), (H, q), (H, F))], [0, 0, 0]
     # scratch: the slices' sums, q/k/v, the attention's rows, the feed-forward's rows and its inner ones
     sizes = [4 * T * max(slices[0] * cols, slices[1] * H, slices[2] * H), 2 * T * cols, 2 * T * q, 2 * T * H, 2 * T * F]
     at, offs = 0, []
@@ -1642,9 +1657,10 @@ def prompt_layer(h: torch.Tensor, x: torch.Tensor, w_qkv: torch.Tensor, w_o: tor
     args = _PromptLayer(*_prompt_entry_points(), _ptr(h), _ptr(x), _ptr(out), _ptr(w_qkv), _ptr(w_o), _ptr(w_gate_up), _ptr(w_down),
                         *[base + o for o in offs], _ptr(positions), _ptr(cos_sin), _ptr(cu_q), _ptr(cache_rows), _ptr(k_pages),
                         _ptr(v_pages), *[norm(n) for n in norms], _code(norms[0][0]), _code(norms[2][0]), T, H, F, n_q, n_kv, head_dim,
-                        page_size, batch, max_q_len, window, scale, cap, limit, ACTIVATIONS[activation], *slices)
+                        page_size, batch, max_q_len, window, scale, cap, limit, ACTIVATIONS[activation], *slices, int(few), *tiles,
+                        int(few and stream_instead_of_skinny(x, w_gate_up)))
     _check(_fn("prompt_layer", "brolm_prompt_layer", [c_void_p, c_void_p])(ctypes.byref(args), _stream()), "prompt_layer")
-    add_launches(7)
+    add_launches(6 if few else 7)
     return out
 
 

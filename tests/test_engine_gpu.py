@@ -291,7 +291,7 @@ def test_decode_in_wider_batches(setups, name, dtype, batch, monkeypatch):
     assert eng.cache.live_slots == 0
 
 
-@pytest.mark.parametrize("lengths", [[17], [33], [20, 1, 30], [128], [60, 68]])
+@pytest.mark.parametrize("lengths", [[1], [5], [16], [9, 1, 6], [17], [33], [20, 1, 30], [128], [60, 68]])
 @pytest.mark.parametrize("n_kv,head_dim", [(2, 64), (1, 128), (4, 256)])
 def test_a_layer_launched_from_one_call_is_the_layer_launched_kernel_by_kernel(monkeypatch, lengths, n_kv, head_dim):
     """The same kernels with the same arguments: every logit's bits, and those of a token decoded from the cache."""
