@@ -1489,6 +1489,7 @@ STREAM_MAX_ROWS = 128
 # 24 rows 9,598 / 9,582; 32 rows 12,708 / 12,660; 48 rows 14,076 / 14,436; 64 rows 18,676 / 19,152;
 # 96 rows 20,727 / 22,622; 128 rows 23,901 / 25,584.  With 64 and 128 token columns a stage of the ring is a
 # third and a half tokens, so fewer bytes of weights are in flight per SM; up to 32 it is at least even.
+# (Prompts of plain layers take the stream up to 128 tokens all the same: there the host sets the pace, ``prompt_layer``.)
 # BROLM_STREAM_ROWS=128 takes every product of up to 128 tokens to the own kernel, =16 none.
 STREAM_ROWS = int(os.environ.get("BROLM_STREAM_ROWS", "32"))
 

@@ -14,7 +14,8 @@ element type in the same way).
   accumulator in tensor memory), float32 accumulation, where there are at
   least as many output tiles as SMs; else, and for operands that kernel does
   not take (a width that is no multiple of 8), the library product (cuBLAS
-  through torch), which so has most products of 33 to 128 rows and, at 2,048
+  through torch), which so has most products of 33 to 128 rows (those of
+  plain layers' prompts excepted, block.py) and, at 2,048
   rows, the narrow ones (o and down of the 2B sizes).  The result is bfloat16
   or, on request, float32.
 """
