@@ -1170,6 +1170,8 @@ def linear_f32_slices_into(x: torch.Tensor, weight: torch.Tensor, sums: torch.Te
 def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
     """Whether the float32 product with these weights runs on tensor cores, whatever the rows are."""
     N, K = weight.shape
+    if N * K < 1 << 20:                                      # (asked for each product of a tiny model's prompt, too)
+        return False
     return not (K % 4 or weight.stride(0) % 4 or weight.data_ptr() % 16) and weight.stride(1) == 1 and linear_f32_tc_slices(N, K) > 0
 
 

@@ -40,7 +40,7 @@ class GatedFeedForward(Part):
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """x (tokens, hidden) -> (tokens, hidden) float32."""
         act = torch.empty((x.shape[0], self.inter), dtype=ctx.dtype, device=x.device)
-        if x.dtype == act.dtype == self.w_gate_up.dtype == torch.float32 and kernels.linear_f32_tc_ok(self.w_gate_up):
+        if ctx.dtype == torch.float32 and kernels.linear_f32_tc_ok(self.w_gate_up) and x.dtype == self.w_gate_up.dtype == torch.float32:
             # float: the activation is the product's last step
             kernels.linear_f32_gated(x, self.w_gate_up, act, self.activation, self.limit)
             return linear(act, self.w_down, out_dtype=torch.float32, parts_ok=True)

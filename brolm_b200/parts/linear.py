@@ -38,7 +38,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if weight.dtype == torch.float32:
         x32 = x if x.dtype == torch.float32 else x.float()
         want = out_dtype or x.dtype
-        parts = kernels.linear_f32_parts(x32, weight) if parts_ok and want == torch.float32 and out is None else 1
+        parts = kernels.linear_f32_parts(x32, weight) if parts_ok and M <= 32 and want == torch.float32 and out is None else 1
         if parts > 1:
             y = torch.empty((parts, M, N), dtype=torch.float32, device=x.device)
             kernels.linear_f32_slices_into(x32, weight, y)
