@@ -620,56 +620,42 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(bf16* __restrict
                                                                 int page_size) {
     const int t = blockIdx.x;
     pdl_trigger();
-    // positions, places and angles are not the product's: they are fetched while it ends
-    const int pos = positions[t];                 // (the host's, written before the step's first kernel)
-    const int crow = k_pages && pos >= 0 ? cache_rows[t] : -1;
+    pdl_wait();
+    const int pos = positions[t];
+    if (pos < 0) return;
     const int half = hd >> 1, per_head = half >> 3;
     const int heads = n_q + 2 * n_kv;
+    const int crow = k_pages ? cache_rows[t] : -1;
     bf16* row = qkv + (size_t)t * heads * hd;
-    float4 cs[4];
-    int item = threadIdx.x, head = item / per_head, i0 = (item - head * per_head) << 3;
-    auto angles = [&] {
-        if (cos_sin != nullptr && pos >= 0 && head < n_q + n_kv) {
-            const float4* at = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * half + i0);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cs[j] = at[j];
-        }
-    };
-    angles();
-    pdl_wait();
-    if (pos < 0) return;
-    for (; item < heads * per_head; ) {
+    for (int item = threadIdx.x; item < heads * per_head; item += blockDim.x) {
+        const int head = item / per_head, i0 = (item - head * per_head) << 3;
         const bool is_v = head >= n_q + n_kv, is_k = !is_v && head >= n_q;
         const bool rotate = !is_v && cos_sin != nullptr;
         const bool keep = crow >= 0 && (is_k || is_v);
-        if (rotate || keep) {
-            bf16* p = row + (size_t)head * hd;
-            uint4 ra = *reinterpret_cast<const uint4*>(p + i0), rb = *reinterpret_cast<const uint4*>(p + half + i0);
-            if (rotate) {
-                __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&ra);
-                __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&rb);
+        if (!rotate && !keep) continue;
+        bf16* p = row + (size_t)head * hd;
+        uint4 ra = *reinterpret_cast<const uint4*>(p + i0), rb = *reinterpret_cast<const uint4*>(p + half + i0);
+        if (rotate) {
+            const float4* cs = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * half + i0);
+            __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&ra);
+            __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&rb);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 c = cs[j];                   // (cos, sin) of pairs 2j and 2j + 1
-                    const float2 fa = __bfloat1622float2(a2[j]), fb = __bfloat1622float2(b2[j]);
-                    a2[j] = __floats2bfloat162_rn(fa.x * c.x - fb.x * c.y, fa.y * c.z - fb.y * c.w);
-                    b2[j] = __floats2bfloat162_rn(fa.x * c.y + fb.x * c.x, fa.y * c.w + fb.y * c.z);
-                }
-                *reinterpret_cast<uint4*>(p + i0) = ra;
-                *reinterpret_cast<uint4*>(p + half + i0) = rb;
+            for (int j = 0; j < 4; ++j) {
+                const float4 c = cs[j];                       // (cos, sin) of pairs 2j and 2j + 1
+                const float2 fa = __bfloat1622float2(a2[j]), fb = __bfloat1622float2(b2[j]);
+                a2[j] = __floats2bfloat162_rn(fa.x * c.x - fb.x * c.y, fa.y * c.z - fb.y * c.w);
+                b2[j] = __floats2bfloat162_rn(fa.x * c.y + fb.x * c.x, fa.y * c.w + fb.y * c.z);
             }
-            if (keep) {
-                const int g = is_k ? head - n_q : head - n_q - n_kv;
-                bf16* dst = (is_k ? k_pages : v_pages) +
-                            (((size_t)(crow / page_size) * n_kv + g) * page_size + crow % page_size) * hd;
-                *reinterpret_cast<uint4*>(dst + i0) = ra;
-                *reinterpret_cast<uint4*>(dst + half + i0) = rb;
-            }
+            *reinterpret_cast<uint4*>(p + i0) = ra;
+            *reinterpret_cast<uint4*>(p + half + i0) = rb;
         }
-        item += blockDim.x;
-        head = item / per_head;
-        i0 = (item - head * per_head) << 3;
-        angles();
+        if (keep) {
+            const int g = is_k ? head - n_q : head - n_q - n_kv;
+            bf16* dst = (is_k ? k_pages : v_pages) +
+                        (((size_t)(crow / page_size) * n_kv + g) * page_size + crow % page_size) * hd;
+            *reinterpret_cast<uint4*>(dst + i0) = ra;
+            *reinterpret_cast<uint4*>(dst + half + i0) = rb;
+        }
     }
 }
 
