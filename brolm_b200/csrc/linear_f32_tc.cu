@@ -28,7 +28,7 @@
 //     4,096 x 2,304         11.2 / 14.0     25.2 / 13.9     91.7 / 25.2     150 / 42.3      445 / 135
 //     2,304 x 2,048          9.8 / 10.1     18.5 / 10.4     54.5 / 18.5    87.4 / 31.5      220 / 120
 //     18,432 x 2,304        38.4 / 34.4     53.0 / 34.3      357 / 56.3     591 / 106     1,845 / 333
-//     2,304 x 9,216         23.0 / 26.9     44.6 / 27.3      182 / 38.1     298 / 70.0      976 / 268
+//     2,304 x 9,216         23.0 / 28.5     44.6 / 28.7      182 / 38.1     298 / 70.0      976 / 268
 // (few tokens would be as fast there; they are here because a row's bits are to be the same however many there are).  The
 // error against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.5 to 1.7e-7 here.  The same with three
 // bfloat16 parts a float and six products: 1.4e-7, but 170 us for 300 tokens of 18,432 x 2,304 and 69 us for 3.
@@ -327,7 +327,15 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             __syncwarp();
             if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
         }
-        if (j == stages) {
+        if (j == stages && g.parts && g.y) {
+            // the kernel behind this one looks for doubtful sums itself
+            float* dst = g.parts + ((size_t)part * g.M + m0 + first) * g.N + n0 + row;
+            if (n0 + row < g.N) {
+#pragma unroll
+                for (int c = 0; c < S::COLS; ++c)
+                    if (first + c < tokens) dst[(size_t)c * g.N] = sum[c];
+            }
+        } else if (j == stages) {
             // the rings are done with: all products have been made
             float* sums = reinterpret_cast<float*>(smem_raw) + row;
 #pragma unroll
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         else __syncthreads();
     };
     all_here();
-    if (!give_up[0]) {
+    if (!(g.parts && g.y) && !give_up[0]) {
         // the blocks of the cluster deal the tokens among them; a thread makes four neighbours of a row of Y, or of this slice's sums
         const int quads = out_rows / 4, ranks = g.parts ? 1 : n_slices, rank = g.parts ? 0 : part;
         float* dst_rows = g.parts ? g.parts + (size_t)part * g.M * g.N : g.y;
@@ -554,10 +562,15 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
     pdl_wait();
     const size_t total = (size_t)g.M * g.N;
     for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
-        float y = g.parts[idx];
+        const size_t token = idx / g.N, n = idx % g.N;
+        float y = 0.0f;
 #pragma unroll 4
-        for (int s = 1; s < slices; ++s) y += g.parts[s * total + idx];
-        g.y[idx / g.N * g.ldy + idx % g.N] = y;
+        for (int s = 0; s < slices; ++s) {
+            float v = g.parts[s * total + idx];
+            if (doubtful(v)) v = plain_dot(g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice));
+            y = s ? y + v : v;
+        }
+        g.y[token * g.ldy + n] = y;
     }
 }
 
