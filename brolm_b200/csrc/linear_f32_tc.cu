@@ -338,11 +338,15 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         } else if (j == stages) {
             // the rings are done with: all products have been made
             float* sums = reinterpret_cast<float*>(smem_raw) + row;
+            bool fine = true;
 #pragma unroll
             for (int c = 0; c < S::COLS; ++c)
-                if (first + c < tokens) sums[(first + c) * BR] = sum[c];
+                if (first + c < tokens) {
+                    sums[(first + c) * BR] = sum[c];
+                    fine &= !doubtful(sum[c]);
+                }
             const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
-            if (w_row < (g.gated ? 2 * g.N : g.N))
+            if (!fine && w_row < (g.gated ? 2 * g.N : g.N))
                 for (int c = first; c < min(first + S::COLS, tokens); ++c)
                     if (doubtful(sums[c * BR]))
                         sums[c * BR] = plain_dot(g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo, min(g.K, k_lo + g.slice));
@@ -563,13 +567,20 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
     const size_t total = (size_t)g.M * g.N;
     for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
         const size_t token = idx / g.N, n = idx % g.N;
-        float y = 0.0f;
-#pragma unroll 4
-        for (int s = 0; s < slices; ++s) {
-            float v = g.parts[s * total + idx];
-            if (doubtful(v)) v = plain_dot(g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice));
-            y = s ? y + v : v;
-        }
+        float v[8];                                            // at most eight slices, all on their way at once
+        bool fine = true;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = s < slices ? g.parts[s * total + idx] : 0.0f;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) fine &= !doubtful(v[s]);
+        if (!fine)
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (doubtful(v[s])) v[s] = plain_dot(g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice));
+        float y = v[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s)
+            if (s < slices) y += v[s];
         g.y[token * g.ldy + n] = y;
     }
 }
