@@ -25,10 +25,10 @@
 // Bound: up to 32 tokens by the memory and by the start and end of short slices, beyond by the warps that split and add (a
 // stage of 64 k with 150 tokens takes 1.5 us, of which the products are 0.5).  us, the kernels of linear_f32.cu / here:
 //     tokens                     3              16              150             300             1,000
-//     4,096 x 2,304         11.2 / 14.0     25.2 / 13.9     91.7 / 25.2     150 / 42.3      445 / 135
-//     2,304 x 2,048          9.8 / 10.1     18.5 / 10.4     54.5 / 18.5    87.4 / 31.5      220 / 120
-//     18,432 x 2,304        38.4 / 34.4     53.0 / 34.3      357 / 56.3     591 / 106     1,845 / 333
-//     2,304 x 9,216         23.0 / 28.5     44.6 / 28.7      182 / 38.1     298 / 70.0      976 / 268
+//     4,096 x 2,304         11.2 / 14.1     25.2 / 14.4     91.7 / 28.2     150 / 48.6      445 / 159
+//     2,304 x 2,048          9.8 / 10.6     18.5 / 11.2     54.5 / 20.9    87.4 / 36.1      220 / 153
+//     18,432 x 2,304        38.4 / 34.6     53.0 / 34.7      357 / 58.8     591 / 110     1,845 / 350
+//     2,304 x 9,216         23.0 / 29.2     44.6 / 29.0      182 / 39.6     298 / 73.4      976 / 303
 // (few tokens would be as fast there; they are here because a row's bits are to be the same however many there are).  The
 // error against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.5 to 1.7e-7 here.  The same with three
 // bfloat16 parts a float and six products: 1.4e-7, but 170 us for 300 tokens of 18,432 x 2,304 and 69 us for 3.
