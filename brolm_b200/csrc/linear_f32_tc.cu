@@ -1,43 +1,49 @@
-// Float matrix product  Y[M,N] = X[M,K] * W[N,K]^T  for large weights, on tcgen05: every float is taken as the sum of two
-// half-precision numbers, and a product of floats as the sum of three products of those.
+// Float matrix product  Y[M,N] = X[M,K] * W[N,K]^T  for large weights, on tcgen05: every float is taken as the sum of three
+// bfloat16 numbers, and a product of floats as the sum of six products of those (Henry, Tang and Heinecke, "Leveraging the
+// bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019).
 //
-// 64 k of a row have a power of two s in common that brings the largest of them to 2^14 .. 2^15.  Then
-//     s x = x0 + x1 + rest:   x0 = half(s x), x1 = half(s x - x0),   |rest| <= 2^-24 |s x|, or 2^-25 where s x is small
-//     x w = (x0 w0 + (x0 w1 + x1 w0)) / (s s') + ...                 what is left out: at most 2^-24 |x w| more
-// so a product is as good as one of numbers rounded to float.  Products of two half-precision numbers are exact in float.
+//     x = x0 + x1 + x2:   x0 = bfloat16(x), x1 = bfloat16(x - x0), x2 = x - x0 - x1,   exact: 8 + 8 + 8 bits, and their signs
+//     x w = x2 w0 + x0 w2 + x1 w1 + x1 w0 + x0 w1 + x0 w0 + ...      what is left out: less than 2^-25 |x w|
+// A bfloat16 has the exponents of a float, so this holds for each number by itself, whatever stands beside it in its row (two
+// halves under a power of two in common, three products, were a sixth faster for 300 tokens and lost what lay 2^15 below its
+// neighbours).
+// Products of two bfloat16 numbers are exact in float.
 // The tensor core adds 16 of them at a time to a float accumulator and cuts off what lies below its last place, so its sums
-// are kept short: the 64 k of the three products, the small ones first, make a partial sum; the partial sums of a slice of K
-// are scaled back and added by float fmas in ascending order, and the slices likewise.  How K is cut hangs on N and K alone, so
+// are kept short: the 64 k of the six products, the small ones first, make a partial sum; the partial sums of a slice of K
+// are added by float additions in ascending order, and the slices likewise.  How K is cut hangs on N and K alone, so
 // a row's bits depend neither on M nor on its place among the rows, nor on how X lies in memory.
 //
 // A block owns 128 rows of W (the M side of the instruction), up to NT tokens (the N side) and one slice of K.  The sums of
 // the slices are added through the shared memory of a cluster of blocks, or by the kernel behind this one.  Roles:
 //   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it;
-//   SPLIT   a lane takes 64 k of a row of W apart and puts the two rows of halves into tensor memory (the A operand);
+//   SPLIT   a lane takes 64 k of a row of W apart and puts the three rows of parts into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
-//           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the halves in by TMA;
-//   MMA     one thread issues 12 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two accumulators;
+//           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the parts in by TMA;
+//   MMA     one lane issues 24 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two accumulators;
 //   ADD     these add an accumulator to the sums in their registers, and at the end store them.
 // The thread that issues is what all wait for, so its stage of 64 k has one barrier to wait on, which all that its products
 // need arrive at (A, the tokens, the emptied accumulator), and one commit, which frees all of it.
 // For W = [gate; up] a block has 64 rows of each, and stores act(gate) * up.
 //
 // Bound: up to 32 tokens by the memory and by the start and end of short slices, beyond by the warps that split and add (a
-// stage of 64 k with 150 tokens takes 1.5 us, of which the products are 0.5).  us, the kernels of linear_f32.cu / here:
+// stage of 64 k with 150 tokens takes 1.7 us, of which the products are 0.9).  us, the kernels of linear_f32.cu / here:
 //     tokens                     3              16              150             300             1,000
-//     4,096 x 2,304         11.2 / 14.1     25.2 / 14.4     91.7 / 28.2     150 / 48.6      445 / 159
-//     2,304 x 2,048          9.8 / 10.6     18.5 / 11.2     54.5 / 20.9    87.4 / 36.1      220 / 153
-//     18,432 x 2,304        38.4 / 34.6     53.0 / 34.7      357 / 58.8     591 / 110     1,845 / 350
-//     2,304 x 9,216         23.0 / 29.2     44.6 / 29.0      182 / 39.6     298 / 73.4      976 / 303
-// (few tokens would be as fast there; they are here because a row's bits are to be the same however many there are).  The
-// error against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.5 to 1.7e-7 here.  The same with three
-// bfloat16 parts a float and six products: 1.4e-7, but 170 us for 300 tokens of 18,432 x 2,304 and 69 us for 3.
-// An infinity or a NaN among the operands ends as a NaN here (infinity minus infinity, infinity times zero), and numbers
-// near the smallest lose their low parts: a slice's sum that is not finite, or so small that this may show, is made again
-// from the floats themselves by the thread that has it.
+//     4,096 x 2,304         11.3 / 12.7     25.3 / 13.5     91.4 / 34.2     150 / 60.6      446 / 197
+//     2,304 x 2,048          9.6 / 10.2     18.5 / 11.0     54.0 / 25.4    87.4 / 46.2      220 / 195
+//     18,432 x 2,304        37.7 / 30.9     53.3 / 31.9      358 / 70.7     592 / 134     1,847 / 419
+//     2,304 x 9,216         23.8 / 33.1     44.6 / 33.2      182 / 48.3     298 / 90.2      978 / 359
+// (a decode step leaves the slices of the second and the fourth to the kernel behind them: 3 tokens 7.6 and 19.5).  The error
+// against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.0 to 1.4e-7 here for normal numbers; 0.7 to 1.2e-7 and
+// 0.9 to 1.2e-7 for sums of one sign, which lose half a last place at each step of the tensor core and none on average to fmas.
+//
+// What three parts cannot say is said by the floats themselves: the thread that has a doubtful sum of a slice makes it again
+// by fmas.  Doubtful are (see doubtful())
+//   a sum that is not finite: an infinity or a NaN among the operands ends as a NaN here, infinity minus infinity;
+//   a sum below 1e-20: the products of low parts end at 2^-126;
+//   a sum with a number below 2^-60 on one side and one of 2^17 or more on the other: numbers below 2^-102 lose their low
+//   parts, up to 2^-125 of each; times less than 2^17 that is far below the last place of a sum of 1e-20;
+//   a zero, where a side has numbers below 2^-60 (or zeros) and neither has zeros alone.
 #include "tcgen05.cuh"
-
-#include <cuda_fp16.h>
 
 namespace {
 
@@ -45,8 +51,8 @@ using namespace tc;
 
 constexpr int BR = 128, KW = 32, KX = 64;          // rows of W; k of a slot of W, and of a stage
 constexpr int W_SLOT = BR * KW * 4;
-constexpr int A_PLANE = KX / 2, A_COLS = 2 * A_PLANE;        // tensor memory: two k a column, two planes a stage
-constexpr int SCALES = 4;                          // stages whose scales are kept: one that is written is not read any more
+constexpr int PARTS = 3;                           // of a float
+constexpr int A_PLANE = KX / 2, A_COLS = PARTS * A_PLANE;    // tensor memory: two k a column, a plane for each part
 
 enum class Role { TMA, MMA, SPLIT, ADD, X, FETCH_X, NONE };
 
@@ -64,14 +70,15 @@ struct Shape {
     static constexpr int X_WARPS = FEW ? 2 : 8;
     static constexpr int READY = 4 + X_WARPS + 4 * GROUPS;                  // arrivals that a stage waits for
     static constexpr int X_RAW = NT * KX * 4;                               // bytes of a stage of X as it is
-    static constexpr int W_SLOTS = !FEW ? 8 : PER_SM == 1 ? 10 : NT == 16 ? 5 : 4;
+    static constexpr int BUFFERS = FEW && PER_SM == 1 ? 4 : 2;              // of A, the tokens and the accumulator
+    static constexpr int W_SLOTS = !FEW ? 6 : PER_SM == 1 ? NT == 16 ? 10 : 8 : NT == 16 ? 5 : 4;
     static constexpr int AHEAD = !FEW ? 0 : PER_SM == 1 ? 4 : 3;           // stages of X that are on their way (FEW)
-    static constexpr int X_PLANE = NT * KX * 2, X_SLOT = 2 * X_PLANE;
-    static constexpr int TMEM = FEW ? 256 : 512;
-    static constexpr int RING = W_SLOTS * W_SLOT + 2 * X_SLOT + AHEAD * X_RAW;
-    static constexpr int BARS = 2 * W_SLOTS + 7;
-    static constexpr int SMEM = RING + SCALES * (BR + NT) * 4 + BARS * 8 + 24;
-    static_assert(2 * NT + 2 * A_COLS <= TMEM && TMEM * PER_SM <= 512, "accumulators and A");
+    static constexpr int X_PLANE = NT * KX * 2, X_SLOT = PARTS * X_PLANE;
+    static constexpr int TMEM = PER_SM == 1 ? 512 : 256;
+    static constexpr int RING = W_SLOTS * W_SLOT + BUFFERS * X_SLOT + AHEAD * X_RAW;
+    static constexpr int BARS = 2 * W_SLOTS + 3 * BUFFERS + 1;
+    static constexpr int SMEM = RING + 2 * BR + NT + BARS * 8 + 24;
+    static_assert(BUFFERS * (NT + A_COLS) <= TMEM && TMEM * PER_SM <= 512, "accumulators and A");
     static_assert((SMEM + 1024) * PER_SM <= 228 * 1024, "the blocks of an SM");
     static_assert(NT * BR * 4 <= RING, "the sums of a slice lie where the rings were");
 
@@ -93,37 +100,49 @@ struct Args {
     const float* x;
     const float* w;
     float* y;
-    const float* x_scale;    // X taken apart ahead: [M][stages of K] scales, and the halves under a map of their own; null: here
+    const uint8_t* x_flags;  // X taken apart ahead: flags [M][stages of K], and the parts under a map of their own; null: here
     float* parts;            // the slices' sums, [slice][M][N], are added by the kernel behind; null: by the cluster
     int ldx, ldw, ldy;
     int M, N, K;
     int tokens;              // of a token tile: a multiple of 16
     int slice;               // k of a slice: a multiple of 64
     int x_vec;               // X's rows lie on 16-byte boundaries
-    int x_stages;            // columns of x_scale
+    int x_stages;            // columns of x_flags
     int gated;               // W is [gate; up] of 2 N rows, a block has 64 of each, and y = act(gate) * up
     int act;
     float limit;
 };
 
-// The power of two that brings `most` to 2^14 .. 2^15, and its inverse; both are normal numbers for every `most`.
-__device__ __forceinline__ void scales_of(float most, float& up, float& down) {
-    const uint32_t e = max((__float_as_uint(most) >> 23) & 255u, 16u);
-    up = __uint_as_float((268u - e) << 23);
-    down = __uint_as_float((e - 14u) << 23);
-}
+// What a row's or a token's numbers of a slice are like, for doubtful().
+enum : uint32_t { SMALL = 1, BIG = 2, SOME = 4 };
+struct Extent {
+    float low = INFINITY, high = 0.0f;
+    __device__ __forceinline__ void add(float v) { low = fminf(low, fabsf(v)), high = fmaxf(high, fabsf(v)); }
+    __device__ __forceinline__ void add(const float4& v) { add(v.x), add(v.y), add(v.z), add(v.w); }
+    __device__ __forceinline__ uint32_t flags() const {
+        return (low < 8.67361738e-19f ? SMALL : 0) | (high >= 131072.0f ? BIG : 0) | (high > 0.0f ? SOME : 0);
+    }
+    // of the eight lanes that share a row's 64 k
+    __device__ __forceinline__ uint32_t flags_of_eight(int lane) const {
+        const uint32_t mine = flags(), eight = 0xffu << (lane & 24);
+        uint32_t all = 0;
+#pragma unroll
+        for (uint32_t bit = SMALL; bit <= SOME; bit <<= 1) all |= __ballot_sync(0xffffffffu, mine & bit) & eight ? bit : 0;
+        return all;
+    }
+};
 // Two neighbours along k, taken apart.
-__device__ __forceinline__ void take_apart(float a, float b, float scale, uint32_t& p0, uint32_t& p1) {
-    a *= scale;
-    b *= scale;
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
-    p0 = *reinterpret_cast<const uint32_t*>(&h);
-    p1 = *reinterpret_cast<const uint32_t*>(&l);
+__device__ __forceinline__ uint32_t take_part(float& a, float& b) {
+    uint32_t p;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(b), "f"(a));
+    a -= __uint_as_float(p << 16);
+    b -= __uint_as_float(p & 0xffff0000u);
+    return p;
 }
-__device__ __forceinline__ float largest(float most, const float4& v) {
-    return fmaxf(fmaxf(fmaxf(most, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+__device__ __forceinline__ void take_apart(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    p0 = take_part(a, b);
+    p1 = take_part(a, b);
+    p2 = take_part(a, b);
 }
 __device__ __forceinline__ float4 lds_float4(uint32_t at) {
     float4 v;
@@ -134,11 +153,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
-// Instruction descriptor of kind::f16: half x half -> f32, both K-major.
-__device__ __forceinline__ uint32_t idesc_half(int m, int n) {
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
 __device__ __noinline__ float plain_dot(const float* x, const float* w, int k, int end) {
     float y = 0.0f;
     for (; k < end; k += 512) {
@@ -154,23 +168,35 @@ __device__ __noinline__ float plain_dot(const float* x, const float* w, int k, i
 }
 __device__ __forceinline__ bool doubtful(float y) {
     const float size = fabsf(y);
-    return !(size <= 3.402823466e38f) || (size < 1e-25f && y != 0.0f);
+    return !(size <= 3.402823466e38f) || (size < 1e-20f && y != 0.0f);
+}
+__device__ __forceinline__ bool doubtful(float y, uint32_t row, uint32_t token) {
+    return doubtful(y) || (((row & token >> 1) | (row >> 1 & token)) & SMALL) || (y == 0.0f && (row & token & SOME) && ((row | token) & SMALL));
+}
+
+// One lane of a warp that is there as a whole, always the same one.  The compiler knows of this one that it is alone, and keeps
+// what the products are given in uniform registers: 24 products of 16 tokens are issued in 0.7 us where `lane == 0` takes 1.2.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
 }
 
 template <int NT, int BLOCKS>
 __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                                                      const __grid_constant__ CUtensorMap map_x, Args g) {
     using S = Shape<NT, BLOCKS>;
+    constexpr int NB = S::BUFFERS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t w_ring = smem_u32(smem_raw), x_ring = w_ring + S::W_SLOTS * W_SLOT;
-    float* row_scale = reinterpret_cast<float*>(smem_raw + S::RING);        // [SCALES][BR]: what a partial sum is multiplied by
-    float* token_scale = row_scale + SCALES * BR;                           // [SCALES][NT]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(token_scale + SCALES * NT);
+    uint8_t* row_flags = smem_raw + S::RING;               // [2][BR]: of the stages that a set of SPLIT had
+    uint8_t* token_flags = row_flags + 2 * BR;             // [NT]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(token_flags + NT);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + S::BARS);
     volatile int* give_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * S::W_SLOTS, ready = w_empty + 8 * S::W_SLOTS, made = ready + 16,
-                   all_made = made + 16, x_full = all_made + 8;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * S::W_SLOTS, ready = w_empty + 8 * S::W_SLOTS,
+                   made = ready + 8 * NB, x_full = made + 8 * NB, all_made = x_full + 8 * NB;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     const int n_slices = gridDim.x, part = blockIdx.x;
     const int out_rows = g.gated ? BR / 2 : BR;                // columns of Y that the block makes
@@ -181,18 +207,19 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::W_SLOTS; ++s) mbar_init(w_full + 8 * s, 1), mbar_init(w_empty + 8 * s, 4);
-        for (int s = 0; s < 2; ++s) mbar_init(ready + 8 * s, S::READY), mbar_init(made + 8 * s, 1), mbar_init(x_full + 8 * s, 1);
+        for (int s = 0; s < NB; ++s) mbar_init(ready + 8 * s, S::READY), mbar_init(made + 8 * s, 1), mbar_init(x_full + 8 * s, 1);
         mbar_init(all_made, 1);
         give_up[0] = 0;
         give_up[1] = 0;
         give_up[2] = tc::g_stall_code;
         mbar_init_fence();
     }
+    if (threadIdx.x < 2 * BR + NT) row_flags[threadIdx.x] = 0;              // (the tokens' too)
     if (warp == 2) tmem_alloc(smem_u32(tmem_slot), S::TMEM);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = *tmem_slot, tmem_a = tmem + 2 * NT;
+    const uint32_t tmem = *tmem_slot, tmem_a = tmem + NB * NT;
 
     auto wait_on = [&](uint32_t bar, uint32_t parity, int code) { return mbar_wait(bar, parity, give_up, &g_linear_f32_tc_error, code); };
     auto all_wait_on = [&](uint32_t bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, wait_on(bar, parity, code)) != 0; };
@@ -215,82 +242,81 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 for (int j = max(0, i - S::W_SLOTS); j < i; ++j)
                     mbar_wait(w_full + 8 * (j % S::W_SLOTS), (j / S::W_SLOTS) & 1, give_up, &g_linear_f32_tc_error, 7, true);
         }
-        if (role == Role::MMA && lane == 0) {
-            const uint32_t id = idesc_half(BR, wide);
+        if (role == Role::MMA) {
+            const uint32_t id = idesc_bf16(BR, wide);
             for (int j = 0; j < stages; ++j) {
-                const int s = j & 1;
-                if (!wait_on(ready + 8 * s, (j >> 1) & 1, 2)) break;
-                if (g.x_scale && !wait_on(x_full + 8 * s, (j >> 1) & 1, 3)) break;
+                const int s = j % NB;
+                if (!all_wait_on(ready + 8 * s, (j / NB) & 1, 2)) break;
+                if (g.x_flags && !all_wait_on(x_full + 8 * s, (j / NB) & 1, 3)) break;
                 fence_after_sync();
-                const uint32_t acc = tmem + s * NT, a = tmem_a + s * A_COLS;
-                const uint64_t b = desc_kmajor(x_ring + s * S::X_SLOT);
-                // (plane of W, plane of X), the small products first
-                constexpr int P[3][2] = {{1, 0}, {0, 1}, {0, 0}};
+                if (elect_one()) {
+                    const uint32_t acc = tmem + s * NT, a = tmem_a + s * A_COLS;
+                    const uint64_t b = desc_kmajor(x_ring + s * S::X_SLOT);
+                    // (plane of W, plane of X), the small products first
+                    constexpr int P[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-                for (int p = 0; p < 3; ++p)
+                    for (int p = 0; p < 6; ++p)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_ts(acc, a + P[p][0] * A_PLANE + 8 * k, b + (uint64_t)(P[p][1] * (S::X_PLANE >> 4) + 2 * k), id, p + k > 0);
-                umma_commit(made + 8 * s);
+                        for (int k = 0; k < 4; ++k)
+                            umma_ts(acc, a + P[p][0] * A_PLANE + 8 * k, b + (uint64_t)(P[p][1] * (S::X_PLANE >> 4) + 2 * k), id, p + k > 0);
+                    umma_commit(made + 8 * s);
+                }
+                __syncwarp();
             }
-            if (*give_up) {                                    // products in flight end before their operands go
+            if (__any_sync(0xffffffffu, *give_up) && elect_one()) {                     // products in flight end before their operands go
                 umma_commit(all_made);
                 mbar_wait(all_made, 0, give_up, &g_linear_f32_tc_error, 10, true);
             }
         }
-        if (role == Role::FETCH_X && lane == 0 && g.x_scale) {
+        if (role == Role::FETCH_X && lane == 0 && g.x_flags) {
             pdl_wait();
             int j = 0;
             for (; j < stages; ++j) {
-                const int s = j & 1;
-                if (j >= 2 && !wait_on(made + 8 * s, ((j >> 1) & 1) ^ 1, 9)) break;
-                mbar_expect_tx(x_full + 8 * s, 2 * g.tokens * KX * 2);
-                for (int q = 0; q < 2; ++q)
+                const int s = j % NB;
+                if (j >= NB && !wait_on(made + 8 * s, ((j / NB) & 1) ^ 1, 9)) break;
+                mbar_expect_tx(x_full + 8 * s, PARTS * g.tokens * KX * 2);
+                for (int q = 0; q < PARTS; ++q)
                     tma_load_3d(x_ring + s * S::X_SLOT + q * S::X_PLANE, &map_x, k_lo + j * KX, m0, q, x_full + 8 * s);
             }
             if (*give_up)
-                for (int i = max(0, j - 2); i < j; ++i)
-                    mbar_wait(x_full + 8 * (i & 1), (i >> 1) & 1, give_up, &g_linear_f32_tc_error, 11, true);
+                for (int i = max(0, j - NB); i < j; ++i)
+                    mbar_wait(x_full + 8 * (i % NB), (i / NB) & 1, give_up, &g_linear_f32_tc_error, 11, true);
         }
     } else if (role == Role::SPLIT) {
         if constexpr (!S::FEW) fewer_registers<48>();
         const int row = (warp & 3) * 32 + lane;
+        Extent extent;
         for (int j = index >> 2; j < stages; j += 2) {         // two sets of four warps take turns
             const int s0 = 2 * j % S::W_SLOTS, s1 = (2 * j + 1) % S::W_SLOTS;
-            // A wait on a slot's phase asks that the phase before it is known to be over.  That was a stage at least four back
-            // where there are eight slots, which this set has seen; where there are fewer, the stage two back has to be over first.
-            constexpr bool AT_ONCE = S::W_SLOTS >= 8;
-            static_assert(S::W_SLOTS >= 4, "two stages");
-            if (!AT_ONCE && j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 6)) break;
+            // A wait on a slot's phase asks that the phase before it is known to be over: it was at least NB stages back.
+            static_assert(S::W_SLOTS >= 2 * NB, "the slots of NB stages");
+            if (j >= NB && !all_wait_on(made + 8 * (j % NB), ((j / NB) & 1) ^ 1, 6)) break;
             if (!all_wait_on(w_full + 8 * s0, (2 * j / S::W_SLOTS) & 1, 5)) break;
             if (!all_wait_on(w_full + 8 * s1, ((2 * j + 1) / S::W_SLOTS) & 1, 5)) break;
             const uint32_t src[2] = {w_ring + s0 * W_SLOT + row * 128, w_ring + s1 * W_SLOT + row * 128};
-            float most = 0.0f, up, down;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) most = largest(most, lds_float4(src[c >> 3] + (((c & 7) ^ (row & 7)) << 4)));
-            scales_of(most, up, down);
-            if (AT_ONCE && j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 6)) break;
             fence_after_sync();
-            row_scale[(j % SCALES) * BR + row] = down;
-            const uint32_t a = tmem_a + (j & 1) * A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+            const uint32_t a = tmem_a + (j % NB) * A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                uint32_t p0[8], p1[8];
+                uint32_t p0[8], p1[8], p2[8];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float4 v = lds_float4(src[h >> 1] + ((((h & 1) * 4 + c) ^ (row & 7)) << 4));
-                    take_apart(v.x, v.y, up, p0[2 * c], p1[2 * c]);
-                    take_apart(v.z, v.w, up, p0[2 * c + 1], p1[2 * c + 1]);
+                    extent.add(v);
+                    take_apart(v.x, v.y, p0[2 * c], p1[2 * c], p2[2 * c]);
+                    take_apart(v.z, v.w, p0[2 * c + 1], p1[2 * c + 1], p2[2 * c + 1]);
                 }
                 tmem_st8(a + 8 * h, p0);
                 tmem_st8(a + A_PLANE + 8 * h, p1);
+                tmem_st8(a + 2 * A_PLANE + 8 * h, p2);
             }
+            if (j + 2 >= stages) row_flags[(index >> 2) * BR + row] = extent.flags();
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * s0), mbar_arrive(w_empty + 8 * s1);       // (every lane has its floats)
             tmem_wait_st();
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
+            if (lane == 0) mbar_arrive(ready + 8 * (j % NB));
         }
     } else if (role == Role::ADD) {
         if constexpr (!S::FEW) more_registers<112>();
@@ -298,15 +324,15 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         float sum[S::COLS];
 #pragma unroll
         for (int c = 0; c < S::COLS; ++c) sum[c] = 0.0f;
-        if (lane == 0) mbar_arrive(ready), mbar_arrive(ready + 8);          // both accumulators are free
+        if (lane == 0)
+            for (int s = 0; s < NB; ++s) mbar_arrive(ready + 8 * s);       // the accumulators are free
         int j = 0;
         for (; j < stages; ++j) {
-            if (!all_wait_on(made + 8 * (j & 1), (j >> 1) & 1, 8)) break;
-            if (!all_wait_on(ready + 8 * (j & 1), (j >> 1) & 1, 8)) break;          // (it has long been: for the scales' sake)
+            if (!all_wait_on(made + 8 * (j % NB), (j / NB) & 1, 8)) break;
+            // (it has long been: for the flags' sake)
+            if (j + 2 >= stages && !all_wait_on(ready + 8 * (j % NB), (j / NB) & 1, 8)) break;
             fence_after_sync();
-            const uint32_t acc = tmem + (j & 1) * NT + first + ((uint32_t)(quarter * 32) << 16);
-            const float mine = row_scale[(j % SCALES) * BR + row];
-            const float4* theirs = reinterpret_cast<const float4*>(token_scale + (j % SCALES) * NT + first);
+            const uint32_t acc = tmem + (j % NB) * NT + first + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll
             for (int c = 0; c < S::COLS; c += 16) {
                 if (first + c < wide) {
@@ -314,26 +340,21 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                     tmem_ld16(acc + c, v);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 16; e += 4) {
-                        const float4 t = theirs[(c + e) / 4];
-                        sum[c + e] = __fmaf_rn(__uint_as_float(v[e]) * mine, t.x, sum[c + e]);
-                        sum[c + e + 1] = __fmaf_rn(__uint_as_float(v[e + 1]) * mine, t.y, sum[c + e + 1]);
-                        sum[c + e + 2] = __fmaf_rn(__uint_as_float(v[e + 2]) * mine, t.z, sum[c + e + 2]);
-                        sum[c + e + 3] = __fmaf_rn(__uint_as_float(v[e + 3]) * mine, t.w, sum[c + e + 3]);
-                    }
+                    for (int e = 0; e < 16; ++e) sum[c + e] += __uint_as_float(v[e]);
                 }
             }
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
+            if (lane == 0) mbar_arrive(ready + 8 * (j % NB));
         }
+        const uint32_t mine = row_flags[row] | row_flags[BR + row];
         if (j == stages && g.parts && g.y) {
-            // the kernel behind this one looks for doubtful sums itself
+            // the kernel behind this one looks for doubtful sums itself; those that their flags make so are told by a NaN
             float* dst = g.parts + ((size_t)part * g.M + m0 + first) * g.N + n0 + row;
             if (n0 + row < g.N) {
 #pragma unroll
                 for (int c = 0; c < S::COLS; ++c)
-                    if (first + c < tokens) dst[(size_t)c * g.N] = sum[c];
+                    if (first + c < tokens) dst[(size_t)c * g.N] = doubtful(sum[c], mine, token_flags[first + c]) ? NAN : sum[c];
             }
         } else if (j == stages) {
             // the rings are done with: all products have been made
@@ -343,12 +364,12 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             for (int c = 0; c < S::COLS; ++c)
                 if (first + c < tokens) {
                     sums[(first + c) * BR] = sum[c];
-                    fine &= !doubtful(sum[c]);
+                    fine &= !doubtful(sum[c], mine, token_flags[first + c]);
                 }
             const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
             if (!fine && w_row < (g.gated ? 2 * g.N : g.N))
                 for (int c = first; c < min(first + S::COLS, tokens); ++c)
-                    if (doubtful(sums[c * BR]))
+                    if (doubtful(sums[c * BR], mine, token_flags[c]))
                         sums[c * BR] = plain_dot(g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo, min(g.K, k_lo + g.slice));
         }
     } else {
@@ -382,37 +403,35 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             }
         };
         auto put = [&](int j, const float (&v)[PER][8]) {      // false: gave up
-            if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 9)) return false;
-            const uint32_t slot = x_ring + (j & 1) * S::X_SLOT;
+            if (j >= NB && !all_wait_on(made + 8 * (j % NB), ((j / NB) & 1) ^ 1, 9)) return false;
+            const uint32_t slot = x_ring + (j % NB) * S::X_SLOT;
 #pragma unroll
             for (int u = 0; u < PER; ++u) {
                 const int token = u * (T / 8) + (xt >> 3);
-                float most = 0.0f, up, down;
+                Extent extent;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) most = fmaxf(most, fabsf(v[u][e]));
-#pragma unroll
-                for (int o = 4; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-                scales_of(most, up, down);
+                for (int e = 0; e < 8; ++e) extent.add(v[u][e]);
+                const uint32_t flags = extent.flags_of_eight(lane);
                 if (token < wide) {
-                    uint32_t p[2][4];
+                    uint32_t p[PARTS][4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) take_apart(v[u][2 * e], v[u][2 * e + 1], up, p[0][e], p[1][e]);
+                    for (int e = 0; e < 4; ++e) take_apart(v[u][2 * e], v[u][2 * e + 1], p[0][e], p[1][e], p[2][e]);
                     const uint32_t at = slot + token * 128 + ((chunk ^ (token & 7)) << 4);
 #pragma unroll
-                    for (int q = 0; q < 2; ++q)
+                    for (int q = 0; q < PARTS; ++q)
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + q * S::X_PLANE), "r"(p[q][0]), "r"(p[q][1]),
                                      "r"(p[q][2]), "r"(p[q][3]) : "memory");
-                    if (chunk == 0) token_scale[(j % SCALES) * NT + token] = down;
+                    if (chunk == 0) token_flags[token] |= flags;
                 }
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
+            if (lane == 0) mbar_arrive(ready + 8 * (j % NB));
             return true;
         };
         if constexpr (S::FEW) {
             // every thread brings in what it will take apart, some stages ahead
-            const uint32_t raw = x_ring + 2 * S::X_SLOT + xt * 32;
+            const uint32_t raw = x_ring + NB * S::X_SLOT + xt * 32;
             auto fetch = [&](int j) {
                 const int k = k_lo + j * KX + chunk * 8;
 #pragma unroll
@@ -450,18 +469,18 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 if (!put(j, v)) break;
             }
             copy_wait<0>();
-        } else if (g.x_scale) {
-            // the halves come by TMA: the scales alone
-            const float* src = g.x_scale + (size_t)(m0 + xt) * g.x_stages + k_lo / KX;
+        } else if (g.x_flags) {
+            // the parts come by TMA: the flags alone
+            const uint8_t* src = g.x_flags + (size_t)(m0 + xt) * g.x_stages + k_lo / KX;
             const bool there = xt < tokens;
-            float next = there ? src[0] : 1.0f;
+            uint32_t all = 0, next = there ? src[0] : 0;
             for (int j = 0; j < stages; ++j) {
-                const float now = next;
+                all |= next;
                 if (there && j + 1 < stages) next = src[j + 1];
-                if (j >= 2 && !all_wait_on(made + 8 * (j & 1), ((j >> 1) & 1) ^ 1, 9)) break;
-                if (xt < NT) token_scale[(j % SCALES) * NT + xt] = now;
+                if (j >= NB && !all_wait_on(made + 8 * (j % NB), ((j / NB) & 1) ^ 1, 9)) break;
+                if (j + 1 == stages && xt < NT) token_flags[xt] = all;
                 __syncwarp();
-                if (lane == 0) mbar_arrive(ready + 8 * (j & 1));
+                if (lane == 0) mbar_arrive(ready + 8 * (j % NB));
             }
         } else {
             float v[PER][8];
@@ -528,8 +547,8 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     if (warp == 2) tmem_dealloc(tmem, S::TMEM);
 }
 
-// X taken apart ahead: eight lanes take 64 k of a token.  halves [2][M][Kp], Kp = 64 stages; scale [M][stages]
-__global__ void __launch_bounds__(256) split_rows_kernel(Args g, __half* __restrict__ halves, float* __restrict__ scale, int stages) {
+// X taken apart ahead: eight lanes take 64 k of a token.  parts [3][M][Kp] bfloat16, Kp = 64 stages; flags [M][stages]
+__global__ void __launch_bounds__(256) split_rows_kernel(Args g, uint16_t* __restrict__ parts, uint8_t* __restrict__ flags, int stages) {
     pdl_trigger();
     const size_t kp = (size_t)stages * KX;
     const long long unit = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
@@ -537,27 +556,24 @@ __global__ void __launch_bounds__(256) split_rows_kernel(Args g, __half* __restr
     pdl_wait();
     const bool there = token < g.M;
     const float* p = g.x + (size_t)(there ? token : 0) * g.ldx + k;
-    float v[8], most = 0.0f, up, down;
+    float4 v[2];
+    Extent extent;
 #pragma unroll
-    for (int e = 0; e < 8; e += 4) {                          // (X's rows lie on 16-byte boundaries)
-        const float4 f = there && k + e < g.K ? *reinterpret_cast<const float4*>(p + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        v[e] = f.x, v[e + 1] = f.y, v[e + 2] = f.z, v[e + 3] = f.w;
+    for (int h = 0; h < 2; ++h) {                             // (X's rows lie on 16-byte boundaries)
+        v[h] = there && k + 4 * h < g.K ? *reinterpret_cast<const float4*>(p + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        extent.add(v[h]);
     }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) most = fmaxf(most, fabsf(v[e]));
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-    scales_of(most, up, down);
+    const uint32_t all = extent.flags_of_eight(threadIdx.x & 31);
     if (!there) return;
-    uint4 q[2];
-    uint32_t* q0 = &q[0].x;
-    uint32_t* q1 = &q[1].x;
+    uint4 q[PARTS];
+    take_apart(v[0].x, v[0].y, q[0].x, q[1].x, q[2].x);
+    take_apart(v[0].z, v[0].w, q[0].y, q[1].y, q[2].y);
+    take_apart(v[1].x, v[1].y, q[0].z, q[1].z, q[2].z);
+    take_apart(v[1].z, v[1].w, q[0].w, q[1].w, q[2].w);
+    uint16_t* dst = parts + (size_t)token * kp + k;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) take_apart(v[2 * e], v[2 * e + 1], up, q0[e], q1[e]);
-    __half* dst = halves + (size_t)token * kp + k;
-    *reinterpret_cast<uint4*>(dst) = q[0];
-    *reinterpret_cast<uint4*>(dst + (size_t)g.M * kp) = q[1];
-    if (chunk == 0) scale[(size_t)token * stages + st] = down;
+    for (int i = 0; i < PARTS; ++i) *reinterpret_cast<uint4*>(dst + i * g.M * kp) = q[i];
+    if (chunk == 0) flags[(size_t)token * stages + st] = (uint8_t)all;
 }
 
 // y = parts[0] + parts[1] + ... in order
@@ -614,10 +630,10 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, dim3 gri
 // Y = X W^T over `slices` slices of K of `slice` k each (a multiple of 64, none empty; at most 8 slices); gated: Y =
 // act(X Wg^T) * (X Wu^T) for W = [Wg; Wu] of 2 N rows.  W's rows lie on 16-byte boundaries, K is a multiple of 4; X's rows
 // may lie anywhere.  parts: room for slices * M * N floats, with which a second kernel adds the slices (y null: the caller's does); null: clusters do.
-// halves: room for X taken apart ahead (more than 32 rows on 16-byte boundaries), 16-byte aligned, M * ceil(K / 64) * 260 bytes;
+// split: room for X taken apart ahead (more than 32 rows on 16-byte boundaries), 16-byte aligned, M * ceil(K / 64) * 385 bytes;
 // null: every block does it.
 BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
-                                  int slices, int slice, int gated, int act, float limit, void* parts, void* halves, cudaStream_t stream) {
+                                  int slices, int slice, int gated, int act, float limit, void* parts, void* split, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;
     if (K <= 0 || K % 4 || ldw % 4 || ((uintptr_t)w & 15)) return BROLM_ERR_ALIGNMENT;
     if (slices < 1 || slices > 8 || slice < 64 || slice % 64 || (long long)(slices - 1) * slice >= K || (long long)slices * slice < K) return BROLM_ERR_BAD_SIZE;
@@ -644,21 +660,21 @@ BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw
     g.slice = slice;
     g.gated = gated; g.act = act; g.limit = limit;
     g.x_vec = ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
-    g.x_scale = nullptr;
+    g.x_flags = nullptr;
     g.x_stages = (K + KX - 1) / KX;
     CUtensorMap mx = mw;
-    if (halves) {
-        if (most <= 32 || !g.x_vec || ((uintptr_t)halves & 15)) return BROLM_ERR_ALIGNMENT;
+    if (split) {
+        if (most <= 32 || !g.x_vec || ((uintptr_t)split & 15)) return BROLM_ERR_ALIGNMENT;
         const cuuint64_t kp = (cuuint64_t)g.x_stages * KX;
-        const cuuint64_t xdims[3] = {kp, (cuuint64_t)M, 2}, xstrides[2] = {kp * 2, kp * M * 2};
+        const cuuint64_t xdims[3] = {kp, (cuuint64_t)M, PARTS}, xstrides[2] = {kp * 2, kp * M * 2};
         const cuuint32_t xbox[3] = {KX, (cuuint32_t)g.tokens, 1}, xelem[3] = {1, 1, 1};
-        if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, halves, xdims, xstrides, xbox, xelem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, split, xdims, xstrides, xbox, xelem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return BROLM_ERR_ALIGNMENT;
-        float* scale = reinterpret_cast<float*>((uint8_t*)halves + (size_t)M * kp * 4);
-        g.x_scale = scale;
+        uint8_t* flags = (uint8_t*)split + (size_t)M * kp * 2 * PARTS;
+        g.x_flags = flags;
         const long long units = (long long)M * g.x_stages;
-        const int st = launch_pdl(split_rows_kernel, dim3((unsigned)((units * 8 + 255) / 256)), dim3(256), 0, stream, g, (__half*)halves, scale, g.x_stages);
+        const int st = launch_pdl(split_rows_kernel, dim3((unsigned)((units * 8 + 255) / 256)), dim3(256), 0, stream, g, (uint16_t*)split, flags, g.x_stages);
         if (st) return st;
     }
     const dim3 grid(slices, (M + g.tokens - 1) / g.tokens, (unsigned)row_tiles);

@@ -70,7 +70,7 @@ __device__ inline bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* fl
     volatile int* give_up = flags + (drain ? 1 : 0);
     const bool stalled = !drain && flags[2] == code;          // (0 in every ordinary launch)
     if (!stalled && mbar_try(bar, parity)) return true;       // (try_wait itself may hold the thread for a while)
-    const long long t0 = clock64(), limit = g_wait_cycles;
+    const long long t0 = clock64(), limit = stalled ? g_wait_cycles / 2 : g_wait_cycles;      // (the stalled one is the first to give up)
     while (true) {
         if (!stalled && mbar_try(bar, parity)) return true;
         if (*give_up) return false;

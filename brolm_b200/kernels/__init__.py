@@ -1206,17 +1206,17 @@ def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, a
 def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], slices: int, gated: bool = False, act: int = 0,
                    limit: float = 0.0, parts: Optional[torch.Tensor] = None) -> None:
     (M, K), N = x.shape, out.shape[1] if out is not None else parts.shape[2]
-    halves = None
+    split = None
     if M > 32 and not (x.stride(0) % 4 or x.data_ptr() % 16):
         if parts is None and slices > 1 and not gated and linear_f32_tc_scratch(M, N, slices):
             parts = torch.empty((slices, M, N), dtype=torch.float32, device=x.device)
-        size = M * -(-K // 64) * 260                         # the rows as halves, and a scale for every 64
+        size = M * -(-K // 64) * 385                         # the rows in three parts of 16 bits, and a byte for every 64
         if size <= F32_PARTS_LIMIT:
-            halves = torch.empty(size, dtype=torch.uint8, device=x.device)
+            split = torch.empty(size, dtype=torch.uint8, device=x.device)
     f = _fn("linear_f32_tc", "brolm_linear_f32_tc", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                                      c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0) if out is not None else N, M, N, K, slices,
-             _f32_tc_slice(K, slices), int(gated), act, limit, _ptr(parts), _ptr(halves), _stream()), "linear_f32_tc")
+             _f32_tc_slice(K, slices), int(gated), act, limit, _ptr(parts), _ptr(split), _stream()), "linear_f32_tc")
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, kind: int, cut: int) -> None:

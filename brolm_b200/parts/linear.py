@@ -2,9 +2,9 @@
 (wlejon/brolm include/brolm/detail/compute.h:49-86 dispatches on the weight's
 element type in the same way).
 
-* float32 weight: the framework's own kernels, at least as precise as float
-  sums: tcgen05 on floats taken apart into halves for large weights, CUDA
-  cores for the others.
+* float32 weight: the framework's own kernels: for large weights tcgen05 on
+  floats taken apart into three bfloat16 numbers, which hold all their bits,
+  CUDA cores for the others.
 * bfloat16 weight, up to 16 rows (decode steps): the framework's own
   weight-streaming tensor-core kernel, float32 accumulation.
 * bfloat16 weight, 17 to 32 rows (``kernels.STREAM_ROWS``; wider decode

@@ -168,6 +168,12 @@ def test_linear_f32_every_kernel_gives_the_same_bits(M, N, K):
         assert torch.equal(out, ref), (kind, cut)
 
 
+def tc_f32_bound(K):
+    """Of the float product on tensor cores, as a share of sum |x w|: a product good to 2^-24; for 64 k four steps of the tensor
+    core with the large parts, each good to 2^-22 of what it adds, and twenty with parts 2^-8 as large; K / 64 float additions."""
+    return (1 + 4 * 4 + 1 + K / 64) * 2.0 ** -24
+
+
 @pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 160, 161, 330])
 @pytest.mark.parametrize("N,K", [(4100, 260), (1024, 1028), (130, 9216), (20000, 256)])
 def test_linear_f32_on_tensor_cores(M, N, K):
@@ -175,17 +181,14 @@ def test_linear_f32_on_tensor_cores(M, N, K):
     assert kernels.linear_f32_tc_slices(N, K) == {4100: 2, 1024: 4, 130: 8, 20000: 1}[N]
     g = torch.Generator(device=DEV).manual_seed(M * N + K)
     x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
-    x[:, ::3] *= 1e-3                                        # (rows whose numbers differ widely)
+    x[:, ::3] *= 1e-3
     wide = torch.full((M, N + 3), float("nan"), device=DEV)
     kernels.linear_f32(x, w, wide[:, :N])
     out = wide[:, :N]
     assert kernels.linear_f32_tc_status(reset=True) == 0 and bool(wide[:, N:].isnan().all())
     ref = x.double() @ w.double().T
-    # a product 3 * 2^-24; per 64 k twelve steps of the tensor core, each good to 2^-22 of what it adds; K / 64 float additions;
-    # what is too small for its row's scale 2^-38 of its largest
     size = x.abs().double() @ w.abs().double().T
-    least = 2.0 ** -38 * K * x.abs().amax(1, keepdim=True).double() * w.abs().amax(1).double()
-    assert bool(((out.double() - ref).abs() <= (3 + 48 + K / 64) * 2.0 ** -24 * size + least).all())
+    assert bool(((out.double() - ref).abs() <= tc_f32_bound(K) * size).all())
     plain_sums = torch.empty(M, N, device=DEV)
     kernels._linear_f32(x, w, plain_sums, 0, 0)
     assert float((out.double() - ref).norm()) <= 1.05 * float((plain_sums.double() - ref).norm())     # no less precise
@@ -195,6 +198,77 @@ def test_linear_f32_on_tensor_cores(M, N, K):
         one = torch.empty(1, N, device=DEV)
         kernels.linear_f32(row[:, 1:], w, one)
         assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("beside", [1e4, 1e8, 1e12, 2.0 ** 40, 1e30])
+@pytest.mark.parametrize("M,off", [(3, 0), (3, 1), (20, 0), (40, 0), (40, 1), (300, 0)])
+@pytest.mark.parametrize("where", ["x", "w"])
+def test_linear_f32_keeps_numbers_beside_much_larger_ones(where, M, off, beside):
+    """A large number in every 64 k that meets a zero: the others' sum is as good as without it."""
+    N, K = 2052, 520
+    assert kernels.linear_f32_tc_slices(N, K) > 1
+    g = torch.Generator(device=DEV).manual_seed(M + off)
+    x, w = torch.randn(M, K + off, generator=g, device=DEV)[:, off:], torch.randn(N, K, generator=g, device=DEV)
+    big, zero = (x, w) if where == "x" else (w, x)
+    big[:, 5::64] *= beside
+    zero[:, 5::64] = 0.0
+    assert kernels.linear_f32_tc_ok(w)
+    out = torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, out)
+    error = (out.double() - x.double() @ w.double().T).abs()
+    assert bool((error <= tc_f32_bound(K) * (x.abs().double() @ w.abs().double().T)).all())
+    gated, both = torch.empty(M, N // 2, device=DEV), torch.empty(M, N // 2, device=DEV)
+    kernels.linear_f32_gated(x, w, gated, "silu")
+    kernels.gated_act(out, both, "silu")
+    assert torch.equal(gated, both)
+
+
+@pytest.mark.parametrize("M", [1, 20, 40, 200])
+def test_linear_f32_on_tensor_cores_at_the_ends_of_the_range(M):
+    """Numbers of which three parts do not hold all bits, beside others that make a sum of ordinary size of them; sums whose
+    terms all end below the smallest normal number; an identity returns x."""
+    N, K = 2048, 640
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    x[:, 7] *= 2.0 ** -118
+    w[:, 7] *= 2.0 ** 110
+    x[:, 8:] *= 2.0 ** -20
+    w[::2, 7] *= 2.0 ** 7 - 1
+    w[1::4, :7], w[1::4, 8:] = 0.0, 0.0                      # rows with nothing but that number
+    w[3::8, 8:] *= 2.0 ** -118
+    x[0, 8:] = 0.0
+    out = torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, out)
+    error = (out.double() - x.double() @ w.double().T).abs()
+    assert bool((error <= tc_f32_bound(K) * (x.abs().double() @ w.abs().double().T) + K * 2.0 ** -149).all())
+    x, w = torch.randn(M, K, generator=g, device=DEV) * 2.0 ** -66, torch.randn(N, K, generator=g, device=DEV) * 2.0 ** -72
+    kernels.linear_f32(x, w, out)
+    error = (out.double() - x.double() @ w.double().T).abs()
+    assert bool((error <= tc_f32_bound(K) * (x.abs().double() @ w.abs().double().T) + K * 2.0 ** -149).all())
+    x, w = torch.randn(M, 1024, generator=g, device=DEV), torch.eye(1024, device=DEV)
+    x[:, ::3] *= 1e9
+    out = torch.empty(M, 1024, device=DEV)
+    kernels.linear_f32(x, w, out)
+    assert kernels.linear_f32_tc_ok(w) and torch.equal(out, x)
+
+
+@pytest.mark.parametrize("kind", ["normal", "positive", "spread"])
+@pytest.mark.parametrize("M,N,K", [(3, 4096, 2304), (300, 2304, 9216)])
+def test_linear_f32_on_tensor_cores_is_no_less_precise_than_fmas(kind, M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) * 0.02
+    if kind == "positive":
+        x, w = x.abs(), w.abs()
+    if kind == "spread":
+        x, w = x * torch.exp(3 * torch.randn(M, K, generator=g, device=DEV)), w * torch.exp(2 * torch.randn(N, K, generator=g, device=DEV))
+    out, fmas = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, out)
+    kernels._linear_f32(x, w, fmas, 0, 0)
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    # sums of one sign: the tensor core cuts off half a last place at each of four steps, with a quarter to the whole of 64 k's sum
+    cut = 1.8 * 2.0 ** -24 * float(ref.norm()) if kind == "positive" else 0.0
+    assert float((out.double() - ref).norm()) <= float((fmas.double() - ref).norm()) + cut
+    assert float(((out.double() - ref).abs() / size).max()) <= float(((fmas.double() - ref).abs() / size).max())
 
 
 def test_linear_f32_on_tensor_cores_of_infinities_and_the_smallest_numbers():
