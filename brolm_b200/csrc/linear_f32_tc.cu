@@ -15,7 +15,7 @@
 //
 // A block owns 128 rows of W (the M side of the instruction), up to NT tokens (the N side) and one slice of K.  The sums of
 // the slices are added through the shared memory of a cluster of blocks, or by the kernel behind this one.  Roles:
-//   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it;
+//   TMA     one thread fetches W, 32 floats of every row at a time, for up to 16 tokens ahead of the kernel before it;
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the three rows of parts into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
 //           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the parts in by TMA;
@@ -229,6 +229,8 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     if (role == Role::TMA || role == Role::MMA || role == Role::FETCH_X || role == Role::NONE) {
         if constexpr (!S::FEW) fewer_registers<48>();
         if (role == Role::TMA && lane == 0) {
+            // W may be the result of the kernel before this one, unless there are at most 16 tokens (the rule of linear_f32.cu)
+            if (g.M > 16) pdl_wait();
             int i = 0;
             for (; i < 2 * stages; ++i) {
                 const int s = i % S::W_SLOTS;

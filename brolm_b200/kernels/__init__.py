@@ -1177,7 +1177,8 @@ def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
     """out (M, N) = x (M, K) @ weight (N, K)^T, all float32, rows may be strided.  A row's bits depend on neither M
-    nor its place among the rows."""
+    nor its place among the rows.  Up to 16 rows, the weights are read ahead of the kernel before this one on the stream: they
+    must not be its result."""
     assert x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32
     assert x.dim() == 2 and weight.dim() == 2 and out.dim() == 2
     assert x.stride(1) == 1 and weight.stride(1) == 1 and out.stride(1) == 1

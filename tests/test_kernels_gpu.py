@@ -271,6 +271,22 @@ def test_linear_f32_on_tensor_cores_is_no_less_precise_than_fmas(kind, M, N, K):
     assert float(((out.double() - ref).abs() / size).max()) <= float(((fmas.double() - ref).abs() / size).max())
 
 
+def test_linear_f32_of_weights_that_the_kernel_before_it_made():
+    """More than 16 rows: the weights are read behind the kernel before."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    made = torch.randn(4096, 2304, generator=g, device=DEV).to(torch.bfloat16)
+    for M in (17, 40, 200):
+        x, out = torch.randn(M, 2304, generator=g, device=DEV), torch.empty(M, 4096, device=DEV)
+        want = torch.empty(M, 4096, device=DEV)
+        kernels.linear_f32(x, made.float(), want)
+        for _ in range(5):
+            w = torch.full((4096, 2304), float("nan"), device=DEV)
+            torch.cuda.synchronize()
+            kernels.cast(made, w)
+            kernels.linear_f32(x, w, out)
+            assert torch.equal(out, want)
+
+
 def test_linear_f32_on_tensor_cores_of_infinities_and_the_smallest_numbers():
     """What a sum of parts cannot say is said by the floats themselves; the rows beside keep their bits."""
     g = torch.Generator(device=DEV).manual_seed(12)
