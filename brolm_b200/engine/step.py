@@ -206,6 +206,7 @@ class Engine:
             weakref.finalize(self, kernels.give_stream, index, self.beside)
         self.last_h2d_bytes = 0          # bytes the last step copied from the host
         self._checked_at = -1            # this library's launches when the kernels' status words were last read
+        self._ran_on: Optional[torch.cuda.Stream] = None      # the stream of the last step
         self._pin: Optional[torch.Tensor] = None      # pinned staging buffer of the steps that are not captured
         self._pin_copied = None
 
@@ -225,19 +226,27 @@ class Engine:
 
     def _check_waits(self, where: str, consequence: str) -> None:
         """Raise if a bounded wait inside one of the tcgen05 kernels ran out since the last check.
-        Reads and resets every status word (each read waits for the device)."""
-        if self.device.type != "cuda" or self._checked_at == kernels.launch_count():
+        Reads and resets every status word, behind the last step: the words are read on the default stream,
+        which waits for no other, so the step's own is waited for first."""
+        launched = kernels.launch_count()
+        if self.device.type != "cuda" or self._checked_at == launched:
             return                       # (nothing of this library has run since: a prompt is checked at its step's end)
-        self._checked_at = kernels.launch_count()
+        if self._ran_on is not None:
+            self._ran_on.synchronize()
         codes = {"linear_f32_tc": kernels.linear_f32_tc_status(reset=True)}
         if self.model.dtype == torch.bfloat16:
             codes |= {"gemm_tc": kernels.gemm_tc_status(reset=True), "attn_tc": kernels.attention_tc_status(reset=True),
                       "gemm_stream": kernels.gemm_stream_status(reset=True),
                       "grouped_tc": kernels.grouped_tc_status(reset=True)}
+        self._checked_at = launched
         bad = {k: v for k, v in codes.items() if v}
         if bad:
             raise StepError(f"{where}: a wait inside a tensor-core kernel ran out ({bad}), in this step or in a "
                             f"decode step since the last check; {consequence}")
+
+    def _note_stream(self) -> None:
+        if self.device.type == "cuda":
+            self._ran_on = torch.cuda.current_stream(self.device)
 
     # the step -------------------------------------------------------------
     def step(self, slots: Sequence[int], tokens: Sequence[Sequence[int]],
@@ -254,6 +263,7 @@ class Engine:
         (wlejon/brolm's ``hidden_out``, include/brolm/gemma2.h:121-125).
         """
         plan = self._plan(slots, tokens, want)
+        self._note_stream()
         if plan.mode == "decode" and self.use_graphs:
             graph = self._graph_for(plan)
             logits = graph.run(plan, self.cache)
@@ -285,6 +295,7 @@ class Engine:
         plan = self._plan(slots, [[0]] * len(slots), None)
         if plan.mode != "decode":
             raise StepError("step_from: only sequences that already hold tokens can go on")
+        self._note_stream()
         if self.use_graphs:
             graph = self._graph_for(plan)
             logits = graph.run(plan, self.cache, ids, [int(p) for p in pick])[:len(plan.slots)]

@@ -113,6 +113,41 @@ def test_a_step_whose_kernel_gave_up_raises_and_the_engine_goes_on():
     eng.close([s])
 
 
+def test_a_step_on_a_stream_of_its_own_whose_kernel_gave_up_raises():
+    """The status words are read behind the step, whatever stream it ran on and whatever stream ``close`` is called on."""
+    cfg = bb.Gemma2Config(vocab_size=1000, num_hidden_layers=1)
+    model = bb.Model(cfg, dtype="bfloat16", device=DEV).init_random(seed=3, on_device=True)
+    eng = bb.Engine(model, max_tokens=4096, max_slots=2)
+    prompt = torch.randint(0, 1000, (2048,), generator=torch.Generator().manual_seed(4)).tolist()
+    stream = torch.cuda.Stream()
+    for library in ("gemm_tc2", "gemm_stream"):                 # (the prompt's products; a decode step's output matrix)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            (s,) = eng.open(1)
+            eng.step([s], [prompt])
+            eng.step([s], [[5]])
+            eng.close([s])
+            (s,) = eng.open(1)
+            if library == "gemm_stream":
+                eng.step([s], [prompt])
+        kernels.wait_control(library, cycles=10 * LIMIT, stall_code=3)
+        try:
+            with torch.cuda.stream(stream):
+                if library == "gemm_tc2":
+                    with pytest.raises(bb.StepError, match="ran out"):
+                        eng.step([s], [prompt])
+                else:
+                    eng.step([s], [[5]])
+            if library == "gemm_stream":
+                with pytest.raises(bb.StepError, match="ran out"):
+                    eng.close([s])
+        finally:
+            torch.cuda.synchronize()
+            kernels.wait_control(library, 0, 0)
+        if library == "gemm_tc2":
+            eng.close([s])
+
+
 def test_routed_experts_whose_wait_runs_out():
     """The tcgen05 grouped product: the epilogue's wait for its accumulator never completes."""
     from brolm_b200.parts import RoutedExperts
