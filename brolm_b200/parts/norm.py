@@ -138,7 +138,10 @@ def add_then_norm(h: torch.Tensor, y: torch.Tensor, post: Optional[Part], nxt: O
             and post.weight.dtype != nxt.weight.dtype:
         fused_next = False
     if y.dim() == 3 and not fused_post:
-        y = y.sum(dim=0)                       # partial sums, and a norm that wants the whole
+        # partial sums, and a norm that wants the whole: added in order, as every other reader adds them
+        whole = torch.empty(h.shape, dtype=torch.float32, device=h.device)
+        kernels.bias_act(y, None, "none", whole)
+        y = whole
     if not fused_post:
         y = post.apply(y, torch.float32)
         post = None

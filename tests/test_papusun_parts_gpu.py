@@ -63,6 +63,23 @@ def test_layer_norm_alone_and_behind_the_sum(W, wd):
             close(out[[0, 3, 4]], ref(h.double() + s)[[0, 3, 4]], what=f"{p} parts, post {with_post}")
 
 
+@pytest.mark.parametrize("parts,W", [(2, 40), (3, 256), (5, 2304), (8, 2304), (8, 41)])
+def test_a_norm_of_the_whole_result_gets_its_slices_added_in_order(parts, W):
+    """A layer norm of the mixer's result: the same bits whether the product left slices or had them added."""
+    g = torch.Generator().manual_seed(parts * W)
+    T = 5
+    h, y = torch.randn(T, W, generator=g).to(DEV), torch.randn(parts, T, W, generator=g).to(DEV)
+    post, nxt = LayerNorm(W, 1e-5), RMSNorm(W, 1e-5)
+    post.bind({"weight": torch.randn(W, generator=g).to(DEV)})
+    nxt.bind({"weight": torch.randn(W, generator=g).to(DEV)})
+    whole = y[0].clone()
+    for s in y[1:]:
+        whole += s
+    one, two = h.clone(), h.clone()
+    a, b = add_then_norm(one, y, post, nxt, torch.float32), add_then_norm(two, whole, post, nxt, torch.float32)
+    assert torch.equal(a, b) and torch.equal(one, two)
+
+
 # --- the gated delta rule ------------------------------------------------------------------------------------------
 def delta_inputs(G, d, H, dv, K, T, seed):
     g = torch.Generator().manual_seed(seed)
