@@ -17,8 +17,9 @@
 // A block owns 32 rows of one (sequence, kv head), a row being a (query token, query head of the group) pair, or 8 where
 // a step has no more (decode), and either walks all spans it sees or, where that leaves SMs idle, one of them, with
 // merge_kernel behind it (attn_f32_splits and attn_f32_worth_sharing in kernels/__init__.py have the rule and what both take): a decode step of three
-// sequences of up to 420 keys is otherwise twelve blocks (30 us shared; 337 us in attn_simt.cu, which served all sizes
-// before; a prompt of 300 tokens 63 and 173 us).  Of a span only the 32-key parts that some row sees are worked on: one,
+// sequences of 420 keys, 4 kv heads of 256, is otherwise twelve blocks (79 us; 27 shared, 11.5 in clusters of four blocks, which
+// take such a span where there are few; 337 in attn_simt.cu, which served all sizes before).  Prompts in tiles of 16 rows where
+// those of 32 leave SMs idle (300 tokens, 8 heads of 256 on 4: 50 us, 62 in tiles of 32).  Of a span only the 32-key parts that some row sees are worked on: one,
 // two or all four (16 tokens, 4 heads of 16: 8.9 us, 13.8 with whole spans; 1,000 tokens, 32 heads of 128 on 8 kv heads, window 64:
 // 129 and 183).  K comes through a ring of cp.async stages in slices of 32 c of all 128 keys, V in
 // slices of 16 keys; both products run on packed fma.rn.f32x2, the scores paired along c, the values along d.  Bound by
@@ -422,7 +423,8 @@ __global__ void __launch_bounds__(THREADS, ROWS == 8 ? 4 : VJ == 4 && ROWS == 32
 // Tiles of eight rows whose spans are shared (decode steps): a cluster of four blocks takes a span, each the scores of 32
 // keys for all rows, and then, with every score handed round through shared memory, a quarter of the value's entries for
 // all 128 keys.  All keys and values of a block are on their way at once, 64 KB with heads of 256, and every chain of fmas
-// has a thread of its own: what is left is the chains' length and the memory's latency.  The same order of operations.
+// has a thread of its own: what is left is the chains' length and the memory's latency.  The same order of operations.  For no more spans than SMs: the
+// cluster's exchange costs more than it gives once blocks queue (brolm_attn_f32 has the figures).
 constexpr int FEW = 8, FEW_THREADS = 32 * FEW, SHARERS = 4;
 
 __host__ __device__ __forceinline__ int few_quarter(int vd) { return (vd + 15) / 16 * 4; }      // value entries of a block
@@ -687,13 +689,17 @@ BROLM_API int brolm_attn_f32(const void* q, int q_stride, void* out, int out_str
     // 8 kv heads, 384 blocks: 27 us where two share an SM)
     a.max_parts = k_pages || max_q_len > 64 || (long long)max_q_len * group <= 8 ? 4 : max_q_len > 32 ? 2 : 1;
     if ((long long)max_q_len * group <= 8) {
-        if (splits) return launch_few(a, batch, max_q_len, stream);
+        // us, a block a span / a cluster a span, by spans (of all sequences and kv heads): heads of 256, two a kv head, 64 28.1 /
+        // 12.5, 128 31.2 / 20.1, 256 36.2 / 35.1, 512 64.6 / 68.2, 1,024 97.7 / 122; heads of 64, one, 128 15.9 / 11.9, 256 19.5 /
+        // 18.6, 512 29.8 / 30.7, 1,024 44.0 / 53.8; heads of 16, two, 128 14.8 / 11.2, 256 16.5 / 17.2, 1,024 37.5 / 49.2
+        if (splits && (long long)splits * n_kv * batch <= device_sm_count()) return launch_few(a, batch, max_q_len, stream);
         if (vd <= 128) return launch<8, 1>(a, batch, max_q_len, stream);
         return launch<8, 2>(a, batch, max_q_len, stream);
     }
     // Shared spans that give an SM hardly more than one block of 32 rows go in tiles of 16: two blocks an SM hide each other's
-    // waits (a prompt of 300 tokens, 8 heads of 256 on 4 kv heads, 152 blocks with something to do: 63.8 us in tiles of 32, 50.7
-    // of 16; of 200 tokens 62.3 / 48.5).
+    // waits (us in tiles of 32 / of 16, prompts of 160 to 400 tokens: 8 heads of 256 on 4 kv heads 59 to 62 / 47 to 50, 8 of 128
+    // on 4 38 to 40 / 32 to 34, 16 of 128 on 4 39.6 / 33.3, 4 of 64 on 2 25 to 27 / 19 to 23).  Beyond, tiles of 16 lose with heads
+    // of 256 (400 tokens, 8 on 4: 63 / 86; 300, 16 on 8: 66 / 94) and gain up to 15 % or lose up to 10 with smaller ones.
     const long long tiles = ((long long)max_q_len * group + 31) / 32;
     if (splits && 2 * tiles * n_kv * batch * (splits + 1) <= 5LL * device_sm_count()) {
         if (vd <= 64) return launch<16, 1>(a, batch, max_q_len, stream);

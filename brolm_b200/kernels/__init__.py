@@ -1698,8 +1698,9 @@ def attn_f32_splits(batch: int, n_kv: int, group: int, vd: int, tokens: int, max
     """How many blocks share the spans of a tile of rows (0: a block walks them all): one per span as long as the tiles
     alone are fewer than four to an SM and the partial results stay below 64 MB.
 
-    Measured, 8 heads of 256 over 4 kv heads, walked / shared: a prompt of 300 tokens (76 tiles) 130 / 71 us, one token of
-    three sequences of 420 keys 84 / 30 us, of eight of 1,024 183 / 42 us, of 64 of 1,280 265 / 204 us.  ``max_keys``: a bound on a sequence's keys (None: none is known)."""
+    Measured, 8 heads of 256 over 4 kv heads, walked / shared: a prompt of 300 tokens (76 tiles) 130 / 50 us, one token of
+    three sequences of 420 keys 79 / 11.5 us, of eight of 1,024 173 / 35 us, of 64 of 1,280 265 / 204 us.  ``max_keys``: a bound
+    on a sequence's keys (None: none is known)."""
     rows = 8 if max_q_len * group <= 8 else 32
     tiles = -(-max_q_len * group // rows)
     spans = [-(-max_keys // F32_SPAN)] if max_keys else []
@@ -1715,9 +1716,11 @@ def attn_f32_worth_sharing(batch: int, n_kv: int, group: int, head_dim: int, vd:
     that walk them.
 
     A span takes a block of 32 rows some 21 us with heads of 64, 30 with 128 and 48 with 256, of 8 rows 10, 14 and 24; two or
-    three blocks share an SM and slow each other down a little.  Measured, walked / shared: a prompt of 300 tokens with 8
-    heads of 256 on 4 kv heads (76 tiles) 147 / 79 us, with a window of 100 92 / 76; with 32 heads of 128 on 8 (304) 93 / 86, with a
-    window of 64 51 / 66; one token of 200 keys, 32 heads of 128 on 8, of one sequence 27 / 18, of 32 sequences 29 / 36."""
+    three blocks share an SM and slow each other down a little.  Up to one span of 8 rows an SM goes to clusters of four blocks:
+    8 us and 4 more for heads of 256, once more where they queue for the SMs' shared memory.  Measured, walked / shared: a prompt of
+    300 tokens with 8 heads of 256 on 4 kv heads (76 tiles) 147 / 79 us (now 50, in tiles of 16), with a window of 100 92 / 76; with 32
+    heads of 128 on 8 (304) 93 / 86, with a window of 64 51 / 66; one token of 200 keys, 32 heads of 128 on 8, of one sequence 22 / 10,
+    of 32 sequences 27 / 31; of 32 sequences of 200 keys, 8 heads of 64 on 1, 19 / 11.5, of as many, 4 of 16 on 2, 16 / 9.6."""
     sms = sms or device_sms()
     rows = 8 if max_q_len * group <= 8 else 32
     size = (head_dim + vd) / 512
@@ -1737,6 +1740,11 @@ def attn_f32_worth_sharing(batch: int, n_kv: int, group: int, head_dim: int, vd:
 
     def round_of(blocks: float) -> float:
         return span * max(1.0, blocks / places) * (1 + slower * min(places / sms - 1, max(0.0, blocks / sms - 1)))
+    if rows == 8 and busy > 1:
+        splits = attn_f32_splits(batch, n_kv, group, vd, batch * max_q_len, max_q_len, max_keys, window, chunk, sms)
+        if 0 < splits * n_kv * batch <= sms:
+            queued = 4 * tiles * busy / ((2 if size > 0.6 else 4) * sms)
+            return (8 + 4 * size) * max(1.0, queued) < 0.93 * walked * span
     merging = 5 + (max_q_len * group * n_kv * batch / 400 if rows == 8 else 0)
     return part * round_of(tiles * busy) + merging < 0.93 * walked * round_of(tiles)
 

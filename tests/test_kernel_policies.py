@@ -202,6 +202,9 @@ def test_float_attention_shares_spans_only_where_the_merge_is_worth_it():
     assert not worth(1, 2, 2, 32, 32, 300, 300, window=16) and not worth(1, 8, 4, 128, 128, 300, 300, window=64)
     assert worth(1, 4, 2, 256, 256, 300, 300, window=100) and not worth(32, 8, 4, 128, 128, 1, 256)
     assert not worth(1, 4, 2, 256, 256, 1, None)                                               # no bound
+    # up to one span an SM in clusters: worth it for the smallest heads, too; beyond, what a block a span takes decides
+    assert worth(8, 2, 2, 16, 16, 1, 200) and worth(32, 1, 8, 64, 64, 1, 200) and worth(3, 4, 2, 256, 256, 1, 200)
+    assert not worth(128, 2, 2, 16, 16, 1, 200) and not worth(8, 2, 2, 16, 16, 1, 120)
 
 
 def test_float_attention_is_cut_by_the_lengths_not_by_the_table():

@@ -1117,6 +1117,51 @@ def test_float_attention_of_a_few_rows_gives_the_bits_of_more(monkeypatch, n_q, 
     close(outs[2], outs[0].double().cpu(), torch.float32, scale=float(outs[0].abs().max()))      # (a share's spans are merged first)
 
 
+@pytest.mark.parametrize("n_kv,hd,vd", [(2, 64, 64), (4, 256, 256), (3, 40, 136)])
+@pytest.mark.parametrize("batch", [6, 60])
+def test_float_attention_of_few_rows_in_clusters_and_a_block_a_span(monkeypatch, batch, n_kv, hd, vd):
+    """Four spans of each sequence: in clusters where they are fewer than SMs, else a block each; the bits of one that walks."""
+    assert (batch * n_kv * 4 <= kernels.device_sms()) == (batch == 6)
+    g = torch.Generator(device=DEV).manual_seed(hd + batch)
+    pages = batch * 8
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32).view(batch, 8)
+    kp, vp = torch.randn(pages, n_kv, 64, hd, generator=g, device=DEV), torch.randn(pages, n_kv, 64, vd, generator=g, device=DEV)
+    q = torch.randn(batch, 2 * n_kv * hd, generator=g, device=DEV)
+    lengths = torch.randint(1, 513, (batch,), generator=g, device=DEV).to(torch.int32)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: True)
+    outs = []
+    for splits in (0, 4):
+        monkeypatch.setattr(kernels, "attn_f32_splits", lambda *a, **kw: splits)
+        outs.append(torch.full((batch, 2 * n_kv * vd), float("nan"), device=DEV))
+        kernels.attention_simt(q, outs[-1], torch.arange(batch + 1, dtype=torch.int32, device=DEV), lengths, n_kv=n_kv, group=2,
+                               head_dim=hd, v_dim=vd, scale=hd ** -0.5, cap=30.0, window=0, batch=batch, max_q_len=1, k_pages=kp,
+                               v_pages=vp, page_table=table, ring=1 << 30, page_size=64)
+    assert torch.equal(outs[0], outs[1]) and not bool(outs[0].isnan().any())
+
+
+@pytest.mark.parametrize("rows", [16, 32])
+@pytest.mark.parametrize("hd,vd", [(64, 64), (64, 128), (40, 72), (256, 256), (128, 200)])
+@pytest.mark.parametrize("n", [131, 300])
+def test_float_attention_of_a_prompt_in_tiles_of_16_and_32_rows(monkeypatch, n, hd, vd, rows):
+    """Shared spans in either tile, every number of value columns a thread: the bits of blocks that walk (tiles of 32)."""
+    batch, n_kv = (1, 3) if rows == 16 else (3, 12)
+    tiles, spans = -(-n * 2 // 32), -(-n // 128)
+    assert (2 * tiles * n_kv * batch * (spans + 1) <= 5 * kernels.device_sms()) == (rows == 16)
+    g = torch.Generator(device=DEV).manual_seed(n + hd + vd)
+    lengths = [n, n - 37, 5][:batch]
+    T, n_q = sum(lengths), 2 * n_kv
+    q, k, v = (torch.randn(T, w, generator=g, device=DEV) for w in (n_q * hd, n_kv * hd, n_kv * vd))
+    cu = torch.tensor([0] + [sum(lengths[:i + 1]) for i in range(batch)], dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(kernels, "attn_f32_worth_sharing", lambda *a, **kw: True)
+    outs = []
+    for cut in (spans, 0):
+        monkeypatch.setattr(kernels, "attn_f32_splits", lambda *a, **kw: cut)
+        outs.append(torch.full((T, n_q * vd), float("nan"), device=DEV))
+        kernels.attention_simt(q, outs[-1], cu, torch.tensor(lengths, dtype=torch.int32, device=DEV), n_kv=n_kv, group=2, head_dim=hd,
+                               v_dim=vd, scale=hd ** -0.5, cap=20.0, window=0, batch=batch, max_q_len=n, k=k, v=v)
+    assert torch.equal(outs[0], outs[1]) and not bool(outs[0].isnan().any())
+
+
 @pytest.mark.parametrize("shared", [False, True])
 @pytest.mark.parametrize("lengths", [[3], [32, 5, 1], [33, 64, 20], [65, 7, 96], [97, 40], [129, 160, 31]])
 @pytest.mark.parametrize("window,chunk", [(0, 0), (1, 0), (40, 0), (70, 0), (0, 33)])
