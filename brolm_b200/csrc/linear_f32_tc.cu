@@ -36,9 +36,10 @@
 // against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.0 to 1.4e-7 here for normal numbers; 0.7 to 1.2e-7 and
 // 0.9 to 1.2e-7 for sums of one sign, which lose half a last place at each step of the tensor core and none on average to fmas.
 //
-// What three parts cannot say is said by the floats themselves: the thread that has a doubtful sum of a slice makes it again
+// What three parts cannot say is said by the floats themselves: the warp that has a doubtful sum of a slice makes it again
 // by fmas.  Doubtful are (see doubtful())
-//   a sum that is not finite: an infinity or a NaN among the operands ends as a NaN here, infinity minus infinity;
+//   a sum that is not finite: an infinity among the operands ends as a NaN here, infinity minus infinity (a NaN among them
+//   is a NaN in any case, and stays);
 //   a sum below 1e-20: the products of low parts end at 2^-126;
 //   a sum with a number below 2^-60 on one side and one of 2^17 or more on the other: numbers below 2^-102 lose their low
 //   parts, up to 2^-125 of each; times less than 2^17 that is far below the last place of a sum of 1e-20;
@@ -114,20 +115,24 @@ struct Args {
 };
 
 // What a row's or a token's numbers of a slice are like, for doubtful().
-enum : uint32_t { SMALL = 1, BIG = 2, SOME = 4 };
+enum : uint32_t { SMALL = 1, BIG = 2, SOME = 4, BROKEN = 8 };
 struct Extent {
-    float low = INFINITY, high = 0.0f;
-    __device__ __forceinline__ void add(float v) { low = fminf(low, fabsf(v)), high = fmaxf(high, fabsf(v)); }
+    float low = INFINITY, high = 0.0f;                         // (a NaN among them makes `high` one)
+    __device__ __forceinline__ void add(float v) {
+        low = fminf(low, fabsf(v));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(v)));
+    }
     __device__ __forceinline__ void add(const float4& v) { add(v.x), add(v.y), add(v.z), add(v.w); }
     __device__ __forceinline__ uint32_t flags() const {
-        return (low < 8.67361738e-19f ? SMALL : 0) | (high >= 131072.0f ? BIG : 0) | (high > 0.0f ? SOME : 0);
+        return (low < 8.67361738e-19f ? SMALL : 0) | (high >= 131072.0f ? BIG : 0) | (high > 0.0f ? SOME : 0) |
+               (high != high ? BROKEN : 0);
     }
     // of the eight lanes that share a row's 64 k
     __device__ __forceinline__ uint32_t flags_of_eight(int lane) const {
         const uint32_t mine = flags(), eight = 0xffu << (lane & 24);
         uint32_t all = 0;
 #pragma unroll
-        for (uint32_t bit = SMALL; bit <= SOME; bit <<= 1) all |= __ballot_sync(0xffffffffu, mine & bit) & eight ? bit : 0;
+        for (uint32_t bit = SMALL; bit <= BROKEN; bit <<= 1) all |= __ballot_sync(0xffffffffu, mine & bit) & eight ? bit : 0;
         return all;
     }
 };
@@ -153,26 +158,39 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
-__device__ __noinline__ float plain_dot(const float* x, const float* w, int k, int end) {
+// A sum from the floats themselves, by a whole warp: a lane's chain of fmas over every 32nd four k, then the lanes' sums in pairs.
+// A token with an infinity is doubtful in all its sums (18,432 x 2,304, 3 tokens: 158 us with one such token, 256 where a thread
+// makes a sum).
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int k, int end, int lane) {
     float y = 0.0f;
-    for (; k < end; k += 512) {
-        float even = 0.0f, odd = 0.0f;
-        const int stop = min(end, k + 512);
-        for (int i = k; i < stop; i += 2) {                   // the ends are multiples of 4
-            even = __fmaf_rn(x[i], w[i], even);
-            odd = __fmaf_rn(x[i + 1], w[i + 1], odd);
-        }
-        y += even + odd;
+    for (k += 4 * lane; k < end; k += 128) {                  // (the ends are multiples of 4, W's rows lie on 16-byte boundaries)
+        const float4 v = *reinterpret_cast<const float4*>(w + k);
+        y = __fmaf_rn(x[k], v.x, y);
+        y = __fmaf_rn(x[k + 1], v.y, y);
+        y = __fmaf_rn(x[k + 2], v.z, y);
+        y = __fmaf_rn(x[k + 3], v.w, y);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
     return y;
 }
-__device__ __forceinline__ bool doubtful(float y) {
-    const float size = fabsf(y);
-    return !(size <= 3.402823466e38f) || (size < 1e-20f && y != 0.0f);
+// The same for every lane of a warp whose sum is doubtful, one after the other.
+__device__ __forceinline__ void make_again(bool again, float& y, const float* x, const float* w, int k, int end, int lane) {
+    for (uint32_t left = __ballot_sync(0xffffffffu, again); left; left &= left - 1) {
+        const int whose = __ffs(left) - 1;
+        const float* xs = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(x), whose));
+        const float* ws = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(w), whose));
+        const float sum = plain_dot(xs, ws, k, end, lane);
+        if (lane == whose) y = sum;
+    }
 }
 __device__ __forceinline__ bool doubtful(float y, uint32_t row, uint32_t token) {
-    return doubtful(y) || (((row & token >> 1) | (row >> 1 & token)) & SMALL) || (y == 0.0f && (row & token & SOME) && ((row | token) & SMALL));
+    const float size = fabsf(y);
+    return !((row | token) & BROKEN) &&                        // (a NaN among the numbers: the sum is one)
+           (!(size <= 3.402823466e38f) || (size < 1e-20f && y != 0.0f) || (((row & token >> 1) | (row >> 1 & token)) & SMALL) ||
+            (y == 0.0f && (row & token & SOME) && ((row | token) & SMALL)));
 }
+constexpr uint32_t AGAIN = 0x7fc0a6a1u;            // a NaN that no sum is: the kernel that adds the slices makes this one again
 
 // One lane of a warp that is there as a whole, always the same one.  The compiler knows of this one that it is alone, and keeps
 // what the products are given in uniform registers: 24 products of 16 tokens are issued in 0.7 us where `lane == 0` takes 1.2.
@@ -351,12 +369,12 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         }
         const uint32_t mine = row_flags[row] | row_flags[BR + row];
         if (j == stages && g.parts && g.y) {
-            // the kernel behind this one looks for doubtful sums itself; those that their flags make so are told by a NaN
+            // the kernel behind this one makes the doubtful sums again
             float* dst = g.parts + ((size_t)part * g.M + m0 + first) * g.N + n0 + row;
             if (n0 + row < g.N) {
 #pragma unroll
                 for (int c = 0; c < S::COLS; ++c)
-                    if (first + c < tokens) dst[(size_t)c * g.N] = doubtful(sum[c], mine, token_flags[first + c]) ? NAN : sum[c];
+                    if (first + c < tokens) dst[(size_t)c * g.N] = doubtful(sum[c], mine, token_flags[first + c]) ? __uint_as_float(AGAIN) : sum[c];
             }
         } else if (j == stages) {
             // the rings are done with: all products have been made
@@ -369,10 +387,14 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                     fine &= !doubtful(sum[c], mine, token_flags[first + c]);
                 }
             const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
-            if (!fine && w_row < (g.gated ? 2 * g.N : g.N))
-                for (int c = first; c < min(first + S::COLS, tokens); ++c)
-                    if (doubtful(sums[c * BR], mine, token_flags[c]))
-                        sums[c * BR] = plain_dot(g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo, min(g.K, k_lo + g.slice));
+            fine |= w_row >= (g.gated ? 2 * g.N : g.N);
+            if (!__all_sync(0xffffffffu, fine))
+                for (int c = first; c < min(first + S::COLS, tokens); ++c) {
+                    float y = sums[c * BR];
+                    make_again(!fine && doubtful(y, mine, token_flags[c]), y, g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo,
+                               min(g.K, k_lo + g.slice), lane);
+                    sums[c * BR] = y;
+                }
         }
     } else {
         // X: eight k of a token at a time, the eight lanes of a token side by side
@@ -583,23 +605,25 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
     pdl_trigger();
     pdl_wait();
     const size_t total = (size_t)g.M * g.N;
-    for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
-        const size_t token = idx / g.N, n = idx % g.N;
+    const int lane = threadIdx.x & 31;
+    for (size_t first = (size_t)blockIdx.x * 256 + threadIdx.x - lane; first < total; first += (size_t)gridDim.x * 256) {
+        const bool there = first + lane < total;              // (a warp stays whole)
+        const size_t idx = there ? first + lane : total - 1, token = idx / g.N, n = idx % g.N;
         float v[8];                                            // at most eight slices, all on their way at once
         bool fine = true;
 #pragma unroll
         for (int s = 0; s < 8; ++s) v[s] = s < slices ? g.parts[s * total + idx] : 0.0f;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) fine &= !doubtful(v[s]);
-        if (!fine)
+        for (int s = 0; s < 8; ++s) fine &= __float_as_uint(v[s]) != AGAIN;
+        if (!__all_sync(0xffffffffu, fine))
 #pragma unroll
             for (int s = 0; s < 8; ++s)
-                if (doubtful(v[s])) v[s] = plain_dot(g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice));
+                make_again(there && __float_as_uint(v[s]) == AGAIN, v[s], g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice), lane);
         float y = v[0];
 #pragma unroll
         for (int s = 1; s < 8; ++s)
             if (s < slices) y += v[s];
-        g.y[token * g.ldy + n] = y;
+        if (there) g.y[token * g.ldy + n] = y;
     }
 }
 
