@@ -1148,8 +1148,11 @@ def _f32_tc_slice(K: int, slices: int) -> int:
 def linear_f32_tc_scratch(M: int, N: int, slices: int) -> bool:
     """Whether the slices of a product of M rows are added by a kernel behind it rather than by clusters of blocks: for more
     than 32 rows a block has an SM to itself, and only about sixteen clusters of eight such blocks find room at a time.
-    Many clusters fill their rounds all the same; then, and where the sums would take more than 256 MB, there is no scratch."""
-    return M > 32 and -(-M // 160) * -(-N // 128) < 64 and slices * M * N * 4 <= F32_PARTS_LIMIT
+    Many clusters fill their rounds all the same; then, and where the sums would take more than 256 MB, there is no scratch.
+    Up to 32 rows those sixteen clusters are the line (3 rows, scratch / clusters: 2,304 x 9,216 20.2 / 33.1 us, 2,304 x 2,304
+    9.1 / 11.5, 2,304 x 2,048 9.3 / 10.2)."""
+    tiles = -(-M // 160) * -(-N // 128)
+    return (tiles < 64 if M > 32 else tiles * slices > 128) and slices * M * N * 4 <= F32_PARTS_LIMIT
 
 
 def linear_f32_parts(x: torch.Tensor, weight: torch.Tensor) -> int:
@@ -1208,9 +1211,10 @@ def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Te
                    limit: float = 0.0, parts: Optional[torch.Tensor] = None) -> None:
     (M, K), N = x.shape, out.shape[1] if out is not None else parts.shape[2]
     split = None
-    if M > 32 and not (x.stride(0) % 4 or x.data_ptr() % 16):
-        if parts is None and slices > 1 and not gated and linear_f32_tc_scratch(M, N, slices):
-            parts = torch.empty((slices, M, N), dtype=torch.float32, device=x.device)
+    aligned = not (x.stride(0) % 4 or x.data_ptr() % 16)
+    if parts is None and slices > 1 and not gated and (aligned or M <= 32) and linear_f32_tc_scratch(M, N, slices):
+        parts = torch.empty((slices, M, N), dtype=torch.float32, device=x.device)
+    if M > 32 and aligned:
         size = M * -(-K // 64) * 385                         # the rows in three parts of 16 bits, and a byte for every 64
         if size <= F32_PARTS_LIMIT:
             split = torch.empty(size, dtype=torch.uint8, device=x.device)

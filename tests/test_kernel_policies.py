@@ -141,6 +141,14 @@ def test_slices_of_the_float_product_on_tensor_cores():
                 assert per % 64 == 0 and (n - 1) * per < K <= n * per and (n == 1 or -(-N // 128) * n <= 148)
 
 
+def test_where_the_slices_of_a_float_product_are_added():
+    """By a kernel behind it where clusters of eight blocks would queue for room, as long as the sums take no more than 256 MB."""
+    scratch = kernels.linear_f32_tc_scratch
+    assert scratch(3, 2304, 8) and scratch(32, 2176, 8) and not scratch(3, 2048, 8) and not scratch(3, 4096, 4)
+    assert scratch(33, 1024, 8) and scratch(300, 2304, 8) and not scratch(3000, 2304, 8)
+    assert scratch(32, 2304, 8) and not scratch(10400, 128, 8) and not scratch(9000, 1024, 8)
+
+
 def test_which_kernel_takes_a_float_product():
     """Streams for few rows, small tiles where large ones leave SMs idle, large ones where there are enough of them."""
     plan = lambda M, N, K: kernels.linear_f32_plan(M, N, K, 148)
