@@ -131,12 +131,13 @@ def test_linear_f32(M, N, K):
 
 
 @pytest.mark.parametrize("M", [1, 2, 5, 16, 17, 33, 70])
-@pytest.mark.parametrize("N,K", [(8, 4), (33, 516), (2304, 2304), (136, 9216), (4750, 1028), (9500, 512)])
+@pytest.mark.parametrize("N,K", [(8, 4), (33, 516), (300, 3072), (112, 9216), (1000, 1028), (2040, 512), (5000, 204)])
 def test_linear_f32_kernels_and_cuts(M, N, K):
     """Streams of 8, 16 and 32 rows a block, tiles of 32 and 64 rows, cut along K and not: float sums, one order."""
     g = torch.Generator(device=DEV).manual_seed(M * N + K)
     x = torch.randn(M, K, generator=g, device=DEV)
     w = torch.randn(N, K, generator=g, device=DEV)
+    assert not kernels.linear_f32_tc_ok(w)
     out = torch.full((M, N), float("nan"), device=DEV)
     kernels.linear_f32(x, w, out)
     ref = x.double() @ w.double().T
@@ -347,9 +348,9 @@ def test_linear_f32_gated(M, F, K, activation, limit):
 
 
 def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
-    x = torch.zeros(300, 2305, device=DEV)[:, 1:]
-    w, out = torch.zeros(2304, 2304, device=DEV), torch.empty(300, 2304, device=DEV)
-    assert kernels.linear_f32_plan(300, 2304, 2304, kernels.device_sms())[1] > 0
+    x = torch.zeros(300, 3073, device=DEV)[:, 1:]
+    w, out = torch.zeros(300, 3072, device=DEV), torch.empty(300, 300, device=DEV)
+    assert not kernels.linear_f32_tc_ok(w) and kernels.linear_f32_plan(300, 300, 3072, kernels.device_sms())[1] > 0
     kernels.linear_f32(x, w, out)
     before = torch.cuda.memory_allocated()
     torch.cuda.reset_peak_memory_stats()
