@@ -312,3 +312,26 @@ def test_a_layer_launched_from_one_call_is_the_layer_launched_kernel_by_kernel(m
         got.append((logits, eng.step(slots, [[7]] * len(prompts)).clone()))
         eng.close(slots)
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and launched[0] == launched[1]
+
+
+@pytest.mark.parametrize("lengths", [[12], [30], [40], [60, 68]])
+def test_a_short_prompt_launched_layer_by_layer_is_as_close_to_64_bits(tmp_path, monkeypatch, lengths):
+    """As the dispatch is: beyond 32 tokens the products are the weight stream's where they were the library's."""
+    from brolm_b200 import kernels
+    cfg = bb.Gemma2Config(vocab_size=500, hidden_size=1024, intermediate_size=2048, num_hidden_layers=4, num_attention_heads=8,
+                          num_key_value_heads=4, head_dim=128, sliding_window=24)
+    folder = str(tmp_path / "m")
+    bb.write_random_model(cfg, folder, seed=2, dtype=torch.bfloat16, device=DEV)
+    config, weights = oracle_inputs(folder)
+    model = bb.load_model(folder, dtype="bfloat16", device=DEV)
+    prompts = random_prompts(500, lengths, seed=9)
+    ref = torch.cat([plain.forward(config, weights, p) for p in prompts])
+    errors = []
+    for at_once in (True, False):
+        monkeypatch.setattr(kernels, "PROMPT_LAYER", at_once)
+        eng = bb.Engine(model, max_tokens=1024, max_slots=4)
+        slots = eng.open(len(prompts))
+        got = eng.step(slots, prompts, want=[list(range(n)) for n in lengths])
+        errors.append(float((got.double().cpu() - ref).norm() / ref.norm()))
+        eng.close(slots)
+    assert errors[0] <= 2e-2 and errors[0] <= 1.1 * errors[1], errors

@@ -253,6 +253,25 @@ def test_linear_f32_on_tensor_cores_at_the_ends_of_the_range(M):
     assert kernels.linear_f32_tc_ok(w) and torch.equal(out, x)
 
 
+@pytest.mark.parametrize("M", [3, 20, 40, 300])
+@pytest.mark.parametrize("N,K", [(2052, 520), (20000, 260), (2304, 2304)])
+def test_linear_f32_on_tensor_cores_of_nan(M, N, K):
+    """A NaN of a token or of a row of W is in all its sums and in no other."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    before, out = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, before)
+    x[M - 1, K - 1], w[5, 0] = torch.nan, torch.nan
+    w[6, 3] = torch.inf
+    kernels.linear_f32(x, w, out)
+    nan = torch.zeros(M, N, dtype=torch.bool, device=DEV)
+    nan[M - 1], nan[:, 5] = True, True
+    assert torch.equal(out.isnan(), nan)
+    keep = torch.ones(M, N, dtype=torch.bool, device=DEV)
+    keep[M - 1], keep[:, 5:7] = False, False
+    assert torch.equal(out[keep], before[keep]) and bool(out[:-1, 6].isinf().all())
+
+
 @pytest.mark.parametrize("kind", ["normal", "positive", "spread"])
 @pytest.mark.parametrize("M,N,K", [(3, 4096, 2304), (300, 2304, 9216)])
 def test_linear_f32_on_tensor_cores_is_no_less_precise_than_fmas(kind, M, N, K):
