@@ -1,9 +1,10 @@
 // True 32-bit matrix product  Y[M,N] = X[M,K] * W[N,K]^T  on CUDA cores
 // (wlejon/brolm include/brolm/detail/compute.h:49-86, the float branch).
 //
-// For weights of up to a million numbers, and those off 16-byte boundaries (linear_f32_tc.cu takes the others; the figures
-// below for larger ones are from before).  No tensor cores and no reduced-precision mode: every product and sum is an
-// IEEE float fma.  One order of sums holds for all kernels of this file,
+// For weights of up to a million numbers, those off 16-byte boundaries, and a K below 256 (linear_f32_tc.cu takes the others).
+// The largest of them, 1,024 x 1,024, take 6.8 / 8.6 / 12.1 / 17.2 us for 1 / 3 / 8 / 16 rows and 22 / 23 / 36 / 62 for 33 / 150 /
+// 300 / 1,000; figures below at more weights than that were measured on these kernels all the same, to see what bounds them.
+// No tensor cores and no reduced-precision mode: every product and sum is an IEEE float fma.  One order of sums holds for all kernels of this file,
 // whatever M is, wherever the row stands in the batch and however the work is
 // cut:
 //
@@ -49,9 +50,7 @@ __device__ __forceinline__ Pair2 lds4(uint32_t addr) {
 // ascending order.
 // A warp's 16-byte read takes shared memory four cycles even where all lanes read one address, so with one row a lane
 // the reads of x set the pace from M = 8 on (256,000 x 2,304: 680 us at M = 8 and 987 us at M = 16, against 370 us at
-// M = 1, which is 6.4 TB/s): a lane then takes two rows for every x it reads (533 and 836 us).  At M = 3 a layer's four
-// products take 15, 14, 41 and 24 us (q/k/v, o, gate and up, down of 2,304 / 9,216); the tiles below, which served all M
-// before, took 317 us each on average.
+// M = 1, which is 6.4 TB/s): a lane then takes two rows for every x it reads (533 and 836 us).
 constexpr int PITCH = 144;                       // bytes of a pair's 32 k, with padding
 
 template <int R> __host__ __device__ constexpr int slots() { return R == 1 ? 5 : 4; }

@@ -5,8 +5,9 @@
 // its eight to nine launches (one prompt of 37 tokens: 4.35 ms, of which the device was busy for 2.0).  Here they are one
 // conversion and seven or eight launches (37 tokens: 2.42 ms).  The kernels are those of the other libraries, whose entry points
 // the caller passes: up to 16 tokens the few-token product (rotation and cache in its epilogue), beyond the weight stream, its
-// slices of K added by the kernels behind it.  Up to 32 tokens these are the launches that were made one by one; beyond, the
-// products were the library's, on the device as fast (q/k/v of 64 tokens 9.2 us with its sums for 7.0, down 12.6 for 14.6).
+// slices of K added by the kernels behind it.  Up to 32 tokens these are the launches that are made one by one otherwise; beyond,
+// the products one by one are the library's and gemm_tc's (q/k/v of 64 tokens 9.2 us here with its sums, 7.0 there; down 12.6 and
+// 14.6).  What a layer takes either way is at prompt_layer_ok in kernels/__init__.py.
 #include "common.cuh"
 
 extern "C" {

@@ -1132,7 +1132,12 @@ def linear_f32_plan(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
 
 def linear_f32_tc_slices(N: int, K: int) -> int:
     """Into how many slices of K the float32 product on tensor cores (linear_f32_tc.cu) is cut; 0: these weights are not
-    for it.  A function of the weights' size alone: every number of rows has to give a row the same bits."""
+    for it.  A function of the weights' size alone: every number of rows has to give a row the same bits.
+
+    The line lies at 2^20 numbers, from where on nearly all numbers of rows are faster there, us on fmas / on tensor cores (with
+    the slices left to the kernel behind): 1,024 x 1,024 1 row 6.8 / 5.9 (4.6), 3 rows 8.6 / 6.0 (4.7), 16 17.2 / 6.8 (5.6), 300
+    36 / 22; 2,048 x 1,024 7.3 / 6.2 (5.8), 9.3 / 6.5 (5.8), 17.7 / 7.5 (6.7), 54 / 39; 2,304 x 2,304 7.0 / 8.9 (7.9), 10.4 / 9.1
+    (8.0), 33 / 10.7 (8.9), 117 / 49.  One row of 2,000 to 4,000 columns is what pays: up to 2 us."""
     if N * K < 1 << 20 or K < 256 or N > 128 * 65535:
         return 0
     tiles, slices = -(-N // 128), 8
@@ -1496,8 +1501,8 @@ STREAM_MAX_ROWS = 128
 # 24 rows 9,598 / 9,582; 32 rows 12,708 / 12,660; 48 rows 14,076 / 14,436; 64 rows 18,676 / 19,152;
 # 96 rows 20,727 / 22,622; 128 rows 23,901 / 25,584.  With 64 and 128 token columns a stage of the ring is a
 # third and a half tokens, so fewer bytes of weights are in flight per SM; up to 32 it is at least even.
-# (Prompts of plain layers take the stream up to 128 tokens all the same: there the host sets the pace, ``prompt_layer``.)
-# BROLM_STREAM_ROWS=128 takes every product of up to 128 tokens to the own kernel, =16 none.
+# (Prompts of plain layers take the stream up to 128 tokens whatever this says: ``prompt_layer_ok`` has the figures.)
+# BROLM_STREAM_ROWS=128 takes every product of up to 128 tokens to the own kernel; =16 none, with BROLM_PROMPT_LAYER=0.
 STREAM_ROWS = int(os.environ.get("BROLM_STREAM_ROWS", "32"))
 
 
@@ -1621,7 +1626,15 @@ def _prompt_entry_points() -> list:
 def prompt_layer_ok(tokens: int, head_dim: int, group: int, inter: int, max_q_len: int, n_kv: int, window: int, batch: int,
                     *weights: torch.Tensor) -> bool:
     """Whether the launches of a layer for a prompt of so many tokens go out from one call (``prompt_layer``): at most what the
-    weight stream takes."""
+    weight stream takes.
+
+    Measured, us a layer of a whole prompt step (12 layers, the call from begin to end), at once / one by one:
+        tokens         16             32             33             64             96             128
+        2B         90 / 176       99 / 185       103 / 195      107 / 195      115 / 195      118 / 194
+        9B        135 / 179      142 / 187       145 / 195      153 / 196      164 / 195      168 / 196
+        27B       251 / 254      250 / 255       256 / 277      267 / 282      288 / 295      297 / 303
+    One by one the host sets the pace of the first two; the 27B sizes' layer is over a gigabyte, 175 us at the memory's rate,
+    and there the products of 33 and more tokens decide: the stream, or the library and gemm_tc."""
     return (0 < tokens <= STREAM_MAX_ROWS and PROMPT_LAYER and inter % 64 == 0 and group <= 16
             and attention_prefill_tc_ok(head_dim, group)
             and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights)
