@@ -15,7 +15,7 @@
 //
 // A block owns 128 rows of W (the M side of the instruction), up to NT tokens (the N side) and one slice of K.  The sums of
 // the slices are added through the shared memory of a cluster of blocks, or by the kernel behind this one.  Roles:
-//   TMA     one thread fetches W, 32 floats of every row at a time, for up to 16 tokens ahead of the kernel before it;
+//   TMA     one thread fetches W, 32 floats of every row at a time, ahead of the kernel before it where W stands;
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the three rows of parts into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
 //           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the parts in by TMA;
@@ -109,6 +109,7 @@ struct Args {
     int slice;               // k of a slice: a multiple of 64
     int x_vec;               // X's rows lie on 16-byte boundaries
     int x_stages;            // columns of x_flags
+    int w_behind;            // W may be the result of the kernel before this one
     int gated;               // W is [gate; up] of 2 N rows, a block has 64 of each, and y = act(gate) * up
     int act;
     float limit;
@@ -184,11 +185,13 @@ __device__ __forceinline__ void make_again(bool again, float& y, const float* x,
         if (lane == whose) y = sum;
     }
 }
+__device__ __forceinline__ bool far_apart(uint32_t row, uint32_t token) { return (((row & token >> 1) | (row >> 1 & token)) & SMALL) != 0; }
 __device__ __forceinline__ bool doubtful(float y, uint32_t row, uint32_t token) {
-    const float size = fabsf(y);
-    return !((row | token) & BROKEN) &&                        // (a NaN among the numbers: the sum is one)
-           (!(size <= 3.402823466e38f) || (size < 1e-20f && y != 0.0f) || (((row & token >> 1) | (row >> 1 & token)) & SMALL) ||
-            (y == 0.0f && (row & token & SOME) && ((row | token) & SMALL)));
+    const float size = fabsf(y);                               // (no branches: every sum of a block is asked)
+    const uint32_t either = row | token;
+    const bool zero = y == 0.0f && !((row & token & SOME) && (either & SMALL));       // (a true one)
+    const bool odd = !(size <= 3.402823466e38f) | ((size < 1e-20f) & !zero) | far_apart(row, token);
+    return odd & !(either & BROKEN);                           // (a NaN among the numbers: the sum is one)
 }
 constexpr uint32_t AGAIN = 0x7fc0a6a1u;            // a NaN that no sum is: the kernel that adds the slices makes this one again
 
@@ -198,6 +201,11 @@ __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
     return one != 0;
+}
+
+__device__ __noinline__ void mark_doubtful(float* sums, int ld, int c, int end, uint32_t row, const uint8_t* token_flags) {
+    for (; c < end; ++c)
+        if (doubtful(sums[(size_t)c * ld], row, token_flags[c])) sums[(size_t)c * ld] = __uint_as_float(AGAIN);
 }
 
 template <int NT, int BLOCKS>
@@ -247,8 +255,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     if (role == Role::TMA || role == Role::MMA || role == Role::FETCH_X || role == Role::NONE) {
         if constexpr (!S::FEW) fewer_registers<48>();
         if (role == Role::TMA && lane == 0) {
-            // W may be the result of the kernel before this one, unless there are at most 16 tokens (the rule of linear_f32.cu)
-            if (g.M > 16) pdl_wait();
+            if (g.w_behind) pdl_wait();
             int i = 0;
             for (; i < 2 * stages; ++i) {
                 const int s = i % S::W_SLOTS;
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float4 v = lds_float4(src[h >> 1] + ((((h & 1) * 4 + c) ^ (row & 7)) << 4));
-                    extent.add(v);
+                    if (k_lo + j * KX + h * 16 + 4 * c < g.K) extent.add(v);
                     take_apart(v.x, v.y, p0[2 * c], p1[2 * c], p2[2 * c]);
                     take_apart(v.z, v.w, p0[2 * c + 1], p1[2 * c + 1], p2[2 * c + 1]);
                 }
@@ -367,31 +374,35 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
             __syncwarp();
             if (lane == 0) mbar_arrive(ready + 8 * (j % NB));
         }
+        // Whether any of the sums can be doubtful: one of ordinary size only by numbers far apart (a zero is not of ordinary size).
         const uint32_t mine = row_flags[row] | row_flags[BR + row];
+        const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2, end = min(first + S::COLS, tokens);
+        uint32_t theirs = 0;
+        for (int c = first + lane; c < end; c += 32) theirs |= token_flags[c];
+        theirs = __reduce_or_sync(0xffffffffu, theirs);
+        bool ask = far_apart(mine, theirs);
+        const auto odd = [](float y) { return !(fabsf(y) <= 3.402823466e38f) | (fabsf(y) < 1e-20f); };
+        const bool real = w_row < (g.gated ? 2 * g.N : g.N);
         if (j == stages && g.parts && g.y) {
             // the kernel behind this one makes the doubtful sums again
-            float* dst = g.parts + ((size_t)part * g.M + m0 + first) * g.N + n0 + row;
+            float* dst = g.parts + ((size_t)part * g.M + m0) * g.N + n0 + row;
             if (n0 + row < g.N) {
 #pragma unroll
                 for (int c = 0; c < S::COLS; ++c)
-                    if (first + c < tokens) dst[(size_t)c * g.N] = doubtful(sum[c], mine, token_flags[first + c]) ? __uint_as_float(AGAIN) : sum[c];
+                    if (first + c < tokens) dst[(size_t)(first + c) * g.N] = sum[c], ask |= odd(sum[c]);
+                if (ask) mark_doubtful(dst, g.N, first, end, mine, token_flags);
             }
         } else if (j == stages) {
             // the rings are done with: all products have been made
             float* sums = reinterpret_cast<float*>(smem_raw) + row;
-            bool fine = true;
 #pragma unroll
             for (int c = 0; c < S::COLS; ++c)
-                if (first + c < tokens) {
-                    sums[(first + c) * BR] = sum[c];
-                    fine &= !doubtful(sum[c], mine, token_flags[first + c]);
-                }
-            const int w_row = row < BR / 2 ? n0 + row : second + row - BR / 2;
-            fine |= w_row >= (g.gated ? 2 * g.N : g.N);
-            if (!__all_sync(0xffffffffu, fine))
-                for (int c = first; c < min(first + S::COLS, tokens); ++c) {
+                if (first + c < tokens) sums[(first + c) * BR] = sum[c], ask |= odd(sum[c]);
+            ask &= real;
+            if (__any_sync(0xffffffffu, ask))
+                for (int c = first; c < end; ++c) {
                     float y = sums[c * BR];
-                    make_again(!fine && doubtful(y, mine, token_flags[c]), y, g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo,
+                    make_again(ask && doubtful(y, mine, token_flags[c]), y, g.x + (size_t)(m0 + c) * g.ldx, g.w + (size_t)w_row * g.ldw, k_lo,
                                min(g.K, k_lo + g.slice), lane);
                     sums[c * BR] = y;
                 }
@@ -434,7 +445,8 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 const int token = u * (T / 8) + (xt >> 3);
                 Extent extent;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) extent.add(v[u][e]);
+                for (int e = 0; e < 8; ++e)
+                    if (k_lo + j * KX + chunk * 8 + e < g.K) extent.add(v[u][e]);
                 const uint32_t flags = extent.flags_of_eight(lane);
                 if (token < wide) {
                     uint32_t p[PARTS][4];
@@ -584,8 +596,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(Args g, uint16_t* __res
     Extent extent;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {                             // (X's rows lie on 16-byte boundaries)
-        v[h] = there && k + 4 * h < g.K ? *reinterpret_cast<const float4*>(p + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        extent.add(v[h]);
+        const bool here = there && k + 4 * h < g.K;
+        v[h] = here ? *reinterpret_cast<const float4*>(p + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (here) extent.add(v[h]);
     }
     const uint32_t all = extent.flags_of_eight(threadIdx.x & 31);
     if (!there) return;
@@ -615,14 +628,16 @@ __global__ void __launch_bounds__(256) add_slices_kernel(Args g, int slices) {
         for (int s = 0; s < 8; ++s) v[s] = s < slices ? g.parts[s * total + idx] : 0.0f;
 #pragma unroll
         for (int s = 0; s < 8; ++s) fine &= __float_as_uint(v[s]) != AGAIN;
-        if (!__all_sync(0xffffffffu, fine))
-#pragma unroll
-            for (int s = 0; s < 8; ++s)
-                make_again(there && __float_as_uint(v[s]) == AGAIN, v[s], g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice), lane);
         float y = v[0];
 #pragma unroll
         for (int s = 1; s < 8; ++s)
             if (s < slices) y += v[s];
+        if (!__all_sync(0xffffffffu, fine))
+            for (int s = 0; s < slices; ++s) {
+                float t = g.parts[s * total + idx];
+                make_again(there && __float_as_uint(t) == AGAIN, t, g.x + token * g.ldx, g.w + n * g.ldw, s * g.slice, min(g.K, (s + 1) * g.slice), lane);
+                y = s ? y + t : t;
+            }
         if (there) g.y[token * g.ldy + n] = y;
     }
 }
@@ -657,9 +672,9 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, dim3 gri
 // act(X Wg^T) * (X Wu^T) for W = [Wg; Wu] of 2 N rows.  W's rows lie on 16-byte boundaries, K is a multiple of 4; X's rows
 // may lie anywhere.  parts: room for slices * M * N floats, with which a second kernel adds the slices (y null: the caller's does); null: clusters do.
 // split: room for X taken apart ahead (more than 32 rows on 16-byte boundaries), 16-byte aligned, M * ceil(K / 64) * 385 bytes;
-// null: every block does it.
+// null: every block does it.  w_behind: W may be the result of a kernel that is still running when this one is let in.
 BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K,
-                                  int slices, int slice, int gated, int act, float limit, void* parts, void* split, cudaStream_t stream) {
+                                  int slices, int slice, int gated, int act, float limit, int w_behind, void* parts, void* split, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return BROLM_OK;
     if (K <= 0 || K % 4 || ldw % 4 || ((uintptr_t)w & 15)) return BROLM_ERR_ALIGNMENT;
     if (slices < 1 || slices > 8 || slice < 64 || slice % 64 || (long long)(slices - 1) * slice >= K || (long long)slices * slice < K) return BROLM_ERR_BAD_SIZE;
@@ -684,6 +699,7 @@ BROLM_API int brolm_linear_f32_tc(const void* x, int ldx, const void* w, int ldw
     g.M = M; g.N = N; g.K = K;
     g.tokens = ((M + tiles - 1) / tiles + 15) / 16 * 16;
     g.slice = slice;
+    g.w_behind = w_behind;
     g.gated = gated; g.act = act; g.limit = limit;
     g.x_vec = ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
     g.x_flags = nullptr;

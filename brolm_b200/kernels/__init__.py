@@ -1166,13 +1166,13 @@ def linear_f32_parts(x: torch.Tensor, weight: torch.Tensor) -> int:
     return max(1, linear_f32_tc_slices(*weight.shape)) if x.shape[0] <= 32 and linear_f32_tc_ok(weight) else 1
 
 
-def linear_f32_slices_into(x: torch.Tensor, weight: torch.Tensor, sums: torch.Tensor) -> None:
+def linear_f32_slices_into(x: torch.Tensor, weight: torch.Tensor, sums: torch.Tensor, standing: bool = False) -> None:
     """sums (slices, M, N) float32: their sum in order is ``linear_f32``, bit by bit."""
     (M, K), N = x.shape, weight.shape[0]
     assert x.dtype == torch.float32 and weight.dtype == torch.float32 and sums.dtype == torch.float32 and sums.is_contiguous()
     assert x.dim() == 2 and x.stride(1) == 1 and weight.shape[1] == K
     assert tuple(sums.shape) == (linear_f32_parts(x, weight), M, N) and sums.shape[0] > 1
-    _linear_f32_tc(x, weight, None, sums.shape[0], parts=sums)
+    _linear_f32_tc(x, weight, None, sums.shape[0], parts=sums, standing=standing)
 
 
 def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
@@ -1183,10 +1183,10 @@ def linear_f32_tc_ok(weight: torch.Tensor) -> bool:
     return not (K % 4 or weight.stride(0) % 4 or weight.data_ptr() % 16) and weight.stride(1) == 1 and linear_f32_tc_slices(N, K) > 0
 
 
-def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
+def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, standing: bool = False) -> None:
     """out (M, N) = x (M, K) @ weight (N, K)^T, all float32, rows may be strided.  A row's bits depend on neither M
-    nor its place among the rows.  Up to 16 rows, the weights are read ahead of the kernel before this one on the stream: they
-    must not be its result."""
+    nor its place among the rows.  Up to 16 rows, and with ``standing`` weights, those are read ahead of the kernels before this
+    one on the stream: they must not be the result of one of this library's that may still be running."""
     assert x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32
     assert x.dim() == 2 and weight.dim() == 2 and out.dim() == 2
     assert x.stride(1) == 1 and weight.stride(1) == 1 and out.stride(1) == 1
@@ -1194,14 +1194,15 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None
     N = weight.shape[0]
     assert weight.shape[1] == K and tuple(out.shape) == (M, N)
     if linear_f32_tc_ok(weight) and M <= 160 * 65535:
-        _linear_f32_tc(x, weight, out, linear_f32_tc_slices(N, K))
+        _linear_f32_tc(x, weight, out, linear_f32_tc_slices(N, K), standing=standing)
         return
     aligned = not (K % 4 or x.stride(0) % 4 or weight.stride(0) % 4 or x.data_ptr() % 16 or weight.data_ptr() % 16)
     kind, cut = linear_f32_plan(M, N, K, device_sms(x.device)) if aligned else (0, 0)
     _linear_f32(x, weight, out, kind, cut)
 
 
-def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, activation: str, limit: float = 0.0) -> None:
+def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, activation: str, limit: float = 0.0,
+                     standing: bool = False) -> None:
     """out (M, F) = act(x @ gate^T) * (x @ up^T) for weight = [gate; up] (2 F, K), all float32: the bits of ``linear_f32``
     and ``gated_act`` behind it, where ``linear_f32_tc_ok``."""
     assert x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32
@@ -1209,11 +1210,11 @@ def linear_f32_gated(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, a
     assert weight.shape == (2 * out.shape[1], x.shape[1]) and x.shape[0] == out.shape[0]
     if activation not in ACTIVATIONS:
         raise KernelError(f"linear_f32_gated: unknown activation '{activation}' (known: {sorted(ACTIVATIONS)})")
-    _linear_f32_tc(x, weight, out, linear_f32_tc_slices(*weight.shape), True, ACTIVATIONS[activation], limit)
+    _linear_f32_tc(x, weight, out, linear_f32_tc_slices(*weight.shape), True, ACTIVATIONS[activation], limit, standing=standing)
 
 
 def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], slices: int, gated: bool = False, act: int = 0,
-                   limit: float = 0.0, parts: Optional[torch.Tensor] = None) -> None:
+                   limit: float = 0.0, parts: Optional[torch.Tensor] = None, standing: bool = False) -> None:
     (M, K), N = x.shape, out.shape[1] if out is not None else parts.shape[2]
     split = None
     aligned = not (x.stride(0) % 4 or x.data_ptr() % 16)
@@ -1224,9 +1225,9 @@ def _linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Te
         if size <= F32_PARTS_LIMIT:
             split = torch.empty(size, dtype=torch.uint8, device=x.device)
     f = _fn("linear_f32_tc", "brolm_linear_f32_tc", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
-                                                     c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p])
+                                                     c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(out), out.stride(0) if out is not None else N, M, N, K, slices,
-             _f32_tc_slice(K, slices), int(gated), act, limit, _ptr(parts), _ptr(split), _stream()), "linear_f32_tc")
+             _f32_tc_slice(K, slices), int(gated), act, limit, int(M > 16 and not standing), _ptr(parts), _ptr(split), _stream()), "linear_f32_tc")
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, kind: int, cut: int) -> None:

@@ -42,7 +42,7 @@ class GatedFeedForward(Part):
         act = torch.empty((x.shape[0], self.inter), dtype=ctx.dtype, device=x.device)
         if ctx.dtype == torch.float32 and kernels.linear_f32_tc_ok(self.w_gate_up) and x.dtype == self.w_gate_up.dtype == torch.float32:
             # float: the activation is the product's last step
-            kernels.linear_f32_gated(x, self.w_gate_up, act, self.activation, self.limit)
+            kernels.linear_f32_gated(x, self.w_gate_up, act, self.activation, self.limit, standing=True)
             return linear(act, self.w_down, out_dtype=torch.float32, parts_ok=True)
         few = kernels.skinny_ok(x, self.w_gate_up)
         stream = kernels.stream_rows(x, self.w_gate_up) or (few and kernels.stream_instead_of_skinny(x, self.w_gate_up))

@@ -30,7 +30,9 @@ from .. import kernels
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            out: Optional[torch.Tensor] = None, parts_ok: bool = False) -> torch.Tensor:
-    """``parts_ok``: the caller adds partial sums itself (the residual kernel
+    """x (tokens, K) -> (tokens, N) for ``weight`` (N, K), a parameter: the kernels may read it ahead of what runs before them.
+
+    ``parts_ok``: the caller adds partial sums itself (the residual kernel
     does); the result may then be [parts, M, N] float32, the slices of a
     product that was cut along K so that more blocks stream the weights."""
     M = x.shape[0]
@@ -41,11 +43,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
         parts = kernels.linear_f32_parts(x32, weight) if parts_ok and M <= 32 and want == torch.float32 and out is None else 1
         if parts > 1:
             y = torch.empty((parts, M, N), dtype=torch.float32, device=x.device)
-            kernels.linear_f32_slices_into(x32, weight, y)
+            kernels.linear_f32_slices_into(x32, weight, y, standing=True)
             return y
         y = out if (out is not None and out.dtype == torch.float32) else \
             torch.empty((M, N), dtype=torch.float32, device=x.device)
-        kernels.linear_f32(x32, weight, y)
+        kernels.linear_f32(x32, weight, y, standing=True)
         if want != torch.float32:
             y = y.to(want)
             if out is not None:

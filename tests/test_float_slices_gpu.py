@@ -80,7 +80,7 @@ def test_slices_left_to_the_kernel_behind_give_the_bits_of_those_added_first(mon
     follow = torch.randint(0, 300, (4, 3), generator=g).tolist()
     sliced = []
     real = kernels.linear_f32_slices_into
-    monkeypatch.setattr(kernels, "linear_f32_slices_into", lambda *a: sliced.append(1) or real(*a))
+    monkeypatch.setattr(kernels, "linear_f32_slices_into", lambda *a, **kw: sliced.append(1) or real(*a, **kw))
 
     def run():
         eng = bb.Engine(model, max_tokens=512, max_slots=3)

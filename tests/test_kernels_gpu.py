@@ -305,6 +305,8 @@ def test_linear_f32_of_weights_that_the_kernel_before_it_made():
             kernels.cast(made, w)
             kernels.linear_f32(x, w, out)
             assert torch.equal(out, want)
+            kernels.linear_f32(x, w, out, standing=True)
+            assert torch.equal(out, want)
 
 
 def test_linear_f32_on_tensor_cores_of_infinities_and_the_smallest_numbers():
