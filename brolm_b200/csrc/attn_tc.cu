@@ -473,7 +473,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
                 } else {
                     own = theirs = 0.0f;
                 }
-                sum_all = total * own + l_o * theirs;
+                // the first half's share is rounded, the second's added by an fma, whichever of them merges
+                sum_all = part == 0 ? fmaf(l_o, theirs, total * own) : fmaf(total, own, l_o * theirs);
                 their_o = reinterpret_cast<const float4*>(a.part_o) + (size_t)(pair * 2 + (part ^ 1)) * (HD / 4) * BM + r;
             }
         }
@@ -504,11 +505,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_tc_kernel(const __gri
                         const float4 t0 = th[i / 4], t1 = th[i / 4 + 1];
                         float f[8];
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(ov[i + e]) * k_own;
-                        f[0] = fmaf(t0.x, k_theirs, f[0]); f[1] = fmaf(t0.y, k_theirs, f[1]);
-                        f[2] = fmaf(t0.z, k_theirs, f[2]); f[3] = fmaf(t0.w, k_theirs, f[3]);
-                        f[4] = fmaf(t1.x, k_theirs, f[4]); f[5] = fmaf(t1.y, k_theirs, f[5]);
-                        f[6] = fmaf(t1.z, k_theirs, f[6]); f[7] = fmaf(t1.w, k_theirs, f[7]);
+                        for (int e = 0; e < 8; ++e) {
+                            const float t = e < 4 ? (&t0.x)[e] : (&t1.x)[e - 4];
+                            const float o = __uint_as_float(ov[i + e]);
+                            f[e] = part <= 0 ? fmaf(t, k_theirs, o * k_own) : fmaf(o, k_own, t * k_theirs);
+                        }
                         uint4 pk;
                         __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll

@@ -368,6 +368,25 @@ def test_linear_f32_gated(M, F, K, activation, limit):
     assert torch.equal(out.nan_to_num(7.0), want.nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("T,n_kv", [(1280, 4), (2048, 4)])
+def test_prompt_attention_cut_in_halves_repeats_itself(T, n_kv):
+    """Which half of a row block comes second and merges is a matter of time; the bits are not."""
+    group, hd = 2, 256
+    assert kernels.attention_prefill_tc_split(T, n_kv, group, 0, 1) > 0
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(T, (n_kv * group + 2 * n_kv) * hd, generator=g, device=DEV).to(torch.bfloat16)
+    cu, q = torch.tensor([0, T], dtype=torch.int32, device=DEV), n_kv * group * hd
+    noise = torch.empty(64 << 20, device=DEV)
+    outs = []
+    for i in range(24):
+        if i % 2:
+            noise.normal_()                                   # (other blocks on the SMs as the launch begins)
+        outs.append(torch.empty(T, q, dtype=torch.bfloat16, device=DEV))
+        kernels.attention_prefill_tc(qkv[:, :q], outs[-1], cu, qkv[:, q:q + n_kv * hd], qkv[:, q + n_kv * hd:], n_kv=n_kv, group=group,
+                                     head_dim=hd, scale=hd ** -0.5, cap=50.0, window=0, batch=1, max_q_len=T)
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
 def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
     x = torch.zeros(300, 3073, device=DEV)[:, 1:]
     w, out = torch.zeros(300, 3072, device=DEV), torch.empty(300, 300, device=DEV)
