@@ -206,7 +206,8 @@ class Engine:
             weakref.finalize(self, kernels.give_stream, index, self.beside)
         self.last_h2d_bytes = 0          # bytes the last step copied from the host
         self._checked_at = -1            # this library's launches when the kernels' status words were last read
-        self._ran_on: Optional[torch.cuda.Stream] = None      # the stream of the last step
+        self._done: Optional[torch.cuda.Event] = None         # behind the last step, if it ran on a stream that is not the default
+        self._on_default = True
         self._pin: Optional[torch.Tensor] = None      # pinned staging buffer of the steps that are not captured
         self._pin_copied = None
 
@@ -227,12 +228,12 @@ class Engine:
     def _check_waits(self, where: str, consequence: str) -> None:
         """Raise if a bounded wait inside one of the tcgen05 kernels ran out since the last check.
         Reads and resets every status word, behind the last step: the words are read on the default stream,
-        which waits for no other, so the step's own is waited for first."""
+        which waits for no other, so a step on one of those is waited for first."""
         launched = kernels.launch_count()
         if self.device.type != "cuda" or self._checked_at == launched:
             return                       # (nothing of this library has run since: a prompt is checked at its step's end)
-        if self._ran_on is not None:
-            self._ran_on.synchronize()
+        if not self._on_default:
+            self._done.synchronize()
         codes = {"linear_f32_tc": kernels.linear_f32_tc_status(reset=True)}
         if self.model.dtype == torch.bfloat16:
             codes |= {"gemm_tc": kernels.gemm_tc_status(reset=True), "attn_tc": kernels.attention_tc_status(reset=True),
@@ -244,9 +245,15 @@ class Engine:
             raise StepError(f"{where}: a wait inside a tensor-core kernel ran out ({bad}), in this step or in a "
                             f"decode step since the last check; {consequence}")
 
-    def _note_stream(self) -> None:
-        if self.device.type == "cuda":
-            self._ran_on = torch.cuda.current_stream(self.device)
+    def _mark_end(self) -> None:
+        """What ``_check_waits`` waits for (an event: a caller's stream may be gone by then)."""
+        if self.device.type != "cuda":
+            return
+        stream = torch.cuda.current_stream(self.device)
+        self._on_default = stream.cuda_stream == 0
+        if not self._on_default:
+            self._done = self._done or torch.cuda.Event()
+            self._done.record(stream)
 
     # the step -------------------------------------------------------------
     def step(self, slots: Sequence[int], tokens: Sequence[Sequence[int]],
@@ -263,7 +270,6 @@ class Engine:
         (wlejon/brolm's ``hidden_out``, include/brolm/gemma2.h:121-125).
         """
         plan = self._plan(slots, tokens, want)
-        self._note_stream()
         if plan.mode == "decode" and self.use_graphs:
             graph = self._graph_for(plan)
             logits = graph.run(plan, self.cache)
@@ -278,8 +284,9 @@ class Engine:
             ctx, tok_dev, rows = self._context(plan)
             logits = self.model.forward(ctx, tok_dev, rows)
             rows_h = self.model.last_hidden
-            if plan.mode == "prefill":
-                self._check_waits("step", "the results of this step are not valid")
+        self._mark_end()
+        if plan.mode == "prefill":
+            self._check_waits("step", "the results of this step are not valid")
         self.cache.commit(dict(zip(plan.slots, plan.new_len)))
         return (logits, rows_h) if hidden else logits
 
@@ -295,7 +302,6 @@ class Engine:
         plan = self._plan(slots, [[0]] * len(slots), None)
         if plan.mode != "decode":
             raise StepError("step_from: only sequences that already hold tokens can go on")
-        self._note_stream()
         if self.use_graphs:
             graph = self._graph_for(plan)
             logits = graph.run(plan, self.cache, ids, [int(p) for p in pick])[:len(plan.slots)]
@@ -304,6 +310,7 @@ class Engine:
             ctx, _, rows = self._context(plan)
             tokens = ids.index_select(0, torch.tensor([int(p) for p in pick], dtype=torch.int32, device=self.device))
             logits = self.model.forward(ctx, tokens, rows)
+        self._mark_end()
         self.cache.commit(dict(zip(plan.slots, plan.new_len)))
         return logits
 
