@@ -26,13 +26,14 @@
 // For W = [gate; up] a block has 64 rows of each, and stores act(gate) * up.
 //
 // Bound: up to 32 tokens by the memory and by the start and end of short slices, beyond by the warps that split and add (a
-// stage of 64 k with 150 tokens takes 1.7 us, of which the products are 0.9).  us, the kernels of linear_f32.cu / here:
+// stage of 64 k with 150 tokens takes 1.6 us, of which the products are 0.9: there is room for two stages of X and of W's parts,
+// so each waits for the products two back, and then for its own X and W).  us, the kernels of linear_f32.cu / here:
 //     tokens                     3              16              150             300             1,000
-//     4,096 x 2,304         11.3 / 12.7     25.3 / 13.5     91.4 / 34.2     150 / 60.6      446 / 197
-//     2,304 x 2,048          9.6 / 10.2     18.5 / 11.0     54.0 / 25.4    87.4 / 46.2      220 / 195
-//     18,432 x 2,304        37.7 / 30.9     53.3 / 31.9      358 / 70.7     592 / 134     1,847 / 419
-//     2,304 x 9,216         23.8 / 33.1     44.6 / 33.2      182 / 48.3     298 / 90.2      978 / 359
-// (a decode step leaves the slices of the second and the fourth to the kernel behind them: 3 tokens 7.6 and 19.5).  The error
+//     4,096 x 2,304         11.3 / 12.2     25.3 / 12.3     91.4 / 28.7     150 / 48.1      446 / 155
+//     2,304 x 2,048          9.6 / 8.8      18.5 / 9.3      54.0 / 20.2    87.4 / 35.6      220 / 141
+//     18,432 x 2,304        37.7 / 30.6     53.3 / 30.9      358 / 67.3     592 / 128     1,847 / 400
+//     2,304 x 9,216         23.8 / 20.2     44.6 / 21.1      182 / 43.5     298 / 78.0      978 / 309
+// (a decode step leaves the slices of the second and the fourth to the kernel behind them: 3 tokens 7.4 and 17.6).  The error
 // against 64 bits, as a share of the result's norm: 2.8 to 3.0e-7 there, 1.0 to 1.4e-7 here for normal numbers; 0.7 to 1.2e-7 and
 // 0.9 to 1.2e-7 for sums of one sign, which lose half a last place at each step of the tensor core and none on average to fmas.
 //
@@ -40,9 +41,10 @@
 // by fmas.  Doubtful are (see doubtful())
 //   a sum that is not finite: an infinity among the operands ends as a NaN here, infinity minus infinity (a NaN among them
 //   is a NaN in any case, and stays);
-//   a sum below 1e-20: the products of low parts end at 2^-126;
-//   a sum with a number below 2^-60 on one side and one of 2^17 or more on the other: numbers below 2^-102 lose their low
-//   parts, up to 2^-125 of each; times less than 2^17 that is far below the last place of a sum of 1e-20;
+//   a sum below 1e-16: the products of low parts end at 2^-126;
+//   a sum with a number below 2^-60 (or a zero, which is not told from it) on one side and one of 2^32 or more on the other:
+//   numbers below 2^-102 lose their low parts, up to 2^-125 of each; times less than 2^32 and 2^15 such terms that is below the
+//   last place of a sum of 1e-16;
 //   a zero, where a side has numbers below 2^-60 (or zeros) and neither has zeros alone.
 #include "tcgen05.cuh"
 
@@ -125,7 +127,7 @@ struct Extent {
     }
     __device__ __forceinline__ void add(const float4& v) { add(v.x), add(v.y), add(v.z), add(v.w); }
     __device__ __forceinline__ uint32_t flags() const {
-        return (low < 8.67361738e-19f ? SMALL : 0) | (high >= 131072.0f ? BIG : 0) | (high > 0.0f ? SOME : 0) |
+        return (low < 8.67361738e-19f ? SMALL : 0) | (high >= 4.294967296e9f ? BIG : 0) | (high > 0.0f ? SOME : 0) |
                (high != high ? BROKEN : 0);
     }
     // of the eight lanes that share a row's 64 k
@@ -135,6 +137,21 @@ struct Extent {
 #pragma unroll
         for (uint32_t bit = SMALL; bit <= BROKEN; bit <<= 1) all |= __ballot_sync(0xffffffffu, mine & bit) & eight ? bit : 0;
         return all;
+    }
+};
+// The same of first parts, two at a time: one instruction a number where that of the floats takes two (few tokens, whose pace
+// the warps that split set beside the memory: 3 of 18,432 x 2,304 30.5 us for 32.0).
+struct PairExtent {
+    uint32_t low = 0x7f807f80u, high = 0;
+    __device__ __forceinline__ void add(uint32_t p) {
+        asm("min.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(low) : "r"(p));
+        asm("max.NaN.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(high) : "r"(p));
+    }
+    __device__ __forceinline__ uint32_t flags() const {
+        Extent e;
+        e.add(__uint_as_float(high << 16)), e.add(__uint_as_float(high & 0xffff0000u));
+        e.low = fminf(fabsf(__uint_as_float(low << 16)), fabsf(__uint_as_float(low & 0xffff0000u)));
+        return e.flags();
     }
 };
 // Two neighbours along k, taken apart.
@@ -160,7 +177,7 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 // A sum from the floats themselves, by a whole warp: a lane's chain of fmas over every 32nd four k, then the lanes' sums in pairs.
-// A token with an infinity is doubtful in all its sums (18,432 x 2,304, 3 tokens: 158 us with one such token, 256 where a thread
+// A token with an infinity is doubtful in all its sums (18,432 x 2,304, 3 tokens: 160 us with one such token, 256 where a thread
 // makes a sum).
 __device__ __noinline__ float plain_dot(const float* x, const float* w, int k, int end, int lane) {
     float y = 0.0f;
@@ -190,7 +207,7 @@ __device__ __forceinline__ bool doubtful(float y, uint32_t row, uint32_t token) 
     const float size = fabsf(y);                               // (no branches: every sum of a block is asked)
     const uint32_t either = row | token;
     const bool zero = y == 0.0f && !((row & token & SOME) && (either & SMALL));       // (a true one)
-    const bool odd = !(size <= 3.402823466e38f) | ((size < 1e-20f) & !zero) | far_apart(row, token);
+    const bool odd = !(size <= 3.402823466e38f) | ((size < 1e-16f) & !zero) | far_apart(row, token);
     return odd & !(either & BROKEN);                           // (a NaN among the numbers: the sum is one)
 }
 constexpr uint32_t AGAIN = 0x7fc0a6a1u;            // a NaN that no sum is: the kernel that adds the slices makes this one again
@@ -312,7 +329,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     } else if (role == Role::SPLIT) {
         if constexpr (!S::FEW) fewer_registers<48>();
         const int row = (warp & 3) * 32 + lane;
-        Extent extent;
+        PairExtent extent;
         for (int j = index >> 2; j < stages; j += 2) {         // two sets of four warps take turns
             const int s0 = 2 * j % S::W_SLOTS, s1 = (2 * j + 1) % S::W_SLOTS;
             // A wait on a slot's phase asks that the phase before it is known to be over: it was at least NB stages back.
@@ -329,9 +346,9 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float4 v = lds_float4(src[h >> 1] + ((((h & 1) * 4 + c) ^ (row & 7)) << 4));
-                    if (k_lo + j * KX + h * 16 + 4 * c < g.K) extent.add(v);
                     take_apart(v.x, v.y, p0[2 * c], p1[2 * c], p2[2 * c]);
                     take_apart(v.z, v.w, p0[2 * c + 1], p1[2 * c + 1], p2[2 * c + 1]);
+                    extent.add(p0[2 * c]), extent.add(p0[2 * c + 1]);
                 }
                 tmem_st8(a + 8 * h, p0);
                 tmem_st8(a + A_PLANE + 8 * h, p1);
@@ -381,7 +398,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
         for (int c = first + lane; c < end; c += 32) theirs |= token_flags[c];
         theirs = __reduce_or_sync(0xffffffffu, theirs);
         bool ask = far_apart(mine, theirs);
-        const auto odd = [](float y) { return !(fabsf(y) <= 3.402823466e38f) | (fabsf(y) < 1e-20f); };
+        const auto odd = [](float y) { return !(fabsf(y) <= 3.402823466e38f) | (fabsf(y) < 1e-16f); };
         const bool real = w_row < (g.gated ? 2 * g.N : g.N);
         if (j == stages && g.parts && g.y) {
             // the kernel behind this one makes the doubtful sums again
@@ -445,8 +462,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
                 const int token = u * (T / 8) + (xt >> 3);
                 Extent extent;
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (k_lo + j * KX + chunk * 8 + e < g.K) extent.add(v[u][e]);
+                for (int e = 0; e < 8; ++e) extent.add(v[u][e]);
                 const uint32_t flags = extent.flags_of_eight(lane);
                 if (token < wide) {
                     uint32_t p[PARTS][4];
@@ -598,7 +614,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(Args g, uint16_t* __res
     for (int h = 0; h < 2; ++h) {                             // (X's rows lie on 16-byte boundaries)
         const bool here = there && k + 4 * h < g.K;
         v[h] = here ? *reinterpret_cast<const float4*>(p + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (here) extent.add(v[h]);
+        extent.add(v[h]);
     }
     const uint32_t all = extent.flags_of_eight(threadIdx.x & 31);
     if (!there) return;

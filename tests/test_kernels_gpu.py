@@ -253,6 +253,24 @@ def test_linear_f32_on_tensor_cores_at_the_ends_of_the_range(M):
     assert kernels.linear_f32_tc_ok(w) and torch.equal(out, x)
 
 
+@pytest.mark.parametrize("M,off", [(3, 0), (20, 1), (40, 0), (40, 1), (200, 0)])
+@pytest.mark.parametrize("low,high,zeros", [(-120, 60, 0.0), (-126, -20, 0.2), (-60, 58, 0.2), (20, 58, 0.0), (-110, -50, 0.9)])
+def test_linear_f32_on_tensor_cores_of_numbers_of_all_sizes(M, off, low, high, zeros):
+    """Every number with an exponent of its own, some of them zeros (up to 2^60: products of 2^126 would run over)."""
+    N, K = 2052, 520
+    g = torch.Generator(device=DEV).manual_seed(M + off - low)
+
+    def draw(*shape):
+        t = torch.randn(*shape, generator=g, device=DEV) * torch.exp2(torch.empty(*shape, device=DEV).uniform_(low, high, generator=g))
+        t[torch.rand(*shape, generator=g, device=DEV) < zeros] = 0.0
+        return t
+    x, w = draw(M, K + off)[:, off:], draw(N, K)
+    out = torch.empty(M, N, device=DEV)
+    kernels.linear_f32(x, w, out)
+    error = (out.double() - x.double() @ w.double().T).abs()
+    assert bool((error <= tc_f32_bound(K) * (x.abs().double() @ w.abs().double().T) + K * 2.0 ** -149).all())
+
+
 @pytest.mark.parametrize("M", [3, 20, 40, 300])
 @pytest.mark.parametrize("N,K", [(2052, 520), (20000, 260), (2304, 2304)])
 def test_linear_f32_on_tensor_cores_of_nan(M, N, K):
