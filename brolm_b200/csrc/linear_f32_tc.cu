@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(Shape<NT, BLOCKS>::THREADS, BLOCKS) linear_f32
     fence_after_sync();
     const uint32_t tmem = *tmem_slot, tmem_a = tmem + NB * NT;
 
-    auto wait_on = [&](uint32_t bar, uint32_t parity, int code) { return mbar_wait(bar, parity, give_up, &g_linear_f32_tc_error, code); };
+    auto wait_on = [&](uint32_t bar, uint32_t parity, int code) { return mbar_wait<2>(bar, parity, give_up, &g_linear_f32_tc_error, code); };
     auto all_wait_on = [&](uint32_t bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, wait_on(bar, parity, code)) != 0; };
 
     int index = 0;

@@ -64,13 +64,15 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // another role of the block had already given up.  give_up: three ints in shared memory that the
 // kernel sets when it starts: [0] the block's give-up flag, [1] that of the drain waits, [2] g_stall_code.
 // `flags`: the three ints; `drain`: one of the waits that let loads in flight land after the block gave up
-// (they watch flags[1] and are never stalled).
+// (they watch flags[1] and are never stalled).  SOONER: a stalled wait has that part of the limit, for kernels where
+// others begin to wait at the same moment.  (A division here for all of them, which is 1, cost a layer of a short prompt 1.4 us.)
+template <int SOONER = 1>
 __device__ inline bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* flags, int* error, int code,
                                  bool drain = false) {
     volatile int* give_up = flags + (drain ? 1 : 0);
     const bool stalled = !drain && flags[2] == code;          // (0 in every ordinary launch)
     if (!stalled && mbar_try(bar, parity)) return true;       // (try_wait itself may hold the thread for a while)
-    const long long t0 = clock64(), limit = stalled ? g_wait_cycles / 2 : g_wait_cycles;      // (the stalled one is the first to give up)
+    const long long t0 = clock64(), limit = SOONER > 1 && stalled ? g_wait_cycles / SOONER : g_wait_cycles;
     while (true) {
         if (!stalled && mbar_try(bar, parity)) return true;
         if (*give_up) return false;
