@@ -19,7 +19,7 @@
 //   SPLIT   a lane takes 64 k of a row of W apart and puts the three rows of parts into tensor memory (the A operand);
 //   X       these do the same for the tokens, into shared memory (the B operand).  Many tokens are taken apart once, by a
 //           kernel ahead of this one, instead of by every block; then FETCH_X, one thread, brings the parts in by TMA;
-//   MMA     one lane issues 24 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two accumulators;
+//   MMA     one lane issues 24 tcgen05.mma for 64 k (M 128, N tokens, K 16) into one of two or four accumulators;
 //   ADD     these add an accumulator to the sums in their registers, and at the end store them.
 // The thread that issues is what all wait for, so its stage of 64 k has one barrier to wait on, which all that its products
 // need arrive at (A, the tokens, the emptied accumulator), and one commit, which frees all of it.

@@ -1135,9 +1135,9 @@ def linear_f32_tc_slices(N: int, K: int) -> int:
     for it.  A function of the weights' size alone: every number of rows has to give a row the same bits.
 
     The line lies at 2^20 numbers, from where on nearly all numbers of rows are faster there, us on fmas / on tensor cores (with
-    the slices left to the kernel behind): 1,024 x 1,024 1 row 6.8 / 5.9 (4.6), 3 rows 8.6 / 6.0 (4.7), 16 17.2 / 6.8 (5.6), 300
-    36 / 22; 2,048 x 1,024 7.3 / 6.2 (5.8), 9.3 / 6.5 (5.8), 17.7 / 7.5 (6.7), 54 / 39; 2,304 x 2,304 7.0 / 8.9 (7.9), 10.4 / 9.1
-    (8.0), 33 / 10.7 (8.9), 117 / 49.  One row of 2,000 to 4,000 columns is what pays: up to 2 us."""
+    the slices left to the kernel behind): 1,024 x 1,024 1 row 6.8 / 6.3 (4.5), 3 rows 8.6 / 6.3 (4.4), 16 17.2 / 6.4 (4.5), 300
+    36 / 16; 2,048 x 1,024 7.3 / 6.9 (5.5), 9.3 / 7.0 (5.5), 17.7 / 7.1 (5.6), 54 / 30; 2,304 x 2,304 7.0 / 8.7 (7.8), 10.4 / 8.7
+    (7.8), 33 / 9.9 (7.9), 117 / 38.  One row of 2,000 to 4,000 columns is what pays: up to 2 us."""
     if N * K < 1 << 20 or K < 256 or N > 128 * 65535:
         return 0
     tiles, slices = -(-N // 128), 8
@@ -1155,7 +1155,7 @@ def linear_f32_tc_scratch(M: int, N: int, slices: int) -> bool:
     than 32 rows a block has an SM to itself, and only about sixteen clusters of eight such blocks find room at a time.
     Many clusters fill their rounds all the same; then, and where the sums would take more than 256 MB, there is no scratch.
     Up to 32 rows those sixteen clusters are the line (3 rows, scratch / clusters: 2,304 x 9,216 20.2 / 33.1 us, 2,304 x 2,304
-    9.1 / 11.5, 2,304 x 2,048 9.3 / 10.2)."""
+    8.7 / 11.5, 2,304 x 2,048 8.8 / 10.2)."""
     tiles = -(-M // 160) * -(-N // 128)
     return (tiles < 64 if M > 32 else tiles * slices > 128) and slices * M * N * 4 <= F32_PARTS_LIMIT
 
