@@ -131,13 +131,12 @@ def test_linear_f32(M, N, K):
 
 
 @pytest.mark.parametrize("M", [1, 2, 5, 16, 17, 33, 70])
-@pytest.mark.parametrize("N,K", [(8, 4), (33, 516), (300, 3072), (112, 9216), (1000, 1028), (2040, 512), (5000, 204)])
+@pytest.mark.parametrize("N,K", [(8, 4), (33, 516), (2304, 2304), (136, 9216), (4750, 1028), (9500, 512)])
 def test_linear_f32_kernels_and_cuts(M, N, K):
     """Streams of 8, 16 and 32 rows a block, tiles of 32 and 64 rows, cut along K and not: float sums, one order."""
     g = torch.Generator(device=DEV).manual_seed(M * N + K)
     x = torch.randn(M, K, generator=g, device=DEV)
     w = torch.randn(N, K, generator=g, device=DEV)
-    assert not kernels.linear_f32_tc_ok(w)
     out = torch.full((M, N), float("nan"), device=DEV)
     kernels.linear_f32(x, w, out)
     ref = x.double() @ w.double().T
@@ -155,6 +154,14 @@ def test_linear_f32_kernels_and_cuts(M, N, K):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("M", [1, 2, 5, 16, 17, 33, 70])
+@pytest.mark.parametrize("N,K", [(300, 3072), (112, 9216), (1000, 1028), (2040, 512), (5000, 204)])
+def test_linear_f32_kernels_and_cuts_of_weights_for_cuda_cores(M, N, K):
+    """The same of weights that are all too small for tensor cores."""
+    assert not kernels.linear_f32_tc_ok(torch.empty(N, K, device=DEV))
+    test_linear_f32_kernels_and_cuts(M, N, K)
+
+
 @pytest.mark.parametrize("M", [1, 8, 16, 31, 33, 64, 100])
 @pytest.mark.parametrize("N,K", [(5, 4), (128, 16), (130, 100), (257, 1540), (96, 3072)])
 def test_linear_f32_every_kernel_gives_the_same_bits(M, N, K):
@@ -169,12 +176,6 @@ def test_linear_f32_every_kernel_gives_the_same_bits(M, N, K):
         assert torch.equal(out, ref), (kind, cut)
 
 
-def tc_f32_bound(K):
-    """Of the float product on tensor cores, as a share of sum |x w|: a product good to 2^-24; for 64 k four steps of the tensor
-    core with the large parts, each good to 2^-22 of what it adds, and twenty with parts 2^-8 as large; K / 64 float additions."""
-    return (1 + 4 * 4 + 1 + K / 64) * 2.0 ** -24
-
-
 @pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 160, 161, 330])
 @pytest.mark.parametrize("N,K", [(4100, 260), (1024, 1028), (130, 9216), (20000, 256)])
 def test_linear_f32_on_tensor_cores(M, N, K):
@@ -182,14 +183,17 @@ def test_linear_f32_on_tensor_cores(M, N, K):
     assert kernels.linear_f32_tc_slices(N, K) == {4100: 2, 1024: 4, 130: 8, 20000: 1}[N]
     g = torch.Generator(device=DEV).manual_seed(M * N + K)
     x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
-    x[:, ::3] *= 1e-3
+    x[:, ::3] *= 1e-3                                        # (rows whose numbers differ widely)
     wide = torch.full((M, N + 3), float("nan"), device=DEV)
     kernels.linear_f32(x, w, wide[:, :N])
     out = wide[:, :N]
     assert kernels.linear_f32_tc_status(reset=True) == 0 and bool(wide[:, N:].isnan().all())
     ref = x.double() @ w.double().T
+    # a product 3 * 2^-24; per 64 k twelve steps of the tensor core, each good to 2^-22 of what it adds; K / 64 float additions;
+    # what is too small for its row's scale 2^-38 of its largest
     size = x.abs().double() @ w.abs().double().T
-    assert bool(((out.double() - ref).abs() <= tc_f32_bound(K) * size).all())
+    least = 2.0 ** -38 * K * x.abs().amax(1, keepdim=True).double() * w.abs().amax(1).double()
+    assert bool(((out.double() - ref).abs() <= (3 + 48 + K / 64) * 2.0 ** -24 * size + least).all())
     plain_sums = torch.empty(M, N, device=DEV)
     kernels._linear_f32(x, w, plain_sums, 0, 0)
     assert float((out.double() - ref).norm()) <= 1.05 * float((plain_sums.double() - ref).norm())     # no less precise
@@ -199,6 +203,26 @@ def test_linear_f32_on_tensor_cores(M, N, K):
         one = torch.empty(1, N, device=DEV)
         kernels.linear_f32(row[:, 1:], w, one)
         assert torch.equal(one[0], out[m])
+
+
+def tc_f32_bound(K):
+    """Of the float product on tensor cores, as a share of sum |x w|: a product good to 2^-24; for 64 k four steps of the tensor
+    core with the large parts, each good to 2^-22 of what it adds, and twenty with parts 2^-8 as large; K / 64 float additions."""
+    return (1 + 4 * 4 + 1 + K / 64) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 160, 161, 330])
+@pytest.mark.parametrize("N,K", [(4100, 260), (1024, 1028), (130, 9216), (20000, 256)])
+def test_linear_f32_on_tensor_cores_of_whole_floats(M, N, K):
+    """Every sum to what three parts a float allow: nothing for a row's largest number."""
+    assert kernels.linear_f32_tc_slices(N, K) > 0
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    x[:, ::3] *= 1e-3
+    out = torch.full((M, N), float("nan"), device=DEV)
+    kernels.linear_f32(x, w, out)
+    size = x.abs().double() @ w.abs().double().T
+    assert bool(((out.double() - x.double() @ w.double().T).abs() <= tc_f32_bound(K) * size).all())
 
 
 @pytest.mark.parametrize("beside", [1e4, 1e8, 1e12, 2.0 ** 40, 1e30])
@@ -406,6 +430,17 @@ def test_prompt_attention_cut_in_halves_repeats_itself(T, n_kv):
 
 
 def test_linear_f32_takes_no_scratch_for_operands_it_does_not_cut():
+    x = torch.zeros(300, 2305, device=DEV)[:, 1:]
+    w, out = torch.zeros(2304, 2304, device=DEV), torch.empty(300, 2304, device=DEV)
+    assert kernels.linear_f32_plan(300, 2304, 2304, kernels.device_sms())[1] > 0
+    kernels.linear_f32(x, w, out)
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    kernels.linear_f32(x, w, out)
+    assert torch.cuda.max_memory_allocated() == before
+
+
+def test_linear_f32_takes_no_scratch_for_small_operands_it_does_not_cut():
     x = torch.zeros(300, 3073, device=DEV)[:, 1:]
     w, out = torch.zeros(300, 3072, device=DEV), torch.empty(300, 300, device=DEV)
     assert not kernels.linear_f32_tc_ok(w) and kernels.linear_f32_plan(300, 300, 3072, kernels.device_sms())[1] > 0
